@@ -63,6 +63,8 @@ typedef enum qmm_variant {
   /* 5 was a tensor-memory decode variant that lost to QMM_VARIANT_MMA on every shape; the value is not reused */
   QMM_VARIANT_I8TC = 6,    /* activations split into int8 limbs, unconverted weights into tcgen05.mma.kind::i8, stream-K
                               over all SMs, 1 <= M <= 64; only through qmm_weight_only (needs workspace) */
+  QMM_VARIANT_I8MMA = 7,   /* decode: activations split into int8 limbs, unconverted weights into warp-level int8 MMAs,
+                              M <= 16, zero points allowed; only through qmm_weight_only (no workspace) */
 } qmm_variant;
 
 typedef enum qmm_op {
@@ -166,7 +168,8 @@ QMM_API size_t qmm_weight_only_workspace_size_for(int wbits, int64_t max_M, int6
  * Replaces: get_tuned_block_sizes (torch_xla/experimental/pallas_kernels/quantized_matmul_kernel.py:537-555).
  */
 QMM_API int qmm_tuned_variant(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_size);
-/* Name of the kernel family qmm_weight_only's AUTO picks for a shape, given a sufficient workspace (static string). */
+/* Name of the kernel family qmm_weight_only's AUTO picks for a shape among those the measured table knows, given a
+ * sufficient workspace (static string).  The few-token calls that QMM_VARIANT_I8MMA takes are decided before it. */
 QMM_API const char* qmm_weight_only_variant_for(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_size, int has_zp);
 QMM_API int qmm_weight_only(int wbits, const void* x, int x_dtype, const void* w, const float* scale, const float* zp,
                     void* out, int out_dtype, int64_t M, int64_t N, int64_t K, int64_t block_size, int variant,

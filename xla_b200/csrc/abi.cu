@@ -190,6 +190,16 @@ static int pick_weight_only(int wbits, int64_t M, int64_t N, int64_t K, int64_t 
   return QMM_VARIANT_GENERIC;
 }
 
+// AUTO's choice between the two warp-level decode kernels.  The integer one streams weights 1.5 times faster, but every
+// CTA of it first splits all activations into limbs, about 0.6 us per token at K = 4096, in proportion to M * K; the
+// gain is proportional to the weight bytes.  K cancels: it wins at one token, and up to one token per 1850 bytes of
+// weight column (14336 int8 outputs: 7 tokens; measured 15.1 against 16.7 us at 4, equal at 8; 4096 outputs: 2).
+// Zero points, scale blocks of 64 and ragged K are beyond the other kernel.
+static bool use_decode_i8(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, const void* x, int x_dt, const void* w, bool has_zp) {
+  if (!decode_i8_supported(wbits, M, N, K, bs, x, x_dt, w, has_zp)) return false;
+  return M == 1 || M * 1850 <= N * wbits / 8 || !decode_mma_supported(wbits, M, N, K, bs, x, x_dt, w, has_zp);
+}
+
 int qmm_w8a16_perchannel(const void* x, int x_dtype, const int8_t* w, const float* scale,
                          const float* zp, void* out, int out_dtype, int64_t M, int64_t N,
                          int64_t K, int variant, void* stream) {
@@ -361,6 +371,7 @@ int qmm_weight_only(int wbits, const void* x, int x_dtype, const void* w, const 
     if (block_size > 0 && K % block_size != 0)
       return fail(QMM_ERR_BAD_SHAPE, "input_dim should be divisible by block_size, got input_dim: %lld, block_size: %lld",
                   (long long)K, (long long)block_size);
+    if (variant == QMM_VARIANT_AUTO && use_decode_i8(wbits, M, N, K, block_size, x, x_dtype, w, zp != nullptr)) variant = QMM_VARIANT_I8MMA;
     const bool can = limb_tc_supported(wbits, M, N, K, block_size, x, x_dtype, w, zp != nullptr) && workspace &&
                      workspace_bytes >= limb_tc_workspace_bytes(M, K) && aligned(workspace, 256);
     // AUTO: the measured table first, the shape rule where the table has no entry for this shape
@@ -380,6 +391,12 @@ int qmm_weight_only(int wbits, const void* x, int x_dtype, const void* w, const 
       return launch_limb_tc(wbits, x, x_dtype, w, scale, out, out_dtype, M, N, K, block_size, 0, workspace, workspace_bytes,
                             as_stream(stream));
     }
+  }
+  if (variant == QMM_VARIANT_I8MMA) {
+    int rc = check_common(x, x_dtype, w, scale, out, out_dtype, M, N, K);
+    if (rc != QMM_OK || M * N == 0) return rc;
+    log_choice("weight_only", "i8mma", M, N, K);
+    return launch_decode_i8(wbits, x, x_dtype, w, scale, zp, out, out_dtype, M, N, K, block_size, 0, as_stream(stream));
   }
   if (wbits == 8) {
     if (block_size > 0)
@@ -408,6 +425,10 @@ int qmm_gate_up_decode(int wbits, const void* x, int x_dtype, const void* w, con
     return fail(QMM_ERR_UNSUPPORTED, "gate_up_decode: needs 1<=M<=32, bf16/f16 activations, K a multiple of %d, 16-byte "
                 "aligned x/w (M=%lld N2=%lld K=%lld bs=%lld)", 512 / wbits, (long long)M, (long long)N2, (long long)K,
                 (long long)block_size);
+  if (use_decode_i8(wbits, M, N2, K, block_size, x, x_dtype, w, false)) {
+    log_choice("gate_up_decode", "i8mma", M, N2, K);
+    return launch_decode_i8(wbits, x, x_dtype, w, scale, nullptr, out, out_dtype, M, N2, K, block_size, 1, st);
+  }
   log_choice("gate_up_decode", "mma", M, N2, K);
   return launch_decode_mma(wbits, x, x_dtype, w, scale, out, out_dtype, M, N2, K, block_size, st, 1);
 }
@@ -476,7 +497,7 @@ int qmm_w8a8_gemm(const int8_t* xq, const int8_t* w, const float* w_scale, const
   if (K > 0 && (!xq || !w)) return fail(QMM_ERR_NULL, "xq or w is NULL");
   cudaStream_t st = as_stream(stream);
   if (variant == QMM_VARIANT_AUTO)
-    variant = (w8a8_tc_supported(M, N, K, xq, w) && M >= 16) ? QMM_VARIANT_TCGEN05 : QMM_VARIANT_GENERIC;
+    variant = w8a8_tc_supported(M, N, K, xq, w) ? QMM_VARIANT_TCGEN05 : QMM_VARIANT_GENERIC;
   switch (variant) {
     case QMM_VARIANT_GENERIC:
       log_choice("w8a8_gemm", "generic", M, N, K);
@@ -488,6 +509,10 @@ int qmm_w8a8_gemm(const int8_t* xq, const int8_t* w, const float* w_scale, const
       return fail(QMM_ERR_UNSUPPORTED, "w8a8_gemm: variant %d is not available", variant);
   }
 }
+
+// Up to here the decode kernel beats the quantizer and the tcgen05 GEMM (4096 x 4096: 6.4 to 19.5 us at 1 to 12 tokens
+// against 20.5; 14336 x 4096: 14 to 27 against 23).
+constexpr int64_t kW8A8DecodeTokens = 12;
 
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
@@ -507,6 +532,11 @@ int qmm_w8a8_perchannel(const void* x, int x_dtype, const int8_t* w, const float
                         size_t workspace_bytes, void* stream) {
   int rc = check_common(x, x_dtype, w, w_scale, out, out_dtype, M, N, K);
   if (rc != QMM_OK || M * N == 0) return rc;
+  // decode batches: one kernel quantizes and multiplies, no scratch
+  if (variant == QMM_VARIANT_AUTO && M <= kW8A8DecodeTokens && decode_w8a8_supported(M, N, K, x, x_dtype, w, zp != nullptr)) {
+    log_choice("w8a8_perchannel", "i8mma", M, N, K);
+    return launch_decode_w8a8(x, x_dtype, w, w_scale, zp, out, out_dtype, M, N, K, saturate, as_stream(stream));
+  }
   const size_t need = qmm_workspace_size(QMM_OP_W8A8_PERCHANNEL, M, N, K);
   if (!workspace || workspace_bytes < need)
     return fail(QMM_ERR_WORKSPACE, "w8a8_perchannel needs %zu bytes of workspace, got %zu", need, workspace_bytes);
@@ -676,7 +706,8 @@ const char* qmm_variant_for(int op, int64_t M, int64_t N, int64_t K, int64_t blo
     case QMM_OP_BLOCKWISE_SBN:
       return "generic";
     case QMM_OP_W8A8_PERCHANNEL:
-      return (M >= 16 && K % 16 == 0 && K >= 16) ? "tcgen05" : "generic";
+      if (K % 16 != 0 || K < 64) return (K % 16 == 0 && K >= 16) ? "tcgen05" : "generic";
+      return M <= kW8A8DecodeTokens && decode_w8a8_supported(M, N, K, ok, QMM_BF16, ok, has_zp != 0) ? "i8mma" : "tcgen05";
     default:
       return "generic";
   }

@@ -13,34 +13,13 @@
 // way HBM sees each activation once: 2 or 4 bytes in, 1 byte out per element.
 #include "common.cuh"
 #include "kernels.h"
+#include "quant.cuh"
 
 namespace qmm {
 
 namespace {
 
 constexpr int kThreads = 256;
-
-template <typename T>
-__device__ __forceinline__ float round_to(float v) {
-  return to_f32(from_f32<T>(v));
-}
-
-__device__ __forceinline__ int8_t to_int8(float r, bool saturate) {
-  if (r != r) return 0;
-  if (saturate) {
-    r = fminf(fmaxf(r, -128.f), 127.f);
-    return (int8_t)(int)r;
-  }
-  // wrap like a float -> int32 -> int8 conversion chain does for values in int32 range
-  if (r > 2147483520.f || r < -2147483648.f) return 0;
-  return (int8_t)(uint8_t)(((int)r) & 0xff);
-}
-
-template <typename T>
-__device__ __forceinline__ int8_t quantize_one(T xv, float scale, bool saturate) {
-  const float q = round_to<T>(__fdiv_rn(to_f32(xv), scale));
-  return to_int8(rintf(q), saturate);
-}
 
 template <typename T, int VEC>
 struct alignas(sizeof(T) * VEC) Pack {
@@ -97,7 +76,7 @@ __global__ void __launch_bounds__(kThreads)
       const float o = s_red[i];
       a = (a != a || o != o) ? __int_as_float(0x7fc00000) : fmaxf(a, o);
     }
-    const float sc = round_to<T>(__fdiv_rn(a, 127.0f));
+    const float sc = quant_scale<T>(a);
     s_scale = sc;
     x_scale[m] = sc;
   }
@@ -115,14 +94,14 @@ __global__ void __launch_bounds__(kThreads)
       Pack<int8_t, VEC> q;
 #pragma unroll
       for (int j = 0; j < VEC; ++j) {
-        q.v[j] = quantize_one<T>(p.v[j], scale, saturate != 0);
+        q.v[j] = quantize_value<T>(to_f32(p.v[j]), scale, saturate != 0);
         isum += q.v[j];
       }
       qv[i] = q;
     }
   } else {
     for (int64_t k = tid; k < K; k += kThreads) {
-      const int8_t q = quantize_one<T>(row[k], scale, saturate != 0);
+      const int8_t q = quantize_value<T>(to_f32(row[k]), scale, saturate != 0);
       qrow[k] = q;
       isum += q;
     }
@@ -145,11 +124,6 @@ __global__ void __launch_bounds__(kThreads)
 //
 // amax is taken on the bit patterns: for non-negative floats the integer order is the float order, and
 // a NaN pattern is larger than every number, so NaN propagates like torch.amax without extra tests.
-//
-// The quotient x / scale must be the correctly rounded fp32 quotient (it is rounded to bf16 next and
-// ties decide).  One Newton step on q0 = x * (1/scale) gives it: both operands have 8-bit significands,
-// so the exact quotient is either a tie (exactly representable: the step lands on it) or at least
-// 2^-17 away from any bf16 rounding boundary, far more than the error of q0.
 template <int CHUNKS>
 __global__ void __launch_bounds__(kThreads)
     quantize_rows_bf16_kernel(const __nv_bfloat16* __restrict__ x, int8_t* __restrict__ xq,
@@ -186,21 +160,15 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
   for (int i = 1; i < kThreads / 32; ++i) a = max(a, s_red[i]);
   const float amax = __uint_as_float(a << 16);
-  const float scale = round_to<__nv_bfloat16>(__fdiv_rn(amax, 127.0f));
+  const float scale = quant_scale<__nv_bfloat16>(amax);
   if (tid == 0) x_scale[m] = scale;
   const float rcp = __frcp_rn(scale);
   // scale == 0 (all-zero row), inf or NaN: the Newton step is not valid there; fall back to IEEE division
-  const bool regular = scale > 1e-30f && scale < 1e30f;
+  const bool regular = quant_regular(scale);
 
   int isum = 0;
   uint2* qv = reinterpret_cast<uint2*>(xq + m * K);
   if (regular) {
-    // Everything after the quotient stays on the FMA and integer pipes (no conversion-unit instruction):
-    //   bf16 rounding   Veltkamp split with 2^16 + 1: g = q * 65537, qb = g + (q - g) is q rounded to 8
-    //                   significant bits, ties to even (each step is one correctly rounded operation; the
-    //                   explicit _rn intrinsics keep the compiler from fusing them)
-    //   rint -> int     qb + 1.5 * 2^23 leaves the integer, rounded ties-to-even, in the low mantissa bits
-    //   int8            clamp (or wrap) in integers, bytes gathered with prmt, row sum with dp4a
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) {
       const int i = tid + c * kThreads;
@@ -209,21 +177,12 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const float xv = __uint_as_float((j & 1) ? (w[j >> 1] & 0xffff0000u) : (w[j >> 1] << 16));
-        const float q0 = xv * rcp;
-        const float r = fmaf(-q0, scale, xv);
-        const float q = fmaf(r, rcp, q0);
-        const float g = __fmul_rn(q, 65537.f);
-        const float qb = __fadd_rn(g, __fsub_rn(q, g));
-        int t = __float_as_int(__fadd_rn(qb, 12582912.f)) - 0x4B400000;
-        if (saturate) t = max(-128, min(127, t));
-        qi[j] = t;
+        qi[j] = quantize_bf16_regular(xv, scale, rcp, saturate != 0);
       }
       uint32_t packed[2];
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const uint32_t lo = __byte_perm((uint32_t)qi[4 * h], (uint32_t)qi[4 * h + 1], 0x0040);
-        const uint32_t hi = __byte_perm((uint32_t)qi[4 * h + 2], (uint32_t)qi[4 * h + 3], 0x0040);
-        packed[h] = __byte_perm(lo, hi, 0x5410);
+        packed[h] = pack_bytes(qi + 4 * h);
         isum = __dp4a((int)packed[h], 0x01010101, isum);
       }
       if (i < nvec) qv[i] = make_uint2(packed[0], packed[1]);

@@ -55,6 +55,17 @@ int launch_decode_mma_allreduce(int wbits, const void* x, int x_dt, const void* 
                                 int64_t M, int64_t N, int64_t K, int64_t block_size, void* const* peer_bufs, int rank,
                                 int world, int64_t slot_floats, cudaStream_t st);
 
+// ---- decode_i8.cu -------------------------------------------------------------------------
+// Decode kernels on the warp-level integer MMAs.  Weight-only: M <= 16, bf16/f16 activations, zero points allowed, the
+// limbs of all tokens have to fit shared memory.  W8A8: M <= 32, activations of any type quantized in the kernel.
+bool decode_i8_supported(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_size, const void* x, int x_dt, const void* w,
+                         bool has_zp);
+int launch_decode_i8(int wbits, const void* x, int x_dt, const void* w, const float* scale, const float* zp, void* out, int out_dt,
+                     int64_t M, int64_t N, int64_t K, int64_t block_size, int gate_up, cudaStream_t st);
+bool decode_w8a8_supported(int64_t M, int64_t N, int64_t K, const void* x, int x_dt, const void* w, bool has_zp);
+int launch_decode_w8a8(const void* x, int x_dt, const int8_t* w, const float* w_scale, const float* zp, void* out, int out_dt,
+                       int64_t M, int64_t N, int64_t K, int saturate, cudaStream_t st);
+
 // ---- limb_gemm.cu (tcgen05 kind::i8 on unconverted weights; activations split into int8 limbs) ----------
 // Weight-only linear for 1 <= M <= 64 (bf16/f16/f32 activations, no zero point): stream-K over all SMs, needs
 // limb_tc_workspace_bytes(M, K) bytes of caller scratch whose first 1024 bytes are zero before the first use (the
