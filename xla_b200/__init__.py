@@ -13,6 +13,7 @@ from . import packed  # noqa: F401
 from .packed import pack_int4, quantized_matmul_packed, unpack_int4  # noqa: F401
 from . import mlp  # noqa: F401
 from .mlp import concat_projections, interleave_gate_up, quantized_gate_up, split_outputs  # noqa: F401
+_capi.register_operators()
 from .host import HostLinear, HostPipeline  # noqa: F401
 
 __all__ = [

@@ -91,6 +91,35 @@ def lib():
   return _lib
 
 
+_torch_lib = None
+
+
+def torch_lib():
+  """The operators' C++ side; loading it registers their CUDA kernels."""
+  global _torch_lib
+  if _torch_lib is None:
+    lib()
+    path = _build.TORCH_LIB_PATH
+    if not os.path.exists(path):
+      raise ImportError(f"{path} is missing: build it with `python -m xla_b200._build` (needs nvcc and g++).")
+    torch.ops.load_library(path)
+    L = ctypes.CDLL(path)
+    L.qmmt_set_thread_state.restype, L.qmmt_set_thread_state.argtypes = None, [_i, _i]
+    L.qmmt_scratch.restype, L.qmmt_scratch.argtypes = None, [_i, _p, _sz, ctypes.POINTER(_p), ctypes.POINTER(_sz)]
+    _torch_lib = L
+  return _torch_lib
+
+
+def register_operators():
+  """Loads the libraries when they have been built from these sources; before that (a fresh or an updated checkout) the
+  package still imports, so that the build can run, and the operators have no CUDA kernels."""
+  if os.path.exists(_build.LIB_PATH) and os.path.exists(_build.TORCH_LIB_PATH):
+    try:
+      torch_lib()
+    except (AttributeError, OSError):
+      pass  # an older build: lib() says what is wrong when it is used
+
+
 def dtype_code(dt):
   try:
     return _DTYPES[dt]
@@ -127,27 +156,18 @@ def on_device(device, fn):
     return fn()
 
 
-_workspaces = {}
-
-
 def workspace(device, max_M, K, N=0, wbits=8):
   """Scratch for ``qmm_weight_only`` on torch's current stream of `device`: (pointer, bytes), or (None, 0) when no
   variant needs one; with N and wbits, including the room that lets a long int4 batch expand its weights to int8
-  once.  One buffer per (device, stream), zero-filled when created (the kernels keep its flag words
-  zero) and grown on demand; a stream capture in progress never allocates - it gets the existing buffer or none."""
+  once.  One buffer per (device, stream), shared with the operators' C++ side, which keeps it (torch_ops.cpp); a stream
+  capture in progress never allocates - it gets the existing buffer or none."""
   need = lib().qmm_weight_only_workspace_size_for(wbits, max_M, N, K) if N else lib().qmm_weight_only_workspace_size(max_M, K)
   if need == 0:
     return None, 0
   idx = device.index if device.index is not None else torch.cuda.current_device()
-  key = (idx, stream_ptr(idx))
-  buf = _workspaces.get(key)
-  if buf is None or buf.numel() < need:
-    if torch.cuda.is_current_stream_capturing():
-      return (None, 0) if buf is None else (buf.data_ptr(), buf.numel())
-    size = max(need, 16 << 20) if buf is None else max(need, 2 * buf.numel())
-    buf = torch.zeros(size, dtype=torch.uint8, device=torch.device("cuda", idx))
-    _workspaces[key] = buf
-  return buf.data_ptr(), buf.numel()
+  p, n = ctypes.c_void_p(), ctypes.c_size_t()
+  torch_lib().qmmt_scratch(idx, stream_ptr(idx), need, ctypes.byref(p), ctypes.byref(n))
+  return p.value, n.value
 
 
 def check(status):

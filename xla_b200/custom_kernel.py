@@ -55,5 +55,6 @@ def quantized_matmul_int8_meta(x, w, scalar, zero_point=None, quant_block_size=N
   return torch.empty(x.shape[0], w.shape[0], device=x.device, dtype=x.dtype)
 
 
-_qm.XLA_LIB.impl("quantized_matmul_int8", quantized_matmul_int8, "CUDA")
+_qm.LIB.define(SCHEMA.replace("quantized_matmul_int8(", "quantized_matmul_int8_any("))
+_qm.LIB.impl("quantized_matmul_int8_any", quantized_matmul_int8, "CUDA")
 _qm.XLA_LIB.impl("quantized_matmul_int8", quantized_matmul_int8_meta, "Meta")

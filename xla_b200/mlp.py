@@ -22,10 +22,8 @@ from . import quantized_matmul as _qm
 from .packed import quantized_matmul_packed
 
 LIB = torch.library.Library("xla_b200", "FRAGMENT")
-try:
-  getattr(torch.ops.xla_b200, "quantized_gate_up")
-except (AttributeError, RuntimeError):
-  LIB.define("quantized_gate_up(Tensor x, Tensor w, Tensor scale, int block_size=-1, bool int4_weight=False, "
+for _name in ("quantized_gate_up", "quantized_gate_up_any"):
+  LIB.define(_name + "(Tensor x, Tensor w, Tensor scale, int block_size=-1, bool int4_weight=False, "
              "bool weight_is_packed=False, ScalarType? out_dtype=None) -> Tensor")
 
 
@@ -118,7 +116,7 @@ def _meta(x, w, scaler, block_size=-1, int4_weight=False, weight_is_packed=False
   return torch.empty(x.shape[:-1] + (w.shape[0] // 2,), dtype=out_dtype, device=x.device)
 
 
-LIB.impl("quantized_gate_up", quantized_gate_up, "CUDA")
+LIB.impl("quantized_gate_up_any", quantized_gate_up, "CUDA")
 LIB.impl("quantized_gate_up", _meta, "Meta")
 
 

@@ -18,10 +18,8 @@ from . import _capi
 from . import quantized_matmul as _qm
 
 LIB = torch.library.Library("xla_b200", "FRAGMENT")
-try:
-  getattr(torch.ops.xla_b200, "quantized_matmul_packed")
-except (AttributeError, RuntimeError):
-  LIB.define("quantized_matmul_packed(Tensor x, Tensor w, Tensor scale, Tensor? zero_point=None, "
+for _name in ("quantized_matmul_packed", "quantized_matmul_packed_any"):
+  LIB.define(_name + "(Tensor x, Tensor w, Tensor scale, Tensor? zero_point=None, "
              "int block_size=-1, bool int4_weight=False, bool weight_is_packed=False, "
              "bool quantize_activation=False, ScalarType? out_dtype=None) -> Tensor")
 
@@ -93,7 +91,8 @@ def _shapes(x, w, scaler, zero_point, block_size, weight_is_packed):
 
 def quantized_matmul_packed(x, w, scaler, zero_point=None, block_size=-1, int4_weight=False,
                             weight_is_packed=False, quantize_activation=False, out_dtype=None, out=None):
-  """CUDA kernel of ``torch.ops.xla_b200.quantized_matmul_packed``.  ``out`` (Python callers only, not part of
+  """The whole operator ``torch.ops.xla_b200.quantized_matmul_packed`` on CUDA tensors (its C++ kernel,
+  csrc/torch_ops.cpp, handles the well-formed calls and comes here with the others).  ``out`` (Python callers only, not part of
   the operator schema) is a preallocated contiguous [M, N] result buffer, e.g. a peer-mapped one."""
   _capi.require_cuda(x, w, scaler, zero_point)
   N, K = _shapes(x, w, scaler, zero_point, block_size, weight_is_packed)
@@ -144,5 +143,5 @@ def _meta(x, w, scaler, zero_point=None, block_size=-1, int4_weight=False, weigh
   return torch.empty(x.shape[:-1] + (w.shape[0],), dtype=out_dtype, device=x.device)
 
 
-LIB.impl("quantized_matmul_packed", quantized_matmul_packed, "CUDA")
+LIB.impl("quantized_matmul_packed_any", quantized_matmul_packed, "CUDA")
 LIB.impl("quantized_matmul_packed", _meta, "Meta")
