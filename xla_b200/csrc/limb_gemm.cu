@@ -449,7 +449,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + kMaxAcc);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
 #ifdef QMM_LIMB_DBG
   const long long dbg_k0 = clock64();
   const unsigned long long dbg_g0 = ptx::globaltimer_ns();
@@ -551,9 +551,9 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
       DBG_FLUSH(8);
     }
   } else if (warp == 1) {
-    // ---------------- MMA issuer: the whole warp walks the loop, lane 0's instructions take effect ----------------
+    // ---------------- MMA issuer: the whole warp walks the loop, one elected thread issues ----------------
     constexpr uint32_t idesc = ptx::make_idesc(/*s32*/ 2, /*s8*/ 1, /*s8*/ 1, BMW, NCOLS);
-    const uint32_t leader = lane == 0 ? 1u : 0u;
+    const bool leader = ptx::elect_one();
     const uint32_t desc_hi = (uint32_t)(ptx::make_sw128_kmajor_desc(0) >> 32);
     const uint32_t lo0 = (uint32_t)ptx::make_sw128_kmajor_desc(ptx::smem_u32(slot_base));
     FragIter it(p);
@@ -565,16 +565,17 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
     // the four MMAs of operand tile t of the current slot into accumulator d
     auto issue_tile = [&](uint32_t d, int t, uint32_t accum) {
       const uint32_t a_lo = lo + t * (kATile >> 4), b_lo = lo + (C::kAInSlot >> 4) + t * (kBTile >> 4);
+      if (!leader) return;
 #pragma unroll
       for (int k = 0; k < kTileK / UMMA_K; ++k) {
         const uint64_t bd = ((uint64_t)desc_hi << 32) | (uint64_t)(b_lo + k * (UMMA_K >> 4));
         if constexpr (C::kATmem) {
           // operand rows = TMEM lanes; one K=32 step = 8 columns = one expanded 16-byte chunk of nibbles
           const uint32_t a_tm = tmem_base + C::kATmemCol0 + slot * C::kATmemSlotCols + (4 * t + k) * 8;
-          ptx::mma_i8_ts_pred(d, a_tm, bd, idesc, accum | (uint32_t)k, leader);
+          ptx::mma_i8_ts(d, a_tm, bd, idesc, accum | (uint32_t)k);
         } else {
           const uint64_t ad = ((uint64_t)desc_hi << 32) | (uint64_t)(a_lo + k * (UMMA_K >> 4));
-          ptx::mma_i8_ss_pred(d, ad, bd, idesc, accum | (uint32_t)k, leader);
+          ptx::mma_i8_ss(d, ad, bd, idesc, accum | (uint32_t)k);
         }
       }
     };
@@ -585,7 +586,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
       ptx::tcgen05_fence_after();
     };
     auto next_acc = [&]() {
-      ptx::mma_commit_pred(&acc_full[buf], leader);
+      if (leader) ptx::mma_commit(&acc_full[buf]);
       if (++buf == nacc) { buf = 0; pacc ^= 1; }
     };
     bool dbg_first = true;
@@ -604,7 +605,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
       ptx::tcgen05_fence_after();
     };
     auto next_slot = [&]() {
-      ptx::mma_commit_pred(&empty[slot], leader);  // frees the slot once the MMAs issued so far have read it
+      if (leader) ptx::mma_commit(&empty[slot]);  // frees the slot once the MMAs issued so far have read it
       lo += kSlot >> 4;
       if (++slot == kSlots) { slot = 0; ph ^= 1; lo = lo0; }
     };

@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
   const int64_t n0 = (int64_t)blockIdx.x * BMW;
   const int64_t m0 = (int64_t)blockIdx.y * MP;
   const uint32_t krank = KSPLIT ? cluster_ctarank() : 0u;
@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const uint32_t a_lo0 = (uint32_t)ptx::make_sw128_kmajor_desc(ptx::smem_u32(a_base));
       const uint32_t b_lo0 = (uint32_t)ptx::make_sw128_kmajor_desc(ptx::smem_u32(b_base));
       int blk = 0, in_blk = 0;
-      const uint32_t leader = lane == 0 ? 1u : 0u;
+      const bool leader = ptx::elect_one();
       // ring positions advance with adds and compares only: this warp's instruction count per tile is what
       // bounds the kernel at small token tiles, and a division by a ring depth costs as much as an MMA issue
       int sa = 0, a_par = 0;           // operand slot of tile t and the parity of its current use
@@ -318,16 +318,18 @@ __global__ void __launch_bounds__(kThreads, 1)
         ptx::mbar_wait(&a_full[sa], a_par, abort_flag, p.err_word, ptx::kErrWaitConv);
         const bool last_in_block = (in_blk + 1 == p.tiles_per_block) || (t == my_tiles - 1);
         const uint32_t d_tmem = tmem_base + buf * MP;
-#pragma unroll
-        for (int k = 0; k < BK / UMMA_K; ++k) {
-          const uint64_t ad = ((uint64_t)desc_hi << 32) | (uint64_t)(a_lo + k * (UMMA_K * 2 >> 4));
-          const uint64_t bd = ((uint64_t)desc_hi << 32) | (uint64_t)(b_lo + k * (UMMA_K * 2 >> 4));
-          ptx::mma_f16_ss_pred(d_tmem, ad, bd, idesc, (in_blk | k) != 0 ? 1u : 0u, leader);
-        }
-        ptx::mma_commit_pred(&a_empty[sa], leader);
         const bool group_done = (jb == kBGroup - 1) || (t == my_tiles - 1);
-        if (group_done) ptx::mma_commit_pred(&b_empty[sb], leader);
-        if (last_in_block) ptx::mma_commit_pred(&acc_full[buf], leader);
+        if (leader) {
+#pragma unroll
+          for (int k = 0; k < BK / UMMA_K; ++k) {
+            const uint64_t ad = ((uint64_t)desc_hi << 32) | (uint64_t)(a_lo + k * (UMMA_K * 2 >> 4));
+            const uint64_t bd = ((uint64_t)desc_hi << 32) | (uint64_t)(b_lo + k * (UMMA_K * 2 >> 4));
+            ptx::mma_f16_ss(d_tmem, ad, bd, idesc, (in_blk | k) != 0 ? 1u : 0u);
+          }
+          ptx::mma_commit(&a_empty[sa]);
+          if (group_done) ptx::mma_commit(&b_empty[sb]);
+          if (last_in_block) ptx::mma_commit(&acc_full[buf]);
+        }
         ++in_blk;
         if (last_in_block) {
           in_blk = 0;

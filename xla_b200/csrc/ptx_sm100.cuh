@@ -81,13 +81,31 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
+// Non-blocking look at a phase: for a barrier that is needed a little later, so that the result's latency (about 45 cycles
+// until a branch on it resolves, 85 behind issued MMAs) passes under other work.
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
 // Bounded wait.  `abort_flag` is a CTA-shared word; `err_word` the library's global error word.
-// The fast path is a bare try_wait loop; the SM cycle counter is looked at only once every 4096
-// polls (a %globaltimer read per wait costs about a microsecond and would dominate short waits).
+// The first try stands alone: a phase that is complete costs 43 cycles this way, 65 to 170 when the loop below is entered
+// for it.  The SM cycle counter is looked at only once every 4096 polls (a %globaltimer read per wait costs about a
+// microsecond and would dominate short waits).
 template <int SLEEP_NS = 0>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
                                           volatile uint32_t* abort_flag, uint32_t* err_word,
                                           uint32_t code) {
+  if (mbar_try_wait(bar, parity)) return true;
   uint32_t spins = 0;
   long long t0 = 0;
   while (!mbar_try_wait(bar, parity)) {
@@ -107,12 +125,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
   return true;
 }
 
-// Whole-warp wait: lane 0 polls, the rest of the warp parks at the warp barrier.  Keeps 31 of 32
-// lanes from hammering the same mbarrier word while the single-thread MMA issuer needs that unit.
+// Whole-warp wait: after one look by all lanes, lane 0 polls and the rest of the warp parks at the warp barrier.  Keeps 31
+// of 32 lanes from hammering the same mbarrier word while the MMA issuer needs that unit.
 template <int SLEEP_NS = 0>
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity,
                                                volatile uint32_t* abort_flag, uint32_t* err_word,
                                                uint32_t code) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   bool ok = true;
   if ((threadIdx.x & 31) == 0) ok = mbar_wait<SLEEP_NS>(bar, parity, abort_flag, err_word, code);
   __syncwarp();
@@ -216,44 +235,12 @@ __device__ __forceinline__ void mma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uin
       : "memory");
 }
 
-// Predicated forms: every lane of the issuing warp executes the same instruction stream and only the
-// lane with `leader` != 0 takes effect.  Keeps the issuing warp converged (no branch around the MMA).
-__device__ __forceinline__ void mma_f16_ss_pred(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                                uint32_t idesc, uint32_t accumulate, uint32_t leader) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p, q;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "setp.ne.b32 q, %5, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader)
-      : "memory");
-}
-
-__device__ __forceinline__ void mma_i8_ss_pred(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                               uint32_t idesc, uint32_t accumulate, uint32_t leader) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p, q;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "setp.ne.b32 q, %5, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t"
-      "}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader)
-      : "memory");
-}
-
-__device__ __forceinline__ void mma_commit_pred(uint64_t* bar, uint32_t leader) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred q;\n\t"
-      "setp.ne.b32 q, %1, 0;\n\t"
-      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
-      "}" ::"r"(smem_u32(bar)),
-      "r"(leader)
-      : "memory");
-}
+// How to issue: the warp index that selects the issuing warp must come from warp_index() and ONE elected thread must issue
+// from inside a branch, so that the compiler keeps descriptors in uniform registers.  Predicating the instruction on a
+// lane instead costs 62 to 77 cycles of instructions per MMA whatever its size; this form issues one in 11 and leaves the
+// tensor pipe as the limit (measured, kind::f16 with A in tensor memory: 11 / 32 / 64 / 96 cycles for N = 16 / 64 / 128 /
+// 192; kind::i8 with A in shared memory: 40 / 48 / 64 / 128 for N = 16 / 64 / 128 / 256).
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 
 // Arrives on `bar` once every tcgen05.mma issued so far by this thread has completed.
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
@@ -326,35 +313,7 @@ __device__ __forceinline__ void tmem_st_wait() {
 }
 
 // D[tmem] (+)= A[tmem] * B[smem]: the A operand is read from tensor memory (row m = lane m, two 16-bit
-// k values per 32-bit column, 8 columns per K=16 step).  Predicated like mma_f16_ss_pred.
-__device__ __forceinline__ void mma_f16_ts_pred(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                                uint32_t accumulate, uint32_t leader) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p, q;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "setp.ne.b32 q, %5, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-      "}" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader)
-      : "memory");
-}
-
-// The same with int8 operands: four k values per 32-bit column, 8 columns per K=32 step.
-__device__ __forceinline__ void mma_i8_ts_pred(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                               uint32_t accumulate, uint32_t leader) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p, q;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "setp.ne.b32 q, %5, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t"
-      "}" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(leader)
-      : "memory");
-}
-
-// Unpredicated form: call from ONE thread.
+// k values per 32-bit column, 8 columns per K=16 step).  Call from ONE thread.
 __device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
                                            uint32_t accumulate) {
   asm volatile(
@@ -362,6 +321,19 @@ __device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uin
       ".reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+      "}" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// The same with int8 operands: four k values per 32-bit column, 8 columns per K=32 step.
+__device__ __forceinline__ void mma_i8_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                           uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t"
       "}" ::"r"(d_tmem),
       "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
