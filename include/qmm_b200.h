@@ -171,6 +171,12 @@ QMM_API int qmm_tuned_variant(int wbits, int64_t M, int64_t N, int64_t K, int64_
 /* Name of the kernel family qmm_weight_only's AUTO picks for a shape among those the measured table knows, given a
  * sufficient workspace (static string).  The few-token calls that QMM_VARIANT_I8MMA takes are decided before it. */
 QMM_API const char* qmm_weight_only_variant_for(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_size, int has_zp);
+/*
+ * Whether qmm_weight_only's AUTO has a fast kernel that applies zero points itself for this shape (given a sufficient
+ * workspace and aligned operands).  Where it has none and the batch is longer than a few tokens, running the symmetric
+ * kernel into fp32 and subtracting the rank-S zero-point term afterwards is faster than the any-shape kernel.
+ */
+QMM_API int qmm_zero_point_in_kernel(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_size, int x_dtype);
 QMM_API int qmm_weight_only(int wbits, const void* x, int x_dtype, const void* w, const float* scale, const float* zp,
                     void* out, int out_dtype, int64_t M, int64_t N, int64_t K, int64_t block_size, int variant,
                     void* workspace, size_t workspace_bytes, void* stream);

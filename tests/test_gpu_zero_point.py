@@ -1,0 +1,31 @@
+"""Zero points inside the tensor-core kernels against the CPU oracle: one and several token tiles, K split over CTAs, scale
+blocks of both kinds, chunked batches, fp32 activations."""
+import pytest
+import torch
+
+import xla_b200
+from oracle import qmm_oracle as qo
+from tests import qmm_cases as qc
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("wbits,bs,N,K,M,dtype", [
+    (8, -1, 300, 1056, 17, torch.bfloat16), (8, 128, 1000, 1280, 33, torch.float16), (8, 256, 129, 768, 70, torch.bfloat16),
+    (4, 128, 4096, 2048, 29, torch.float16), (4, 128, 777, 1024, 64, torch.bfloat16), (4, -1, 520, 4096, 130, torch.bfloat16),
+    (4, 256, 300, 1024, 513, torch.float16), (8, -1, 260, 272, 1100, torch.float32), (4, 128, 4096, 1024, 40, torch.float32),
+    (8, 512, 200, 1024, 9, torch.float32),
+])
+def test_zero_points_above_eight_tokens(wbits, bs, N, K, M, dtype):
+  g = qc.gen(N + K + M)
+  x = qc.activations(g, M, K, dtype, outliers=True)
+  w = qc.int4_weight(g, N, K) if wbits == 4 else qc.int8_weight(g, N, K)
+  s = qc.per_channel_scale(g, N) if bs == -1 else qc.blockwise_scale(g, K // bs, N)
+  zp = torch.randint(-3, 4, s.shape, generator=g).float() * s
+  exact = qo.quantized_matmul(x.float(), w if bs == -1 else qc.to_sbn(w, bs), s, zp, block_size=bs, dot_round=None)
+  wd = xla_b200.pack_int4(w.to(DEV)) if wbits == 4 else w.to(DEV)
+  for out_dtype, tol in ((torch.float32, 1e-5), (torch.bfloat16, 1e-2)):
+    out = torch.ops.xla_b200.quantized_matmul_packed(x.to(DEV), wd, s.to(DEV), zp.to(DEV), block_size=bs, int4_weight=wbits == 4,
+                                                     weight_is_packed=wbits == 4, out_dtype=out_dtype)
+    assert qo.max_abs_rel(out, exact) < tol, out_dtype

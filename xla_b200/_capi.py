@@ -33,6 +33,7 @@ SIGNATURES = {
     "qmm_weight_only_workspace_size_for": (_sz, [ctypes.c_int, _i64, _i64, _i64]),
     "qmm_tuned_variant": (_i, [_i, _i64, _i64, _i64, _i64]),
     "qmm_weight_only_variant_for": (ctypes.c_char_p, [_i, _i64, _i64, _i64, _i64, _i]),
+    "qmm_zero_point_in_kernel": (_i, [_i, _i64, _i64, _i64, _i64, _i]),
     "qmm_weight_only": (_i, [_i, _p, _i, _p, _p, _p, _p, _i, _i64, _i64, _i64, _i64, _i, _p, _sz, _p]),
     "qmm_host_pipeline_create": (_i, [_sz, _sz, _i, ctypes.POINTER(ctypes.c_void_p)]),
     "qmm_host_weight_only": (_i, [_p, _i, _p, _i, _p, _p, _p, _p, _i, _i64, _i64, _i64, _i64, _i]),
@@ -116,8 +117,9 @@ def register_operators():
   if os.path.exists(_build.LIB_PATH) and os.path.exists(_build.TORCH_LIB_PATH):
     try:
       torch_lib()
-    except (AttributeError, OSError):
-      pass  # an older build: lib() says what is wrong when it is used
+    except (AttributeError, OSError) as e:  # an older build
+      import warnings
+      warnings.warn(f"xla_b200: the built libraries do not match the sources ({e}); run `python -m xla_b200._build`")
 
 
 def dtype_code(dt):

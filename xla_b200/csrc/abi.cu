@@ -335,13 +335,22 @@ int qmm_tuned_variant(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_
   return tuned_variant(wbits, block_size < 0 ? 0 : block_size, M, N, K);
 }
 
+int qmm_zero_point_in_kernel(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_size, int x_dtype) {
+  if (block_size < 0) block_size = 0;
+  const void* ok = reinterpret_cast<const void*>(uintptr_t(256));
+  return M <= 8 || limb_tc_shape_ok(wbits, M, N, K, block_size, x_dtype, true) ||
+         decode_i8_supported(wbits, M, N, K, block_size, ok, x_dtype, ok, true);
+}
+
 const char* qmm_weight_only_variant_for(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_size, int has_zp) {
   // Shape-only view of qmm_weight_only's AUTO choice, for a caller that passes a sufficient workspace and aligned pointers.
   if (block_size < 0) block_size = 0;
   const void* ok = reinterpret_cast<const void*>(uintptr_t(256));
   const bool can = limb_tc_shape_ok(wbits, M, N, K, block_size, QMM_BF16, has_zp != 0);
   const int tuned = tuned_variant(wbits, block_size, M, N, K);
-  if (can && (tuned ? tuned == QMM_VARIANT_I8TC : limb_tc_preferred(wbits, M, N, K, block_size))) return "i8tc";
+  if (can && has_zp) {
+    if (M > 8) return "i8tc";
+  } else if (can && (tuned ? tuned == QMM_VARIANT_I8TC : limb_tc_preferred(wbits, M, N, K, block_size))) return "i8tc";
   if (!has_zp && tuned == QMM_VARIANT_MMA && decode_mma_supported(wbits, M, N, K, block_size, ok, QMM_BF16, ok, false)) return "mma";
   if (!has_zp && tuned == QMM_VARIANT_TCGEN05 && mixed_tc_shape_ok(wbits, M, N, K, block_size, QMM_BF16, false)) return "tcgen05";
   if (decode_mma_supported(wbits, M, N, K, block_size, ok, QMM_BF16, ok, has_zp != 0)) return "mma";
@@ -377,7 +386,13 @@ int qmm_weight_only(int wbits, const void* x, int x_dtype, const void* w, const 
     // AUTO: the measured table first, the shape rule where the table has no entry for this shape
     const int tuned = variant == QMM_VARIANT_AUTO ? tuned_variant(wbits, block_size, M, N, K) : 0;
     bool use = variant == QMM_VARIANT_I8TC;
-    if (variant == QMM_VARIANT_AUTO && can) use = tuned ? tuned == QMM_VARIANT_I8TC : limb_tc_preferred(wbits, M, N, K, block_size);
+    if (variant == QMM_VARIANT_AUTO && can) {
+      use = tuned ? tuned == QMM_VARIANT_I8TC : limb_tc_preferred(wbits, M, N, K, block_size);
+      // Zero points and fp32 activations: the other kernels for more than a few tokens take neither, and the any-shape
+      // kernel is a hundred times slower (333 tokens of fp32 on [5120,6912] int8 with zero points: 12.2 ms, here 56 us).
+      // Up to eight tokens the register-dequant GEMV takes both.
+      if (zp || x_dtype == QMM_F32) use = M > 8;
+    }
     if (!use && tuned && tuned != QMM_VARIANT_I8TC && !zp) {
       // the table names one of the kernels behind the entry points below; they refuse what they cannot run, and AUTO
       // then decides there
@@ -387,8 +402,7 @@ int qmm_weight_only(int wbits, const void* x, int x_dtype, const void* w, const 
     }
     if (use) {
       log_choice("weight_only", "i8tc", M, N, K);
-      if (zp) return fail(QMM_ERR_UNSUPPORTED, "the split-activation tensor-core kernel does not take a zero point");
-      return launch_limb_tc(wbits, x, x_dtype, w, scale, out, out_dtype, M, N, K, block_size, 0, workspace, workspace_bytes,
+      return launch_limb_tc(wbits, x, x_dtype, w, scale, zp, out, out_dtype, M, N, K, block_size, 0, workspace, workspace_bytes,
                             as_stream(stream));
     }
   }
@@ -444,7 +458,7 @@ int qmm_gate_up(int wbits, const void* x, int x_dtype, const void* w, const floa
     return fail(QMM_ERR_BAD_SHAPE, "gate_up: K (%lld) must be a multiple of block_size (%lld)", (long long)K, (long long)block_size);
   if (M == 0 || N2 == 0) return QMM_OK;
   log_choice("gate_up", "i8tc", M, N2, K);
-  return launch_limb_tc(wbits, x, x_dtype, w, scale, out, out_dtype, M, N2, K, block_size, 1, workspace, workspace_bytes, st);
+  return launch_limb_tc(wbits, x, x_dtype, w, scale, nullptr, out, out_dtype, M, N2, K, block_size, 1, workspace, workspace_bytes, st);
 }
 
 int qmm_w4a16_perchannel_packed(const void* x, int x_dtype, const uint8_t* wp, const float* scale,

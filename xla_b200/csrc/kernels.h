@@ -67,7 +67,7 @@ int launch_decode_w8a8(const void* x, int x_dt, const int8_t* w, const float* w_
                        int64_t M, int64_t N, int64_t K, int saturate, cudaStream_t st);
 
 // ---- limb_gemm.cu (tcgen05 kind::i8 on unconverted weights; activations split into int8 limbs) ----------
-// Weight-only linear for 1 <= M <= 64 (bf16/f16/f32 activations, no zero point): stream-K over all SMs, needs
+// Weight-only linear (bf16/f16/f32 activations): stream-K over all SMs, needs
 // limb_tc_workspace_bytes(M, K) bytes of caller scratch whose first 1024 bytes are zero before the first use (the
 // kernel leaves them zero).  gate_up as in launch_decode_mma.
 constexpr int kLimbMaxCtas = 320;  // two CTAs per SM on up to 160 SMs
@@ -80,7 +80,7 @@ bool limb_tc_supported(int wbits, int64_t M, int64_t N, int64_t K, int64_t block
                        const void* w, bool has_zp);
 // AUTO's shape rule: true where this kernel is the fastest measured choice.
 bool limb_tc_preferred(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_size);
-int launch_limb_tc(int wbits, const void* x, int x_dt, const void* w, const float* scale, void* out, int out_dt, int64_t M,
+int launch_limb_tc(int wbits, const void* x, int x_dt, const void* w, const float* scale, const float* zp, void* out, int out_dt, int64_t M,
                    int64_t N, int64_t K, int64_t block_size, int gate_up, void* workspace, size_t workspace_bytes,
                    cudaStream_t st);
 

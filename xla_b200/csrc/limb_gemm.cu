@@ -95,6 +95,10 @@ enum Mode : int {
 
 struct Params {
   const float* scale;  // [N] or [S,N]
+  const float* zp;     // like scale, or null
+  const float* xs;     // with zp: [S][xs_pitch] sums of the fixed-point activations over each scale block
+  int xs_pitch;
+  float zp_mul;        // factor that the weight bytes carry (16 for int4 weights)
   const float* pw;     // [M]: 2^(e_m - 21) (times 1/16 for int4 weights)
   void* out;
   int out_dt;
@@ -228,12 +232,18 @@ __device__ __forceinline__ int64_t gate_up_column(int64_t n) { return ((n >> 4) 
 // Order of k inside the operand rows.  int8 weights: natural.  int4 weights: the nibble expansion emits, per raw
 // 16-byte chunk (32 nibbles, k = 32c + 8j + i), the 16 even-k values and then the 16 odd-k values, so value k sits at
 // 32c + 16*(i & 1) + 4j + i/2; the limb rows are written in the same order.
+constexpr int kMaxZpBlocks = 512;  // scale blocks of a weight with zero points
+
 // One CTA per token row.  xl: [NL*M][K] int8, row NL*m + l = limb l of token m; pw[m] = 2^(e_m - q) * pw_mul.
+// xs (for zero points; may be null): xs[b * xs_pitch + m] = sum of the row's fixed-point values over scale block b, which
+// covers block_groups groups of eight values (a multiple of 16 groups, or all of them); summed exactly in integers.
 // A row with a non-finite entry gets pw = NaN (its outputs are NaN); an all-zero row gets zeros.
 template <typename XT, int NL>
 __global__ void __launch_bounds__(1024) split_rows_kernel(const XT* __restrict__ x, int8_t* __restrict__ xl, float* __restrict__ pw,
-                                                          int64_t K, int perm4, float pw_mul) {
+                                                          int64_t K, int perm4, float pw_mul, float* __restrict__ xs, int xs_pitch,
+                                                          int block_groups) {
   __shared__ uint32_t s_max[32];
+  __shared__ unsigned long long s_sum[kMaxZpBlocks];
   if (blockIdx.x == 0 && threadIdx.x == 0) { DBG_STAMP(10); }
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");  // x may come from the previous kernel of the stream
@@ -263,14 +273,31 @@ __global__ void __launch_bounds__(1024) split_rows_kernel(const XT* __restrict__
   float mult, pwv;
   row_factors<NL>(mx, pw_mul, mult, pwv);
   if (threadIdx.x == 0) pw[m] = pwv;
+  const int blocks = xs ? (int)((groups + block_groups - 1) / block_groups) : 0;
+  if (xs) {
+    for (int b = threadIdx.x; b < blocks; b += blockDim.x) s_sum[b] = 0ull;
+    __syncthreads();
+  }
   int8_t* r0 = xl + (int64_t)(NL * m) * K;
   int8_t* r1 = r0 + K;
   int8_t* r2 = r1 + K;
-  for (int64_t gi = threadIdx.x; gi < groups; gi += blockDim.x) {
-    float v[8];
-    load8<XT>(xr + gi * 8, v);
+  const int lane = threadIdx.x & 31;
+  for (int64_t g0 = threadIdx.x - lane; g0 < groups; g0 += blockDim.x) {
+    const int64_t gi = g0 + lane;
+    float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (gi < groups) load8<XT>(xr + gi * 8, v);
     uint32_t l0[2], l1[2], l2[2] = {0u, 0u};  // bytes of limb l for k = 8*gi + i, packed in k order
     split8<NL>(v, mult, l0, l1, l2);
+    if (xs) {
+      // sixteen neighbouring groups are inside one scale block: one 64-bit atomic for them (all lanes of a row adding to
+      // one word took three times as long as the GEMM)
+      auto sum = [](const uint32_t* l) { return __dp4a((int)l[1], 0x01010101, __dp4a((int)l[0], 0x01010101, 0)); };
+      int t = sum(l0) + 256 * sum(l1) + (NL == 3 ? 65536 * sum(l2) : 0);
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if ((lane & 15) == 0 && gi < groups) atomicAdd(s_sum + (int)(gi / block_groups), (unsigned long long)(long long)t);
+    }
+    if (gi >= groups) continue;
     if (!perm4) {
       const int64_t o = gi * 8;
       *reinterpret_cast<uint2*>(r0 + o) = make_uint2(l0[0], l0[1]);
@@ -290,6 +317,10 @@ __global__ void __launch_bounds__(1024) split_rows_kernel(const XT* __restrict__
         *reinterpret_cast<uint32_t*>(r2 + base + 16) = odds(l2);
       }
     }
+  }
+  if (xs) {
+    __syncthreads();
+    for (int b = threadIdx.x; b < blocks; b += blockDim.x) xs[(int64_t)b * xs_pitch + m] = (float)(long long)s_sum[b];
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) { DBG_STAMP(12); }
 }
@@ -427,7 +458,7 @@ __device__ __forceinline__ void fold_regions_pipelined(uint32_t taddr, uint32_t 
   }
 }
 
-template <int WBITS, int NCOLS, int NL>
+template <int WBITS, int NCOLS, int NL, bool ZP>
 __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NCOLS, NL>::kOcc)
     limb_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const Params p) {
   using C = Cfg<WBITS, NCOLS, NL>;
@@ -859,6 +890,30 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
         if (warp == kDrainWarp0) { DBG_STAMP(16); }
       }
       drain_bar();  // the factors written at the top of the fragment are visible
+      float psv = ps;
+      if constexpr (ZP) {
+        // the zero points' term, once per tile: minus sum_b zp[b,n] * xs[b,m], in units of the fixed point; every lane
+        // reads the same token sums.  The zero points come from HBM and are fetched four blocks ahead.
+        if (p.mode == kPerChannel) {
+#pragma unroll
+          for (int t = 0; t < MTD; ++t) total[t] *= ps;
+          psv = 1.f;
+        }
+        const float* zp = p.zp + min(n, p.N - 1);
+        auto fetch_zp = [&](int b) { return -p.zp_mul * __ldg(zp + (int64_t)min(b, p.S - 1) * p.ld); };
+        float zq[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) zq[i] = fetch_zp(i);
+        const float* xs = p.xs + mt0;
+        for (int b = 0; b < p.S; ++b, xs += p.xs_pitch) {
+          const float z = zq[0];
+#pragma unroll
+          for (int i = 0; i < 3; ++i) zq[i] = zq[i + 1];
+          zq[3] = fetch_zp(b + 4);
+#pragma unroll
+          for (int t = 0; t < MTD; ++t) total[t] = fmaf(z, __ldg(xs + t), total[t]);
+        }
+      }
       float pwv[MTD];
 #pragma unroll
       for (int t = 0; t < MTD; ++t) pwv[t] = pw_s[half * MTD + t];
@@ -866,12 +921,12 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
 #pragma unroll
         for (int t = 0; t < MTD; ++t)
           if (t < mcount && n_ok)
-            store_from_f32(p.out, (int64_t)(p.m0 + mt0 + t) * p.ld + n, p.out_dt, total[t] * ps * pwv[t]);
+            store_from_f32(p.out, (int64_t)(p.m0 + mt0 + t) * p.ld + n, p.out_dt, total[t] * psv * pwv[t]);
       } else {
         // rows come in groups of 16: eight gate rows, then the eight up rows of the same outputs
 #pragma unroll
         for (int t = 0; t < MTD; ++t) {
-          const float v = t < mcount ? total[t] * ps * pwv[t] : 0.f;
+          const float v = t < mcount ? total[t] * psv * pwv[t] : 0.f;
           const float u = __shfl_down_sync(0xffffffffu, v, 8);
           if (t < mcount && n_ok && (rl & 8) == 0)
             store_from_f32(p.out, (int64_t)(p.m0 + mt0 + t) * (p.ld >> 1) + gate_up_column(n), p.out_dt, silu_mul(v, u));
@@ -967,6 +1022,8 @@ size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 struct Scratch {
   int8_t* limbs;
   float* pw;
+  float* xs;
+  int xs_pitch;
   float* partial;
   uint32_t* flags;
   size_t bytes;
@@ -986,13 +1043,13 @@ std::atomic<int> g_limb_policy{0};
 // there.  Wider batches pay per limb column: when the output is a 16-bit type, two limbs (15 bits below the row's
 // largest value, error at most 2^-15 of it per activation, under the output's own rounding) carry 64 tokens per
 // 128-column tile instead of 42.  fp32 outputs always get three.
-Plan plan_for(int wbits, int64_t M, int out_dt) {
-  const bool two_ok = g_limb_policy.load(std::memory_order_relaxed) != 3 && (out_dt == QMM_BF16 || out_dt == QMM_F16);
+Plan plan_for(int wbits, int64_t M, int out_dt, bool has_zp) {
+  const bool two_ok = !has_zp && g_limb_policy.load(std::memory_order_relaxed) != 3 && (out_dt == QMM_BF16 || out_dt == QMM_F16);
   Plan pl;
   pl.nl = 3;
   pl.items = false;
-  if (M <= 5) pl.ncols = 16;
-  else if (M <= 10) pl.ncols = 32;
+  if (M <= 5 && !has_zp) pl.ncols = 16;  // (zero points: fewer instances, shorter batches run elsewhere)
+  else if (M <= 10 && !has_zp) pl.ncols = 32;
   else if (M <= 16) pl.ncols = 48;
   else if (M <= 32 && !(wbits == 4 && two_ok)) pl.ncols = 96;
   else {
@@ -1007,7 +1064,7 @@ Plan plan_for(int wbits, int64_t M, int out_dt) {
 // tokens per launch above which a batch is chunked (24 tiles of 42, 16 tiles of 64)
 int64_t max_rows(int nl) { return nl == 2 ? 1024 : 1008; }
 
-// Layout of the caller's scratch: [flags: 1 KB][pw][limbs][partial tiles]; the flag words come first so that a
+// Layout of the caller's scratch: [flags][pw][block sums][limbs][partial tiles]; the flag words come first so that a
 // caller who clears only the head of the buffer clears them.  partial_tokens: tokens of a token tile.
 Scratch carve(void* base, int64_t M, int64_t K, int nl, int partial_tokens, int max_ctas) {
   Scratch s;
@@ -1017,6 +1074,9 @@ Scratch carve(void* base, int64_t M, int64_t K, int nl, int partial_tokens, int 
   off += align_up((size_t)max_ctas * 4, 1024);
   s.pw = reinterpret_cast<float*>(b + off);
   off += align_up((size_t)M * 4, 256);
+  s.xs = reinterpret_cast<float*>(b + off);
+  s.xs_pitch = (int)M + 64;  // a token tile may reach beyond the batch
+  off += align_up((size_t)(K / kTileK + 1) * s.xs_pitch * 4, 256);
   s.limbs = reinterpret_cast<int8_t*>(b + off);
   off += align_up((size_t)nl * M * K, 256);
   s.partial = reinterpret_cast<float*>(b + off);
@@ -1025,10 +1085,10 @@ Scratch carve(void* base, int64_t M, int64_t K, int nl, int partial_tokens, int 
   return s;
 }
 
-template <int WBITS, int NCOLS, int NL = 3>
+template <int WBITS, int NCOLS, int NL = 3, bool ZP = false>
 int launch_cfg(const CUtensorMap& map_w, const CUtensorMap& map_x, const Params& p, int grid, cudaStream_t st) {
   using C = Cfg<WBITS, NCOLS, NL>;
-  auto kern = limb_tc_kernel<WBITS, NCOLS, NL>;
+  auto kern = limb_tc_kernel<WBITS, NCOLS, NL, ZP>;
   static bool attr_set[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -1057,6 +1117,11 @@ int launch_cfg(const CUtensorMap& map_w, const CUtensorMap& map_x, const Params&
 
 template <int WBITS>
 int launch_ncols(int ncols, int nl, const CUtensorMap& map_w, const CUtensorMap& map_x, const Params& p, int grid, cudaStream_t st) {
+  if (p.zp) {
+    if (ncols == 48) return launch_cfg<WBITS, 48, 3, true>(map_w, map_x, p, grid, st);
+    if (ncols == 96) return launch_cfg<WBITS, 96, 3, true>(map_w, map_x, p, grid, st);
+    return launch_cfg<WBITS, 128, 3, true>(map_w, map_x, p, grid, st);
+  }
   if (nl == 2) return launch_cfg<WBITS, 128, 2>(map_w, map_x, p, grid, st);
   switch (ncols) {
     case 16: return launch_cfg<WBITS, 16>(map_w, map_x, p, grid, st);
@@ -1068,7 +1133,8 @@ int launch_ncols(int ncols, int nl, const CUtensorMap& map_w, const CUtensorMap&
 }
 
 template <typename XT>
-cudaError_t launch_split(const void* x, int8_t* xl, float* pw, int64_t M, int64_t K, int nl, int perm4, float pw_mul, cudaStream_t st) {
+cudaError_t launch_split(const void* x, int8_t* xl, float* pw, int64_t M, int64_t K, int nl, int perm4, float pw_mul, float* xs, int xs_pitch,
+                         int block_groups, cudaStream_t st) {
   int threads = (int)std::min<int64_t>(1024, std::max<int64_t>(64, align_up((size_t)(K / 8), 32)));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)M);
@@ -1079,8 +1145,8 @@ cudaError_t launch_split(const void* x, int8_t* xl, float* pw, int64_t M, int64_
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (nl == 2) return cudaLaunchKernelEx(&cfg, split_rows_kernel<XT, 2>, reinterpret_cast<const XT*>(x), xl, pw, K, perm4, pw_mul);
-  return cudaLaunchKernelEx(&cfg, split_rows_kernel<XT, 3>, reinterpret_cast<const XT*>(x), xl, pw, K, perm4, pw_mul);
+  if (nl == 2) return cudaLaunchKernelEx(&cfg, split_rows_kernel<XT, 2>, reinterpret_cast<const XT*>(x), xl, pw, K, perm4, pw_mul, xs, xs_pitch, block_groups);
+  return cudaLaunchKernelEx(&cfg, split_rows_kernel<XT, 3>, reinterpret_cast<const XT*>(x), xl, pw, K, perm4, pw_mul, xs, xs_pitch, block_groups);
 }
 
 }  // namespace
@@ -1185,7 +1251,7 @@ size_t limb_tc_workspace_bytes(int64_t M, int64_t K) {
 }
 
 bool limb_tc_shape_ok(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_size, int x_dt, bool has_zp) {
-  if (has_zp) return false;
+  if (has_zp && block_size > 0 && K / block_size > kMaxZpBlocks) return false;
   if (x_dt != QMM_BF16 && x_dt != QMM_F16 && x_dt != QMM_F32) return false;
   if (M < 1 || N < 1 || K < 128) return false;
   if (wbits == 8 ? (K % 16 != 0) : (K % 32 != 0)) return false;  // TMA row pitches of the weights and the limbs
@@ -1235,17 +1301,18 @@ cudaError_t launch_expand(const void* src, void* dst, int64_t rows, int64_t K, c
 
 // pw_mul: factor folded into the per-token power of two (1/16 when the weight bytes hold value * 16); w_dep: the
 // weights are written by a kernel earlier in the stream that the weight producer has to wait for.
-int launch_limb_impl(int wbits, const void* x, int x_dt, const void* w, const float* scale, void* out, int out_dt, int64_t M,
+int launch_limb_impl(int wbits, const void* x, int x_dt, const void* w, const float* scale, const float* zp, void* out, int out_dt, int64_t M,
                      int64_t N, int64_t K, int64_t block_size, int gate_up, void* workspace, size_t workspace_bytes,
                      float pw_mul, int w_dep, cudaStream_t st) {
-  if (!limb_tc_supported(wbits, M, N, K, block_size, x, x_dt, w, false))
+  if (!limb_tc_supported(wbits, M, N, K, block_size, x, x_dt, w, zp != nullptr))
     return fail(QMM_ERR_UNSUPPORTED,
                 "split-activation tensor-core kernel: needs an sm_100 device, K >= 128 and a multiple of %d, "
-                "block_size 128 or a multiple of 256, 16-byte aligned x/w, no zero point (M=%lld N=%lld K=%lld bs=%lld)",
+                "block_size 128 or a multiple of 256, 16-byte aligned x/w (M=%lld N=%lld K=%lld bs=%lld)",
                 wbits == 8 ? 16 : 32, (long long)M, (long long)N, (long long)K, (long long)block_size);
+  if (gate_up && zp) return fail(QMM_ERR_UNSUPPORTED, "fused gate/up epilogue: no zero points");
   if (gate_up && N % 16 != 0)
     return fail(QMM_ERR_BAD_SHAPE, "fused gate/up epilogue: the interleaved weight needs a multiple of 16 rows, got %lld", (long long)N);
-  const Plan pl = plan_for(wbits, M, out_dt);
+  const Plan pl = plan_for(wbits, M, out_dt, zp != nullptr);
   const int nl = pl.nl;
   const size_t need = carve(nullptr, std::min(M, max_rows(nl)), K, nl, pl.tile_tokens, kLimbMaxCtas).bytes;
   if (!workspace || workspace_bytes < need)
@@ -1262,7 +1329,7 @@ int launch_limb_impl(int wbits, const void* x, int x_dt, const void* w, const fl
       cudaGetLastError();
       return fail(QMM_ERR_LAUNCH, "expand_int4_kernel launch: %s", cudaGetErrorString(e));
     }
-    return launch_limb_impl(8, x, x_dt, wide, scale, out, out_dt, M, N, K, block_size, 0, workspace, wide_off, 0.0625f, 1, st);
+    return launch_limb_impl(8, x, x_dt, wide, scale, zp, out, out_dt, M, N, K, block_size, 0, workspace, wide_off, 0.0625f, 1, st);
   }
   if (M > max_rows(nl)) {
     // long batches run in chunks of whole token tiles that share the scratch (same stream: ordered)
@@ -1271,7 +1338,7 @@ int launch_limb_impl(int wbits, const void* x, int x_dt, const void* w, const fl
     const size_t xb = dtype_size(x_dt), ob = dtype_size(out_dt);
     for (int64_t m0 = 0; m0 < M; m0 += rows) {
       const int64_t mc = std::min(rows, M - m0);
-      const int rc = launch_limb_impl(wbits, reinterpret_cast<const uint8_t*>(x) + (size_t)m0 * K * xb, x_dt, w, scale,
+      const int rc = launch_limb_impl(wbits, reinterpret_cast<const uint8_t*>(x) + (size_t)m0 * K * xb, x_dt, w, scale, zp,
                                       reinterpret_cast<uint8_t*>(out) + (size_t)m0 * N * ob, out_dt, mc, N, K, block_size, 0, workspace,
                                       workspace_bytes, pw_mul, w_dep, st);
       if (rc != QMM_OK) return rc;
@@ -1299,11 +1366,12 @@ int launch_limb_impl(int wbits, const void* x, int x_dt, const void* w, const fl
   {
     // the limbs are made by a kernel of their own (one CTA per token) and reach the main kernel as TMA tiles; the two
     // are chained with programmatic dependent launch, so the main kernel's set-up and first weight loads run under it
+    const int block_groups = (int)((block_size > 0 ? block_size : K) / 8);
     const int perm4 = wbits == 4 && slice_rows == 0;  // the expanded weights are in natural k order
     cudaError_t e;
-    if (x_dt == QMM_F32) e = launch_split<float>(x, sc.limbs, sc.pw, M, K, nl, perm4, pw_mul, st);
-    else if (x_dt == QMM_BF16) e = launch_split<__nv_bfloat16>(x, sc.limbs, sc.pw, M, K, nl, perm4, pw_mul, st);
-    else e = launch_split<__half>(x, sc.limbs, sc.pw, M, K, nl, perm4, pw_mul, st);
+    if (x_dt == QMM_F32) e = launch_split<float>(x, sc.limbs, sc.pw, M, K, nl, perm4, pw_mul, zp ? sc.xs : nullptr, sc.xs_pitch, block_groups, st);
+    else if (x_dt == QMM_BF16) e = launch_split<__nv_bfloat16>(x, sc.limbs, sc.pw, M, K, nl, perm4, pw_mul, zp ? sc.xs : nullptr, sc.xs_pitch, block_groups, st);
+    else e = launch_split<__half>(x, sc.limbs, sc.pw, M, K, nl, perm4, pw_mul, zp ? sc.xs : nullptr, sc.xs_pitch, block_groups, st);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return fail(QMM_ERR_LAUNCH, "split_rows_kernel launch: %s", cudaGetErrorString(e));
@@ -1315,6 +1383,9 @@ int launch_limb_impl(int wbits, const void* x, int x_dt, const void* w, const fl
 
   Params p;
   p.pw = sc.pw;
+  p.xs = sc.xs;
+  p.xs_pitch = sc.xs_pitch;
+  p.zp_mul = 1.f / pw_mul;
   p.out_dt = out_dt;
   p.M = (int)M;
   p.ld = N;
@@ -1331,6 +1402,7 @@ int launch_limb_impl(int wbits, const void* x, int x_dt, const void* w, const fl
   p.m0 = 0;
   if (slice_rows == 0) {
     p.scale = scale;
+    p.zp = zp;
     p.out = out;
     p.w_dep = w_dep;
     return launch_main(wbits, w, N, K, pl, p, map_x, st);
@@ -1344,6 +1416,7 @@ int launch_limb_impl(int wbits, const void* x, int x_dt, const void* w, const fl
       return fail(QMM_ERR_LAUNCH, "expand_int4_kernel launch: %s", cudaGetErrorString(e));
     }
     p.scale = scale + n0;
+    p.zp = zp ? zp + n0 : nullptr;
     p.out = reinterpret_cast<uint8_t*>(out) + (size_t)n0 * ob;
     p.w_dep = 1;
     rc = launch_main(8, wide, rows, K, pl, p, map_x, st);
@@ -1354,10 +1427,10 @@ int launch_limb_impl(int wbits, const void* x, int x_dt, const void* w, const fl
 
 }  // namespace
 
-int launch_limb_tc(int wbits, const void* x, int x_dt, const void* w, const float* scale, void* out, int out_dt, int64_t M,
+int launch_limb_tc(int wbits, const void* x, int x_dt, const void* w, const float* scale, const float* zp, void* out, int out_dt, int64_t M,
                    int64_t N, int64_t K, int64_t block_size, int gate_up, void* workspace, size_t workspace_bytes,
                    cudaStream_t st) {
-  return launch_limb_impl(wbits, x, x_dt, w, scale, out, out_dt, M, N, K, block_size, gate_up, workspace, workspace_bytes,
+  return launch_limb_impl(wbits, x, x_dt, w, scale, zp, out, out_dt, M, N, K, block_size, gate_up, workspace, workspace_bytes,
                           wbits == 4 ? 0.0625f : 1.f, 0, st);
 }
 

@@ -108,9 +108,10 @@ Tensor output(const Tensor& x, int64_t N, at::ScalarType dt) {
   return at::empty(shape, x.options().dtype(dt));
 }
 
-// Zero points above eight tokens with 16-bit activations are applied after the kernel in the Python form.
-bool zero_point_outside(int64_t M, const Tensor& x, const optional<Tensor>& zp) {
-  return zp.has_value() && M > 8 && tl_variant == QMM_VARIANT_AUTO && x.scalar_type() != at::kFloat;
+// The few shapes whose zero points are applied after the kernel (in the Python form).
+bool zero_point_outside(const Tensor& x, int64_t N, int wbits, int64_t block, const optional<Tensor>& zp) {
+  return zp.has_value() && tl_variant == QMM_VARIANT_AUTO && x.scalar_type() != at::kFloat &&
+         !qmm_zero_point_in_kernel(wbits, x.numel() / x.size(-1), N, x.size(-1), block, dtype_code(x.scalar_type()));
 }
 
 struct Call {
@@ -190,7 +191,7 @@ Tensor quantized_matmul(const Tensor& x, const Tensor& w, const Tensor& scale, c
     c10::cuda::OptionalCUDAGuard guard(x.device());
     const bool qact = quantize_activation.value_or(false);
     const at::ScalarType dt = promote(x, scale, zp);
-    if (dtype_code(dt) >= 0 && (qact || !zero_point_outside(x.numel() / x.size(-1), x, zp))) {
+    if (dtype_code(dt) >= 0 && (qact || !zero_point_outside(x, w.size(0), 8, -1, zp))) {
       const Call c = make_call(x, w, scale, zp, -1, false);
       Tensor out = output(x, c.N, dt);
       if (qact ? w8a8(c, out) : weight_only(c, out)) return out;
@@ -218,7 +219,7 @@ Tensor quantized_matmul_packed(const Tensor& x, const Tensor& w, const Tensor& s
   if (!(quantize_activation && (weight_is_packed || block_size != -1)) && plain(x, w, scale, zp, block_size, weight_is_packed)) {
     c10::cuda::OptionalCUDAGuard guard(x.device());
     const at::ScalarType dt = out_dtype.has_value() ? *out_dtype : promote(x, scale, zp);
-    if (dtype_code(dt) >= 0 && (quantize_activation || !zero_point_outside(x.numel() / x.size(-1), x, zp))) {
+    if (dtype_code(dt) >= 0 && (quantize_activation || !zero_point_outside(x, w.size(0), weight_is_packed ? 4 : 8, block_size, zp))) {
       const Call c = make_call(x, w, scale, zp, block_size, weight_is_packed);
       Tensor out = output(x, c.N, dt);
       if (quantize_activation ? w8a8(c, out) : weight_only(c, out)) return out;

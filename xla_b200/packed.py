@@ -107,7 +107,7 @@ def quantized_matmul_packed(x, w, scaler, zero_point=None, block_size=-1, int4_w
   s32, zp32 = _qm._f32(scaler), _qm._f32(zero_point)
   L = _capi.lib()
   variant = _capi.VARIANTS[_qm.current_variant()]
-  zp_after = not quantize_activation and _qm._zero_point_outside(M, x2, zero_point)
+  zp_after = not quantize_activation and _qm._zero_point_outside(x2, N, 4 if weight_is_packed else 8, block_size, zero_point)
   out_buf = None if quantize_activation else out
 
   def run():
