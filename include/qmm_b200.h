@@ -65,6 +65,8 @@ typedef enum qmm_variant {
                               over all SMs, 1 <= M <= 64; only through qmm_weight_only (needs workspace) */
   QMM_VARIANT_I8MMA = 7,   /* decode: activations split into int8 limbs, unconverted weights into warp-level int8 MMAs,
                               M <= 16, zero points allowed; only through qmm_weight_only (no workspace) */
+  QMM_VARIANT_TMEM = 8,    /* weights converted into tensor memory as the A operand of tcgen05.mma.kind::f16, any M, bf16/f16
+                              activations, zero points allowed; only through qmm_weight_only (needs workspace) */
 } qmm_variant;
 
 typedef enum qmm_op {

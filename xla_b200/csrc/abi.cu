@@ -1,6 +1,7 @@
 // extern "C" entry points of libqmm_b200 (declared in include/qmm_b200.h): argument checks,
 // kernel-family selection, and the host-side helpers the kernels share.
 #include <cuda.h>
+#include <algorithm>
 #include <atomic>
 #include <stdarg.h>
 #include <stdio.h>
@@ -360,11 +361,11 @@ const char* qmm_weight_only_variant_for(int wbits, int64_t M, int64_t N, int64_t
 }
 
 size_t qmm_weight_only_workspace_size(int64_t max_M, int64_t K) {
-  return limb_tc_workspace_bytes(max_M, K);
+  return std::max(limb_tc_workspace_bytes(max_M, K), tmem_gemm_workspace_bytes(max_M, K));
 }
 
 size_t qmm_weight_only_workspace_size_for(int wbits, int64_t max_M, int64_t N, int64_t K) {
-  const size_t base = limb_tc_workspace_bytes(max_M, K);
+  const size_t base = qmm_weight_only_workspace_size(max_M, K);
   if (base == 0 || N < 1) return base;
   return (base + 255) / 256 * 256 + limb_tc_wide_bytes(wbits, max_M, N, K);
 }
@@ -411,6 +412,13 @@ int qmm_weight_only(int wbits, const void* x, int x_dtype, const void* w, const 
     if (rc != QMM_OK || M * N == 0) return rc;
     log_choice("weight_only", "i8mma", M, N, K);
     return launch_decode_i8(wbits, x, x_dtype, w, scale, zp, out, out_dtype, M, N, K, block_size, 0, as_stream(stream));
+  }
+  if (variant == QMM_VARIANT_TMEM) {
+    int rc = check_common(x, x_dtype, w, scale, out, out_dtype, M, N, K);
+    if (rc != QMM_OK || M * N == 0) return rc;
+    log_choice("weight_only", "tmem", M, N, K);
+    return launch_tmem_gemm(wbits, x, x_dtype, w, scale, zp, out, out_dtype, M, N, K, block_size, 0, workspace, workspace_bytes,
+                            as_stream(stream));
   }
   if (wbits == 8) {
     if (block_size > 0)

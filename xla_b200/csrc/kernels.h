@@ -84,6 +84,16 @@ int launch_limb_tc(int wbits, const void* x, int x_dt, const void* w, const floa
                    int64_t N, int64_t K, int64_t block_size, int gate_up, void* workspace, size_t workspace_bytes,
                    cudaStream_t st);
 
+// ---- tmem_gemm.cu (tcgen05 kind::f16, weights converted into tensor memory) -------------------------------------------
+// Weight-only linear for batches of bf16/f16 activations, zero points allowed; scratch as limb_gemm.cu's (its first 2 KB
+// are flag words that are zero between launches).
+size_t tmem_gemm_workspace_bytes(int64_t max_M, int64_t K);
+bool tmem_gemm_shape_ok(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_size, int x_dt);
+bool tmem_gemm_supported(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_size, const void* x, int x_dt, const void* w);
+int launch_tmem_gemm(int wbits, const void* x, int x_dt, const void* w, const float* scale, const float* zp, void* out, int out_dt,
+                     int64_t M, int64_t N, int64_t K, int64_t block_size, int gate_up, void* workspace, size_t workspace_bytes,
+                     cudaStream_t st);
+
 // ---- peer_reduce.cu -----------------------------------------------------------------------
 // One-shot all-reduce of fp32 partial results that every rank keeps in peer-mapped memory.
 int launch_peer_allreduce(void* const* data_ptrs, void* const* flag_ptrs, int rank, int world, uint32_t epoch, void* out,
