@@ -1,0 +1,47 @@
+"""The tensor-memory kernel against the CPU oracle where its tiling can go wrong: every accumulator width, partial row and
+token tiles, K that ends inside a step or a raw tile, items split over CTAs, scale blocks of 64 to several steps."""
+import pytest
+import torch
+
+import xla_b200
+from oracle import qmm_oracle as qo
+from tests import qmm_cases as qc
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("wbits,bs,N,K,M", [
+    (8, -1, 128, 64, 1), (8, -1, 300, 1056, 20), (8, 64, 130, 320, 33), (8, 128, 1000, 1280, 64), (8, 256, 129, 768, 65),
+    (8, -1, 260, 2064, 128), (4, -1, 77, 4000, 16), (4, 128, 300, 1152, 50), (4, 64, 300, 1984, 40), (4, 64, 512, 192, 129),
+    (4, 128, 128 * 149, 256, 130), (4, 256, 300, 1024, 193), (4, 128, 640, 4096, 400), (8, 512, 200, 1024, 577),
+])
+def test_against_the_oracle(dtype, wbits, bs, N, K, M):
+  g = qc.gen(N + K + M)
+  x = qc.activations(g, M, K, dtype, outliers=True)
+  w = qc.int4_weight(g, N, K) if wbits == 4 else qc.int8_weight(g, N, K)
+  s = qc.per_channel_scale(g, N) if bs == -1 else qc.blockwise_scale(g, K // bs, N)
+  rows = torch.tensor(sorted({0, M // 3, M // 2, M - 2 if M > 1 else 0, M - 1}))
+  exact = qo.quantized_matmul(x[rows].float(), w if bs == -1 else qc.to_sbn(w, bs), s, block_size=bs, dot_round=None)
+  wd = xla_b200.pack_int4(w.to(DEV)) if wbits == 4 else w.to(DEV)
+  with xla_b200.force_variant("tmem"):
+    out = torch.ops.xla_b200.quantized_matmul_packed(x.to(DEV), wd, s.to(DEV), block_size=bs, int4_weight=wbits == 4,
+                                                     weight_is_packed=wbits == 4, out_dtype=torch.float32)
+  assert qo.max_abs_rel(out[rows.to(DEV)], exact) < 1e-5
+
+
+@pytest.mark.parametrize("M", [65, 200, 1100])
+def test_gate_up(M):
+  g = qc.gen(M)
+  N, K, bs = 128 * 101, 512, 128
+  x = qc.activations(g, M, K)
+  wg, wu = qc.int4_weight(g, N // 2, K), qc.int4_weight(g, N // 2, K)
+  sg, su = qc.blockwise_scale(g, K // bs, N // 2), qc.blockwise_scale(g, K // bs, N // 2)
+  w, s = xla_b200.interleave_gate_up(xla_b200.pack_int4(wg.to(DEV)), xla_b200.pack_int4(wu.to(DEV)), sg.to(DEV), su.to(DEV), bs)
+  rows = torch.tensor([0, M // 2, M - 1])
+  gate = qo.quantized_matmul(x[rows].float(), qc.to_sbn(wg, bs), sg, block_size=bs, dot_round=None)
+  up = qo.quantized_matmul(x[rows].float(), qc.to_sbn(wu, bs), su, block_size=bs, dot_round=None)
+  out = torch.ops.xla_b200.quantized_gate_up(x.to(DEV), w, s, block_size=bs, int4_weight=True, weight_is_packed=True,
+                                             out_dtype=torch.float32)
+  assert qo.max_abs_rel(out[rows.to(DEV)], torch.nn.functional.silu(torch.as_tensor(gate)) * torch.as_tensor(up)) < 1e-4

@@ -363,27 +363,34 @@ __global__ void __launch_bounds__(kThreads, 1)
           for (int q = 0; q < kSPR; ++q) {
             const uint32_t j = i + q;
             if (s + q >= s1 || (int)(j & 1) != grp) continue;
-            uint4 v[kPieces];
-#pragma unroll
-            for (int c = 0; c < kPieces; ++c) v[c] = lds128(row + (((uint32_t)(q * kPieces + c) ^ sw) << 4));
+            auto piece = [&](int c) { return lds128(row + (((uint32_t)(q * kPieces + c) ^ sw) << 4)); };
+            uint4 v = piece(0);
             // the MMAs that read this operand slot last are complete
             if (j >= (uint32_t)kASlots)
               ptx::mbar_wait_warp(&done[(j - kASlots) % kDone], ((j - kASlots) / kDone) & 1, abort_flag, p.err_word, ptx::kErrWaitEmpty);
             ptx::tcgen05_fence_after();
-            const uint32_t t = t_row + (j % kASlots) * kACols;
-            constexpr int kWords = WBITS == 4 ? 4 : 8;  // raw words per 16 columns
-#pragma unroll
-            for (int c = 0; c < KS / 32; ++c) {
+            uint32_t t = t_row + (j % kASlots) * kACols;
+            // Rolled: the three kinds of warps of a scheduler share its instruction cache, and this body is the longest.
+#pragma unroll 1
+            for (int c = 0; c < kPieces; ++c) {
+              const uint4 nx = piece(min(c + 1, kPieces - 1));
               uint32_t o[16];
-#pragma unroll
-              for (int e = 0; e < kWords; ++e) {
-                const int wi = c * kWords + e;
-                const uint4& q4 = v[wi / 4];
-                const uint32_t w = wi % 4 == 0 ? q4.x : wi % 4 == 1 ? q4.y : wi % 4 == 2 ? q4.z : q4.w;
-                if constexpr (WBITS == 4) cvt_s4x8<XT>(w, o + 4 * e);
-                else cvt_s8x4<XT>(w, o + 2 * e);
+              if constexpr (WBITS == 4) {
+                cvt_s4x8<XT>(v.x, o);
+                cvt_s4x8<XT>(v.y, o + 4);
+                cvt_s4x8<XT>(v.z, o + 8);
+                cvt_s4x8<XT>(v.w, o + 12);
+                ptx::tmem_st_32x32b_x16(t, o);
+                t += 16;
+              } else {
+                cvt_s8x4<XT>(v.x, o);
+                cvt_s8x4<XT>(v.y, o + 2);
+                cvt_s8x4<XT>(v.z, o + 4);
+                cvt_s8x4<XT>(v.w, o + 6);
+                ptx::tmem_st_32x32b_x8(t, o);
+                t += 8;
               }
-              ptx::tmem_st_32x32b_x16(t + 16 * c, o);
+              v = nx;
             }
             ptx::tmem_st_wait();
             ptx::tcgen05_fence_before();

@@ -237,7 +237,7 @@ Tensor quantized_gate_up(const Tensor& x, const Tensor& w, const Tensor& scale, 
     const bool half = x.scalar_type() != at::kFloat;
     const bool decode = M <= 32 && half && K % (512 / wbits) == 0 && (block_size == -1 || block_size % (512 / wbits) == 0) &&
                         (tl_variant == QMM_VARIANT_AUTO || tl_variant == QMM_VARIANT_MMA);
-    const bool batch = !decode && M > 32 && M <= 1008 && K >= 128 && K % (128 / wbits) == 0 &&
+    const bool batch = !decode && M > 32 && K >= 128 && K % (128 / wbits) == 0 &&
                        (block_size == -1 || block_size == 128 || block_size % 256 == 0) &&
                        (tl_variant == QMM_VARIANT_AUTO || tl_variant == QMM_VARIANT_I8TC);
     const at::ScalarType dt = out_dtype.has_value() ? *out_dtype : promote(x, scale, {});
