@@ -582,6 +582,9 @@ int qmm_w8a8_perchannel(const void* x, int x_dtype, const int8_t* w, const float
   int rc = check_common(x, x_dtype, w, w_scale, out, out_dtype, M, N, K);
   if (rc != QMM_OK || M * N == 0) return rc;
   // decode batches: one kernel quantizes and multiplies, no scratch
+  // Nine to fifteen tokens on a small weight with short rows: the any-shape GEMM is done in the 8 us that the others need
+  // to start ([300,512] at 15 tokens 8.2 us, tcgen05 17; at 10 fp16 tokens 8.8, decode kernel 11).
+  if (variant == QMM_VARIANT_AUTO && M > 8 && M < 16 && K <= 512 && N * K <= (1 << 20)) variant = QMM_VARIANT_GENERIC;
   if (variant == QMM_VARIANT_AUTO && M <= kW8A8DecodeTokens && decode_w8a8_supported(M, N, K, x, x_dtype, w, zp != nullptr)) {
     log_choice("w8a8_perchannel", "i8mma", M, N, K);
     return launch_decode_w8a8(x, x_dtype, w, w_scale, zp, out, out_dtype, M, N, K, saturate, as_stream(stream));
