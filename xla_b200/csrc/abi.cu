@@ -211,12 +211,18 @@ static bool use_decode_i8(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs
 //                  to the split-activation kernel's narrower ones ([4096,4096] at 128 tokens 23 us against 19;
 //                  [14336,4096] at 96 tokens 27 against 35, [28672,8192] at 512 tokens 284 against 340).  Per channel up
 //                  to 384 tokens, from where that kernel expands the weights once.
-static bool use_tmem(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, int x_dt, bool has_zp) {
+//   fp32 results   above 64 tokens, when the items fill half of the SMs: the other kernel needs a third limb per token
+//                  there (int8 [28672,8192] at 512 tokens 257 us against 312, [2432,9248] at 763 tokens 49 against 74).
+//   narrow int8    up to 2048 outputs and above the 1024 tokens of one launch of the other kernel, whose launches are then
+//                  a round or two of items each ([1536,14592] at 4178 tokens 189 us against 313).
+static bool use_tmem(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, int x_dt, int out_dt, bool has_zp) {
   if (!tmem_gemm_shape_ok(wbits, M, N, K, bs, x_dt)) return false;
   if (has_zp) return M > 8;
   if (bs == 64) return M > 32;
   const int64_t items = ceil_div(N, 128) * ceil_div(M, 192);
-  return wbits == 4 && M > 64 && 3 * items >= 2 * sm_count() && (bs > 0 || M < 384);
+  if (out_dt == QMM_F32 && M > 64 && 2 * items >= sm_count() && (wbits == 8 || bs > 0 || M < 384)) return true;
+  if (wbits == 8) return M > 1024 && N <= 2048;
+  return M > 64 && 3 * items >= 2 * sm_count() && (bs > 0 || M < 384);
 }
 
 int qmm_w8a16_perchannel(const void* x, int x_dtype, const int8_t* w, const float* scale,
@@ -357,7 +363,7 @@ int qmm_tuned_variant(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_
 int qmm_zero_point_in_kernel(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_size, int x_dtype) {
   if (block_size < 0) block_size = 0;
   const void* ok = reinterpret_cast<const void*>(uintptr_t(256));
-  return M <= 8 || use_tmem(wbits, M, N, K, block_size, x_dtype, true) || limb_tc_shape_ok(wbits, M, N, K, block_size, x_dtype, true) ||
+  return M <= 8 || use_tmem(wbits, M, N, K, block_size, x_dtype, QMM_F32, true) || limb_tc_shape_ok(wbits, M, N, K, block_size, x_dtype, true) ||
          decode_i8_supported(wbits, M, N, K, block_size, ok, x_dtype, ok, true);
 }
 
@@ -365,7 +371,7 @@ const char* qmm_weight_only_variant_for(int wbits, int64_t M, int64_t N, int64_t
   // Shape-only view of qmm_weight_only's AUTO choice, for a caller that passes a sufficient workspace and aligned pointers.
   if (block_size < 0) block_size = 0;
   const void* ok = reinterpret_cast<const void*>(uintptr_t(256));
-  if (use_tmem(wbits, M, N, K, block_size, QMM_BF16, has_zp != 0)) return "tmem";
+  if (use_tmem(wbits, M, N, K, block_size, QMM_BF16, QMM_BF16, has_zp != 0)) return "tmem";
   const bool can = limb_tc_shape_ok(wbits, M, N, K, block_size, QMM_BF16, has_zp != 0);
   const int tuned = tuned_variant(wbits, block_size, M, N, K);
   if (can && has_zp) {
@@ -401,7 +407,7 @@ int qmm_weight_only(int wbits, const void* x, int x_dtype, const void* w, const 
       return fail(QMM_ERR_BAD_SHAPE, "input_dim should be divisible by block_size, got input_dim: %lld, block_size: %lld",
                   (long long)K, (long long)block_size);
     if (variant == QMM_VARIANT_AUTO && use_decode_i8(wbits, M, N, K, block_size, x, x_dtype, w, zp != nullptr)) variant = QMM_VARIANT_I8MMA;
-    if (variant == QMM_VARIANT_AUTO && use_tmem(wbits, M, N, K, block_size, x_dtype, zp != nullptr) && aligned(x, 16) && aligned(w, 16) &&
+    if (variant == QMM_VARIANT_AUTO && use_tmem(wbits, M, N, K, block_size, x_dtype, out_dtype, zp != nullptr) && aligned(x, 16) && aligned(w, 16) &&
         device_is_sm100() && workspace && aligned(workspace, 256) && workspace_bytes >= tmem_gemm_workspace_bytes(M, K))
       variant = QMM_VARIANT_TMEM;
     const bool can = limb_tc_supported(wbits, M, N, K, block_size, x, x_dtype, w, zp != nullptr) && workspace &&
@@ -487,7 +493,7 @@ int qmm_gate_up(int wbits, const void* x, int x_dtype, const void* w, const floa
   if (block_size < 0 || (block_size > 0 && K % block_size != 0))
     return fail(QMM_ERR_BAD_SHAPE, "gate_up: K (%lld) must be a multiple of block_size (%lld)", (long long)K, (long long)block_size);
   if (M == 0 || N2 == 0) return QMM_OK;
-  if (use_tmem(wbits, M, N2, K, block_size, x_dtype, false) && aligned(x, 16) && aligned(w, 16) && workspace &&
+  if (use_tmem(wbits, M, N2, K, block_size, x_dtype, out_dtype, false) && aligned(x, 16) && aligned(w, 16) && workspace &&
       workspace_bytes >= tmem_gemm_workspace_bytes(M, K)) {
     log_choice("gate_up", "tmem", M, N2, K);
     return launch_tmem_gemm(wbits, x, x_dtype, w, scale, nullptr, out, out_dtype, M, N2, K, block_size, 1, workspace, workspace_bytes, st);
