@@ -236,14 +236,14 @@ constexpr int kMaxZpBlocks = 512;  // scale blocks of a weight with zero points
 
 // One CTA per token row.  xl: [NL*M][K] int8, row NL*m + l = limb l of token m; pw[m] = 2^(e_m - q) * pw_mul.
 // xs (for zero points; may be null): xs[b * xs_pitch + m] = sum of the row's fixed-point values over scale block b, which
-// covers block_groups groups of eight values (a multiple of 16 groups, or all of them); summed exactly in integers.
+// covers block_groups groups of eight values (a multiple of eight groups, or all of them); summed exactly in integers.
 // A row with a non-finite entry gets pw = NaN (its outputs are NaN); an all-zero row gets zeros.
 template <typename XT, int NL>
 __global__ void __launch_bounds__(1024) split_rows_kernel(const XT* __restrict__ x, int8_t* __restrict__ xl, float* __restrict__ pw,
                                                           int64_t K, int perm4, float pw_mul, float* __restrict__ xs, int xs_pitch,
                                                           int block_groups) {
   __shared__ uint32_t s_max[32];
-  __shared__ unsigned long long s_sum[kMaxZpBlocks];
+  __shared__ int s_lo[kMaxZpBlocks], s_hi[kMaxZpBlocks];
   if (blockIdx.x == 0 && threadIdx.x == 0) { DBG_STAMP(10); }
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");  // x may come from the previous kernel of the stream
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(1024) split_rows_kernel(const XT* __restrict__
   if (threadIdx.x == 0) pw[m] = pwv;
   const int blocks = xs ? (int)((groups + block_groups - 1) / block_groups) : 0;
   if (xs) {
-    for (int b = threadIdx.x; b < blocks; b += blockDim.x) s_sum[b] = 0ull;
+    for (int b = threadIdx.x; b < blocks; b += blockDim.x) s_lo[b] = s_hi[b] = 0;
     __syncthreads();
   }
   int8_t* r0 = xl + (int64_t)(NL * m) * K;
@@ -289,13 +289,19 @@ __global__ void __launch_bounds__(1024) split_rows_kernel(const XT* __restrict__
     uint32_t l0[2], l1[2], l2[2] = {0u, 0u};  // bytes of limb l for k = 8*gi + i, packed in k order
     split8<NL>(v, mult, l0, l1, l2);
     if (xs) {
-      // sixteen neighbouring groups are inside one scale block: one 64-bit atomic for them (all lanes of a row adding to
-      // one word took three times as long as the GEMM)
+      // Eight neighbouring groups (64 values) are inside one scale block and add to it together, in two 32-bit halves:
+      // at most 1024 times, so neither overflows.  (The machine adds 32-bit words in shared memory by itself; 64-bit ones
+      // are retried until no other lane was faster: 333 rows of 6912 fp32 values in one block each 52.1 us with the GEMM
+      // and sixteen groups to an add, now 47.4.)
       auto sum = [](const uint32_t* l) { return __dp4a((int)l[1], 0x01010101, __dp4a((int)l[0], 0x01010101, 0)); };
       int t = sum(l0) + 256 * sum(l1) + (NL == 3 ? 65536 * sum(l2) : 0);
 #pragma unroll
-      for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      if ((lane & 15) == 0 && gi < groups) atomicAdd(s_sum + (int)(gi / block_groups), (unsigned long long)(long long)t);
+      for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if ((lane & 7) == 0 && gi < groups) {
+        const int b = (int)(gi / block_groups);
+        atomicAdd(s_lo + b, t & 0xffff);
+        atomicAdd(s_hi + b, t >> 16);
+      }
     }
     if (gi >= groups) continue;
     if (!perm4) {
@@ -320,7 +326,7 @@ __global__ void __launch_bounds__(1024) split_rows_kernel(const XT* __restrict__
   }
   if (xs) {
     __syncthreads();
-    for (int b = threadIdx.x; b < blocks; b += blockDim.x) xs[(int64_t)b * xs_pitch + m] = (float)(long long)s_sum[b];
+    for (int b = threadIdx.x; b < blocks; b += blockDim.x) xs[(int64_t)b * xs_pitch + m] = (float)((long long)s_hi[b] * 65536 + s_lo[b]);
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) { DBG_STAMP(12); }
 }
