@@ -15,7 +15,8 @@ DEV = "cuda:0"
     (8, -1, 300, 1056, 17, torch.bfloat16), (8, 128, 1000, 1280, 33, torch.float16), (8, 256, 129, 768, 70, torch.bfloat16),
     (4, 128, 4096, 2048, 29, torch.float16), (4, 128, 777, 1024, 64, torch.bfloat16), (4, -1, 520, 4096, 130, torch.bfloat16),
     (4, 256, 300, 1024, 513, torch.float16), (8, -1, 260, 272, 1100, torch.float32), (4, 128, 4096, 1024, 40, torch.float32),
-    (8, 512, 200, 1024, 9, torch.float32),
+    (8, 512, 200, 1024, 9, torch.float32), (8, 64, 300, 832, 40, torch.float32), (4, 64, 520, 1088, 9, torch.float32),
+  (4, 64, 300, 4096, 200, torch.float32),
 ])
 def test_zero_points_above_eight_tokens(wbits, bs, N, K, M, dtype):
   g = qc.gen(N + K + M)

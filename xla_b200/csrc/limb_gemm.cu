@@ -91,6 +91,7 @@ enum Mode : int {
   kPerChannel = 0,  // one accumulation per (tile, K range of the CTA)
   kBlock128 = 1,    // scale blocks of 128: two blocks per slot
   kBlockSlots = 2,  // scale blocks of spb whole slots
+  kBlock64 = 3,     // scale blocks of 64: four blocks per slot, a hand-over each
 };
 
 struct Params {
@@ -599,23 +600,25 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
     int slot = 0, buf = 0;
     uint32_t ph = 0, pacc = 0;
     uint32_t lo = lo0;
-    // the four MMAs of operand tile t of the current slot into accumulator d
-    auto issue_tile = [&](uint32_t d, int t, uint32_t accum) {
+    // the MMAs k0 <= k < k1 (of four) of operand tile t of the current slot into accumulator d
+    auto issue_part = [&](uint32_t d, int t, int k0, int k1, uint32_t accum) {
       const uint32_t a_lo = lo + t * (kATile >> 4), b_lo = lo + (C::kAInSlot >> 4) + t * (kBTile >> 4);
       if (!leader) return;
 #pragma unroll
       for (int k = 0; k < kTileK / UMMA_K; ++k) {
+        if (k < k0 || k >= k1) continue;
         const uint64_t bd = ((uint64_t)desc_hi << 32) | (uint64_t)(b_lo + k * (UMMA_K >> 4));
         if constexpr (C::kATmem) {
           // operand rows = TMEM lanes; one K=32 step = 8 columns = one expanded 16-byte chunk of nibbles
           const uint32_t a_tm = tmem_base + C::kATmemCol0 + slot * C::kATmemSlotCols + (4 * t + k) * 8;
-          ptx::mma_i8_ts(d, a_tm, bd, idesc, accum | (uint32_t)k);
+          ptx::mma_i8_ts(d, a_tm, bd, idesc, accum | (uint32_t)(k - k0));
         } else {
           const uint64_t ad = ((uint64_t)desc_hi << 32) | (uint64_t)(a_lo + k * (UMMA_K >> 4));
-          ptx::mma_i8_ss(d, ad, bd, idesc, accum | (uint32_t)k);
+          ptx::mma_i8_ss(d, ad, bd, idesc, accum | (uint32_t)(k - k0));
         }
       }
     };
+    auto issue_tile = [&](uint32_t d, int t, uint32_t accum) { issue_part(d, t, 0, kTileK / UMMA_K, accum); };
     auto wait_acc = [&]() {
       DBG_BEGIN();
       ptx::mbar_wait(&acc_empty[buf], pacc ^ 1, abort_flag, p.err_word, ptx::kErrWaitTmemEmpty);
@@ -648,7 +651,18 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
     };
     while (it.next(tile, u0, u1)) {
       const int s0 = u0 * p.spu, s1 = min(p.slots, u1 * p.spu);
-      if (p.mode == kBlock128) {
+      if (p.mode == kBlock64) {
+        for (int s = s0; s < s1; ++s) {
+#pragma unroll
+          for (int h = 0; h < 4; ++h) {
+            wait_acc();
+            if (h == 0) wait_slot();
+            issue_part(tmem_base + buf * NCOLS, h >> 1, 2 * (h & 1), 2 * (h & 1) + 2, 0);
+            if (h == 3) next_slot();
+            next_acc();
+          }
+        }
+      } else if (p.mode == kBlock128) {
         for (int s = s0; s < s1; ++s) {
           if (C::kPair) {
             wait_acc();
@@ -699,7 +713,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
     const int half = (C::kHalves == 2 && warp >= C::kXDrainWarp0) ? 1 : 0;
     const uint32_t col0 = (uint32_t)(half * NL * MTD);
     constexpr int kDT = 128 * C::kHalves;                     // drain threads
-    const bool small = p.mode == kBlock128 || (p.mode == kBlockSlots && p.spu == 1);
+    const bool small = p.mode == kBlock128 || p.mode == kBlock64 || (p.mode == kBlockSlots && p.spu == 1);
     asm volatile("griddepcontrol.wait;" ::: "memory");  // pw, the scratch and `out` belong to earlier kernels until here
     if (warp == kDrainWarp0) { DBG_STAMP(5); }
     const int quad = warp & 3;
@@ -824,10 +838,12 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
           sc2[1] = nx1;
         }
       } else {
-        int s = s0, b = p.mode == kBlockSlots ? s0 / p.spu : 0;
+        // hand-overs, and slots per hand-over in quarters (blocks of 64: one quarter)
+        const int per = p.mode == kBlockSlots ? 4 * p.spu : (p.mode == kBlock64 ? 1 : 4 * (s1 - s0));
+        int s = 4 * s0, b = p.mode == kBlockSlots ? s0 / p.spu : 4 * s0;
         float sc = p.mode == kPerChannel ? 1.f : fetch_scale(b);
-        while (s < s1) {
-          const int g_end = p.mode == kBlockSlots ? min(s1, s + p.spu) : s1;
+        while (s < 4 * s1) {
+          const int g_end = s + per;
           const float nx = p.mode == kPerChannel ? 1.f : fetch_scale(++b);
           wait_acc();
           DBG_BEGIN();
@@ -1073,7 +1089,7 @@ Scratch carve(void* base, int64_t M, int64_t K, int nl, int partial_tokens, int 
   off += align_up((size_t)M * 4, 256);
   s.xs = reinterpret_cast<float*>(b + off);
   s.xs_pitch = (int)M + 64;  // a token tile may reach beyond the batch
-  off += align_up((size_t)(K / kTileK + 1) * s.xs_pitch * 4, 256);
+  off += align_up((size_t)(K / 64 + 1) * s.xs_pitch * 4, 256);
   s.limbs = reinterpret_cast<int8_t*>(b + off);
   off += align_up((size_t)nl * M * K, 256);
   s.partial = reinterpret_cast<float*>(b + off);
@@ -1252,8 +1268,8 @@ bool limb_tc_shape_ok(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_
   if (x_dt != QMM_BF16 && x_dt != QMM_F16 && x_dt != QMM_F32) return false;
   if (M < 1 || N < 1 || K < 128) return false;
   if (wbits == 8 ? (K % 16 != 0) : (K % 32 != 0)) return false;  // TMA row pitches of the weights and the limbs
-  // scale blocks of 128 (two per slot) or of whole 256-value slots
-  if (block_size > 0 && ((block_size != kTileK && block_size % kSlotK != 0) || K % block_size != 0)) return false;
+  // scale blocks of 64 (four per slot), 128 (two) or of whole 256-value slots
+  if (block_size > 0 && ((block_size != 64 && block_size != kTileK && block_size % kSlotK != 0) || K % block_size != 0)) return false;
   // one int32 accumulation runs over a scale block (all of K per-channel): |limb * weight| <= 2^14 per term
   if ((block_size > 0 ? block_size : K) > (1 << 16)) return false;
   if (N > (1LL << 30) || K > (1LL << 24)) return false;
@@ -1272,7 +1288,7 @@ bool limb_tc_preferred(int wbits, int64_t M, int64_t N, int64_t K, int64_t block
   // back by its streaming rate once the weight is large enough, sooner the larger the batch (thresholds read off
   // the tuner's measurements over the reference's shape families); above 64 tokens it beats the conversion-based
   // tensor-core kernel on every shape measured.
-  (void)block_size;
+  if (block_size == 64) return false;  // a hand-over per block: only where the alternative is the any-shape kernel
   const int64_t mib = N * K * wbits / 8 >> 20;
   if (M > 64) return N * K >= (1 << 20);
   if (M > 32) return mib >= 24;
@@ -1304,7 +1320,7 @@ int launch_limb_impl(int wbits, const void* x, int x_dt, const void* w, const fl
   if (!limb_tc_supported(wbits, M, N, K, block_size, x, x_dt, w, zp != nullptr))
     return fail(QMM_ERR_UNSUPPORTED,
                 "split-activation tensor-core kernel: needs an sm_100 device, K >= 128 and a multiple of %d, "
-                "block_size 128 or a multiple of 256, 16-byte aligned x/w (M=%lld N=%lld K=%lld bs=%lld)",
+                "block_size 64, 128 or a multiple of 256, 16-byte aligned x/w (M=%lld N=%lld K=%lld bs=%lld)",
                 wbits == 8 ? 16 : 32, (long long)M, (long long)N, (long long)K, (long long)block_size);
   if (gate_up && zp) return fail(QMM_ERR_UNSUPPORTED, "fused gate/up epilogue: no zero points");
   if (gate_up && N % 16 != 0)
@@ -1387,7 +1403,7 @@ int launch_limb_impl(int wbits, const void* x, int x_dt, const void* w, const fl
   p.M = (int)M;
   p.ld = N;
   p.slots = (int)ceil_div(K, kSlotK);
-  p.mode = block_size <= 0 ? kPerChannel : (block_size == kTileK ? kBlock128 : kBlockSlots);
+  p.mode = block_size <= 0 ? kPerChannel : (block_size == kTileK ? kBlock128 : block_size == 64 ? kBlock64 : kBlockSlots);
   p.S = block_size > 0 ? (int)(K / block_size) : 1;
   p.spu = p.mode == kBlockSlots ? (int)(block_size / kSlotK) : 1;
   p.ut = (int)ceil_div(p.slots, p.spu);
