@@ -261,3 +261,18 @@ def test_auto_picks_it_and_reference_op_reaches_it():
   assert out.dtype == torch.float32
   assert qo.max_abs_rel(out, _exact(x, w, s, 0)) < TOL_F32
   assert _capi.lib().qmm_weight_only_workspace_size(16, 4096) > 0
+
+
+# weights long enough for two CTAs per SM to have a dozen slots each: block scales through the shared-memory ring, and the
+# 64-column instance of 17 to 32 tokens
+@pytest.mark.parametrize("M,bs", [(4, 128), (9, 64), (16, 128), (17, 0), (25, 128), (32, 256)])
+def test_long_int4_weights(M, bs):
+  g = qc.gen(700 + M)
+  N, K = 128 * 149 - 9, 6272 if bs != 256 else 6400
+  x = qc.activations(g, M, K)
+  w = qc.int4_weight(g, N, K)
+  s = qc.blockwise_scale(g, K // bs, N) if bs > 0 else qc.per_channel_scale(g, N)
+  out = _run(x, w, s, bs, 4, torch.bfloat16)
+  rows = torch.cat([torch.arange(300), torch.arange(N - 300, N)])
+  exact = _exact(x, w[rows], s[..., rows], bs)
+  assert qo.max_abs_rel(out[:, rows.to(DEV)], exact) < TOL_BF16

@@ -112,6 +112,7 @@ struct Params {
   int spu;     // slots per scheduling unit (= slots per scale block in kBlockSlots mode, else 1)
   int ut;      // units per tile
   int mode;
+  int scale_ring;  // block scales through the ring in shared memory (instances that have one)
   int S;       // scale blocks
   long long units;
   float* partial;   // [grid][MT][128] fp32
@@ -132,11 +133,11 @@ struct Params {
 template <int WBITS, int NCOLS, int NL = 3>
 struct Cfg {
   static constexpr uint32_t kBTile = NCOLS * 128;
-  // CTAs per SM.  With int4 weights and up to 48 limb columns a CTA takes at most half of an SM's shared memory, tensor memory and
+  // CTAs per SM.  With int4 weights and up to 64 limb columns a CTA takes at most half of an SM's shared memory, tensor memory and
   // registers, and two run side by side: whenever one pipeline waits (a hand-over between warps, the partial-tile
   // exchange at the end of a K range, its own start-up) the other's MMAs keep the tensor pipe and the weight stream
   // busy, and a kernel's first CTAs overlap the last ones of the kernel before it.
-  static constexpr int kOcc = (WBITS == 4 && NCOLS <= 48) ? 2 : 1;
+  static constexpr int kOcc = (WBITS == 4 && NCOLS <= 64) ? 2 : 1;
   static constexpr int kTmemCols = 512 / kOcc;
   static constexpr uint32_t kBudget = kOcc == 2 ? 110 * 1024 - 2048 : kSmemBudget;
   // int4 with up to 96 limb columns: the expanded weight operand lives in tensor memory (64 columns per slot, in the
@@ -152,7 +153,10 @@ struct Cfg {
   static constexpr int kSlots = kATmem ? kATmemSlots : (WBITS == 4 ? 2 : std::min<int>(6, kBudget / kSlot));
   // expanding warps: two groups of four that take alternate slots, or one group where two CTAs share the SM
   static constexpr int kGroups = WBITS == 4 ? (kOcc == 2 ? 1 : 2) : 0;
-  static constexpr int kRawFit = WBITS == 4 ? (int)((kBudget - kSlots * kSlot) / kRawBytes) : 0;
+  // block scales on their way to the drain warps, per drain thread: where the raw tiles leave room for them
+  static constexpr int kScaleRing = kOcc == 2 ? 8 : 0;
+  static constexpr uint32_t kScaleBytes = kScaleRing * 128 * 4;
+  static constexpr int kRawFit = WBITS == 4 ? (int)((kBudget - kScaleBytes - kSlots * kSlot) / kRawBytes) : 0;
   static constexpr int kRaw = WBITS == 4 ? std::min(10, kGroups == 2 ? (kRawFit & ~1) : kRawFit) : 0;
   static constexpr int kAccCols = kATmem ? kATmemCol0 : kTmemCols;
   static constexpr int kRegions = std::min(2 * kMaxAcc, kAccCols / NCOLS);   // accumulators that fit in TMEM
@@ -167,7 +171,7 @@ struct Cfg {
   static constexpr bool kPipeDrain = NCOLS >= 96 && !(WBITS == 4 && NCOLS == 128);
   static constexpr int kXDrainWarp0 = 8 + 4 * kGroups;
   static constexpr int kThreads = 256 + 128 * kGroups + 128 * (kHalves - 1);
-  static constexpr size_t kSmem = 1024 + (size_t)kRaw * kRawBytes + (size_t)kSlots * kSlot + 1024;
+  static constexpr size_t kSmem = 1024 + (size_t)kRaw * kRawBytes + (size_t)kSlots * kSlot + kScaleBytes + 1024;
   static_assert(kSlots >= 2 && (WBITS == 8 || kRaw >= 2), "ring depths");
   static_assert(kGroups != 2 || (kSlots % 2 == 0 && kRaw % 2 == 0), "a ring slot always belongs to the same group");
   static_assert(kRegions >= 2, "two accumulators, so that drain and MMA overlap");
@@ -216,6 +220,9 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
 }
 __device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ void cp_async4(uint32_t dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void st_release_gpu(uint32_t* p, uint32_t v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
@@ -477,7 +484,8 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* raw_base = smem;
   uint8_t* slot_base = raw_base + (size_t)kRaw * kRawBytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(slot_base + (size_t)kSlots * kSlot);
+  float* scale_base = reinterpret_cast<float*>(slot_base + (size_t)kSlots * kSlot);  // [kScaleRing][128]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(scale_base) + C::kScaleBytes);
   uint64_t* raw_full = bars;                       // [kRaw]    TMA bytes
   uint64_t* raw_empty = raw_full + (kRaw ? kRaw : 1);  // [kRaw]    4 expanding warps
   uint64_t* full = raw_empty + (kRaw ? kRaw : 1);      // [kSlots]  int8: both TMA producers; int4: 4 expanding warps + limb producer
@@ -803,7 +811,49 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
       // hand-over put a whole memory round trip into each: int4 block 128 [28672,8192] at 512 tokens 363 us, now 337.)
       const float* scale_n = p.scale + min(n, p.N - 1);
       auto fetch_scale = [&](int b) { return __ldg(scale_n + (int64_t)min(b, p.S - 1) * p.ld); };
-      if (p.mode == kBlock128) {
+      if (C::kScaleRing > 0 && p.scale_ring) {
+        // A hand-over here is shorter than a round trip to HBM, so the scales come eight blocks ahead, into a ring of the
+        // thread's own (one hand-over ahead, in registers: int4 block 128 [57344,8192] 53.9 us at 4 tokens and 82.0 at 16,
+        // now 46.4 and 74.3).
+        constexpr int R = C::kScaleRing > 0 ? C::kScaleRing : 1;
+        const int per_slot = p.mode == kBlock128 ? 2 : p.mode == kBlock64 ? 4 : 1;  // blocks
+        const int b0 = p.mode == kBlockSlots ? u0 : s0 * per_slot, b1 = p.mode == kBlockSlots ? u1 : s1 * per_slot;
+        float* ring = scale_base + rl;
+        const uint32_t ring_u32 = ptx::smem_u32(ring);
+        auto fetch = [&](int b) {
+          // (a last slot may hold fewer blocks than the others: their sums are zero, but the factor has to be a number)
+          if (b < b1) cp_async4(ring_u32 + (uint32_t)(b % R) * 512, scale_n + (int64_t)min(b, p.S - 1) * p.ld);
+          asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+#pragma unroll 1
+        for (int b = b0; b < b0 + R; ++b) fetch(b);
+        if (C::kPair && p.mode == kBlock128) {
+#pragma unroll 1
+          for (int b = b0; b < b1; b += 2) {
+            wait_acc();
+            asm volatile("cp.async.wait_group %0;" ::"n"(R - 2) : "memory");
+            const float sc0 = ring[(b % R) * 128], sc1 = ring[((b + 1) % R) * 128];
+            const uint32_t a = lane_addr + buf * (2 * NCOLS) + col0;
+            fold_region<DC, MTD, NL, true>(a, sc0, total, false, release);
+            fold_region<DC, MTD, NL, true>(a + NCOLS, sc1, total, true, release);
+            next_acc();
+            fetch(b + R);
+            fetch(b + R + 1);
+          }
+        } else {
+#pragma unroll 1
+          for (int b = b0; b < b1; ++b) {
+            wait_acc();
+            asm volatile("cp.async.wait_group %0;" ::"n"(R - 1) : "memory");
+            const float sc = ring[(b % R) * 128];
+            if (small) fold_region<DC, MTD, NL, true>(lane_addr + buf * NCOLS + col0, sc, total, true, release);
+            else fold_region<DC, MTD, NL, false>(lane_addr + buf * NCOLS + col0, sc, total, true, release);
+            next_acc();
+            fetch(b + R);
+          }
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");  // the ring is refilled from any place
+      } else if (p.mode == kBlock128) {
         float sc2[2] = {fetch_scale(2 * s0), fetch_scale(2 * s0 + 1)};
         for (int s = s0; s < s1; ++s) {
           const float nx0 = fetch_scale(2 * s + 2), nx1 = fetch_scale(2 * s + 3);
@@ -1052,11 +1102,14 @@ struct Plan {
 // limb_tc_set_limbs(3) keeps three limbs everywhere (process-wide).
 std::atomic<int> g_limb_policy{0};
 
+// Fewer than a dozen slots for each of two CTAs per SM
+bool few_slots(int64_t slots) { return slots < 24LL * sm_count(); }
+
 // Limbs per token.  In narrow tiles the MMA costs the same with three limbs as with two, so the exact form is kept
 // there.  Wider batches pay per limb column: when the output is a 16-bit type, two limbs (15 bits below the row's
 // largest value, error at most 2^-15 of it per activation, under the output's own rounding) carry 64 tokens per
 // 128-column tile instead of 42.  fp32 outputs always get three.
-Plan plan_for(int wbits, int64_t M, int out_dt, bool has_zp) {
+Plan plan_for(int wbits, int64_t M, int64_t N, int64_t K, bool per_channel, int out_dt, bool has_zp) {
   const bool two_ok = !has_zp && g_limb_policy.load(std::memory_order_relaxed) != 3 && (out_dt == QMM_BF16 || out_dt == QMM_F16);
   Plan pl;
   pl.nl = 3;
@@ -1064,7 +1117,13 @@ Plan plan_for(int wbits, int64_t M, int out_dt, bool has_zp) {
   if (M <= 5 && !has_zp) pl.ncols = 16;  // (zero points: fewer instances, shorter batches run elsewhere)
   else if (M <= 10 && !has_zp) pl.ncols = 32;
   else if (M <= 16) pl.ncols = 48;
-  else if (M <= 32 && !(wbits == 4 && two_ok)) pl.ncols = 96;
+  else if (M <= 32 && wbits == 4 && two_ok && (per_channel || !few_slots(ceil_div(N, BMW) * ceil_div(K, kSlotK)))) {
+    // 64 columns, two CTAs per SM: 29 tokens, int4 block 128 [57344,8192] 83 us against 99 of the 128-column instance,
+    // block 256 [28672,8192] 36 against 52; with few slots per CTA the hand-overs' latency shows (block 128 [14336,4096]
+    // 24 against 19)
+    pl.ncols = 64;
+    pl.nl = 2;
+  } else if (M <= 32 && !(wbits == 4 && two_ok)) pl.ncols = 96;
   else {
     // 128 columns: 42 tokens of three limbs or 64 of two; one tile is split over K, more run as items
     pl.ncols = 128;
@@ -1135,6 +1194,8 @@ int launch_ncols(int ncols, int nl, const CUtensorMap& map_w, const CUtensorMap&
     if (ncols == 96) return launch_cfg<WBITS, 96, 3, true>(map_w, map_x, p, grid, st);
     return launch_cfg<WBITS, 128, 3, true>(map_w, map_x, p, grid, st);
   }
+  if constexpr (WBITS == 4)
+    if (nl == 2 && ncols == 64) return launch_cfg<4, 64, 2>(map_w, map_x, p, grid, st);
   if (nl == 2) return launch_cfg<WBITS, 128, 2>(map_w, map_x, p, grid, st);
   switch (ncols) {
     case 16: return launch_cfg<WBITS, 16>(map_w, map_x, p, grid, st);
@@ -1178,9 +1239,11 @@ struct Split {
   int grid;
   long long cost;  // slots of streaming per SM, exchange included
 };
-Split split_one_tile(int wbits, const Plan& pl, long long tiles, long long slots, int spu) {
+Split split_one_tile(int wbits, const Plan& pl, long long tiles, long long slots, int spu, bool per_channel) {
   const long long ut = ceil_div(slots, spu), units = tiles * ut;
-  const int occ = (wbits == 4 && pl.ncols <= 48) ? 2 : 1;  // Cfg::kOcc
+  // CTAs per SM: Cfg::kOcc.  Per channel one where there are few slots: half of the exchanges, and the second place is the
+  // next kernel's ([14336,4096] at 16 tokens 14.3 us against 16.9).  With scale blocks two hide each other's hand-overs.
+  const int occ = (wbits == 4 && pl.ncols <= 64 && !(per_channel && few_slots(tiles * slots))) ? 2 : 1;
   const long long ctas_max = std::min<long long>((long long)occ * sm_count(), kLimbMaxCtas);
   const long long min_units = std::max<long long>(1, 2 / spu);
   Split sp;
@@ -1217,7 +1280,7 @@ int launch_main(int wbits, const void* w, int64_t rows, int64_t K, const Plan& p
   // to split every tile, and whole tiles alone leave the last round partly filled)
   if (pl.items || (ncols == 128 && p.tiles > sm_count())) {
     // the CTAs walk the (weight tile, token tile) items, whole items each: nothing is exchanged between them
-    const int occ = (wbits == 4 && ncols <= 48) ? 2 : 1;  // Cfg::kOcc
+    const int occ = (wbits == 4 && ncols <= 64) ? 2 : 1;  // Cfg::kOcc
     const long long items = (long long)p.tiles * p.ytiles, ctas = (long long)occ * sm_count();
     grid = (int)std::min<long long>(ctas, items);
     p.items1 = items;
@@ -1240,12 +1303,14 @@ int launch_main(int wbits, const void* w, int64_t rows, int64_t K, const Plan& p
       }
     }
   } else {
-    const Split sp = split_one_tile(wbits, pl, p.tiles, p.slots, p.spu);
+    const Split sp = split_one_tile(wbits, pl, p.tiles, p.slots, p.spu, p.mode == kPerChannel);
     grid = sp.grid;
     p.items1 = 0;
     p.units = (long long)p.tiles * p.ut;
     p.g2 = grid;
   }
+  // the ring costs a few dozen instructions per hand-over and pays from a dozen slots per CTA ([14336,4096], six: 3 % slower)
+  p.scale_ring = p.mode != kPerChannel && (long long)p.tiles * p.ytiles * p.slots >= 12LL * grid;
   CUtensorMap map_w;
   const int rc = encode_tmap_2d(&map_w, w, 1, false, (uint64_t)rows, (uint64_t)(K * wbits / 8), BMW, 128);
   if (rc != QMM_OK) return rc;
@@ -1325,7 +1390,7 @@ int launch_limb_impl(int wbits, const void* x, int x_dt, const void* w, const fl
   if (gate_up && zp) return fail(QMM_ERR_UNSUPPORTED, "fused gate/up epilogue: no zero points");
   if (gate_up && N % 16 != 0)
     return fail(QMM_ERR_BAD_SHAPE, "fused gate/up epilogue: the interleaved weight needs a multiple of 16 rows, got %lld", (long long)N);
-  const Plan pl = plan_for(wbits, M, out_dt, zp != nullptr);
+  const Plan pl = plan_for(wbits, M, N, K, block_size <= 0, out_dt, zp != nullptr);
   const int nl = pl.nl;
   const size_t need = carve(nullptr, std::min(M, max_rows(nl)), K, nl, pl.tile_tokens, kLimbMaxCtas).bytes;
   if (!workspace || workspace_bytes < need)
