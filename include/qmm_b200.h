@@ -147,7 +147,7 @@ QMM_API int qmm_w8a16_blockwise(const void* x, int x_dtype, const int8_t* w, con
  *   wbits 8: w int8 [N,K];  wbits 4: w uint8 [N,K/2], nibble order as qmm_w4a16_blockwise_packed.
  *   block_size <= 0: per-channel, scale/zp f32 [N];  block_size > 0: scale/zp f32 [K/block_size, N].
  *   workspace: qmm_weight_only_workspace_size(max M, K) bytes of device memory, 256-byte aligned, whose first
- *   1024 bytes are ZERO before the first call (the kernel leaves them zero); calls that share a workspace must be
+ *   2048 bytes are ZERO before the first call (the kernel leaves them zero); calls that share a workspace must be
  *   ordered on the GPU (same stream).  NULL / 0 is allowed and rules the I8TC variant out.  A workspace of
  *   qmm_weight_only_workspace_size_for(wbits, max M, N, K) bytes additionally lets long int4 batches (384 tokens
  *   and more per channel, 512 with scale blocks) expand the weights to int8 once per call (N*K bytes behind the
@@ -200,8 +200,8 @@ QMM_API int qmm_gate_up_decode(int wbits, const void* x, int x_dtype, const void
 /*
  * The same fused operation for any batch up to 1008 tokens on the split-activation kernel (QMM_VARIANT_I8TC), whose
  * drain warps apply silu(gate) * up before the one store: bf16 / f16 / f32 activations, K >= 128 and a multiple of
- * 16 (int8) or 32 (int4), block_size 0, 128 or a multiple of 256.  workspace: as for qmm_weight_only
- * (qmm_weight_only_workspace_size(M, K) bytes, 256-byte aligned, first 1024 bytes zero before the first use).
+ * 16 (int8) or 32 (int4), block_size 0, 64, 128 or a multiple of 256.  workspace: as for qmm_weight_only
+ * (qmm_weight_only_workspace_size(M, K) bytes, 256-byte aligned, first 2048 bytes zero before the first use).
  * Returns QMM_ERR_UNSUPPORTED outside that range.  No counterpart in the reference (see qmm_gate_up_decode).
  */
 QMM_API int qmm_gate_up(int wbits, const void* x, int x_dtype, const void* w, const float* scale, void* out, int out_dtype,
