@@ -202,11 +202,13 @@ static bool use_decode_i8(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs
 }
 
 // Where AUTO takes the tensor-memory kernel (16-bit activations).
-//   zero points    above eight tokens, everywhere: it applies them in the drain it runs anyway (int4 block 128
+//   zero points    above eight tokens: it applies them in the drain it runs anyway (int4 block 128
 //                  [37888,3584] at 29 tokens 42 us against 59 on the split-activation kernel, [14336,4096] at 512: 147
-//                  against 211).
-//   blocks of 64   above 32 tokens: the split-activation kernel has none (int4 [14336,4096] at 512 tokens 135 us against
-//                  199 on the shared-memory kernel).
+//                  against 211).  Not per channel with int8 weights, or with larger int4 weights up to the 42 tokens of one
+//                  tile of the other kernel, which hands over once per tile then (20 tokens on [14336,4096]: int8 17.7 us
+//                  against 23.0, int4 14.1 against 20.1; int4 [4096,4096] 12.8 against 11.8; 64 tokens 28 against 22).
+//   blocks of 64   above 32 tokens: the split-activation kernel hands over four times per slot there (int4 [14336,4096] at
+//                  512 tokens 135 us against 232).
 //   int4           above 64 tokens, when the (128-row, up to 192-token) items fill two thirds of the SMs: fewer leave it
 //                  to the split-activation kernel's narrower ones ([4096,4096] at 128 tokens 23 us against 19;
 //                  [14336,4096] at 96 tokens 27 against 35, [28672,8192] at 512 tokens 284 against 340).  Per channel up
@@ -217,6 +219,7 @@ static bool use_decode_i8(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs
 //                  a round or two of items each ([1536,14592] at 4178 tokens 189 us against 313).
 static bool use_tmem(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, int x_dt, int out_dt, bool has_zp) {
   if (!tmem_gemm_shape_ok(wbits, M, N, K, bs, x_dt)) return false;
+  if (has_zp && bs <= 0 && (wbits == 8 || (M <= 42 && N * K >= 1 << 25)) && limb_tc_shape_ok(wbits, M, N, K, bs, x_dt, true)) return false;
   if (has_zp) return M > 8;
   if (bs == 64) return M > 32;
   const int64_t items = ceil_div(N, 128) * ceil_div(M, 192);
