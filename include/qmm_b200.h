@@ -182,6 +182,16 @@ QMM_API int qmm_zero_point_in_kernel(int wbits, int64_t M, int64_t N, int64_t K,
 QMM_API int qmm_weight_only(int wbits, const void* x, int x_dtype, const void* w, const float* scale, const float* zp,
                     void* out, int out_dtype, int64_t M, int64_t N, int64_t K, int64_t block_size, int variant,
                     void* workspace, size_t workspace_bytes, void* stream);
+/*
+ * The same with scales and zero points of type scale_dtype (one type for both): what the buffers of a quantized 16-bit
+ * model hold, read as they are.  Results are those of the fp32 call with the same values.  QMM_ERR_UNSUPPORTED, before
+ * anything is launched, where the kernel that `variant` stands for at this shape reads fp32 only: the any-shape, GEMV
+ * and TCGEN05 kernels; MMA unless scale_dtype is x_dtype; blockwise scales with an odd N or not 4-byte aligned.  Callers
+ * then convert the scales and call qmm_weight_only.
+ */
+QMM_API int qmm_weight_only_typed(int wbits, const void* x, int x_dtype, const void* w, const void* scale, const void* zp,
+                    int scale_dtype, void* out, int out_dtype, int64_t M, int64_t N, int64_t K, int64_t block_size, int variant,
+                    void* workspace, size_t workspace_bytes, void* stream);
 
 /*
  * Fused gate + up projection of a gated MLP for decode batches (1 <= M <= 32, bf16/f16 activations):
@@ -246,6 +256,11 @@ QMM_API int qmm_w8a8_perchannel(const void* x, int x_dtype, const int8_t* w, con
                         const float* zp, void* out, int out_dtype, int64_t M, int64_t N,
                         int64_t K, int saturate, int variant, void* workspace,
                         size_t workspace_bytes, void* stream);
+/* The same with scales and zero points of type scale_dtype, as in qmm_weight_only_typed (QMM_ERR_UNSUPPORTED where only the
+ * any-shape kernel takes the shape). */
+QMM_API int qmm_w8a8_perchannel_typed(const void* x, int x_dtype, const int8_t* w, const void* w_scale, const void* zp,
+                        int scale_dtype, void* out, int out_dtype, int64_t M, int64_t N, int64_t K, int saturate, int variant,
+                        void* workspace, size_t workspace_bytes, void* stream);
 
 /*
  * qmm_w8a8_perchannel for callers that cannot hand over device memory of their own: plugins inside

@@ -1,0 +1,55 @@
+"""A module's scales and zero points are read on every call, in the type they are held in: 16-bit ones give the bits of the
+fp32 call with the same values in every kernel that a module reaches, and a write to the buffers shows in the next call
+however it was made.  (N odd or a buffer at an odd element: the calls that convert the scales first.)"""
+import pytest
+import torch
+
+import xla_b200
+from tests import qmm_cases as qc
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+# weight bits, block size, zero points, activation quantization, N, K, M, whether the buffers start at an odd element
+CASES = [
+    (8, -1, False, False, 261, 1056, 1, True), (8, -1, True, False, 512, 1024, 2, False), (4, 128, False, False, 1024, 4096, 1, False),
+    (4, 128, True, False, 1024, 4096, 3, False), (4, 64, True, False, 130, 320, 2, False), (8, 128, False, False, 4096, 512, 2, False),
+    (4, 128, False, False, 1024, 2048, 8, False), (8, -1, False, False, 512, 1024, 14, False), (8, 256, False, False, 514, 1024, 29, True),
+    (4, 128, True, False, 4096, 1024, 29, False), (4, -1, True, False, 777, 4096, 130, True), (4, 64, False, False, 300, 1024, 40, False),
+    (8, 128, False, False, 1000, 2048, 70, False), (8, -1, False, False, 1025, 2048, 300, True), (8, 256, True, False, 2048, 1024, 9, False),
+    (4, 256, False, False, 4096, 2048, 520, False), (8, -1, False, True, 514, 1024, 4, False), (8, -1, True, True, 300, 1024, 40, True),
+    (8, -1, True, True, 300, 512, 10, False), (4, 128, True, False, 301, 1024, 29, False), (8, 64, True, False, 300, 832, 9, True),
+]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("wbits,bs,zp,qact,N,K,M,odd", CASES)
+def test_module_follows_its_scales(dtype, wbits, bs, zp, qact, N, K, M, odd):
+  g = qc.gen(N + K + M)
+  x = qc.activations(g, M, K, dtype).to(DEV)
+  w = (qc.int4_weight if wbits == 4 else qc.int8_weight)(g, N, K)
+  native = xla_b200.pack_int4(w.to(DEV)) if wbits == 4 and K % 2 == 0 and not qact else w.to(DEV)
+
+  def held(t):
+    flat = torch.empty(t.numel() + 1, dtype=dtype, device=DEV)[1 if odd else 0:][:t.numel()]
+    return flat.copy_(t.flatten()).view(t.shape)
+
+  def draw():
+    s = qc.per_channel_scale(g, N) if bs == -1 else qc.blockwise_scale(g, K // bs, N)
+    return s.to(dtype), (torch.randint(-3, 4, s.shape, generator=g) * s).to(dtype) if zp else None
+
+  def in_f32(s, z):
+    return torch.ops.xla_b200.quantized_matmul_packed(x, native, s.float().to(DEV), None if z is None else z.float().to(DEV),
+                                                      block_size=bs, int4_weight=wbits == 4, weight_is_packed=native.dtype == torch.uint8,
+                                                      quantize_activation=qact, out_dtype=dtype)
+
+  mod = xla_b200.XlaQuantizedLinear(K, N, is_symmetric=not zp, block_size=bs, int4_weight=wbits == 4, quantize_activation=qact)
+  s, z = draw()
+  mod.load_quantized_weight((w if bs == -1 else qc.to_sbn(w, bs)).to(DEV), held(s), None if z is None else held(z))
+  assert torch.equal(mod(x), in_f32(s, z))
+  s, z = draw()
+  mod.weight_scaler.data.copy_(s)  # leaves the version counter as it is, as a replayed graph does
+  if z is not None:
+    mod.zero_point.data.copy_(z)
+  y = mod(x)
+  assert y.dtype == dtype and torch.equal(y, in_f32(s, z))

@@ -35,6 +35,7 @@ SIGNATURES = {
     "qmm_weight_only_variant_for": (ctypes.c_char_p, [_i, _i64, _i64, _i64, _i64, _i]),
     "qmm_zero_point_in_kernel": (_i, [_i, _i64, _i64, _i64, _i64, _i]),
     "qmm_weight_only": (_i, [_i, _p, _i, _p, _p, _p, _p, _i, _i64, _i64, _i64, _i64, _i, _p, _sz, _p]),
+    "qmm_weight_only_typed": (_i, [_i, _p, _i, _p, _p, _p, _i, _p, _i, _i64, _i64, _i64, _i64, _i, _p, _sz, _p]),
     "qmm_host_pipeline_create": (_i, [_sz, _sz, _i, ctypes.POINTER(ctypes.c_void_p)]),
     "qmm_host_weight_only": (_i, [_p, _i, _p, _i, _p, _p, _p, _p, _i, _i64, _i64, _i64, _i64, _i]),
     "qmm_host_pipeline_wait_stream": (_i, [_p, _p]),
@@ -55,6 +56,7 @@ SIGNATURES = {
     "qmm_quantize_activation": (_i, [_p, _i, _p, _p, _p, _i64, _i64, _i, _p]),
     "qmm_w8a8_gemm": (_i, [_p, _p, _p, _p, _p, _p, _p, _p, _i, _i64, _i64, _i64, _i, _p]),
     "qmm_w8a8_perchannel": (_i, [_p, _i, _p, _p, _p, _p, _i, _i64, _i64, _i64, _i, _i, _p, _sz, _p]),
+    "qmm_w8a8_perchannel_typed": (_i, [_p, _i, _p, _p, _p, _i, _p, _i, _i64, _i64, _i64, _i, _i, _p, _sz, _p]),
     "qmm_w8a8_perchannel_static": (_i, [_p, _i, _p, _p, _p, _p, _i, _i64, _i64, _i64, _i, _i, _p]),
     "qmm_workspace_size": (_sz, [_i, _i64, _i64, _i64]),
     "qmm_pack_int4_nk": (_i, [_p, _p, _i64, _i64, _p]),

@@ -130,7 +130,7 @@ int encode_tmap_2d(CUtensorMap* map, const void* base, int elem_bytes, bool is_f
 }
 
 // ---- argument checks ----------------------------------------------------------------------
-static int check_common(const void* x, int x_dt, const void* w, const float* scale, void* out,
+static int check_common(const void* x, int x_dt, const void* w, const void* scale, void* out,
                         int out_dt, int64_t M, int64_t N, int64_t K) {
   if (M < 0 || N < 0 || K < 0) return fail(QMM_ERR_BAD_SHAPE, "negative dimension (M=%lld N=%lld K=%lld)",
                                            (long long)M, (long long)N, (long long)K);
@@ -245,7 +245,7 @@ int qmm_w8a16_perchannel(const void* x, int x_dtype, const int8_t* w, const floa
     case QMM_VARIANT_MMA:
       log_choice("w8a16_perchannel", "mma", M, N, K);
       if (zp) return fail(QMM_ERR_UNSUPPORTED, "the register-dequant decode kernel does not take a zero point");
-      return launch_decode_mma(8, x, x_dtype, w, scale, out, out_dtype, M, N, K, 0, st);
+      return launch_decode_mma(8, x, x_dtype, w, scale, QMM_F32, out, out_dtype, M, N, K, 0, st);
     case QMM_VARIANT_TCGEN05:
       log_choice("w8a16_perchannel", "tcgen05", M, N, K);
       if (zp) return fail(QMM_ERR_UNSUPPORTED, "tcgen05 weight-only kernel does not take a zero point");
@@ -295,7 +295,7 @@ int qmm_w4a16_blockwise_packed(const void* x, int x_dtype, const uint8_t* wp, co
     case QMM_VARIANT_MMA:
       log_choice("w4a16_blockwise_packed", "mma", M, N, K);
       if (zp) return fail(QMM_ERR_UNSUPPORTED, "the register-dequant decode kernel does not take a zero point");
-      return launch_decode_mma(4, x, x_dtype, wp, scale, out, out_dtype, M, N, K, block_size, st);
+      return launch_decode_mma(4, x, x_dtype, wp, scale, QMM_F32, out, out_dtype, M, N, K, block_size, st);
     case QMM_VARIANT_TCGEN05:
       log_choice("w4a16_blockwise_packed", "tcgen05", M, N, K);
       if (zp) return fail(QMM_ERR_UNSUPPORTED, "tcgen05 weight-only kernel does not take a zero point");
@@ -325,7 +325,7 @@ int qmm_w8a16_blockwise(const void* x, int x_dtype, const int8_t* w, const float
     case QMM_VARIANT_MMA:
       log_choice("w8a16_blockwise", "mma", M, N, K);
       if (zp) return fail(QMM_ERR_UNSUPPORTED, "the register-dequant decode kernel does not take a zero point");
-      return launch_decode_mma(8, x, x_dtype, w, scale, out, out_dtype, M, N, K, block_size, st);
+      return launch_decode_mma(8, x, x_dtype, w, scale, QMM_F32, out, out_dtype, M, N, K, block_size, st);
     case QMM_VARIANT_TCGEN05:
       log_choice("w8a16_blockwise", "tcgen05", M, N, K);
       if (zp) return fail(QMM_ERR_UNSUPPORTED, "tcgen05 weight-only kernel does not take a zero point");
@@ -401,7 +401,16 @@ size_t qmm_weight_only_workspace_size_for(int wbits, int64_t max_M, int64_t N, i
 int qmm_weight_only(int wbits, const void* x, int x_dtype, const void* w, const float* scale, const float* zp, void* out,
                     int out_dtype, int64_t M, int64_t N, int64_t K, int64_t block_size, int variant, void* workspace,
                     size_t workspace_bytes, void* stream) {
+  return qmm_weight_only_typed(wbits, x, x_dtype, w, scale, zp, QMM_F32, out, out_dtype, M, N, K, block_size, variant, workspace,
+                               workspace_bytes, stream);
+}
+
+int qmm_weight_only_typed(int wbits, const void* x, int x_dtype, const void* w, const void* scale, const void* zp, int scale_dtype,
+                          void* out, int out_dtype, int64_t M, int64_t N, int64_t K, int64_t block_size, int variant,
+                          void* workspace, size_t workspace_bytes, void* stream) {
   if (wbits != 4 && wbits != 8) return fail(QMM_ERR_BAD_SHAPE, "weight_only: wbits must be 4 or 8, got %d", wbits);
+  if (!valid_float_dtype(scale_dtype)) return fail(QMM_ERR_UNSUPPORTED, "weight_only: bad scale dtype %d", scale_dtype);
+  const Scales sc{scale, zp, scale_dtype};
   if (block_size < 0) block_size = 0;
   if (variant == QMM_VARIANT_AUTO || variant == QMM_VARIANT_I8TC) {
     int rc = check_common(x, x_dtype, w, scale, out, out_dtype, M, N, K);
@@ -434,7 +443,7 @@ int qmm_weight_only(int wbits, const void* x, int x_dtype, const void* w, const 
     }
     if (use) {
       log_choice("weight_only", "i8tc", M, N, K);
-      return launch_limb_tc(wbits, x, x_dtype, w, scale, zp, out, out_dtype, M, N, K, block_size, 0, workspace, workspace_bytes,
+      return launch_limb_tc(wbits, x, x_dtype, w, sc, out, out_dtype, M, N, K, block_size, 0, workspace, workspace_bytes,
                             as_stream(stream));
     }
   }
@@ -442,25 +451,36 @@ int qmm_weight_only(int wbits, const void* x, int x_dtype, const void* w, const 
     int rc = check_common(x, x_dtype, w, scale, out, out_dtype, M, N, K);
     if (rc != QMM_OK || M * N == 0) return rc;
     log_choice("weight_only", "i8mma", M, N, K);
-    return launch_decode_i8(wbits, x, x_dtype, w, scale, zp, out, out_dtype, M, N, K, block_size, 0, as_stream(stream));
+    return launch_decode_i8(wbits, x, x_dtype, w, sc, out, out_dtype, M, N, K, block_size, 0, as_stream(stream));
   }
   if (variant == QMM_VARIANT_TMEM) {
     int rc = check_common(x, x_dtype, w, scale, out, out_dtype, M, N, K);
     if (rc != QMM_OK || M * N == 0) return rc;
     log_choice("weight_only", "tmem", M, N, K);
-    return launch_tmem_gemm(wbits, x, x_dtype, w, scale, zp, out, out_dtype, M, N, K, block_size, 0, workspace, workspace_bytes,
+    return launch_tmem_gemm(wbits, x, x_dtype, w, sc, out, out_dtype, M, N, K, block_size, 0, workspace, workspace_bytes,
                             as_stream(stream));
   }
+  if (scale_dtype != QMM_F32) {
+    // the entry points below read fp32 scales; the one kernel behind them that also takes others is called here
+    int rc = check_common(x, x_dtype, w, scale, out, out_dtype, M, N, K);
+    if (rc != QMM_OK || M * N == 0) return rc;
+    if (block_size > 0 && K % block_size != 0) return fail(QMM_ERR_BAD_SHAPE, "weight_only: block_size must divide K");
+    if (variant == QMM_VARIANT_AUTO) variant = pick_weight_only(wbits, M, N, K, block_size, x, x_dtype, w, zp != nullptr);
+    if (variant != QMM_VARIANT_MMA || zp) return fail(QMM_ERR_UNSUPPORTED, "weight_only: variant %d reads fp32 scales only", variant);
+    log_choice("weight_only", "mma", M, N, K);
+    return launch_decode_mma(wbits, x, x_dtype, w, scale, scale_dtype, out, out_dtype, M, N, K, block_size, as_stream(stream));
+  }
+  const float *s32 = static_cast<const float*>(scale), *z32 = static_cast<const float*>(zp);
   if (wbits == 8) {
     if (block_size > 0)
-      return qmm_w8a16_blockwise(x, x_dtype, static_cast<const int8_t*>(w), scale, zp, out, out_dtype, M, N, K, block_size, variant,
+      return qmm_w8a16_blockwise(x, x_dtype, static_cast<const int8_t*>(w), s32, z32, out, out_dtype, M, N, K, block_size, variant,
                                  stream);
-    return qmm_w8a16_perchannel(x, x_dtype, static_cast<const int8_t*>(w), scale, zp, out, out_dtype, M, N, K, variant, stream);
+    return qmm_w8a16_perchannel(x, x_dtype, static_cast<const int8_t*>(w), s32, z32, out, out_dtype, M, N, K, variant, stream);
   }
   if (block_size > 0)
-    return qmm_w4a16_blockwise_packed(x, x_dtype, static_cast<const uint8_t*>(w), scale, zp, out, out_dtype, M, N, K, block_size,
+    return qmm_w4a16_blockwise_packed(x, x_dtype, static_cast<const uint8_t*>(w), s32, z32, out, out_dtype, M, N, K, block_size,
                                       variant, stream);
-  return qmm_w4a16_perchannel_packed(x, x_dtype, static_cast<const uint8_t*>(w), scale, zp, out, out_dtype, M, N, K, variant, stream);
+  return qmm_w4a16_perchannel_packed(x, x_dtype, static_cast<const uint8_t*>(w), s32, z32, out, out_dtype, M, N, K, variant, stream);
 }
 
 int qmm_gate_up_decode(int wbits, const void* x, int x_dtype, const void* w, const float* scale, void* out,
@@ -480,10 +500,10 @@ int qmm_gate_up_decode(int wbits, const void* x, int x_dtype, const void* w, con
                 (long long)block_size);
   if (use_decode_i8(wbits, M, N2, K, block_size, x, x_dtype, w, false)) {
     log_choice("gate_up_decode", "i8mma", M, N2, K);
-    return launch_decode_i8(wbits, x, x_dtype, w, scale, nullptr, out, out_dtype, M, N2, K, block_size, 1, st);
+    return launch_decode_i8(wbits, x, x_dtype, w, Scales{scale, nullptr, QMM_F32}, out, out_dtype, M, N2, K, block_size, 1, st);
   }
   log_choice("gate_up_decode", "mma", M, N2, K);
-  return launch_decode_mma(wbits, x, x_dtype, w, scale, out, out_dtype, M, N2, K, block_size, st, 1);
+  return launch_decode_mma(wbits, x, x_dtype, w, scale, QMM_F32, out, out_dtype, M, N2, K, block_size, st, 1);
 }
 
 int qmm_gate_up(int wbits, const void* x, int x_dtype, const void* w, const float* scale, void* out, int out_dtype, int64_t M,
@@ -496,13 +516,14 @@ int qmm_gate_up(int wbits, const void* x, int x_dtype, const void* w, const floa
   if (block_size < 0 || (block_size > 0 && K % block_size != 0))
     return fail(QMM_ERR_BAD_SHAPE, "gate_up: K (%lld) must be a multiple of block_size (%lld)", (long long)K, (long long)block_size);
   if (M == 0 || N2 == 0) return QMM_OK;
+  const Scales sc{scale, nullptr, QMM_F32};
   if (use_tmem(wbits, M, N2, K, block_size, x_dtype, out_dtype, false) && aligned(x, 16) && aligned(w, 16) && workspace &&
       workspace_bytes >= tmem_gemm_workspace_bytes(M, K)) {
     log_choice("gate_up", "tmem", M, N2, K);
-    return launch_tmem_gemm(wbits, x, x_dtype, w, scale, nullptr, out, out_dtype, M, N2, K, block_size, 1, workspace, workspace_bytes, st);
+    return launch_tmem_gemm(wbits, x, x_dtype, w, sc, out, out_dtype, M, N2, K, block_size, 1, workspace, workspace_bytes, st);
   }
   log_choice("gate_up", "i8tc", M, N2, K);
-  return launch_limb_tc(wbits, x, x_dtype, w, scale, nullptr, out, out_dtype, M, N2, K, block_size, 1, workspace, workspace_bytes, st);
+  return launch_limb_tc(wbits, x, x_dtype, w, sc, out, out_dtype, M, N2, K, block_size, 1, workspace, workspace_bytes, st);
 }
 
 int qmm_w4a16_perchannel_packed(const void* x, int x_dtype, const uint8_t* wp, const float* scale,
@@ -524,7 +545,7 @@ int qmm_w4a16_perchannel_packed(const void* x, int x_dtype, const uint8_t* wp, c
     case QMM_VARIANT_MMA:
       log_choice("w4a16_perchannel_packed", "mma", M, N, K);
       if (zp) return fail(QMM_ERR_UNSUPPORTED, "the register-dequant decode kernel does not take a zero point");
-      return launch_decode_mma(4, x, x_dtype, wp, scale, out, out_dtype, M, N, K, 0, st);
+      return launch_decode_mma(4, x, x_dtype, wp, scale, QMM_F32, out, out_dtype, M, N, K, 0, st);
     case QMM_VARIANT_TCGEN05:
       log_choice("w4a16_perchannel_packed", "tcgen05", M, N, K);
       if (zp) return fail(QMM_ERR_UNSUPPORTED, "tcgen05 weight-only kernel does not take a zero point");
@@ -543,6 +564,24 @@ int qmm_quantize_activation(const void* x, int x_dtype, int8_t* xq, float* x_sca
   return launch_quantize_activation(x, x_dtype, xq, x_scale, xq_rowsum, M, K, saturate, as_stream(stream));
 }
 
+static int w8a8_gemm(const int8_t* xq, const int8_t* w, const Scales& sc, const float* x_scale, const int32_t* xq_rowsum,
+                     int32_t* acc_out, void* out, int out_dtype, int64_t M, int64_t N, int64_t K, int variant, cudaStream_t st) {
+  if (variant == QMM_VARIANT_AUTO)
+    variant = w8a8_tc_supported(M, N, K, xq, w) ? QMM_VARIANT_TCGEN05 : QMM_VARIANT_GENERIC;
+  switch (variant) {
+    case QMM_VARIANT_GENERIC:
+      log_choice("w8a8_gemm", "generic", M, N, K);
+      if (sc.dt != QMM_F32) return fail(QMM_ERR_UNSUPPORTED, "w8a8_gemm: the any-shape kernel reads fp32 scales only");
+      return launch_generic_w8a8(xq, w, static_cast<const float*>(sc.scale), static_cast<const float*>(sc.zp), x_scale, xq_rowsum, acc_out,
+                                 out, out_dtype, M, N, K, st);
+    case QMM_VARIANT_TCGEN05:
+      log_choice("w8a8_gemm", "tcgen05", M, N, K);
+      return launch_w8a8_tc(xq, w, sc, x_scale, xq_rowsum, acc_out, out, out_dtype, M, N, K, st);
+    default:
+      return fail(QMM_ERR_UNSUPPORTED, "w8a8_gemm: variant %d is not available", variant);
+  }
+}
+
 int qmm_w8a8_gemm(const int8_t* xq, const int8_t* w, const float* w_scale, const float* zp,
                   const float* x_scale, const int32_t* xq_rowsum, int32_t* acc_out, void* out,
                   int out_dtype, int64_t M, int64_t N, int64_t K, int variant, void* stream) {
@@ -553,19 +592,7 @@ int qmm_w8a8_gemm(const int8_t* xq, const int8_t* w, const float* w_scale, const
   if (out && (!w_scale || !x_scale)) return fail(QMM_ERR_NULL, "w_scale or x_scale is NULL");
   if (zp && !xq_rowsum) return fail(QMM_ERR_NULL, "a zero point needs xq_rowsum");
   if (K > 0 && (!xq || !w)) return fail(QMM_ERR_NULL, "xq or w is NULL");
-  cudaStream_t st = as_stream(stream);
-  if (variant == QMM_VARIANT_AUTO)
-    variant = w8a8_tc_supported(M, N, K, xq, w) ? QMM_VARIANT_TCGEN05 : QMM_VARIANT_GENERIC;
-  switch (variant) {
-    case QMM_VARIANT_GENERIC:
-      log_choice("w8a8_gemm", "generic", M, N, K);
-      return launch_generic_w8a8(xq, w, w_scale, zp, x_scale, xq_rowsum, acc_out, out, out_dtype, M, N, K, st);
-    case QMM_VARIANT_TCGEN05:
-      log_choice("w8a8_gemm", "tcgen05", M, N, K);
-      return launch_w8a8_tc(xq, w, w_scale, zp, x_scale, xq_rowsum, acc_out, out, out_dtype, M, N, K, st);
-    default:
-      return fail(QMM_ERR_UNSUPPORTED, "w8a8_gemm: variant %d is not available", variant);
-  }
+  return w8a8_gemm(xq, w, Scales{w_scale, zp, QMM_F32}, x_scale, xq_rowsum, acc_out, out, out_dtype, M, N, K, variant, as_stream(stream));
 }
 
 // Up to here the decode kernel beats the quantizer and the tcgen05 GEMM (4096 x 4096: 6.4 to 19.5 us at 1 to 12 tokens
@@ -588,6 +615,15 @@ int qmm_w8a8_perchannel(const void* x, int x_dtype, const int8_t* w, const float
                         const float* zp, void* out, int out_dtype, int64_t M, int64_t N,
                         int64_t K, int saturate, int variant, void* workspace,
                         size_t workspace_bytes, void* stream) {
+  return qmm_w8a8_perchannel_typed(x, x_dtype, w, w_scale, zp, QMM_F32, out, out_dtype, M, N, K, saturate, variant, workspace,
+                                   workspace_bytes, stream);
+}
+
+int qmm_w8a8_perchannel_typed(const void* x, int x_dtype, const int8_t* w, const void* w_scale, const void* zp, int scale_dtype,
+                              void* out, int out_dtype, int64_t M, int64_t N, int64_t K, int saturate, int variant,
+                              void* workspace, size_t workspace_bytes, void* stream) {
+  if (!valid_float_dtype(scale_dtype)) return fail(QMM_ERR_UNSUPPORTED, "w8a8_perchannel: bad scale dtype %d", scale_dtype);
+  const Scales sc{w_scale, zp, scale_dtype};
   int rc = check_common(x, x_dtype, w, w_scale, out, out_dtype, M, N, K);
   if (rc != QMM_OK || M * N == 0) return rc;
   // decode batches: one kernel quantizes and multiplies, no scratch
@@ -596,7 +632,7 @@ int qmm_w8a8_perchannel(const void* x, int x_dtype, const int8_t* w, const float
   if (variant == QMM_VARIANT_AUTO && M > 8 && M < 16 && K <= 512 && N * K <= (1 << 20)) variant = QMM_VARIANT_GENERIC;
   if (variant == QMM_VARIANT_AUTO && M <= kW8A8DecodeTokens && decode_w8a8_supported(M, N, K, x, x_dtype, w, zp != nullptr)) {
     log_choice("w8a8_perchannel", "i8mma", M, N, K);
-    return launch_decode_w8a8(x, x_dtype, w, w_scale, zp, out, out_dtype, M, N, K, saturate, as_stream(stream));
+    return launch_decode_w8a8(x, x_dtype, w, sc, out, out_dtype, M, N, K, saturate, as_stream(stream));
   }
   const size_t need = qmm_workspace_size(QMM_OP_W8A8_PERCHANNEL, M, N, K);
   if (!workspace || workspace_bytes < need)
@@ -606,10 +642,12 @@ int qmm_w8a8_perchannel(const void* x, int x_dtype, const int8_t* w, const float
   int8_t* xq = reinterpret_cast<int8_t*>(base);
   float* xs = reinterpret_cast<float*>(base + align_up((size_t)M * (size_t)K, 256));
   int32_t* rowsum = reinterpret_cast<int32_t*>(reinterpret_cast<uint8_t*>(xs) + align_up((size_t)M * 4, 256));
+  // (refused before the quantizer is launched)
+  if (scale_dtype != QMM_F32 && (variant == QMM_VARIANT_GENERIC || !w8a8_tc_supported(M, N, K, xq, w)))
+    return fail(QMM_ERR_UNSUPPORTED, "w8a8_perchannel: the any-shape kernel reads fp32 scales only");
   rc = qmm_quantize_activation(x, x_dtype, xq, xs, zp ? rowsum : nullptr, M, K, saturate, stream);
   if (rc != QMM_OK) return rc;
-  return qmm_w8a8_gemm(xq, w, w_scale, zp, xs, zp ? rowsum : nullptr, nullptr, out, out_dtype, M, N, K,
-                       variant, stream);
+  return w8a8_gemm(xq, w, sc, xs, zp ? rowsum : nullptr, nullptr, out, out_dtype, M, N, K, variant, as_stream(stream));
 }
 
 int qmm_pack_int4_nk(const int8_t* w, uint8_t* wp, int64_t N, int64_t K, void* stream) {

@@ -84,6 +84,38 @@ __device__ __forceinline__ void store_from_f32(void* p, int64_t i, int dt, float
     reinterpret_cast<__half*>(p)[i] = __float2half_rn(v);
 }
 
+// ---- weight scales and zero points ---------------------------------------------------------
+// In fp32 or in a 16-bit type (the buffers of a quantized 16-bit model), both in the same one.
+struct Scales {
+  const void* scale;
+  const void* zp;  // or null
+  int dt;
+};
+
+inline const void* elements_from(const void* p, int64_t n, int dt) {
+  return p ? static_cast<const uint8_t*>(p) + n * (int64_t)dtype_size(dt) : nullptr;
+}
+
+// Kernels that stream block scales copy them in 32-bit words: one fp32 value, or the pair of 16-bit values that holds the
+// wanted one.  For that every row of a 16-bit [S,N] tensor has to start on a word.  (Per channel they are read one by one.)
+inline bool scale_words_ok(const Scales& s, int64_t N, int64_t block_size) {
+  return s.dt == QMM_F32 || block_size <= 0 || (N % 2 == 0 && aligned(s.scale, 4) && aligned(s.zp, 4));
+}
+
+// Byte offset of the word that holds element n
+__device__ __forceinline__ int64_t scale_word_offset(int64_t n, int dt) { return dt == QMM_F32 ? n * 4 : (n & ~1ll) * 2; }
+
+// A word's value for the element n that it was fetched for
+struct ScaleWord {
+  uint32_t shift, mask;
+  bool half;
+  __device__ ScaleWord(int dt, int n) : shift(dt == QMM_F32 || (n & 1) ? 0u : 16u), mask(dt == QMM_F32 ? ~0u : 0xffff0000u), half(dt == QMM_F16) {}
+  __device__ float operator()(uint32_t w) const {
+    w = (w << shift) & mask;
+    return half ? __half2float(__ushort_as_half((unsigned short)(w >> 16))) : __uint_as_float(w);
+  }
+};
+
 // 128-bit streaming load that does not pollute L1 (weights are read exactly once).
 __device__ __forceinline__ uint4 ld_stream_u4(const void* p) {
   uint4 r;

@@ -47,11 +47,11 @@ constexpr size_t kSmemMax = 227 * 1024 - 512;  // static shared memory beside it
 struct Args {
   const void* x;
   const uint8_t* w;
-  const float* scale;  // [N] or [S,N]
-  const float* zp;     // like scale, or null
+  const void* scale;   // [N] or [S,N], of type s_dt
+  const void* zp;      // like scale, or null
   void* out;
   int64_t N, K;
-  int x_dt, out_dt, M;
+  int x_dt, out_dt, s_dt, M;
   int steps;           // 64-byte steps per weight row (the last one may be partly outside the row)
   int tiles_lo, tiles_extra;  // tiles per CTA, and how many CTAs take one more
   int fold_steps;      // steps per scale block (0: per channel)
@@ -215,6 +215,8 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 2 : 1) decode_i8_kernel(const
   const int64_t pitch = p.K * WBITS / 8;
   const int cols = NL * p.M;
   const int n_last = (int)p.N - 1;
+  const int64_t sc_pitch = p.N * (p.s_dt == QMM_F32 ? 4 : 2);  // bytes from one scale block to the next
+  const ScaleWord word(p.s_dt, g);                             // (rows g and g + 8 of a tile; tiles start at even rows)
 
   if ((int)threadIdx.x < nt_cta) {
     int wv = 0;
@@ -228,13 +230,14 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 2 : 1) decode_i8_kernel(const
   const int piece_first = ls;
   uint32_t ldst = ring;
   const uint8_t *lp0, *lp1;
-  const float* lsc = nullptr;  // this lane's row of the scales (lanes 0..15) or zero points (lanes 16..31)
+  const uint8_t* lsc = nullptr;  // this lane's row of the scales (lanes 0..15) or zero points (lanes 16..31)
   auto set_tile = [&]() {
     // rows beyond N repeat the last one; they are not stored
     const int n0 = min(ltile * kRows + g, n_last), n1 = min(ltile * kRows + g + 8, n_last);
     lp0 = p.w + n0 * pitch + (HALF ? 8 : 16) * t;
     lp1 = p.w + n1 * pitch + (HALF ? 8 : 16) * t;
-    if (BLOCKED) lsc = (ZP && lane >= 16 ? p.zp : p.scale) + min(ltile * kRows + (lane & 15), n_last);
+    if (BLOCKED)
+      lsc = static_cast<const uint8_t*>(ZP && lane >= 16 ? p.zp : p.scale) + scale_word_offset(min(ltile * kRows + (lane & 15), n_last), p.s_dt);
   };
   set_tile();
   lp0 += (int64_t)ls * 64;
@@ -258,11 +261,11 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 2 : 1) decode_i8_kernel(const
       if constexpr (BLOCKED) {
         if (ZP || lane < 16) {
           if constexpr (HALF) {
-            cp_async_small<4>(ldst + 1024 + lane * 4, lsc + (int64_t)(2 * ls) * p.N);
-            if (2 * ls + 1 < p.S) cp_async_small<4>(ldst + 1152 + lane * 4, lsc + (int64_t)(2 * ls + 1) * p.N);
+            cp_async_small<4>(ldst + 1024 + lane * 4, lsc + (2 * ls) * sc_pitch);
+            if (2 * ls + 1 < p.S) cp_async_small<4>(ldst + 1152 + lane * 4, lsc + (2 * ls + 1) * sc_pitch);
           } else {
             const int b = p.fold_shift >= 0 ? ls >> p.fold_shift : ls / p.fold_steps;
-            cp_async_small<4>(ldst + 1024 + lane * 4, lsc + (int64_t)b * p.N);
+            cp_async_small<4>(ldst + 1024 + lane * 4, lsc + b * sc_pitch);
           }
         }
       }
@@ -346,9 +349,9 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 2 : 1) decode_i8_kernel(const
 
   // scale block b ends here: total += scale * sums, and (once per block: by the warp that runs its last step) the
   // zero-point term
-  auto fold = [&](const float* sc, int b, bool zp_too) {
+  auto fold = [&](const uint32_t* sc, int b, bool zp_too) {
     if constexpr (BLOCKED) {
-      const float s0 = sc[g], s1 = sc[g + 8];
+      const float s0 = word(sc[g]), s1 = word(sc[g + 8]);
 #pragma unroll
       for (int i = 0; i < NT; ++i) {
         total[i][0] = fmaf(s0, __int2float_rn(sum_of(i, 0)), total[i][0]);
@@ -360,7 +363,7 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 2 : 1) decode_i8_kernel(const
       if constexpr (ZP) {
         if (zp_too) {
           constexpr float kW = WBITS == 4 ? 16.f : 1.f;  // the weight sums carry this factor
-          const float z0 = -kW * sc[16 + g], z1 = -kW * sc[24 + g];
+          const float z0 = -kW * word(sc[16 + g]), z1 = -kW * word(sc[24 + g]);
 #pragma unroll
           for (int i = 0; i < NT; ++i) {
             const int c = 8 * i + 2 * t;
@@ -384,7 +387,7 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 2 : 1) decode_i8_kernel(const
     issue();  // into the slot of the step before this one, which every lane has read
     const uint8_t* slot = cring + cslot;
     cslot = cslot + kSlot == D * kSlot ? 0 : cslot + kSlot;
-    const float* sc = reinterpret_cast<const float*>(slot + 1024);
+    const uint32_t* sc = reinterpret_cast<const uint32_t*>(slot + 1024);
     const uint4 a = *reinterpret_cast<const uint4*>(slot + lane * 16), b = *reinterpret_cast<const uint4*>(slot + 512 + lane * 16);
     if constexpr (WBITS == 8) {
 #pragma unroll
@@ -447,15 +450,16 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 2 : 1) decode_i8_kernel(const
       }
     }
     if constexpr (NL == 1) {
-      return w8a8_dequant(ai, __ldg(p.scale + n), ZP ? p.zp + n : nullptr, ZP ? s_xs[m] : 0, s_pw[m]);
+      const float z = ZP ? load_as_f32(p.zp, n, p.s_dt) : 0.f;
+      return w8a8_dequant(ai, load_as_f32(p.scale, n, p.s_dt), ZP ? &z : nullptr, ZP ? s_xs[m] : 0, s_pw[m]);
     } else {
       float v = fmaf(65536.f, a[2], fmaf(256.f, a[1], a[0]));
       if constexpr (!BLOCKED) {
-        v *= __ldg(p.scale + n);
+        v *= load_as_f32(p.scale, n, p.s_dt);
         if constexpr (ZP) {
           constexpr float kW = WBITS == 4 ? 16.f : 1.f;
           const float xsum = fmaf(65536.f, (float)s_xs[3 * m + 2], fmaf(256.f, (float)s_xs[3 * m + 1], (float)s_xs[3 * m]));
-          v = fmaf(-kW * __ldg(p.zp + n), xsum, v);
+          v = fmaf(-kW * load_as_f32(p.zp, n, p.s_dt), xsum, v);
         }
       }
       return v * s_pw[m];
@@ -587,13 +591,14 @@ bool shape_ok(int wbits, int nl, int xbytes, int64_t M, int64_t N, int64_t K, in
   return layout_for(wbits, nl, xbytes, M, N, K, block_size > 0 ? K / block_size : 1, block_size > 0, half_blocks(wbits, block_size), zp).bytes <= kSmemMax;
 }
 
-Args make_args(int wbits, const void* x, int x_dt, const void* w, const float* scale, const float* zp, void* out, int out_dt,
-               int64_t M, int64_t N, int64_t K, int64_t block_size, const Layout& l) {
+Args make_args(int wbits, const void* x, int x_dt, const void* w, const Scales& sc, void* out, int out_dt, int64_t M,
+               int64_t N, int64_t K, int64_t block_size, const Layout& l) {
   Args a = {};
   a.x = x;
   a.w = reinterpret_cast<const uint8_t*>(w);
-  a.scale = scale;
-  a.zp = zp;
+  a.scale = sc.scale;
+  a.zp = sc.zp;
+  a.s_dt = sc.dt;
   a.out = out;
   a.N = N;
   a.K = K;
@@ -627,16 +632,17 @@ bool decode_i8_supported(int wbits, int64_t M, int64_t N, int64_t K, int64_t blo
   return aligned(x, 16) && aligned(w, 16);
 }
 
-int launch_decode_i8(int wbits, const void* x, int x_dt, const void* w, const float* scale, const float* zp, void* out, int out_dt,
-                     int64_t M, int64_t N, int64_t K, int64_t block_size, int gate_up, cudaStream_t st) {
+int launch_decode_i8(int wbits, const void* x, int x_dt, const void* w, const Scales& sc, void* out, int out_dt, int64_t M, int64_t N,
+                     int64_t K, int64_t block_size, int gate_up, cudaStream_t st) {
+  const bool zp = sc.zp != nullptr;
   if (gate_up && N % 16 != 0)
     return fail(QMM_ERR_BAD_SHAPE, "fused gate/up epilogue: the interleaved weight needs a multiple of 16 rows, got %lld", (long long)N);
-  if (!decode_i8_supported(wbits, M, N, K, block_size, x, x_dt, w, zp != nullptr))
+  if (!decode_i8_supported(wbits, M, N, K, block_size, x, x_dt, w, zp) || !scale_words_ok(sc, N, block_size))
     return fail(QMM_ERR_UNSUPPORTED, "integer decode kernel: M=%lld N=%lld K=%lld bs=%lld not supported", (long long)M, (long long)N,
                 (long long)K, (long long)block_size);
   const bool half = half_blocks(wbits, block_size);
-  const Layout l = layout_for(wbits, 3, 2, M, N, K, block_size > 0 ? K / block_size : 1, block_size > 0, half, zp != nullptr);
-  Args a = make_args(wbits, x, x_dt, w, scale, zp, out, out_dt, M, N, K, block_size, l);
+  const Layout l = layout_for(wbits, 3, 2, M, N, K, block_size > 0 ? K / block_size : 1, block_size > 0, half, zp);
+  Args a = make_args(wbits, x, x_dt, w, sc, out, out_dt, M, N, K, block_size, l);
   a.gate_up = gate_up;
   const int nt = tiles_n((int)(3 * M));
   const bool blocked = block_size > 0;
@@ -650,12 +656,13 @@ bool decode_w8a8_supported(int64_t M, int64_t N, int64_t K, const void* x, int x
   return aligned(x, 16) && aligned(w, 16);
 }
 
-int launch_decode_w8a8(const void* x, int x_dt, const int8_t* w, const float* w_scale, const float* zp, void* out, int out_dt,
-                       int64_t M, int64_t N, int64_t K, int saturate, cudaStream_t st) {
-  if (!decode_w8a8_supported(M, N, K, x, x_dt, w, zp != nullptr))
+int launch_decode_w8a8(const void* x, int x_dt, const int8_t* w, const Scales& sc, void* out, int out_dt, int64_t M, int64_t N,
+                       int64_t K, int saturate, cudaStream_t st) {
+  const bool zp = sc.zp != nullptr;
+  if (!decode_w8a8_supported(M, N, K, x, x_dt, w, zp))
     return fail(QMM_ERR_UNSUPPORTED, "W8A8 decode kernel: M=%lld N=%lld K=%lld not supported", (long long)M, (long long)N, (long long)K);
-  const Layout l = layout_for(8, 1, (int)dtype_size(x_dt), M, N, K, 1, false, false, zp != nullptr);
-  Args a = make_args(8, x, x_dt, w, w_scale, zp, out, out_dt, M, N, K, 0, l);
+  const Layout l = layout_for(8, 1, (int)dtype_size(x_dt), M, N, K, 1, false, false, zp);
+  Args a = make_args(8, x, x_dt, w, sc, out, out_dt, M, N, K, 0, l);
   a.saturate = saturate;
   const int nt = tiles_n((int)M);
   return zp ? launch_nt<8, 1, false, true, false>(nt, a, l, st) : launch_nt<8, 1, false, false, false>(nt, a, l, st);

@@ -164,9 +164,9 @@ __device__ __forceinline__ float ar_ld_peer(const float* p) {
 // step and reuses its activation registers for all of them); WARPS = warps splitting K.
 // One "fold" = the end of a scale block (blockwise) or of a single step (per-channel): the partial tile,
 // minus bias * sum(x), is added into the totals.
-template <int WBITS, typename XT, int NT, int RG, int WARPS, bool AR = false>
+template <int WBITS, typename XT, typename ST, int NT, int RG, int WARPS, bool AR = false>
 __global__ void __launch_bounds__(WARPS * 32)
-    decode_mma_kernel(const XT* __restrict__ x, const uint8_t* __restrict__ w, const float* __restrict__ scale,
+    decode_mma_kernel(const XT* __restrict__ x, const uint8_t* __restrict__ w, const ST* __restrict__ scale,
                       void* __restrict__ out, int out_dt, int M, int64_t N, int64_t K, int steps_per_block,
                       int spb_shift, int blockwise, int gate_up, const ArParams ar, uint32_t* err_word) {
   // ar.wait_cycles bounds the wait for the peers' tiles (AR only)
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(WARPS * 32)
   const int steps = (int)(K / VPS);
   // lane rows: group r -> rows n0 + 16r + g and n0 + 16r + g + 8 (clamped: tail rows are computed, not stored)
   const uint8_t* wrow[2 * RG];
-  const float* srow[2 * RG];
+  const ST* srow[2 * RG];
 #pragma unroll
   for (int r = 0; r < 2 * RG; ++r) {
     int64_t n = n0 + 16 * (r >> 1) + g + 8 * (r & 1);
@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(WARPS * 32)
       fold = sn >= steps || bn != b;
       if (fold) {
 #pragma unroll
-        for (int r = 0; r < 2 * RG; ++r) sc[r] = __ldg(srow[r] + (int64_t)b * N);
+        for (int r = 0; r < 2 * RG; ++r) sc[r] = to_f32(__ldg(srow[r] + (int64_t)b * N));
       }
     }
     if (!kPrefetchX) load_x(s, xr);
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(WARPS * 32)
         float v = 0.f;
 #pragma unroll
         for (int wi = 0; wi < WARPS; ++wi) v += s_part[wi][row][tok];
-        if (!blockwise) v *= __ldg(scale + n);
+        if (!blockwise) v *= to_f32(__ldg(scale + n));
         const size_t o = region + (size_t)tok * N + n;
 #pragma unroll
         for (int r = 0; r < kArMaxRanks; ++r)
@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(WARPS * 32)
       float v = 0.f;
 #pragma unroll
       for (int wi = 0; wi < WARPS; ++wi) v += s_part[wi][row][tok];
-      if (!blockwise) v *= __ldg(scale + n);
+      if (!blockwise) v *= to_f32(__ldg(scale + n));
       if (!gate_up) {
         store_from_f32(out, (int64_t)tok * N + n, out_dt, v);
       } else if ((row & 8) == 0) {
@@ -459,7 +459,7 @@ __global__ void __launch_bounds__(WARPS * 32)
         float u = 0.f;
 #pragma unroll
         for (int wi = 0; wi < WARPS; ++wi) u += s_part[wi][row + 8][tok];
-        if (!blockwise) u *= __ldg(scale + n + 8);
+        if (!blockwise) u *= to_f32(__ldg(scale + n + 8));
         store_from_f32(out, (int64_t)tok * (N >> 1) + gate_up_column(n), out_dt, silu_mul(v, u));
       }
     }
@@ -502,14 +502,15 @@ __device__ __forceinline__ void mma_16816_nv_first(float* c, const uint32_t* a, 
   }
 }
 
+template <typename ST>
 struct StagedStep {  // one K step of a warp in flight: 16 bytes of two weight rows and their block scales
   uint4 w[2];
-  float sc[2];
+  ST sc[2];
 };
 
-template <int WBITS, typename XT, int NT, bool FOLD_EVERY>
+template <int WBITS, typename XT, typename ST, int NT, bool FOLD_EVERY>
 __global__ void __launch_bounds__(kStagedWarps * 32, 1)
-    decode_mma_staged_kernel(const XT* __restrict__ x, const uint8_t* __restrict__ w, const float* __restrict__ scale,
+    decode_mma_staged_kernel(const XT* __restrict__ x, const uint8_t* __restrict__ w, const ST* __restrict__ scale,
                              void* __restrict__ out, int out_dt, int M, int N, int K, int steps_per_block,
                              int spb_shift, int blockwise, int tiles, int TR, int WK, int rounds, int gate_up) {
   constexpr int VPS = 512 / WBITS;            // weight values per row per step
@@ -576,7 +577,7 @@ __global__ void __launch_bounds__(kStagedWarps * 32, 1)
     const int tile = blockIdx.x + (round * TR + ts) * gridDim.x;
     const bool active = ts < TR && tile < tiles;
     const uint8_t* wrow[2];
-    const float* srow[2];
+    const ST* srow[2];
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       int n = (active ? tile : 0) * 16 + g + 8 * r;
@@ -600,14 +601,14 @@ __global__ void __launch_bounds__(kStagedWarps * 32, 1)
     const uint8_t* wp0 = wrow[0] + wk * 64;
     const uint8_t* wp1 = wrow[1] + wk * 64;
     const int64_t wstride = (int64_t)WK * 64;
-    const float *sp0 = srow[0], *sp1 = srow[1];
+    const ST *sp0 = srow[0], *sp1 = srow[1];
     int64_t sstride = 0;
     if constexpr (FOLD_EVERY && kLateFetch) {
       sp0 += (int64_t)(wk >> spb_shift) * N;
       sp1 += (int64_t)(wk >> spb_shift) * N;
       sstride = (int64_t)(WK >> spb_shift) * N;
     }
-    auto fetch = [&](int s, StagedStep& d) {
+    auto fetch = [&](int s, StagedStep<ST>& d) {
       if constexpr (FOLD_EVERY && kLateFetch) {
         d.w[0] = ld_stream_u4(wp0);
         d.w[1] = ld_stream_u4(wp1);
@@ -630,11 +631,11 @@ __global__ void __launch_bounds__(kStagedWarps * 32, 1)
         }
       }
     };
-    StagedStep qa, qb;
+    StagedStep<ST> qa, qb;
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
       qa.w[r] = qb.w[r] = make_uint4(0, 0, 0, 0);
-      qa.sc[r] = qb.sc[r] = 1.f;
+      qa.sc[r] = qb.sc[r] = from_f32<ST>(1.f);
     }
     if (active && wk < steps) {
       fetch(wk, qa);
@@ -657,9 +658,9 @@ __global__ void __launch_bounds__(kStagedWarps * 32, 1)
       for (int j = 0; j < 4; ++j) total[i][j] = part[i][j] = 0.f;
 
     // one K step: convert q's weights, multiply with the chunk's activations, fold, refill q two steps ahead
-    auto do_step = [&](int s, int c, StagedStep& q) {
+    auto do_step = [&](int s, int c, StagedStep<ST>& q) {
       const uint4 w0 = q.w[0], w1 = q.w[1];
-      const float sc0 = q.sc[0], sc1 = q.sc[1];
+      const float sc0 = to_f32(q.sc[0]), sc1 = to_f32(q.sc[1]);
       if constexpr (!kLateFetch) fetch(s + 2 * WK, q);
       const int ls = s - c * kChunkSteps;
       const unsigned char* xs = smem + ((uint32_t)(c & 1) * STAGE_BYTES + (uint32_t)ls * (UPS * 16));
@@ -770,7 +771,7 @@ __global__ void __launch_bounds__(kStagedWarps * 32, 1)
         if (s < s_end) {  // odd count in this chunk: run one step and swap the slots
           do_step(s, c, qa);
           s += WK;
-          const StagedStep tmp = qa;
+          const StagedStep<ST> tmp = qa;
           qa = qb;
           qb = tmp;
         }
@@ -801,13 +802,13 @@ __global__ void __launch_bounds__(kStagedWarps * 32, 1)
       if (otile < tiles && n < N && tok < M) {
         float v = 0.f;
         for (int j = 0; j < WK; ++j) v += red[((slot * WK + j) * ROWS_X + tok) * kRedPitch + row];
-        if (!blockwise) v *= __ldg(scale + n);
+        if (!blockwise) v *= to_f32(__ldg(scale + n));
         if (!gate_up) {
           store_from_f32(out, (int64_t)tok * N + n, out_dt, v);
         } else if ((row & 8) == 0) {
           float u = 0.f;
           for (int j = 0; j < WK; ++j) u += red[((slot * WK + j) * ROWS_X + tok) * kRedPitch + row + 8];
-          if (!blockwise) u *= __ldg(scale + n + 8);
+          if (!blockwise) u *= to_f32(__ldg(scale + n + 8));
           store_from_f32(out, (int64_t)tok * (N >> 1) + gate_up_column(n), out_dt, silu_mul(v, u));
         }
       }
@@ -833,8 +834,8 @@ cudaError_t launch_pdl(Kernel kern, unsigned grid, unsigned block, size_t smem_b
   return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
-template <int WBITS, typename XT, int NT>
-cudaError_t launch_staged(const XT* xp, const uint8_t* wp, const float* scale, void* out, int out_dt, int64_t M,
+template <int WBITS, typename XT, typename ST, int NT>
+cudaError_t launch_staged(const XT* xp, const uint8_t* wp, const ST* scale, void* out, int out_dt, int64_t M,
                           int64_t N, int64_t K, int spb, int shift, int bw, int gate_up, cudaStream_t st) {
   constexpr int VPS = 512 / WBITS;
   constexpr int PITCH = kChunkSteps * (VPS * 2 / 16) * 16 + 16;
@@ -847,7 +848,7 @@ cudaError_t launch_staged(const XT* xp, const uint8_t* wp, const float* scale, v
   const int wk = std::min(kStagedWarps / tr, 8);   // warps sharing the K steps of one tile
   const int rounds = (int)ceil_div(per_cta, tr);
   const bool fold_every = bw && wk % spb == 0;
-  auto kern = fold_every ? decode_mma_staged_kernel<WBITS, XT, NT, true> : decode_mma_staged_kernel<WBITS, XT, NT, false>;
+  auto kern = fold_every ? decode_mma_staged_kernel<WBITS, XT, ST, NT, true> : decode_mma_staged_kernel<WBITS, XT, ST, NT, false>;
   static bool configured[64][2] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -860,8 +861,8 @@ cudaError_t launch_staged(const XT* xp, const uint8_t* wp, const float* scale, v
                     shift, bw, tiles, tr, wk, rounds, gate_up);
 }
 
-template <int WBITS, typename XT>
-int launch_nt(const void* x, const void* w, const float* scale, void* out, int out_dt, int64_t M, int64_t N,
+template <int WBITS, typename XT, typename ST>
+int launch_nt(const void* x, const void* w, const ST* scale, void* out, int out_dt, int64_t M, int64_t N,
               int64_t K, int64_t block_size, int gate_up, cudaStream_t st, const ArParams* ar = nullptr) {
   constexpr int VPS = 512 / WBITS;
   const int spb = block_size > 0 ? (int)(block_size / VPS) : 1;
@@ -874,7 +875,7 @@ int launch_nt(const void* x, const void* w, const float* scale, void* out, int o
   const XT* xp = reinterpret_cast<const XT*>(x);
   const uint8_t* wp = reinterpret_cast<const uint8_t*>(w);
 #define QMM_DECODE_LAUNCH(NT, RG, WARPS)                                                                        \
-  launch_pdl(decode_mma_kernel<WBITS, XT, NT, RG, WARPS>, (unsigned)ceil_div(N, 16 * RG), WARPS * 32, 0, st, xp, wp, \
+  launch_pdl(decode_mma_kernel<WBITS, XT, ST, NT, RG, WARPS>, (unsigned)ceil_div(N, 16 * RG), WARPS * 32, 0, st, xp, wp, \
              scale, out, out_dt, (int)M, N, K, spb, shift, bw, gate_up, ArParams{}, (uint32_t*)nullptr)
   // one token tile: many small CTAs, activations through L1 (64 KB for 8 tokens of 4096);
   // two or four tiles: one CTA per SM with the activations staged in shared memory
@@ -894,13 +895,17 @@ int launch_nt(const void* x, const void* w, const float* scale, void* out, int o
   cudaError_t err;
   if (ar) {
     if (M > 8 || gate_up) return fail(QMM_ERR_UNSUPPORTED, "fused row-parallel exchange: M <= 8 only (got %lld)", (long long)M);
-    ArParams a = *ar;
-    a.tiles = (uint32_t)tiles;
-    // always four warps per tile here: a CTA that waits for its peers' tiles holds its SM slot, and with 16-warp
-    // CTAs only one is resident per SM, so nothing else would run under the wait (measured: 86 vs 81 us on the
-    // two-GPU MLP)
-    err = launch_pdl(decode_mma_kernel<WBITS, XT, 1, 1, 4, true>, (unsigned)tiles, 128, 0, st, xp, wp, scale, out, out_dt,
-                     (int)M, N, K, spb, shift, bw, 0, a, device_error_word());
+    if constexpr (!std::is_same<ST, float>::value) {
+      return fail(QMM_ERR_UNSUPPORTED, "fused row-parallel exchange: fp32 scales only");
+    } else {
+      ArParams a = *ar;
+      a.tiles = (uint32_t)tiles;
+      // always four warps per tile here: a CTA that waits for its peers' tiles holds its SM slot, and with 16-warp
+      // CTAs only one is resident per SM, so nothing else would run under the wait (measured: 86 vs 81 us on the
+      // two-GPU MLP)
+      err = launch_pdl(decode_mma_kernel<WBITS, XT, float, 1, 1, 4, true>, (unsigned)tiles, 128, 0, st, xp, wp, scale, out, out_dt,
+                       (int)M, N, K, spb, shift, bw, 0, a, device_error_word());
+    }
   } else if (M <= 8) {
     if (warps >= 16)
       err = QMM_DECODE_LAUNCH(1, 1, 16);
@@ -910,9 +915,9 @@ int launch_nt(const void* x, const void* w, const float* scale, void* out, int o
       err = QMM_DECODE_LAUNCH(1, 1, 4);
   }
   else if (M <= 16)
-    err = launch_staged<WBITS, XT, 2>(xp, wp, scale, out, out_dt, M, N, K, spb, shift, bw, gate_up, st);
+    err = launch_staged<WBITS, XT, ST, 2>(xp, wp, scale, out, out_dt, M, N, K, spb, shift, bw, gate_up, st);
   else
-    err = launch_staged<WBITS, XT, 4>(xp, wp, scale, out, out_dt, M, N, K, spb, shift, bw, gate_up, st);
+    err = launch_staged<WBITS, XT, ST, 4>(xp, wp, scale, out, out_dt, M, N, K, spb, shift, bw, gate_up, st);
   if (err != cudaSuccess) {
     cudaGetLastError();
     return fail(QMM_ERR_LAUNCH, "decode_mma_kernel launch: %s", cudaGetErrorString(err));
@@ -962,7 +967,20 @@ bool decode_mma_supported(int wbits, int64_t M, int64_t N, int64_t K, int64_t bl
   return true;
 }
 
-int launch_decode_mma(int wbits, const void* x, int x_dt, const void* w, const float* scale, void* out, int out_dt,
+namespace {
+
+// The scales are fp32 or of the activations' type (a model's buffers share one type).
+template <int WBITS, typename XT>
+int launch_st(const void* x, const void* w, const void* scale, int scale_dt, void* out, int out_dt, int64_t M, int64_t N, int64_t K,
+              int64_t block_size, int gate_up, cudaStream_t st) {
+  if (scale_dt == QMM_F32)
+    return launch_nt<WBITS, XT>(x, w, reinterpret_cast<const float*>(scale), out, out_dt, M, N, K, block_size, gate_up, st);
+  return launch_nt<WBITS, XT>(x, w, reinterpret_cast<const XT*>(scale), out, out_dt, M, N, K, block_size, gate_up, st);
+}
+
+}  // namespace
+
+int launch_decode_mma(int wbits, const void* x, int x_dt, const void* w, const void* scale, int scale_dt, void* out, int out_dt,
                       int64_t M, int64_t N, int64_t K, int64_t block_size, cudaStream_t st, int gate_up) {
   if (gate_up && N % 16 != 0)
     return fail(QMM_ERR_BAD_SHAPE, "fused gate/up epilogue: the interleaved weight needs a multiple of 16 rows, got %lld",
@@ -972,12 +990,14 @@ int launch_decode_mma(int wbits, const void* x, int x_dt, const void* w, const f
                 "decode kernel: needs bf16/f16 activations, 1<=M<=32, K a multiple of %d, block_size a multiple of %d, "
                 "16-byte aligned x/w, no zero point (M=%lld N=%lld K=%lld bs=%lld)",
                 512 / wbits, 512 / wbits, (long long)M, (long long)N, (long long)K, (long long)block_size);
+  if (scale_dt != QMM_F32 && scale_dt != x_dt)
+    return fail(QMM_ERR_UNSUPPORTED, "decode kernel: scales are fp32 or of the activations' type");
   if (wbits == 4) {
-    if (x_dt == QMM_BF16) return launch_nt<4, __nv_bfloat16>(x, w, scale, out, out_dt, M, N, K, block_size, gate_up, st);
-    return launch_nt<4, __half>(x, w, scale, out, out_dt, M, N, K, block_size, gate_up, st);
+    if (x_dt == QMM_BF16) return launch_st<4, __nv_bfloat16>(x, w, scale, scale_dt, out, out_dt, M, N, K, block_size, gate_up, st);
+    return launch_st<4, __half>(x, w, scale, scale_dt, out, out_dt, M, N, K, block_size, gate_up, st);
   }
-  if (x_dt == QMM_BF16) return launch_nt<8, __nv_bfloat16>(x, w, scale, out, out_dt, M, N, K, block_size, gate_up, st);
-  return launch_nt<8, __half>(x, w, scale, out, out_dt, M, N, K, block_size, gate_up, st);
+  if (x_dt == QMM_BF16) return launch_st<8, __nv_bfloat16>(x, w, scale, scale_dt, out, out_dt, M, N, K, block_size, gate_up, st);
+  return launch_st<8, __half>(x, w, scale, scale_dt, out, out_dt, M, N, K, block_size, gate_up, st);
 }
 
 }  // namespace qmm

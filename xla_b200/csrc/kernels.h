@@ -6,6 +6,8 @@
 
 namespace qmm {
 
+struct Scales;  // common.cuh
+
 // fp32 dequant of one W8A8 accumulator in the reference's operation order
 // (torch_xla/experimental/xla_quantized_matmul.py:159, 172-182): every product is rounded
 // separately, so the result matches the reference's fp32 output bit for bit.
@@ -45,7 +47,8 @@ bool decode_mma_supported(int wbits, int64_t M, int64_t N, int64_t K, int64_t bl
                           const void* w, bool has_zp);
 // gate_up != 0: the weight rows are interleaved gate/up groups of eight and the kernel writes
 // silu(gate) * up as [M, N/2].
-int launch_decode_mma(int wbits, const void* x, int x_dt, const void* w, const float* scale, void* out, int out_dt,
+// scale: fp32, or the activations' type.
+int launch_decode_mma(int wbits, const void* x, int x_dt, const void* w, const void* scale, int scale_dt, void* out, int out_dt,
                       int64_t M, int64_t N, int64_t K, int64_t block_size, cudaStream_t st, int gate_up = 0);
 
 // The same kernel for the K-sharded (row-parallel) linear with the sum over ranks fused into its epilogue:
@@ -60,11 +63,11 @@ int launch_decode_mma_allreduce(int wbits, const void* x, int x_dt, const void* 
 // limbs of all tokens have to fit shared memory.  W8A8: M <= 32, activations of any type quantized in the kernel.
 bool decode_i8_supported(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_size, const void* x, int x_dt, const void* w,
                          bool has_zp);
-int launch_decode_i8(int wbits, const void* x, int x_dt, const void* w, const float* scale, const float* zp, void* out, int out_dt,
-                     int64_t M, int64_t N, int64_t K, int64_t block_size, int gate_up, cudaStream_t st);
+int launch_decode_i8(int wbits, const void* x, int x_dt, const void* w, const Scales& sc, void* out, int out_dt, int64_t M, int64_t N,
+                     int64_t K, int64_t block_size, int gate_up, cudaStream_t st);
 bool decode_w8a8_supported(int64_t M, int64_t N, int64_t K, const void* x, int x_dt, const void* w, bool has_zp);
-int launch_decode_w8a8(const void* x, int x_dt, const int8_t* w, const float* w_scale, const float* zp, void* out, int out_dt,
-                       int64_t M, int64_t N, int64_t K, int saturate, cudaStream_t st);
+int launch_decode_w8a8(const void* x, int x_dt, const int8_t* w, const Scales& sc, void* out, int out_dt, int64_t M, int64_t N,
+                       int64_t K, int saturate, cudaStream_t st);
 
 // ---- limb_gemm.cu (tcgen05 kind::i8 on unconverted weights; activations split into int8 limbs) ----------
 // Weight-only linear (bf16/f16/f32 activations): stream-K over all SMs, needs
@@ -80,9 +83,8 @@ bool limb_tc_supported(int wbits, int64_t M, int64_t N, int64_t K, int64_t block
                        const void* w, bool has_zp);
 // AUTO's shape rule: true where this kernel is the fastest measured choice.
 bool limb_tc_preferred(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_size);
-int launch_limb_tc(int wbits, const void* x, int x_dt, const void* w, const float* scale, const float* zp, void* out, int out_dt, int64_t M,
-                   int64_t N, int64_t K, int64_t block_size, int gate_up, void* workspace, size_t workspace_bytes,
-                   cudaStream_t st);
+int launch_limb_tc(int wbits, const void* x, int x_dt, const void* w, const Scales& sc, void* out, int out_dt, int64_t M, int64_t N,
+                   int64_t K, int64_t block_size, int gate_up, void* workspace, size_t workspace_bytes, cudaStream_t st);
 
 // ---- tmem_gemm.cu (tcgen05 kind::f16, weights converted into tensor memory) -------------------------------------------
 // Weight-only linear for batches of bf16/f16 activations, zero points allowed; scratch as limb_gemm.cu's (its first 2 KB
@@ -90,9 +92,8 @@ int launch_limb_tc(int wbits, const void* x, int x_dt, const void* w, const floa
 size_t tmem_gemm_workspace_bytes(int64_t max_M, int64_t K);
 bool tmem_gemm_shape_ok(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_size, int x_dt);
 bool tmem_gemm_supported(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_size, const void* x, int x_dt, const void* w);
-int launch_tmem_gemm(int wbits, const void* x, int x_dt, const void* w, const float* scale, const float* zp, void* out, int out_dt,
-                     int64_t M, int64_t N, int64_t K, int64_t block_size, int gate_up, void* workspace, size_t workspace_bytes,
-                     cudaStream_t st);
+int launch_tmem_gemm(int wbits, const void* x, int x_dt, const void* w, const Scales& sc, void* out, int out_dt, int64_t M, int64_t N,
+                     int64_t K, int64_t block_size, int gate_up, void* workspace, size_t workspace_bytes, cudaStream_t st);
 
 // ---- peer_reduce.cu -----------------------------------------------------------------------
 // One-shot all-reduce of fp32 partial results that every rank keeps in peer-mapped memory.
@@ -112,9 +113,8 @@ int launch_unpack_int4_nk(const uint8_t* wp, int8_t* w, int64_t N, int64_t K, cu
 
 // ---- w8a8_gemm.cu (tcgen05 kind::i8) ------------------------------------------------------
 bool w8a8_tc_supported(int64_t M, int64_t N, int64_t K, const void* xq, const void* w);
-int launch_w8a8_tc(const int8_t* xq, const int8_t* w, const float* w_scale, const float* zp,
-                   const float* x_scale, const int32_t* rowsum, int32_t* acc_out, void* out,
-                   int out_dt, int64_t M, int64_t N, int64_t K, cudaStream_t st);
+int launch_w8a8_tc(const int8_t* xq, const int8_t* w, const Scales& sc, const float* x_scale, const int32_t* rowsum,
+                   int32_t* acc_out, void* out, int out_dt, int64_t M, int64_t N, int64_t K, cudaStream_t st);
 
 // ---- mixed_gemm.cu (tcgen05 kind::f16 after shared-memory dequant) ------------------------
 bool mixed_tc_shape_ok(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_size, int x_dt, bool has_zp);

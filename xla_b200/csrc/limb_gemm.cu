@@ -95,8 +95,9 @@ enum Mode : int {
 };
 
 struct Params {
-  const float* scale;  // [N] or [S,N]
-  const float* zp;     // like scale, or null
+  const void* scale;   // [N] or [S,N], of type s_dt
+  const void* zp;      // like scale, or null
+  int s_dt;
   const float* xs;     // with zp: [S][xs_pitch] sums of the fixed-point activations over each scale block
   int xs_pitch;
   float zp_mul;        // factor that the weight bytes carry (16 for int4 weights)
@@ -221,7 +222,7 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
 __device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
-__device__ __forceinline__ void cp_async4(uint32_t dst, const float* src) {
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void st_release_gpu(uint32_t* p, uint32_t v) {
@@ -484,7 +485,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* raw_base = smem;
   uint8_t* slot_base = raw_base + (size_t)kRaw * kRawBytes;
-  float* scale_base = reinterpret_cast<float*>(slot_base + (size_t)kSlots * kSlot);  // [kScaleRing][128]
+  uint32_t* scale_base = reinterpret_cast<uint32_t*>(slot_base + (size_t)kSlots * kSlot);  // [kScaleRing][128]
   uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(scale_base) + C::kScaleBytes);
   uint64_t* raw_full = bars;                       // [kRaw]    TMA bytes
   uint64_t* raw_empty = raw_full + (kRaw ? kRaw : 1);  // [kRaw]    4 expanding warps
@@ -737,6 +738,8 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
     __shared__ float s_pw[2][64];
     static_assert(MT <= 64, "per-token factors of a tile");
     int frag = 0;
+    const int64_t sc_pitch = p.ld * (p.s_dt == QMM_F32 ? 4 : 2);
+    const ScaleWord word(p.s_dt, rl);
     auto wait_acc = [&]() {
       DBG_BEGIN();
       ptx::mbar_wait_warp<32>(&acc_full[buf], pacc, abort_flag, p.err_word, ptx::kErrWaitTmemFull);
@@ -763,7 +766,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
       // readers of one from the writers of its next use).  Fetched at the end they are two L2 round trips per tile.
       float* pw_s = s_pw[frag & 1];
       ++frag;
-      const float ps = (p.mode != kPerChannel || !n_ok || !first) ? 1.f : __ldg(p.scale + n);
+      const float ps = (p.mode != kPerChannel || !n_ok || !first) ? 1.f : load_as_f32(p.scale, n, p.s_dt);
       if (first && dt < MT) pw_s[dt] = it.y * MT + dt < p.M ? __ldg(p.pw + it.y * MT + dt) : 0.f;
       float total[MTD];
 #pragma unroll
@@ -809,8 +812,9 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
       // Block scales are fetched one hand-over ahead, from clamped addresses, and change registers at its end.  (A longer
       // register queue does not fetch further ahead: its shift waits for the youngest load, and shifting twice per
       // hand-over put a whole memory round trip into each: int4 block 128 [28672,8192] at 512 tokens 363 us, now 337.)
-      const float* scale_n = p.scale + min(n, p.N - 1);
-      auto fetch_scale = [&](int b) { return __ldg(scale_n + (int64_t)min(b, p.S - 1) * p.ld); };
+      const int64_t sc_off = scale_word_offset(min(n, p.N - 1), p.s_dt);
+      const uint8_t* scale_n = static_cast<const uint8_t*>(p.scale) + sc_off;
+      auto fetch_scale = [&](int b) { return __ldg(reinterpret_cast<const uint32_t*>(scale_n + min(b, p.S - 1) * sc_pitch)); };
       if (C::kScaleRing > 0 && p.scale_ring) {
         // A hand-over here is shorter than a round trip to HBM, so the scales come eight blocks ahead, into a ring of the
         // thread's own (one hand-over ahead, in registers: int4 block 128 [57344,8192] 53.9 us at 4 tokens and 82.0 at 16,
@@ -818,11 +822,11 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
         constexpr int R = C::kScaleRing > 0 ? C::kScaleRing : 1;
         const int per_slot = p.mode == kBlock128 ? 2 : p.mode == kBlock64 ? 4 : 1;  // blocks
         const int b0 = p.mode == kBlockSlots ? u0 : s0 * per_slot, b1 = p.mode == kBlockSlots ? u1 : s1 * per_slot;
-        float* ring = scale_base + rl;
+        const uint32_t* ring = scale_base + rl;
         const uint32_t ring_u32 = ptx::smem_u32(ring);
         auto fetch = [&](int b) {
           // (a last slot may hold fewer blocks than the others: their sums are zero, but the factor has to be a number)
-          if (b < b1) cp_async4(ring_u32 + (uint32_t)(b % R) * 512, scale_n + (int64_t)min(b, p.S - 1) * p.ld);
+          if (b < b1) cp_async4(ring_u32 + (uint32_t)(b % R) * 512, scale_n + min(b, p.S - 1) * sc_pitch);
           asm volatile("cp.async.commit_group;" ::: "memory");
         };
 #pragma unroll 1
@@ -832,7 +836,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
           for (int b = b0; b < b1; b += 2) {
             wait_acc();
             asm volatile("cp.async.wait_group %0;" ::"n"(R - 2) : "memory");
-            const float sc0 = ring[(b % R) * 128], sc1 = ring[((b + 1) % R) * 128];
+            const float sc0 = word(ring[(b % R) * 128]), sc1 = word(ring[((b + 1) % R) * 128]);
             const uint32_t a = lane_addr + buf * (2 * NCOLS) + col0;
             fold_region<DC, MTD, NL, true>(a, sc0, total, false, release);
             fold_region<DC, MTD, NL, true>(a + NCOLS, sc1, total, true, release);
@@ -845,7 +849,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
           for (int b = b0; b < b1; ++b) {
             wait_acc();
             asm volatile("cp.async.wait_group %0;" ::"n"(R - 1) : "memory");
-            const float sc = ring[(b % R) * 128];
+            const float sc = word(ring[(b % R) * 128]);
             if (small) fold_region<DC, MTD, NL, true>(lane_addr + buf * NCOLS + col0, sc, total, true, release);
             else fold_region<DC, MTD, NL, false>(lane_addr + buf * NCOLS + col0, sc, total, true, release);
             next_acc();
@@ -854,9 +858,10 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");  // the ring is refilled from any place
       } else if (p.mode == kBlock128) {
-        float sc2[2] = {fetch_scale(2 * s0), fetch_scale(2 * s0 + 1)};
+        uint32_t w0 = fetch_scale(2 * s0), w1 = fetch_scale(2 * s0 + 1);
         for (int s = s0; s < s1; ++s) {
-          const float nx0 = fetch_scale(2 * s + 2), nx1 = fetch_scale(2 * s + 3);
+          const float sc2[2] = {word(w0), word(w1)};
+          const uint32_t nx0 = fetch_scale(2 * s + 2), nx1 = fetch_scale(2 * s + 3);
           if (C::kPair) {
             wait_acc();
             DBG_BEGIN();
@@ -884,17 +889,18 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
               next_acc();
             }
           }
-          sc2[0] = nx0;
-          sc2[1] = nx1;
+          w0 = nx0;
+          w1 = nx1;
         }
       } else {
         // hand-overs, and slots per hand-over in quarters (blocks of 64: one quarter)
         const int per = p.mode == kBlockSlots ? 4 * p.spu : (p.mode == kBlock64 ? 1 : 4 * (s1 - s0));
         int s = 4 * s0, b = p.mode == kBlockSlots ? s0 / p.spu : 4 * s0;
-        float sc = p.mode == kPerChannel ? 1.f : fetch_scale(b);
+        uint32_t w = p.mode == kPerChannel ? 0u : fetch_scale(b);
         while (s < 4 * s1) {
           const int g_end = s + per;
-          const float nx = p.mode == kPerChannel ? 1.f : fetch_scale(++b);
+          const float sc = p.mode == kPerChannel ? 1.f : word(w);
+          const uint32_t nx = p.mode == kPerChannel ? 0u : fetch_scale(++b);
           wait_acc();
           DBG_BEGIN();
           if constexpr (C::kPipeDrain) {
@@ -908,7 +914,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
           DBG_END(1);
           next_acc();
           s = g_end;
-          sc = nx;
+          w = nx;
         }
       }
       DBG_BEGIN();
@@ -962,14 +968,18 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
           for (int t = 0; t < MTD; ++t) total[t] *= ps;
           psv = 1.f;
         }
-        const float* zp = p.zp + min(n, p.N - 1);
-        auto fetch_zp = [&](int b) { return -p.zp_mul * __ldg(zp + (int64_t)min(b, p.S - 1) * p.ld); };
-        float zq[4];
+        const uint8_t* zp = static_cast<const uint8_t*>(p.zp) + sc_off;
+        // (one block: a single value, which need not lie in a word of the tensor)
+        auto fetch_zp = [&](int b) {
+          return p.mode == kPerChannel ? __float_as_uint(load_as_f32(p.zp, min(n, p.N - 1), p.s_dt))
+                                       : __ldg(reinterpret_cast<const uint32_t*>(zp + min(b, p.S - 1) * sc_pitch));
+        };
+        uint32_t zq[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) zq[i] = fetch_zp(i);
         const float* xs = p.xs + mt0;
         for (int b = 0; b < p.S; ++b, xs += p.xs_pitch) {
-          const float z = zq[0];
+          const float z = -p.zp_mul * (p.mode == kPerChannel ? __uint_as_float(zq[0]) : word(zq[0]));
 #pragma unroll
           for (int i = 0; i < 3; ++i) zq[i] = zq[i + 1];
           zq[3] = fetch_zp(b + 4);
@@ -1379,10 +1389,11 @@ cudaError_t launch_expand(const void* src, void* dst, int64_t rows, int64_t K, c
 
 // pw_mul: factor folded into the per-token power of two (1/16 when the weight bytes hold value * 16); w_dep: the
 // weights are written by a kernel earlier in the stream that the weight producer has to wait for.
-int launch_limb_impl(int wbits, const void* x, int x_dt, const void* w, const float* scale, const float* zp, void* out, int out_dt, int64_t M,
-                     int64_t N, int64_t K, int64_t block_size, int gate_up, void* workspace, size_t workspace_bytes,
-                     float pw_mul, int w_dep, cudaStream_t st) {
-  if (!limb_tc_supported(wbits, M, N, K, block_size, x, x_dt, w, zp != nullptr))
+int launch_limb_impl(int wbits, const void* x, int x_dt, const void* w, const Scales& scales, void* out, int out_dt, int64_t M, int64_t N,
+                     int64_t K, int64_t block_size, int gate_up, void* workspace, size_t workspace_bytes, float pw_mul, int w_dep,
+                     cudaStream_t st) {
+  const bool zp = scales.zp != nullptr;
+  if (!limb_tc_supported(wbits, M, N, K, block_size, x, x_dt, w, zp) || !scale_words_ok(scales, N, block_size))
     return fail(QMM_ERR_UNSUPPORTED,
                 "split-activation tensor-core kernel: needs an sm_100 device, K >= 128 and a multiple of %d, "
                 "block_size 64, 128 or a multiple of 256, 16-byte aligned x/w (M=%lld N=%lld K=%lld bs=%lld)",
@@ -1390,7 +1401,7 @@ int launch_limb_impl(int wbits, const void* x, int x_dt, const void* w, const fl
   if (gate_up && zp) return fail(QMM_ERR_UNSUPPORTED, "fused gate/up epilogue: no zero points");
   if (gate_up && N % 16 != 0)
     return fail(QMM_ERR_BAD_SHAPE, "fused gate/up epilogue: the interleaved weight needs a multiple of 16 rows, got %lld", (long long)N);
-  const Plan pl = plan_for(wbits, M, N, K, block_size <= 0, out_dt, zp != nullptr);
+  const Plan pl = plan_for(wbits, M, N, K, block_size <= 0, out_dt, zp);
   const int nl = pl.nl;
   const size_t need = carve(nullptr, std::min(M, max_rows(nl)), K, nl, pl.tile_tokens, kLimbMaxCtas).bytes;
   if (!workspace || workspace_bytes < need)
@@ -1407,7 +1418,7 @@ int launch_limb_impl(int wbits, const void* x, int x_dt, const void* w, const fl
       cudaGetLastError();
       return fail(QMM_ERR_LAUNCH, "expand_int4_kernel launch: %s", cudaGetErrorString(e));
     }
-    return launch_limb_impl(8, x, x_dt, wide, scale, zp, out, out_dt, M, N, K, block_size, 0, workspace, wide_off, 0.0625f, 1, st);
+    return launch_limb_impl(8, x, x_dt, wide, scales, out, out_dt, M, N, K, block_size, 0, workspace, wide_off, 0.0625f, 1, st);
   }
   if (M > max_rows(nl)) {
     // long batches run in chunks of whole token tiles that share the scratch (same stream: ordered)
@@ -1416,7 +1427,7 @@ int launch_limb_impl(int wbits, const void* x, int x_dt, const void* w, const fl
     const size_t xb = dtype_size(x_dt), ob = dtype_size(out_dt);
     for (int64_t m0 = 0; m0 < M; m0 += rows) {
       const int64_t mc = std::min(rows, M - m0);
-      const int rc = launch_limb_impl(wbits, reinterpret_cast<const uint8_t*>(x) + (size_t)m0 * K * xb, x_dt, w, scale, zp,
+      const int rc = launch_limb_impl(wbits, reinterpret_cast<const uint8_t*>(x) + (size_t)m0 * K * xb, x_dt, w, scales,
                                       reinterpret_cast<uint8_t*>(out) + (size_t)m0 * N * ob, out_dt, mc, N, K, block_size, 0, workspace,
                                       workspace_bytes, pw_mul, w_dep, st);
       if (rc != QMM_OK) return rc;
@@ -1464,6 +1475,7 @@ int launch_limb_impl(int wbits, const void* x, int x_dt, const void* w, const fl
   p.xs = sc.xs;
   p.xs_pitch = sc.xs_pitch;
   p.zp_mul = 1.f / pw_mul;
+  p.s_dt = scales.dt;
   p.out_dt = out_dt;
   p.M = (int)M;
   p.ld = N;
@@ -1479,8 +1491,8 @@ int launch_limb_impl(int wbits, const void* x, int x_dt, const void* w, const fl
   p.ytiles = pl.items ? (int)ceil_div(M, pl.tile_tokens) : 1;
   p.m0 = 0;
   if (slice_rows == 0) {
-    p.scale = scale;
-    p.zp = zp;
+    p.scale = scales.scale;
+    p.zp = scales.zp;
     p.out = out;
     p.w_dep = w_dep;
     return launch_main(wbits, w, N, K, pl, p, map_x, st);
@@ -1493,8 +1505,8 @@ int launch_limb_impl(int wbits, const void* x, int x_dt, const void* w, const fl
       cudaGetLastError();
       return fail(QMM_ERR_LAUNCH, "expand_int4_kernel launch: %s", cudaGetErrorString(e));
     }
-    p.scale = scale + n0;
-    p.zp = zp ? zp + n0 : nullptr;
+    p.scale = elements_from(scales.scale, n0, scales.dt);
+    p.zp = elements_from(scales.zp, n0, scales.dt);
     p.out = reinterpret_cast<uint8_t*>(out) + (size_t)n0 * ob;
     p.w_dep = 1;
     rc = launch_main(8, wide, rows, K, pl, p, map_x, st);
@@ -1505,10 +1517,9 @@ int launch_limb_impl(int wbits, const void* x, int x_dt, const void* w, const fl
 
 }  // namespace
 
-int launch_limb_tc(int wbits, const void* x, int x_dt, const void* w, const float* scale, const float* zp, void* out, int out_dt, int64_t M,
-                   int64_t N, int64_t K, int64_t block_size, int gate_up, void* workspace, size_t workspace_bytes,
-                   cudaStream_t st) {
-  return launch_limb_impl(wbits, x, x_dt, w, scale, zp, out, out_dt, M, N, K, block_size, gate_up, workspace, workspace_bytes,
+int launch_limb_tc(int wbits, const void* x, int x_dt, const void* w, const Scales& scales, void* out, int out_dt, int64_t M, int64_t N,
+                   int64_t K, int64_t block_size, int gate_up, void* workspace, size_t workspace_bytes, cudaStream_t st) {
+  return launch_limb_impl(wbits, x, x_dt, w, scales, out, out_dt, M, N, K, block_size, gate_up, workspace, workspace_bytes,
                           wbits == 4 ? 0.0625f : 1.f, 0, st);
 }
 

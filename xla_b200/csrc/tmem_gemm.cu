@@ -50,8 +50,9 @@ constexpr int kMiscRegs = 40, kConvRegs = 64, kDrainRegs = 152;  // x 128, 256, 
 constexpr uint32_t kErrPartial = 10;      // owner CTA never saw a partial tile arrive
 
 struct Params {
-  const float* scale;  // [N] or [S,N]
-  const float* zp;     // like scale, or null
+  const void* scale;   // [N] or [S,N], of type s_dt
+  const void* zp;      // like scale, or null
+  int s_dt;
   const float* xs;     // with zp: [S][xs_pitch] sums of the activations over each scale block
   int xs_pitch;
   void* out;
@@ -132,7 +133,7 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
   asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
   return v;
 }
-__device__ __forceinline__ void cp_async4(uint32_t dst, const float* src) {
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void st_release_gpu(uint32_t* p, uint32_t v) {
@@ -217,7 +218,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* raw_base = smem;
   uint8_t* b_base = raw_base + (size_t)kRaw * kRawBytes;
-  float* s_scale = reinterpret_cast<float*>(b_base + (size_t)kB * C::kBStage);  // [scale, zero point][kScaleRing][kDrain]
+  uint32_t* s_scale = reinterpret_cast<uint32_t*>(b_base + (size_t)kB * C::kBStage);  // [scale, zero point][kScaleRing][kDrain]
   uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(s_scale) + C::kScaleBytes);
   uint64_t* raw_full = bars;                 // [kRaw]    TMA bytes
   uint64_t* raw_empty = raw_full + kRaw;     // [kRaw]    the converting warps that share the tile
@@ -416,8 +417,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + grp * DT;
     auto drain_bar = [&]() { asm volatile("bar.sync 1, 256;" ::: "memory"); };
     __shared__ int s_npart;
-    float* my_scale = s_scale + dt;
+    const uint32_t* my_scale = s_scale + dt;
     const uint32_t my_scale_u32 = ptx::smem_u32(my_scale);
+    const ScaleWord word(p.s_dt, rl);
     bool waited = false;
     FragIter it(p);
     int buf = 0;
@@ -434,14 +436,14 @@ __global__ void __launch_bounds__(kThreads, 1)
       // Block scales and zero points are a stream of their own (a round trip to HBM each): every thread copies its own
       // row's, seven folds ahead, into a ring of its own.  (Held in registers that shift from fold to fold, the shift
       // waits for the load of the fold before, whatever the nominal distance.)
-      const int64_t nc = min(n, p.N - 1);
-      const float* scp = p.scale + nc;
-      const float* zpp = p.zp ? p.zp + nc : nullptr;
+      const int64_t sc_off = scale_word_offset(min(n, p.N - 1), p.s_dt), sc_pitch = p.N * (p.s_dt == QMM_F32 ? 4 : 2);
+      const uint8_t* scp = static_cast<const uint8_t*>(p.scale) + sc_off;
+      const uint8_t* zpp = static_cast<const uint8_t*>(p.zp) + sc_off;
       auto fetch = [&](int f) {
         if (p.blocked && f < it.u1) {
           const uint32_t dst = my_scale_u32 + (uint32_t)(f % kScaleRing) * (kDrain * 4);
-          cp_async4(dst, scp + (int64_t)f * p.N);
-          if (p.zp) cp_async4(dst + kScaleRing * kDrain * 4, zpp + (int64_t)f * p.N);
+          cp_async4(dst, scp + f * sc_pitch);
+          if (p.zp) cp_async4(dst + kScaleRing * kDrain * 4, zpp + f * sc_pitch);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
       };
@@ -465,7 +467,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         uint32_t r[2][16];
         ptx::tmem_ld_32x32b_x16(a, r[0]);
         asm volatile("cp.async.wait_group %0;" ::"n"(kScaleRing - 1) : "memory");
-        const float sc = p.blocked ? my_scale[(f % kScaleRing) * kDrain] : 1.f;
+        const float sc = p.blocked ? word(my_scale[(f % kScaleRing) * kDrain]) : 1.f;
 #pragma unroll
         for (int c = 0; c < DT / 16; ++c) {
           uint32_t* cur = r[c & 1];
@@ -486,7 +488,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           pacc ^= 1;
         }
         if (p.blocked && p.zp) {
-          const float z = -my_scale[(kScaleRing + f % kScaleRing) * kDrain];
+          const float z = -word(my_scale[(kScaleRing + f % kScaleRing) * kDrain]);
           const float* xs = p.xs + (int64_t)f * p.xs_pitch + m0;  // the same for all lanes; the pitch covers whole tiles
 #pragma unroll
           for (int t = 0; t < DT; t += 4) {
@@ -528,8 +530,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         drain_bar();
       }
-      const float ps = p.blocked || !n_ok ? 1.f : __ldg(p.scale + n);
-      const float z1 = !p.blocked && p.zp && n_ok ? -__ldg(p.zp + n) : 0.f;
+      const float ps = p.blocked || !n_ok ? 1.f : load_as_f32(p.scale, n, p.s_dt);
+      const float z1 = !p.blocked && p.zp && n_ok ? -load_as_f32(p.zp, n, p.s_dt) : 0.f;
 #pragma unroll 1
       for (int c = 0; c < DT / 16; ++c) {
         const int l0 = grp * DT + 16 * c;  // token inside the item
@@ -731,10 +733,10 @@ bool tmem_gemm_supported(int wbits, int64_t M, int64_t N, int64_t K, int64_t blo
   return tmem_gemm_shape_ok(wbits, M, N, K, block_size, x_dt) && aligned(x, 16) && aligned(w, 16) && device_is_sm100();
 }
 
-int launch_tmem_gemm(int wbits, const void* x, int x_dt, const void* w, const float* scale, const float* zp, void* out, int out_dt,
-                     int64_t M, int64_t N, int64_t K, int64_t block_size, int gate_up, void* workspace, size_t workspace_bytes,
-                     cudaStream_t st) {
-  if (!tmem_gemm_supported(wbits, M, N, K, block_size, x, x_dt, w))
+int launch_tmem_gemm(int wbits, const void* x, int x_dt, const void* w, const Scales& scales, void* out, int out_dt, int64_t M, int64_t N,
+                     int64_t K, int64_t block_size, int gate_up, void* workspace, size_t workspace_bytes, cudaStream_t st) {
+  const bool zp = scales.zp != nullptr;
+  if (!tmem_gemm_supported(wbits, M, N, K, block_size, x, x_dt, w) || !scale_words_ok(scales, N, block_size))
     return fail(QMM_ERR_UNSUPPORTED,
                 "tensor-memory kernel: needs an sm_100 device, bf16/f16 activations, 16-byte row pitches, block_size 64 or a "
                 "multiple of 128, 16-byte aligned x/w (M=%lld N=%lld K=%lld bs=%lld)",
@@ -749,8 +751,9 @@ int launch_tmem_gemm(int wbits, const void* x, int x_dt, const void* w, const fl
   if (!aligned(workspace, 256)) return fail(QMM_ERR_MISALIGNED, "workspace must be 256-byte aligned");
 
   Params p = {};
-  p.scale = scale;
-  p.zp = zp;
+  p.scale = scales.scale;
+  p.zp = scales.zp;
+  p.s_dt = scales.dt;
   p.xs = sc.xs;
   p.xs_pitch = sc.xs_pitch;
   p.out = out;

@@ -120,22 +120,43 @@ struct Call {
   Tensor scale, zp;
   int wbits;
   int64_t M, N, K, block;  // block 0: per channel
+
+  // Scales (and zero points) in the one type that the kernels read besides fp32, or fp32
+  void scales_to_f32() {
+    scale = as_f32(scale);
+    if (zp.defined()) zp = as_f32(zp);
+  }
+  bool scales_f32() const { return scale.scalar_type() == at::kFloat; }
+  const void* zp_ptr() const { return zp.defined() ? zp.data_ptr() : nullptr; }
 };
 
+// Scales in 16 bits go to the kernel as they are; where the one that this shape takes reads fp32 only, they are converted.
+template <typename F>
+bool with_scales(Call& c, F run) {
+  int rc = run();
+  if (rc == QMM_ERR_UNSUPPORTED && !c.scales_f32()) {
+    c.scales_to_f32();
+    rc = run();
+  }
+  return rc == QMM_OK;
+}
+
 // Runs one linear; false when the library refused it (the Python form repeats the call and raises its error).
-bool weight_only(const Call& c, Tensor& out) {
+bool weight_only(Call& c, Tensor& out) {
   const int dev = c.x.get_device();
   const cudaStream_t st = c10::cuda::getCurrentCUDAStream(dev).stream();
   std::lock_guard<std::mutex> hold(g_scratch_lock);
   void* ws;
   size_t ws_bytes;
   scratch(dev, st, qmm_weight_only_workspace_size_for(c.wbits, c.M, c.N, c.K), &ws, &ws_bytes);
-  return qmm_weight_only(c.wbits, c.x.data_ptr(), dtype_code(c.x.scalar_type()), c.w.data_ptr(), (const float*)c.scale.data_ptr(),
-                         c.zp.defined() ? (const float*)c.zp.data_ptr() : nullptr, out.data_ptr(), dtype_code(out.scalar_type()), c.M,
-                         c.N, c.K, c.block, tl_variant, ws, ws_bytes, st) == QMM_OK;
+  return with_scales(c, [&] {
+    return qmm_weight_only_typed(c.wbits, c.x.data_ptr(), dtype_code(c.x.scalar_type()), c.w.data_ptr(), c.scale.data_ptr(), c.zp_ptr(),
+                                 dtype_code(c.scale.scalar_type()), out.data_ptr(), dtype_code(out.scalar_type()), c.M, c.N, c.K,
+                                 c.block, tl_variant, ws, ws_bytes, st);
+  });
 }
 
-bool w8a8(const Call& c, Tensor& out) {
+bool w8a8(Call& c, Tensor& out) {
   const int dev = c.x.get_device();
   const cudaStream_t st = c10::cuda::getCurrentCUDAStream(dev).stream();
   std::lock_guard<std::mutex> hold(g_scratch_lock);
@@ -151,9 +172,11 @@ bool w8a8(const Call& c, Tensor& out) {
   } else {
     ws = static_cast<uint8_t*>(ws) + kFlags;
   }
-  return qmm_w8a8_perchannel(c.x.data_ptr(), dtype_code(c.x.scalar_type()), (const int8_t*)c.w.data_ptr(),
-                             (const float*)c.scale.data_ptr(), c.zp.defined() ? (const float*)c.zp.data_ptr() : nullptr, out.data_ptr(),
-                             dtype_code(out.scalar_type()), c.M, c.N, c.K, tl_saturate, tl_variant, ws, need, st) == QMM_OK;
+  return with_scales(c, [&] {
+    return qmm_w8a8_perchannel_typed(c.x.data_ptr(), dtype_code(c.x.scalar_type()), (const int8_t*)c.w.data_ptr(), c.scale.data_ptr(),
+                                     c.zp_ptr(), dtype_code(c.scale.scalar_type()), out.data_ptr(), dtype_code(out.scalar_type()), c.M,
+                                     c.N, c.K, tl_saturate, tl_variant, ws, need, st);
+  });
 }
 
 // The shapes and layouts the kernels take as they are: contiguous activations, a contiguous K-minor weight, scales (and
@@ -175,8 +198,11 @@ bool plain(const Tensor& x, const Tensor& w, const Tensor& scale, const optional
 
 Call make_call(const Tensor& x, const Tensor& w, const Tensor& scale, const optional<Tensor>& zp, int64_t block, bool packed) {
   const int64_t K = x.size(-1);
-  return Call{x, w, as_f32(scale), zp.has_value() ? as_f32(*zp) : Tensor(), packed ? 4 : 8, x.numel() / K, w.size(0), K,
-              block == -1 ? 0 : block};
+  Call c{x, w, scale, zp.has_value() ? *zp : Tensor(), packed ? 4 : 8, x.numel() / K, w.size(0), K, block == -1 ? 0 : block};
+  const bool as_they_are = dtype_code(scale.scalar_type()) >= 0 && scale.is_contiguous() &&
+                           (!zp.has_value() || (zp->scalar_type() == scale.scalar_type() && zp->is_contiguous()));
+  if (!as_they_are) c.scales_to_f32();
+  return c;
 }
 
 template <typename Sig, typename... A>
@@ -192,7 +218,7 @@ Tensor quantized_matmul(const Tensor& x, const Tensor& w, const Tensor& scale, c
     const bool qact = quantize_activation.value_or(false);
     const at::ScalarType dt = promote(x, scale, zp);
     if (dtype_code(dt) >= 0 && (qact || !zero_point_outside(x, w.size(0), 8, -1, zp))) {
-      const Call c = make_call(x, w, scale, zp, -1, false);
+      Call c = make_call(x, w, scale, zp, -1, false);
       Tensor out = output(x, c.N, dt);
       if (qact ? w8a8(c, out) : weight_only(c, out)) return out;
     }
@@ -206,7 +232,7 @@ Tensor quantized_matmul_int8(const Tensor& x, const Tensor& w, const Tensor& sca
                              optional<int64_t> out_block_size, optional<int64_t> in_block_size) {
   if (!zp.has_value() && !quant_block_size.has_value() && x.dim() == 2 && plain(x, w, scalar, zp, -1, false)) {
     c10::cuda::OptionalCUDAGuard guard(x.device());
-    const Call c = make_call(x, w, scalar, zp, -1, false);
+    Call c = make_call(x, w, scalar, zp, -1, false);
     Tensor out = output(x, c.N, x.scalar_type());
     if (quantize_activation ? w8a8(c, out) : weight_only(c, out)) return out;
   }
@@ -220,7 +246,7 @@ Tensor quantized_matmul_packed(const Tensor& x, const Tensor& w, const Tensor& s
     c10::cuda::OptionalCUDAGuard guard(x.device());
     const at::ScalarType dt = out_dtype.has_value() ? *out_dtype : promote(x, scale, zp);
     if (dtype_code(dt) >= 0 && (quantize_activation || !zero_point_outside(x, w.size(0), weight_is_packed ? 4 : 8, block_size, zp))) {
-      const Call c = make_call(x, w, scale, zp, block_size, weight_is_packed);
+      Call c = make_call(x, w, scale, zp, block_size, weight_is_packed);
       Tensor out = output(x, c.N, dt);
       if (quantize_activation ? w8a8(c, out) : weight_only(c, out)) return out;
     }
@@ -243,7 +269,8 @@ Tensor quantized_gate_up(const Tensor& x, const Tensor& w, const Tensor& scale, 
     const at::ScalarType dt = out_dtype.has_value() ? *out_dtype : promote(x, scale, {});
     if (dtype_code(dt) >= 0 && (decode || batch)) {
       c10::cuda::OptionalCUDAGuard guard(x.device());
-      const Call c = make_call(x, w, scale, {}, block_size, weight_is_packed);
+      Call c = make_call(x, w, scale, {}, block_size, weight_is_packed);
+      c.scales_to_f32();
       const int dev = x.get_device();
       const cudaStream_t st = c10::cuda::getCurrentCUDAStream(dev).stream();
       Tensor out = output(x, c.N / 2, dt);

@@ -38,8 +38,9 @@ constexpr uint32_t kScaleBytes = 2 * BN * 4;              // w_scale and zero po
 constexpr size_t kSmemBytes = 1024 /*align slack*/ + (size_t)kStages * kStageBytes + kOutStaging + kScaleBytes + 256;
 
 struct Params {
-  const float* w_scale;
-  const float* zp;
+  const void* w_scale;  // [N], of type s_dt
+  const void* zp;       // like w_scale, or null
+  int s_dt;
   const float* x_scale;
   const int32_t* rowsum;
   int32_t* acc_out;
@@ -190,8 +191,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         asm volatile("bar.sync 1, 128;" ::: "memory");
         for (int j = e; j < BN; j += 128) {
           const int64_t n = (int64_t)tn * BN + j;
-          s_ws[j] = n < p.N ? __ldg(p.w_scale + n) : 0.f;
-          s_zp[j] = (p.zp && n < p.N) ? __ldg(p.zp + n) : 0.f;
+          s_ws[j] = n < p.N ? load_as_f32(p.w_scale, n, p.s_dt) : 0.f;
+          s_zp[j] = (p.zp && n < p.N) ? load_as_f32(p.zp, n, p.s_dt) : 0.f;
         }
         asm volatile("bar.sync 1, 128;" ::: "memory");
         const int rl = quad * 32 + lane;  // row inside the tile
@@ -267,7 +268,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
             const int64_t n = (n0 + j < p.N) ? n0 + j : p.N - 1;
-            v[j] = w8a8_dequant((int32_t)r[j], __ldg(p.w_scale + n), p.zp ? p.zp + n : nullptr, rs, xs);
+            const float z = p.zp ? load_as_f32(p.zp, n, p.s_dt) : 0.f;
+            v[j] = w8a8_dequant((int32_t)r[j], load_as_f32(p.w_scale, n, p.s_dt), p.zp ? &z : nullptr, rs, xs);
           }
           if (p.out_dt == QMM_F32)
             store_row_chunk<float>(reinterpret_cast<float*>(p.out) + m * p.N + n0, v, ncols, p.out_vec != 0);
@@ -304,9 +306,8 @@ bool w8a8_tc_supported(int64_t M, int64_t N, int64_t K, const void* xq, const vo
   return device_is_sm100();
 }
 
-int launch_w8a8_tc(const int8_t* xq, const int8_t* w, const float* w_scale, const float* zp,
-                   const float* x_scale, const int32_t* rowsum, int32_t* acc_out, void* out,
-                   int out_dt, int64_t M, int64_t N, int64_t K, cudaStream_t st) {
+int launch_w8a8_tc(const int8_t* xq, const int8_t* w, const Scales& sc, const float* x_scale, const int32_t* rowsum,
+                   int32_t* acc_out, void* out, int out_dt, int64_t M, int64_t N, int64_t K, cudaStream_t st) {
   if (!w8a8_tc_supported(M, N, K, xq, w))
     return fail(QMM_ERR_UNSUPPORTED,
                 "w8a8 tcgen05 kernel: needs an sm_100 device, K a multiple of 16 and 16-byte aligned "
@@ -341,8 +342,9 @@ int launch_w8a8_tc(const int8_t* xq, const int8_t* w, const float* w_scale, cons
   // vector stores only where every row start is 16-byte aligned; anything else takes the scalar path
   p.out_vec = (out && aligned(out, 16) && (N * (int64_t)dtype_size(out_dt)) % 16 == 0) ? 1 : 0;
   p.acc_vec = (acc_out && aligned(acc_out, 16) && N % 4 == 0) ? 1 : 0;
-  p.w_scale = w_scale;
-  p.zp = zp;
+  p.w_scale = sc.scale;
+  p.zp = sc.zp;
+  p.s_dt = sc.dt;
   p.x_scale = x_scale;
   p.rowsum = rowsum;
   p.acc_out = acc_out;
