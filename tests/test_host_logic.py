@@ -91,6 +91,26 @@ def test_module_mirrors_reference_buffers(golden):
   sym2.load_state_dict(sym.state_dict())
 
 
+def test_a_used_module_can_be_saved_and_copied():
+  """torch.save, pickle and deepcopy of a module in the state that a forward pass on a GPU leaves: the buffers come back,
+  what was derived from them does not travel."""
+  import copy
+  import io
+  import pickle
+  m = xla_b200.XlaQuantizedLinear(32, 16, is_symmetric=True, int4_weight=True)
+  m.load_quantized_weight(torch.randint(-8, 8, (16, 32), dtype=torch.int8), torch.rand(16))
+  w = m.weight
+  m._packed = ((w.data_ptr(), w._version, w.device), torch.zeros(16, 16, dtype=torch.uint8), True)
+  m._plan = (w, w._version, w.data_ptr(), m._packed[1], True, torch.ops.xla_b200.quantized_matmul_packed.default)
+  buf = io.BytesIO()
+  torch.save(m, buf)
+  buf.seek(0)
+  for c in (torch.load(buf, weights_only=False), pickle.loads(pickle.dumps(m)), copy.deepcopy(m)):
+    assert c._plan is None and c._packed is None
+    assert torch.equal(c.weight, m.weight) and torch.equal(c.weight_scaler, m.weight_scaler) and c.zero_point is None
+    assert c.input_dim == 32 and c.int4_weight and c.prepack
+
+
 def test_blockwise_rejects_activation_quantization_before_touching_the_gpu():
   x = torch.zeros(2, 6, device="meta")
   with pytest.raises(Exception):
