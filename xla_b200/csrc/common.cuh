@@ -5,6 +5,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <type_traits>
 
 #include "../../include/qmm_b200.h"
 
@@ -84,6 +85,15 @@ __device__ __forceinline__ void store_from_f32(void* p, int64_t i, int dt, float
     reinterpret_cast<__half*>(p)[i] = __float2half_rn(v);
 }
 
+// ---- data of earlier kernels (device) --------------------------------------------------------
+// A kernel launched with programmatic stream serialization starts while the kernel before it still runs.  What
+// it may have written is read with ordinary loads: __ldg and const __restrict__ stand for data that nobody writes
+// while the kernel runs, so such a load may be moved ahead of the wait or served from a stale cache line.
+template <typename T>
+__device__ __forceinline__ T ld_ordered(const T* p) {
+  return *p;
+}
+
 // ---- weight scales and zero points ---------------------------------------------------------
 // In fp32 or in a 16-bit type (the buffers of a quantized 16-bit model), both in the same one.
 struct Scales {
@@ -103,18 +113,29 @@ inline bool scale_words_ok(const Scales& s, int64_t N, int64_t block_size) {
 }
 
 // Byte offset of the word that holds element n
-__device__ __forceinline__ int64_t scale_word_offset(int64_t n, int dt) { return dt == QMM_F32 ? n * 4 : (n & ~1ll) * 2; }
+template <bool W16>
+__device__ __forceinline__ int64_t scale_word_offset(int64_t n) {
+  return W16 ? (n & ~1ll) * 2 : n * 4;
+}
 
-// A word's value for the element n that it was fetched for
-struct ScaleWord {
-  uint32_t shift, mask;
-  bool half;
-  __device__ ScaleWord(int dt, int n) : shift(dt == QMM_F32 || (n & 1) ? 0u : 16u), mask(dt == QMM_F32 ? ~0u : 0xffff0000u), half(dt == QMM_F16) {}
-  __device__ float operator()(uint32_t w) const {
-    w = (w << shift) & mask;
-    return half ? __half2float(__ushort_as_half((unsigned short)(w >> 16))) : __uint_as_float(w);
-  }
-};
+// The scale of element n in the word that was copied for it.  W16: 16-bit scales, of type T if that is given.  A template
+// parameter of the kernels, because their loops have no register to spare for the conversion (decided at run time it cost
+// fp32 scales 2 to 25 %: int4 block 128, [57344,8192] and [8192,28672] at 64 tokens 182 us, up to 228).
+template <bool W16, typename T = void>
+__device__ __forceinline__ float scale_in(const uint32_t* word, int n, int dt) {
+  if (!W16) return __uint_as_float(*word);
+  const unsigned short h = reinterpret_cast<const unsigned short*>(word)[n & 1];
+  if (std::is_same<T, __half>::value || (std::is_void<T>::value && dt == QMM_F16)) return __half2float(__ushort_as_half(h));
+  return __uint_as_float((uint32_t)h << 16);
+}
+
+// A single scale as its bits, and their value: apart, because the conversion waits for the load
+__device__ __forceinline__ uint32_t load_scale_bits(const void* p, int64_t n, int dt) {
+  return dt == QMM_F32 ? ld_ordered(static_cast<const uint32_t*>(p) + n) : (uint32_t)ld_ordered(static_cast<const unsigned short*>(p) + n);
+}
+__device__ __forceinline__ float scale_value(uint32_t bits, int dt) {
+  return dt == QMM_F32 ? __uint_as_float(bits) : dt == QMM_BF16 ? __uint_as_float(bits << 16) : __half2float(__ushort_as_half((unsigned short)bits));
+}
 
 // 128-bit streaming load that does not pollute L1 (weights are read exactly once).
 __device__ __forceinline__ uint4 ld_stream_u4(const void* p) {

@@ -51,6 +51,7 @@ struct Args {
   const void* zp;      // like scale, or null
   void* out;
   int64_t N, K;
+  int64_t sc_pitch;    // bytes from one scale block to the next
   int x_dt, out_dt, s_dt, M;
   int steps;           // 64-byte steps per weight row (the last one may be partly outside the row)
   int tiles_lo, tiles_extra;  // tiles per CTA, and how many CTAs take one more
@@ -190,7 +191,7 @@ __host__ __device__ constexpr int slot_bytes(bool blocked, int nb) { return 1024
 template <int W>
 constexpr int kDepth = W == 8 ? 7 : 4;  // ring slots per warp
 
-template <int WBITS, int NL, int NT, bool BLOCKED, bool ZP, bool HALF, int W>
+template <int WBITS, int NL, int NT, bool BLOCKED, bool ZP, bool HALF, int W, bool W16>
 __global__ void __launch_bounds__(W * 32, W == 8 ? 2 : 1) decode_i8_kernel(const Args p) {
   constexpr int kWarps = W, kThreads = W * 32, D = kDepth<W>;
   constexpr int VPS = 512 / WBITS;
@@ -215,8 +216,6 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 2 : 1) decode_i8_kernel(const
   const int64_t pitch = p.K * WBITS / 8;
   const int cols = NL * p.M;
   const int n_last = (int)p.N - 1;
-  const int64_t sc_pitch = p.N * (p.s_dt == QMM_F32 ? 4 : 2);  // bytes from one scale block to the next
-  const ScaleWord word(p.s_dt, g);                             // (rows g and g + 8 of a tile; tiles start at even rows)
 
   if ((int)threadIdx.x < nt_cta) {
     int wv = 0;
@@ -231,18 +230,31 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 2 : 1) decode_i8_kernel(const
   uint32_t ldst = ring;
   const uint8_t *lp0, *lp1;
   const uint8_t* lsc = nullptr;  // this lane's row of the scales (lanes 0..15) or zero points (lanes 16..31)
+  auto scale_row = [&](int tile) {
+    return static_cast<const uint8_t*>(ZP && lane >= 16 ? p.zp : p.scale) + scale_word_offset<W16>(min(tile * kRows + (lane & 15), n_last));
+  };
+  // the block scales and zero points of a step, into its ring slot
+  auto copy_scales = [&](uint32_t slot, const uint8_t* row, int step) {
+    if (!ZP && lane >= 16) return;
+    if constexpr (HALF) {
+      cp_async_small<4>(slot + 1024 + lane * 4, row + (2 * step) * p.sc_pitch);
+      if (2 * step + 1 < p.S) cp_async_small<4>(slot + 1152 + lane * 4, row + (2 * step + 1) * p.sc_pitch);
+    } else {
+      const int b = p.fold_shift >= 0 ? step >> p.fold_shift : step / p.fold_steps;
+      cp_async_small<4>(slot + 1024 + lane * 4, row + b * p.sc_pitch);
+    }
+  };
   auto set_tile = [&]() {
     // rows beyond N repeat the last one; they are not stored
     const int n0 = min(ltile * kRows + g, n_last), n1 = min(ltile * kRows + g + 8, n_last);
     lp0 = p.w + n0 * pitch + (HALF ? 8 : 16) * t;
     lp1 = p.w + n1 * pitch + (HALF ? 8 : 16) * t;
-    if (BLOCKED)
-      lsc = static_cast<const uint8_t*>(ZP && lane >= 16 ? p.zp : p.scale) + scale_word_offset(min(ltile * kRows + (lane & 15), n_last), p.s_dt);
+    if (BLOCKED) lsc = scale_row(ltile);
   };
   set_tile();
   lp0 += (int64_t)ls * 64;
   lp1 += (int64_t)ls * 64;
-  auto issue = [&]() {
+  auto issue = [&](bool with_scales) {
     if (left > 0) {
       --left;
       const uint32_t d = ldst + lane * 16;
@@ -258,17 +270,7 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 2 : 1) decode_i8_kernel(const
         cp_async16(d, lp0);
         cp_async16(d + 512, lp1);
       }
-      if constexpr (BLOCKED) {
-        if (ZP || lane < 16) {
-          if constexpr (HALF) {
-            cp_async_small<4>(ldst + 1024 + lane * 4, lsc + (2 * ls) * sc_pitch);
-            if (2 * ls + 1 < p.S) cp_async_small<4>(ldst + 1152 + lane * 4, lsc + (2 * ls + 1) * sc_pitch);
-          } else {
-            const int b = p.fold_shift >= 0 ? ls >> p.fold_shift : ls / p.fold_steps;
-            cp_async_small<4>(ldst + 1024 + lane * 4, lsc + b * sc_pitch);
-          }
-        }
-      }
+      if (BLOCKED && with_scales) copy_scales(ldst, lsc, ls);
       ldst = ldst + kSlot == ring + D * kSlot ? ring : ldst + kSlot;
       lp0 += 64;
       lp1 += 64;
@@ -281,7 +283,7 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 2 : 1) decode_i8_kernel(const
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
 #pragma unroll
-  for (int d = 0; d < D - 1; ++d) issue();
+  for (int d = 0; d < D - 1; ++d) issue(true);
   // The weights are static: their first loads run under the kernel before this one.  The activations, and every store
   // of this kernel, come after the wait.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -351,7 +353,8 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 2 : 1) decode_i8_kernel(const
   // zero-point term
   auto fold = [&](const uint32_t* sc, int b, bool zp_too) {
     if constexpr (BLOCKED) {
-      const float s0 = word(sc[g]), s1 = word(sc[g + 8]);
+      auto value = [&](int i) { return scale_in<W16>(sc + i, g, p.s_dt); };  // (rows g and g + 8; tiles start at even rows)
+      const float s0 = value(g), s1 = value(g + 8);
 #pragma unroll
       for (int i = 0; i < NT; ++i) {
         total[i][0] = fmaf(s0, __int2float_rn(sum_of(i, 0)), total[i][0]);
@@ -363,7 +366,7 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 2 : 1) decode_i8_kernel(const
       if constexpr (ZP) {
         if (zp_too) {
           constexpr float kW = WBITS == 4 ? 16.f : 1.f;  // the weight sums carry this factor
-          const float z0 = -kW * word(sc[16 + g]), z1 = -kW * word(sc[24 + g]);
+          const float z0 = -kW * value(16 + g), z1 = -kW * value(24 + g);
 #pragma unroll
           for (int i = 0; i < NT; ++i) {
             const int c = 8 * i + 2 * t;
@@ -384,7 +387,7 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 2 : 1) decode_i8_kernel(const
   for (int j = lo; j < hi; ++j) {
     asm volatile("cp.async.wait_group %0;" ::"n"(D - 2) : "memory");
     __syncwarp();
-    issue();  // into the slot of the step before this one, which every lane has read
+    issue(true);  // into the slot of the step before this one, which every lane has read
     const uint8_t* slot = cring + cslot;
     cslot = cslot + kSlot == D * kSlot ? 0 : cslot + kSlot;
     const uint32_t* sc = reinterpret_cast<const uint32_t*>(slot + 1024);
@@ -527,9 +530,9 @@ Layout layout_for(int wbits, int nl, int xbytes, int64_t M, int64_t N, int64_t K
   return layout_with(16, wbits, nl, xbytes, M, N, K, S, blocked, half, zp);
 }
 
-template <int WBITS, int NL, int NT, bool BLOCKED, bool ZP, bool HALF, int W>
-int launch_one(const Args& a, const Layout& l, cudaStream_t st) {
-  auto kern = decode_i8_kernel<WBITS, NL, NT, BLOCKED, ZP, HALF, W>;
+template <int WBITS, int NL, int NT, bool BLOCKED, bool ZP, bool HALF, int W, bool W16>
+int launch_with(const Args& a, const Layout& l, cudaStream_t st) {
+  auto kern = decode_i8_kernel<WBITS, NL, NT, BLOCKED, ZP, HALF, W, W16>;
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -554,6 +557,13 @@ int launch_one(const Args& a, const Layout& l, cudaStream_t st) {
     return fail(QMM_ERR_LAUNCH, "decode_i8_kernel launch: %s", cudaGetErrorString(e));
   }
   return QMM_OK;
+}
+
+template <int WBITS, int NL, int NT, bool BLOCKED, bool ZP, bool HALF, int W>
+int launch_one(const Args& a, const Layout& l, cudaStream_t st) {
+  if constexpr (BLOCKED)
+    if (a.s_dt != QMM_F32) return launch_with<WBITS, NL, NT, BLOCKED, ZP, HALF, W, true>(a, l, st);
+  return launch_with<WBITS, NL, NT, BLOCKED, ZP, HALF, W, false>(a, l, st);
 }
 
 template <int WBITS, int NL, bool BLOCKED, bool ZP, bool HALF>
@@ -599,6 +609,7 @@ Args make_args(int wbits, const void* x, int x_dt, const void* w, const Scales& 
   a.scale = sc.scale;
   a.zp = sc.zp;
   a.s_dt = sc.dt;
+  a.sc_pitch = N * (int64_t)dtype_size(sc.dt);
   a.out = out;
   a.N = N;
   a.K = K;

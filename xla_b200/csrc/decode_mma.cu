@@ -166,7 +166,7 @@ __device__ __forceinline__ float ar_ld_peer(const float* p) {
 // minus bias * sum(x), is added into the totals.
 template <int WBITS, typename XT, typename ST, int NT, int RG, int WARPS, bool AR = false>
 __global__ void __launch_bounds__(WARPS * 32)
-    decode_mma_kernel(const XT* __restrict__ x, const uint8_t* __restrict__ w, const ST* __restrict__ scale,
+    decode_mma_kernel(const XT* x, const uint8_t* __restrict__ w, const ST* scale,
                       void* __restrict__ out, int out_dt, int M, int64_t N, int64_t K, int steps_per_block,
                       int spb_shift, int blockwise, int gate_up, const ArParams ar, uint32_t* err_word) {
   // ar.wait_cycles bounds the wait for the peers' tiles (AR only)
@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(WARPS * 32)
       const uint4* xp = reinterpret_cast<const uint4*>(xrow[i] + (int64_t)step * VPS);
 #pragma unroll
       for (int q = 0; q < XREGS / 4; ++q) {
-        const uint4 v = __ldg(xp + q);  // an absent token reads token 0: its column is computed, never stored
+        const uint4 v = ld_ordered(xp + q);  // an absent token reads token 0: its column is computed, never stored
         dst[i][4 * q] = v.x;
         dst[i][4 * q + 1] = v.y;
         dst[i][4 * q + 2] = v.z;
@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(WARPS * 32)
       fold = sn >= steps || bn != b;
       if (fold) {
 #pragma unroll
-        for (int r = 0; r < 2 * RG; ++r) sc[r] = to_f32(__ldg(srow[r] + (int64_t)b * N));
+        for (int r = 0; r < 2 * RG; ++r) sc[r] = to_f32(ld_ordered(srow[r] + (int64_t)b * N));
       }
     }
     if (!kPrefetchX) load_x(s, xr);
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(WARPS * 32)
         float v = 0.f;
 #pragma unroll
         for (int wi = 0; wi < WARPS; ++wi) v += s_part[wi][row][tok];
-        if (!blockwise) v *= to_f32(__ldg(scale + n));
+        if (!blockwise) v *= to_f32(ld_ordered(scale + n));
         const size_t o = region + (size_t)tok * N + n;
 #pragma unroll
         for (int r = 0; r < kArMaxRanks; ++r)
@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(WARPS * 32)
       float v = 0.f;
 #pragma unroll
       for (int wi = 0; wi < WARPS; ++wi) v += s_part[wi][row][tok];
-      if (!blockwise) v *= to_f32(__ldg(scale + n));
+      if (!blockwise) v *= to_f32(ld_ordered(scale + n));
       if (!gate_up) {
         store_from_f32(out, (int64_t)tok * N + n, out_dt, v);
       } else if ((row & 8) == 0) {
@@ -459,7 +459,7 @@ __global__ void __launch_bounds__(WARPS * 32)
         float u = 0.f;
 #pragma unroll
         for (int wi = 0; wi < WARPS; ++wi) u += s_part[wi][row + 8][tok];
-        if (!blockwise) u *= to_f32(__ldg(scale + n + 8));
+        if (!blockwise) u *= to_f32(ld_ordered(scale + n + 8));
         store_from_f32(out, (int64_t)tok * (N >> 1) + gate_up_column(n), out_dt, silu_mul(v, u));
       }
     }
@@ -510,7 +510,7 @@ struct StagedStep {  // one K step of a warp in flight: 16 bytes of two weight r
 
 template <int WBITS, typename XT, typename ST, int NT, bool FOLD_EVERY>
 __global__ void __launch_bounds__(kStagedWarps * 32, 1)
-    decode_mma_staged_kernel(const XT* __restrict__ x, const uint8_t* __restrict__ w, const ST* __restrict__ scale,
+    decode_mma_staged_kernel(const XT* x, const uint8_t* __restrict__ w, const ST* scale,
                              void* __restrict__ out, int out_dt, int M, int N, int K, int steps_per_block,
                              int spb_shift, int blockwise, int tiles, int TR, int WK, int rounds, int gate_up) {
   constexpr int VPS = 512 / WBITS;            // weight values per row per step
@@ -608,28 +608,40 @@ __global__ void __launch_bounds__(kStagedWarps * 32, 1)
       sp1 += (int64_t)(wk >> spb_shift) * N;
       sstride = (int64_t)(WK >> spb_shift) * N;
     }
-    auto fetch = [&](int s, StagedStep<ST>& d) {
+    auto fetch_w = [&](int s, StagedStep<ST>& d) {
       if constexpr (FOLD_EVERY && kLateFetch) {
         d.w[0] = ld_stream_u4(wp0);
         d.w[1] = ld_stream_u4(wp1);
-        d.sc[0] = __ldg(sp0);
-        d.sc[1] = __ldg(sp1);
         if (s + WK < steps) {
           wp0 += wstride;
           wp1 += wstride;
-          sp0 += sstride;
-          sp1 += sstride;
         }
       } else {
         const int sf = min(s, last_step);
 #pragma unroll
         for (int r = 0; r < 2; ++r) d.w[r] = ld_stream_u4(wrow[r] + sf * 64);
+      }
+    };
+    auto fetch_sc = [&](int s, StagedStep<ST>& d) {
+      if constexpr (FOLD_EVERY && kLateFetch) {
+        d.sc[0] = ld_ordered(sp0);
+        d.sc[1] = ld_ordered(sp1);
+        if (s + WK < steps) {
+          sp0 += sstride;
+          sp1 += sstride;
+        }
+      } else {
+        const int sf = min(s, last_step);
         if (blockwise) {
           const int b = spb_shift >= 0 ? (sf >> spb_shift) : (sf / steps_per_block);
 #pragma unroll
-          for (int r = 0; r < 2; ++r) d.sc[r] = __ldg(srow[r] + (int64_t)b * N);
+          for (int r = 0; r < 2; ++r) d.sc[r] = ld_ordered(srow[r] + (int64_t)b * N);
         }
       }
+    };
+    auto fetch = [&](int s, StagedStep<ST>& d) {
+      fetch_w(s, d);
+      fetch_sc(s, d);
     };
     StagedStep<ST> qa, qb;
 #pragma unroll
@@ -802,13 +814,13 @@ __global__ void __launch_bounds__(kStagedWarps * 32, 1)
       if (otile < tiles && n < N && tok < M) {
         float v = 0.f;
         for (int j = 0; j < WK; ++j) v += red[((slot * WK + j) * ROWS_X + tok) * kRedPitch + row];
-        if (!blockwise) v *= to_f32(__ldg(scale + n));
+        if (!blockwise) v *= to_f32(ld_ordered(scale + n));
         if (!gate_up) {
           store_from_f32(out, (int64_t)tok * N + n, out_dt, v);
         } else if ((row & 8) == 0) {
           float u = 0.f;
           for (int j = 0; j < WK; ++j) u += red[((slot * WK + j) * ROWS_X + tok) * kRedPitch + row + 8];
-          if (!blockwise) u *= to_f32(__ldg(scale + n + 8));
+          if (!blockwise) u *= to_f32(ld_ordered(scale + n + 8));
           store_from_f32(out, (int64_t)tok * (N >> 1) + gate_up_column(n), out_dt, silu_mul(v, u));
         }
       }

@@ -98,6 +98,8 @@ struct Params {
   const void* scale;   // [N] or [S,N], of type s_dt
   const void* zp;      // like scale, or null
   int s_dt;
+  int64_t sc_pitch;    // bytes from one scale block to the next
+  uint32_t as_is;      // the byte permutation that changes nothing
   const float* xs;     // with zp: [S][xs_pitch] sums of the fixed-point activations over each scale block
   int xs_pitch;
   float zp_mul;        // factor that the weight bytes carry (16 for int4 weights)
@@ -248,7 +250,7 @@ constexpr int kMaxZpBlocks = 512;  // scale blocks of a weight with zero points
 // covers block_groups groups of eight values (a multiple of eight groups, or all of them); summed exactly in integers.
 // A row with a non-finite entry gets pw = NaN (its outputs are NaN); an all-zero row gets zeros.
 template <typename XT, int NL>
-__global__ void __launch_bounds__(1024) split_rows_kernel(const XT* __restrict__ x, int8_t* __restrict__ xl, float* __restrict__ pw,
+__global__ void __launch_bounds__(1024) split_rows_kernel(const XT* x, int8_t* __restrict__ xl, float* __restrict__ pw,
                                                           int64_t K, int perm4, float pw_mul, float* __restrict__ xs, int xs_pitch,
                                                           int block_groups) {
   __shared__ uint32_t s_max[32];
@@ -473,7 +475,7 @@ __device__ __forceinline__ void fold_regions_pipelined(uint32_t taddr, uint32_t 
   }
 }
 
-template <int WBITS, int NCOLS, int NL, bool ZP>
+template <int WBITS, int NCOLS, int NL, bool ZP, bool W16>
 __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NCOLS, NL>::kOcc)
     limb_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const Params p) {
   using C = Cfg<WBITS, NCOLS, NL>;
@@ -738,8 +740,13 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
     __shared__ float s_pw[2][64];
     static_assert(MT <= 64, "per-token factors of a tile");
     int frag = 0;
-    const int64_t sc_pitch = p.ld * (p.s_dt == QMM_F32 ? 4 : 2);
-    const ScaleWord word(p.s_dt, rl);
+    // a fetched scale's value: the fp32 bits, or a 16-bit value's
+    auto value = [&](uint32_t w) { return W16 ? scale_value(w, p.s_dt) : __uint_as_float(w); };
+    // A scale fetched one hand-over ahead, at the end of the current one.  The permutation is one that the compiler does not
+    // know: without it the value needs no register of its own, and the load moves down to behind the last use of its
+    // predecessor, a few hundred cycles before its own (int4 block 128, [57344,8192] and [8192,28672] at 64 tokens 224 us
+    // that way, 180 this way).
+    auto arrived = [&](uint32_t w) { return W16 ? value(w) : __uint_as_float(__byte_perm(w, 0u, p.as_is)); };
     auto wait_acc = [&]() {
       DBG_BEGIN();
       ptx::mbar_wait_warp<32>(&acc_full[buf], pacc, abort_flag, p.err_word, ptx::kErrWaitTmemFull);
@@ -766,8 +773,9 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
       // readers of one from the writers of its next use).  Fetched at the end they are two L2 round trips per tile.
       float* pw_s = s_pw[frag & 1];
       ++frag;
-      const float ps = (p.mode != kPerChannel || !n_ok || !first) ? 1.f : load_as_f32(p.scale, n, p.s_dt);
-      if (first && dt < MT) pw_s[dt] = it.y * MT + dt < p.M ? __ldg(p.pw + it.y * MT + dt) : 0.f;
+      const bool own_scale = p.mode == kPerChannel && n_ok && first;
+      const uint32_t ps_bits = own_scale ? load_scale_bits(p.scale, n, p.s_dt) : 0u;
+      if (first && dt < MT) pw_s[dt] = it.y * MT + dt < p.M ? ld_ordered(p.pw + it.y * MT + dt) : 0.f;
       float total[MTD];
 #pragma unroll
       for (int t = 0; t < MTD; ++t) total[t] = 0.f;
@@ -812,9 +820,10 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
       // Block scales are fetched one hand-over ahead, from clamped addresses, and change registers at its end.  (A longer
       // register queue does not fetch further ahead: its shift waits for the youngest load, and shifting twice per
       // hand-over put a whole memory round trip into each: int4 block 128 [28672,8192] at 512 tokens 363 us, now 337.)
-      const int64_t sc_off = scale_word_offset(min(n, p.N - 1), p.s_dt);
-      const uint8_t* scale_n = static_cast<const uint8_t*>(p.scale) + sc_off;
-      auto fetch_scale = [&](int b) { return __ldg(reinterpret_cast<const uint32_t*>(scale_n + min(b, p.S - 1) * sc_pitch)); };
+      using SBits = typename std::conditional<W16, unsigned short, uint32_t>::type;
+      const int64_t nc = min(n, p.N - 1);
+      const uint8_t* scale_n = static_cast<const uint8_t*>(p.scale) + nc * sizeof(SBits);
+      auto fetch_scale = [&](int b) -> uint32_t { return ld_ordered(reinterpret_cast<const SBits*>(scale_n + min(b, p.S - 1) * p.sc_pitch)); };
       if (C::kScaleRing > 0 && p.scale_ring) {
         // A hand-over here is shorter than a round trip to HBM, so the scales come eight blocks ahead, into a ring of the
         // thread's own (one hand-over ahead, in registers: int4 block 128 [57344,8192] 53.9 us at 4 tokens and 82.0 at 16,
@@ -824,9 +833,11 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
         const int b0 = p.mode == kBlockSlots ? u0 : s0 * per_slot, b1 = p.mode == kBlockSlots ? u1 : s1 * per_slot;
         const uint32_t* ring = scale_base + rl;
         const uint32_t ring_u32 = ptx::smem_u32(ring);
+        const uint8_t* word_n = static_cast<const uint8_t*>(p.scale) + scale_word_offset<W16>(nc);
+        auto copied = [&](int i) { return scale_in<W16>(ring + i * 128, rl, p.s_dt); };
         auto fetch = [&](int b) {
           // (a last slot may hold fewer blocks than the others: their sums are zero, but the factor has to be a number)
-          if (b < b1) cp_async4(ring_u32 + (uint32_t)(b % R) * 512, scale_n + min(b, p.S - 1) * sc_pitch);
+          if (b < b1) cp_async4(ring_u32 + (uint32_t)(b % R) * 512, word_n + min(b, p.S - 1) * p.sc_pitch);
           asm volatile("cp.async.commit_group;" ::: "memory");
         };
 #pragma unroll 1
@@ -836,7 +847,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
           for (int b = b0; b < b1; b += 2) {
             wait_acc();
             asm volatile("cp.async.wait_group %0;" ::"n"(R - 2) : "memory");
-            const float sc0 = word(ring[(b % R) * 128]), sc1 = word(ring[((b + 1) % R) * 128]);
+            const float sc0 = copied(b % R), sc1 = copied((b + 1) % R);
             const uint32_t a = lane_addr + buf * (2 * NCOLS) + col0;
             fold_region<DC, MTD, NL, true>(a, sc0, total, false, release);
             fold_region<DC, MTD, NL, true>(a + NCOLS, sc1, total, true, release);
@@ -849,7 +860,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
           for (int b = b0; b < b1; ++b) {
             wait_acc();
             asm volatile("cp.async.wait_group %0;" ::"n"(R - 1) : "memory");
-            const float sc = word(ring[(b % R) * 128]);
+            const float sc = copied(b % R);
             if (small) fold_region<DC, MTD, NL, true>(lane_addr + buf * NCOLS + col0, sc, total, true, release);
             else fold_region<DC, MTD, NL, false>(lane_addr + buf * NCOLS + col0, sc, total, true, release);
             next_acc();
@@ -858,48 +869,63 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");  // the ring is refilled from any place
       } else if (p.mode == kBlock128) {
-        uint32_t w0 = fetch_scale(2 * s0), w1 = fetch_scale(2 * s0 + 1);
-        for (int s = s0; s < s1; ++s) {
-          const float sc2[2] = {word(w0), word(w1)};
-          const uint32_t nx0 = fetch_scale(2 * s + 2), nx1 = fetch_scale(2 * s + 3);
-          if (C::kPair) {
+        if constexpr (C::kPair && C::kPipeDrain && W16) {
+          // two hand-overs ahead, in two sets of registers ([8192,8192] int8 at 200 tokens 68.8 us as below, 54.3 so)
+          uint32_t even[2] = {fetch_scale(2 * s0), fetch_scale(2 * s0 + 1)}, odd[2] = {fetch_scale(2 * s0 + 2), fetch_scale(2 * s0 + 3)};
+          auto step = [&](int s, uint32_t(&w)[2]) {
             wait_acc();
-            DBG_BEGIN();
-            const uint32_t a = lane_addr + buf * (2 * NCOLS) + col0;
-            if constexpr (C::kPipeDrain) {
-              fold_regions_pipelined<DC, MTD, NL, true, 2>(a, NCOLS, sc2, total, release);
-            } else {
-              fold_region<DC, MTD, NL, true>(a, sc2[0], total, false, release);
-              fold_region<DC, MTD, NL, true>(a + NCOLS, sc2[1], total, true, release);
-            }
-            DBG_END(1);
+            const float sc2[2] = {value(w[0]), value(w[1])};
+            fold_regions_pipelined<DC, MTD, NL, true, 2>(lane_addr + buf * (2 * NCOLS) + col0, NCOLS, sc2, total, release);
             next_acc();
-          } else {
-#pragma unroll 1
-            for (int h = 0; h < 2; ++h) {
+            w[0] = fetch_scale(2 * s + 4);
+            w[1] = fetch_scale(2 * s + 5);
+          };
+          for (int s = s0; s < s1; s += 2) {
+            step(s, even);
+            if (s + 1 < s1) step(s + 1, odd);
+          }
+        } else {
+          float sc2[2] = {value(fetch_scale(2 * s0)), value(fetch_scale(2 * s0 + 1))};
+          for (int s = s0; s < s1; ++s) {
+            const uint32_t nx0 = fetch_scale(2 * s + 2), nx1 = fetch_scale(2 * s + 3);
+            if (C::kPair) {
               wait_acc();
               DBG_BEGIN();
-              const float sc1[1] = {h ? sc2[1] : sc2[0]};
+              const uint32_t a = lane_addr + buf * (2 * NCOLS) + col0;
               if constexpr (C::kPipeDrain) {
-                fold_regions_pipelined<DC, MTD, NL, true, 1>(lane_addr + buf * NCOLS + col0, 0, sc1, total, release);
+                fold_regions_pipelined<DC, MTD, NL, true, 2>(a, NCOLS, sc2, total, release);
               } else {
-                fold_region<DC, MTD, NL, true>(lane_addr + buf * NCOLS + col0, sc1[0], total, true, release);
+                fold_region<DC, MTD, NL, true>(a, sc2[0], total, false, release);
+                fold_region<DC, MTD, NL, true>(a + NCOLS, sc2[1], total, true, release);
               }
               DBG_END(1);
               next_acc();
+            } else {
+#pragma unroll 1
+              for (int h = 0; h < 2; ++h) {
+                wait_acc();
+                DBG_BEGIN();
+                const float sc1[1] = {h ? sc2[1] : sc2[0]};
+                if constexpr (C::kPipeDrain) {
+                  fold_regions_pipelined<DC, MTD, NL, true, 1>(lane_addr + buf * NCOLS + col0, 0, sc1, total, release);
+                } else {
+                  fold_region<DC, MTD, NL, true>(lane_addr + buf * NCOLS + col0, sc1[0], total, true, release);
+                }
+                DBG_END(1);
+                next_acc();
+              }
             }
+            sc2[0] = arrived(nx0);
+            sc2[1] = arrived(nx1);
           }
-          w0 = nx0;
-          w1 = nx1;
         }
       } else {
         // hand-overs, and slots per hand-over in quarters (blocks of 64: one quarter)
         const int per = p.mode == kBlockSlots ? 4 * p.spu : (p.mode == kBlock64 ? 1 : 4 * (s1 - s0));
         int s = 4 * s0, b = p.mode == kBlockSlots ? s0 / p.spu : 4 * s0;
-        uint32_t w = p.mode == kPerChannel ? 0u : fetch_scale(b);
+        float sc = p.mode == kPerChannel ? 1.f : value(fetch_scale(b));
         while (s < 4 * s1) {
           const int g_end = s + per;
-          const float sc = p.mode == kPerChannel ? 1.f : word(w);
           const uint32_t nx = p.mode == kPerChannel ? 0u : fetch_scale(++b);
           wait_acc();
           DBG_BEGIN();
@@ -914,7 +940,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
           DBG_END(1);
           next_acc();
           s = g_end;
-          w = nx;
+          if (p.mode != kPerChannel) sc = arrived(nx);
         }
       }
       DBG_BEGIN();
@@ -959,32 +985,31 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
         if (warp == kDrainWarp0) { DBG_STAMP(16); }
       }
       drain_bar();  // the factors written at the top of the fragment are visible
-      float psv = ps;
+      float psv = own_scale ? scale_value(ps_bits, p.s_dt) : 1.f;
       if constexpr (ZP) {
         // the zero points' term, once per tile: minus sum_b zp[b,n] * xs[b,m], in units of the fixed point; every lane
         // reads the same token sums.  The zero points come from HBM and are fetched four blocks ahead.
         if (p.mode == kPerChannel) {
 #pragma unroll
-          for (int t = 0; t < MTD; ++t) total[t] *= ps;
+          for (int t = 0; t < MTD; ++t) total[t] *= psv;
           psv = 1.f;
         }
-        const uint8_t* zp = static_cast<const uint8_t*>(p.zp) + sc_off;
-        // (one block: a single value, which need not lie in a word of the tensor)
-        auto fetch_zp = [&](int b) {
-          return p.mode == kPerChannel ? __float_as_uint(load_as_f32(p.zp, min(n, p.N - 1), p.s_dt))
-                                       : __ldg(reinterpret_cast<const uint32_t*>(zp + min(b, p.S - 1) * sc_pitch));
+        // (per channel the instance for fp32 serves all types)
+        const uint8_t* zp = static_cast<const uint8_t*>(p.zp) + nc * sizeof(SBits);
+        auto fetch_zp = [&](int b) -> uint32_t {
+          return p.mode == kPerChannel ? load_scale_bits(p.zp, nc, p.s_dt) : ld_ordered(reinterpret_cast<const SBits*>(zp + min(b, p.S - 1) * p.sc_pitch));
         };
         uint32_t zq[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) zq[i] = fetch_zp(i);
         const float* xs = p.xs + mt0;
         for (int b = 0; b < p.S; ++b, xs += p.xs_pitch) {
-          const float z = -p.zp_mul * (p.mode == kPerChannel ? __uint_as_float(zq[0]) : word(zq[0]));
+          const float z = -p.zp_mul * (p.mode == kPerChannel ? scale_value(zq[0], p.s_dt) : value(zq[0]));
 #pragma unroll
           for (int i = 0; i < 3; ++i) zq[i] = zq[i + 1];
           zq[3] = fetch_zp(b + 4);
 #pragma unroll
-          for (int t = 0; t < MTD; ++t) total[t] = fmaf(z, __ldg(xs + t), total[t]);
+          for (int t = 0; t < MTD; ++t) total[t] = fmaf(z, ld_ordered(xs + t), total[t]);
         }
       }
       float pwv[MTD];
@@ -1167,10 +1192,10 @@ Scratch carve(void* base, int64_t M, int64_t K, int nl, int partial_tokens, int 
   return s;
 }
 
-template <int WBITS, int NCOLS, int NL = 3, bool ZP = false>
-int launch_cfg(const CUtensorMap& map_w, const CUtensorMap& map_x, const Params& p, int grid, cudaStream_t st) {
+template <int WBITS, int NCOLS, int NL, bool ZP, bool W16>
+int launch_with(const CUtensorMap& map_w, const CUtensorMap& map_x, const Params& p, int grid, cudaStream_t st) {
   using C = Cfg<WBITS, NCOLS, NL>;
-  auto kern = limb_tc_kernel<WBITS, NCOLS, NL, ZP>;
+  auto kern = limb_tc_kernel<WBITS, NCOLS, NL, ZP, W16>;
   static bool attr_set[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -1195,6 +1220,12 @@ int launch_cfg(const CUtensorMap& map_w, const CUtensorMap& map_x, const Params&
     return fail(QMM_ERR_LAUNCH, "limb_tc_kernel launch: %s", cudaGetErrorString(e));
   }
   return check_launch("limb_tc_kernel");
+}
+
+template <int WBITS, int NCOLS, int NL = 3, bool ZP = false>
+int launch_cfg(const CUtensorMap& map_w, const CUtensorMap& map_x, const Params& p, int grid, cudaStream_t st) {
+  return p.mode != kPerChannel && p.s_dt != QMM_F32 ? launch_with<WBITS, NCOLS, NL, ZP, true>(map_w, map_x, p, grid, st)
+                                                    : launch_with<WBITS, NCOLS, NL, ZP, false>(map_w, map_x, p, grid, st);
 }
 
 template <int WBITS>
@@ -1476,6 +1507,8 @@ int launch_limb_impl(int wbits, const void* x, int x_dt, const void* w, const Sc
   p.xs_pitch = sc.xs_pitch;
   p.zp_mul = 1.f / pw_mul;
   p.s_dt = scales.dt;
+  p.as_is = 0x3210u;
+  p.sc_pitch = N * (int64_t)dtype_size(scales.dt);
   p.out_dt = out_dt;
   p.M = (int)M;
   p.ld = N;

@@ -53,6 +53,7 @@ struct Params {
   const void* scale;   // [N] or [S,N], of type s_dt
   const void* zp;      // like scale, or null
   int s_dt;
+  int64_t sc_pitch;    // bytes from one scale block to the next
   const float* xs;     // with zp: [S][xs_pitch] sums of the activations over each scale block
   int xs_pitch;
   void* out;
@@ -208,7 +209,7 @@ __device__ __forceinline__ void reg_dec() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS));
 }
 
-template <int WBITS, typename XT, int NC, int KS>
+template <int WBITS, typename XT, int NC, int KS, bool W16>
 __global__ void __launch_bounds__(kThreads, 1)
     tmem_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const Params p) {
   using C = Cfg<WBITS, NC, KS>;
@@ -419,7 +420,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     __shared__ int s_npart;
     const uint32_t* my_scale = s_scale + dt;
     const uint32_t my_scale_u32 = ptx::smem_u32(my_scale);
-    const ScaleWord word(p.s_dt, rl);
+    auto value = [&](int i) { return scale_in<W16, XT>(my_scale + i * kDrain, rl, p.s_dt); };
     bool waited = false;
     FragIter it(p);
     int buf = 0;
@@ -436,14 +437,14 @@ __global__ void __launch_bounds__(kThreads, 1)
       // Block scales and zero points are a stream of their own (a round trip to HBM each): every thread copies its own
       // row's, seven folds ahead, into a ring of its own.  (Held in registers that shift from fold to fold, the shift
       // waits for the load of the fold before, whatever the nominal distance.)
-      const int64_t sc_off = scale_word_offset(min(n, p.N - 1), p.s_dt), sc_pitch = p.N * (p.s_dt == QMM_F32 ? 4 : 2);
+      const int64_t sc_off = scale_word_offset<W16>(min(n, p.N - 1));
       const uint8_t* scp = static_cast<const uint8_t*>(p.scale) + sc_off;
       const uint8_t* zpp = static_cast<const uint8_t*>(p.zp) + sc_off;
       auto fetch = [&](int f) {
         if (p.blocked && f < it.u1) {
           const uint32_t dst = my_scale_u32 + (uint32_t)(f % kScaleRing) * (kDrain * 4);
-          cp_async4(dst, scp + f * sc_pitch);
-          if (p.zp) cp_async4(dst + kScaleRing * kDrain * 4, zpp + f * sc_pitch);
+          cp_async4(dst, scp + f * p.sc_pitch);
+          if (p.zp) cp_async4(dst + kScaleRing * kDrain * 4, zpp + f * p.sc_pitch);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
       };
@@ -467,7 +468,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         uint32_t r[2][16];
         ptx::tmem_ld_32x32b_x16(a, r[0]);
         asm volatile("cp.async.wait_group %0;" ::"n"(kScaleRing - 1) : "memory");
-        const float sc = p.blocked ? word(my_scale[(f % kScaleRing) * kDrain]) : 1.f;
+        const float sc = p.blocked ? value(f % kScaleRing) : 1.f;
 #pragma unroll
         for (int c = 0; c < DT / 16; ++c) {
           uint32_t* cur = r[c & 1];
@@ -488,11 +489,11 @@ __global__ void __launch_bounds__(kThreads, 1)
           pacc ^= 1;
         }
         if (p.blocked && p.zp) {
-          const float z = -word(my_scale[(kScaleRing + f % kScaleRing) * kDrain]);
+          const float z = -value(kScaleRing + f % kScaleRing);
           const float* xs = p.xs + (int64_t)f * p.xs_pitch + m0;  // the same for all lanes; the pitch covers whole tiles
 #pragma unroll
           for (int t = 0; t < DT; t += 4) {
-            const float4 v = __ldg(reinterpret_cast<const float4*>(xs + t));
+            const float4 v = ld_ordered(reinterpret_cast<const float4*>(xs + t));
             total[t] = fmaf(z, v.x, total[t]);
             total[t + 1] = fmaf(z, v.y, total[t + 1]);
             total[t + 2] = fmaf(z, v.z, total[t + 2]);
@@ -530,8 +531,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         drain_bar();
       }
-      const float ps = p.blocked || !n_ok ? 1.f : load_as_f32(p.scale, n, p.s_dt);
-      const float z1 = !p.blocked && p.zp && n_ok ? -load_as_f32(p.zp, n, p.s_dt) : 0.f;
+      const float ps = p.blocked || !n_ok ? 1.f : scale_value(load_scale_bits(p.scale, n, p.s_dt), p.s_dt);
+      const float z1 = !p.blocked && p.zp && n_ok ? -scale_value(load_scale_bits(p.zp, n, p.s_dt), p.s_dt) : 0.f;
 #pragma unroll 1
       for (int c = 0; c < DT / 16; ++c) {
         const int l0 = grp * DT + 16 * c;  // token inside the item
@@ -556,7 +557,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
             for (int t = 0; t < 16; ++t) {
               total[t] *= ps;
-              if (p.zp && t < count) total[t] = fmaf(z1, __ldg(p.xs + m0 + 16 * c + t), total[t]);
+              if (p.zp && t < count) total[t] = fmaf(z1, ld_ordered(p.xs + m0 + 16 * c + t), total[t]);
             }
           }
           const int64_t row_out = m0 + 16 * c;
@@ -601,7 +602,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 // Sums of the activations over each scale block, for the zero points: xs[b * pitch + m], one warp per (token, block);
 // tokens from M up to the pitch get zeros.
 template <typename XT>
-__global__ void __launch_bounds__(256) block_sums_kernel(const XT* __restrict__ x, float* __restrict__ xs, int pitch, int M, int K, int S) {
+__global__ void __launch_bounds__(256) block_sums_kernel(const XT* x, float* __restrict__ xs, int pitch, int M, int K, int S) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const int lane = threadIdx.x & 31;
@@ -637,10 +638,10 @@ cudaError_t launch_pdl(Kernel kern, unsigned grid, unsigned block, size_t smem, 
   return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
-template <int WBITS, typename XT, int NC, int KS>
-int launch_cfg(const CUtensorMap& map_w, const CUtensorMap& map_x, const Params& p, int grid, cudaStream_t st) {
+template <int WBITS, typename XT, int NC, int KS, bool W16>
+int launch_with(const CUtensorMap& map_w, const CUtensorMap& map_x, const Params& p, int grid, cudaStream_t st) {
   using C = Cfg<WBITS, NC, KS>;
-  auto kern = tmem_gemm_kernel<WBITS, XT, NC, KS>;
+  auto kern = tmem_gemm_kernel<WBITS, XT, NC, KS, W16>;
   static bool attr_set[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -655,6 +656,12 @@ int launch_cfg(const CUtensorMap& map_w, const CUtensorMap& map_x, const Params&
     return fail(QMM_ERR_LAUNCH, "tmem_gemm_kernel launch: %s", cudaGetErrorString(e));
   }
   return QMM_OK;
+}
+
+template <int WBITS, typename XT, int NC, int KS>
+int launch_cfg(const CUtensorMap& map_w, const CUtensorMap& map_x, const Params& p, int grid, cudaStream_t st) {
+  return p.blocked && p.s_dt != QMM_F32 ? launch_with<WBITS, XT, NC, KS, true>(map_w, map_x, p, grid, st)
+                                        : launch_with<WBITS, XT, NC, KS, false>(map_w, map_x, p, grid, st);
 }
 
 template <int WBITS, typename XT>
@@ -736,7 +743,8 @@ bool tmem_gemm_supported(int wbits, int64_t M, int64_t N, int64_t K, int64_t blo
 int launch_tmem_gemm(int wbits, const void* x, int x_dt, const void* w, const Scales& scales, void* out, int out_dt, int64_t M, int64_t N,
                      int64_t K, int64_t block_size, int gate_up, void* workspace, size_t workspace_bytes, cudaStream_t st) {
   const bool zp = scales.zp != nullptr;
-  if (!tmem_gemm_supported(wbits, M, N, K, block_size, x, x_dt, w) || !scale_words_ok(scales, N, block_size))
+  if (!tmem_gemm_supported(wbits, M, N, K, block_size, x, x_dt, w) || !scale_words_ok(scales, N, block_size) ||
+      (block_size > 0 && scales.dt != QMM_F32 && scales.dt != x_dt))
     return fail(QMM_ERR_UNSUPPORTED,
                 "tensor-memory kernel: needs an sm_100 device, bf16/f16 activations, 16-byte row pitches, block_size 64 or a "
                 "multiple of 128, 16-byte aligned x/w (M=%lld N=%lld K=%lld bs=%lld)",
@@ -754,6 +762,7 @@ int launch_tmem_gemm(int wbits, const void* x, int x_dt, const void* w, const Sc
   p.scale = scales.scale;
   p.zp = scales.zp;
   p.s_dt = scales.dt;
+  p.sc_pitch = N * (int64_t)dtype_size(scales.dt);
   p.xs = sc.xs;
   p.xs_pitch = sc.xs_pitch;
   p.out = out;
