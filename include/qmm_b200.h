@@ -15,6 +15,10 @@
  *   - Every function returns a qmm_status; 0 is success.  No exception or abort crosses the ABI.
  *     qmm_last_error_string() gives a per-thread description of the last failure.
  *   - There is no CPU fallback: a call that cannot run on the current device fails with a status.
+ *   - Kernels are launched with programmatic stream serialization and read their first weight bytes while the kernel in
+ *     front of them on the stream may still run.  So that kernel must not be the one that writes the weights: put any other
+ *     launch, or a synchronisation, between the two.  (The packing functions below are such kernels.)  Every other operand
+ *     may come from the kernel directly in front.
  *   - `variant` picks the kernel family; QMM_VARIANT_AUTO chooses by shape.  A variant that
  *     cannot take the given shape fails with QMM_ERR_UNSUPPORTED rather than running another one.
  */

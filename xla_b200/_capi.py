@@ -174,6 +174,14 @@ def workspace(device, max_M, K, N=0, wbits=8):
   return p.value, n.value
 
 
+def settled(w):
+  """`w`, a weight that has just been written on the current stream, with one more launch behind it: the linears read their
+  first weights while the kernel in front of them may still run, so that kernel must not be the one that writes them."""
+  if w.is_cuda:
+    torch.zeros(1, device=w.device)
+  return w
+
+
 def check(status):
   """Turns a non-zero qmm_status into the Python exception the reference would raise."""
   if status == 0:

@@ -86,13 +86,17 @@ __device__ __forceinline__ void store_from_f32(void* p, int64_t i, int dt, float
 }
 
 // ---- data of earlier kernels (device) --------------------------------------------------------
-// A kernel launched with programmatic stream serialization starts while the kernel before it still runs.  What
-// it may have written is read with ordinary loads: __ldg and const __restrict__ stand for data that nobody writes
+// A kernel launched with programmatic stream serialization starts while the kernel before it still runs.  Only the raw
+// weights, which no kernel directly in front may write, are read before griddepcontrol.wait; activations, scratch, scales
+// and zero points come after it, and with ordinary loads: __ldg and const __restrict__ stand for data that nobody writes
 // while the kernel runs, so such a load may be moved ahead of the wait or served from a stale cache line.
 template <typename T>
 __device__ __forceinline__ T ld_ordered(const T* p) {
   return *p;
 }
+
+// Brings a line into L2, where all SMs see the same data: allowed ahead of the wait for data that is loaded after it.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // ---- weight scales and zero points ---------------------------------------------------------
 // In fp32 or in a 16-bit type (the buffers of a quantized 16-bit model), both in the same one.

@@ -283,9 +283,23 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 2 : 1) decode_i8_kernel(const
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
 #pragma unroll
-  for (int d = 0; d < D - 1; ++d) issue(true);
-  // The weights are static: their first loads run under the kernel before this one.  The activations, and every store
+  for (int d = 0; d < D - 1; ++d) issue(false);
+  // The weights are static: their first loads run under the kernel before this one.  Scales, activations, and every store
   // of this kernel, come after the wait.
+  auto first_scales = [&](auto take) {
+    int step = piece_first, scale_tile = t0 + lo / SP;
+#pragma unroll 1
+    for (int d = 0; d < min(D - 1, hi - lo); ++d) {
+      take(ring + d * kSlot, scale_row(scale_tile), step);
+      if (++step == SP) {
+        step = 0;
+        ++scale_tile;
+      }
+    }
+  };
+  if constexpr (BLOCKED) first_scales([&](uint32_t, const uint8_t* row, int step) {
+    prefetch_l2(row + (HALF ? 2 * step : p.fold_shift >= 0 ? step >> p.fold_shift : step / p.fold_steps) * p.sc_pitch);
+  });
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   {
@@ -294,11 +308,14 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 2 : 1) decode_i8_kernel(const
     for (int o = threadIdx.x * 16; o < bytes; o += kThreads * 16)
       cp_async16((uint32_t)__cvta_generic_to_shared(raw + o), reinterpret_cast<const uint8_t*>(p.x) + o);
     asm volatile("cp.async.commit_group;" ::: "memory");
+    // the first steps' scales, behind the weights under way, are waited for when the activations have been split
+    if constexpr (BLOCKED) first_scales(copy_scales);
+    asm volatile("cp.async.commit_group;" ::: "memory");
     if (threadIdx.x < kMaxTokens * 2) s_max[threadIdx.x] = 0;
     if (ZP)
       for (int i = threadIdx.x; i < p.S * cols; i += kThreads) s_xs[i] = 0;
-    // groups complete in order: this one last, the weights' first steps with it
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    // groups complete in order: the activations' with the weights' first steps
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncthreads();
     if (p.x_dt == QMM_BF16)
       stage_activations<WBITS, NL, ZP, kThreads>(p, xs, reinterpret_cast<const __nv_bfloat16*>(raw), s_pw, s_xs, s_max);
@@ -381,6 +398,7 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 2 : 1) decode_i8_kernel(const
     }
   };
 
+  asm volatile("cp.async.wait_group 0;" ::: "memory");  // the first scales
   int cs = piece_first, tile = lo / SP;  // compute position
   const uint8_t* cring = smem + p.ring_off + warp * (D * kSlot);
   int cslot = 0;

@@ -650,11 +650,16 @@ __global__ void __launch_bounds__(kStagedWarps * 32, 1)
       qa.sc[r] = qb.sc[r] = from_f32<ST>(1.f);
     }
     if (active && wk < steps) {
-      fetch(wk, qa);
-      fetch(wk + WK, qb);
+      fetch_w(wk, qa);
+      fetch_w(wk + WK, qb);
+      if (first && blockwise) {
+        const int b = spb_shift >= 0 ? (wk >> spb_shift) : (wk / steps_per_block);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) prefetch_l2(srow[r] + (int64_t)b * N);
+      }
     }
     if (first) {
-      // weights are static: their first loads may overlap the previous kernel of the stream; the
+      // weights are static: their first loads may overlap the previous kernel of the stream; the scales, the
       // activations and every store of this kernel come after the wait
       asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
       asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -662,6 +667,10 @@ __global__ void __launch_bounds__(kStagedWarps * 32, 1)
     }
     issue_chunk(0);
     if (nchunks > 1) issue_chunk(1);
+    if (active && wk < steps) {
+      fetch_sc(wk, qa);
+      fetch_sc(wk + WK, qb);
+    }
 
     float total[NT][4], part[NT][4];
 #pragma unroll

@@ -448,12 +448,20 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
       };
-#pragma unroll 1
-      for (int f = 0; f < kScaleRing - 1; ++f) fetch(it.u0 + f);
       if (!waited) {
-        asm volatile("griddepcontrol.wait;" ::: "memory");  // block sums, scratch and `out` belong to earlier kernels until here
+        if (p.blocked) {
+#pragma unroll 1
+          for (int f = it.u0; f < min(it.u0 + kScaleRing - 1, it.u1); ++f) {
+            prefetch_l2(scp + f * p.sc_pitch);
+            if (p.zp) prefetch_l2(zpp + f * p.sc_pitch);
+          }
+        }
+        // scales (a conversion may be the kernel in front), block sums, scratch and `out` belong to earlier kernels until here
+        asm volatile("griddepcontrol.wait;" ::: "memory");
         waited = true;
       }
+#pragma unroll 1
+      for (int f = 0; f < kScaleRing - 1; ++f) fetch(it.u0 + f);
       for (int f = it.u0; f < it.u1; ++f) {
         fetch(f + kScaleRing - 1);
         if (p.fu == 1) {

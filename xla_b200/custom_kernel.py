@@ -34,7 +34,7 @@ def quantized_matmul_int8(x, w, scalar, zero_point=None, quant_block_size=None,
   x2 = _qm._rows(x)
   M, K = x2.shape
   N = w.shape[0]
-  w = w if w.is_contiguous() else w.contiguous()
+  w = w if w.is_contiguous() else _capi.settled(w.contiguous())
   s32 = _qm._f32(scalar)
   with torch.cuda.device(x.device):
     if quantize_activation:

@@ -72,7 +72,7 @@ def quantized_gate_up(x, w, scaler, block_size=-1, int4_weight=False, weight_is_
   if fused:
     expect = (N2,) if block_size == -1 else (K // block_size, N2)
     assert tuple(s32.shape) == expect, f"weight scaler shape is expect to be {list(expect)}, got {list(s32.shape)}."
-    wc = w if w.is_contiguous() else w.contiguous()
+    wc = w if w.is_contiguous() else _capi.settled(w.contiguous())
 
     def run():
       out = torch.empty((M, N2 // 2), dtype=out_dtype, device=x.device)
@@ -89,7 +89,7 @@ def quantized_gate_up(x, w, scaler, block_size=-1, int4_weight=False, weight_is_
       # larger batches: the split-activation tensor-core kernel applies silu(gate) * up in its drain
       expect = (N2,) if block_size == -1 else (K // block_size, N2)
       assert tuple(s32.shape) == expect, f"weight scaler shape is expect to be {list(expect)}, got {list(s32.shape)}."
-      wc = w if w.is_contiguous() else w.contiguous()
+      wc = w if w.is_contiguous() else _capi.settled(w.contiguous())
 
       def run():
         ws, ws_bytes = _capi.workspace(x.device, M, K)

@@ -43,7 +43,7 @@ def pack_int4(w, layout="nk"):
       _capi.check(L.qmm_pack_int4_sbn(_capi.ptr(w), _capi.ptr(out), s, bs, n, _capi.stream_ptr(w.device)))
     else:
       raise ValueError(f"unknown layout {layout!r}")
-  return out
+    return _capi.settled(out)
 
 
 def unpack_int4(wp):
@@ -103,7 +103,7 @@ def quantized_matmul_packed(x, w, scaler, zero_point=None, block_size=-1, int4_w
     out_dtype = _qm._out_dtype(x, scaler, zero_point)
   x2 = _qm._rows(x)
   M = x2.shape[0]
-  w = w if w.is_contiguous() else w.contiguous()
+  w = w if w.is_contiguous() else _capi.settled(w.contiguous())
   s32, zp32 = _qm._f32(scaler), _qm._f32(zero_point)
   L = _capi.lib()
   variant = _capi.VARIANTS[_qm.current_variant()]

@@ -17,6 +17,8 @@ operator; the CPU tests of the sharding arithmetic pass the CPU oracle instead.
 import torch
 import torch.distributed as dist
 
+from . import _capi
+
 
 def _world(group=None):
   if dist.is_available() and dist.is_initialized():
@@ -49,9 +51,9 @@ def shard_row(w, scaler, zero_point, rank, world, in_features, block_size=-1, we
     assert kl % block_size == 0, f"each rank's K slice ({kl}) must hold whole blocks of {block_size}"
   if weight_is_packed:
     assert kl % 2 == 0
-    wl = w[:, rank * kl // 2:(rank + 1) * kl // 2].contiguous()
+    wl = _capi.settled(w[:, rank * kl // 2:(rank + 1) * kl // 2].contiguous())
   else:
-    wl = w[:, rank * kl:(rank + 1) * kl].contiguous()
+    wl = _capi.settled(w[:, rank * kl:(rank + 1) * kl].contiguous())
   if block_size == -1:
     return wl, scaler, zero_point  # per-channel scale/zero point apply to every rank's partial
   sl = kl // block_size
