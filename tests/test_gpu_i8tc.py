@@ -276,3 +276,33 @@ def test_long_int4_weights(M, bs):
   rows = torch.cat([torch.arange(300), torch.arange(N - 300, N)])
   exact = _exact(x, w[rows], s[..., rows], bs)
   assert qo.max_abs_rel(out[:, rows.to(DEV)], exact) < TOL_BF16
+
+
+@pytest.mark.parametrize("variant", ["i8tc", "tmem"])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("wbits,bs", [(4, 128), (8, -1)])
+def test_a_workspace_of_the_stated_size_suffices(variant, out_dtype, wbits, bs):
+  """qmm_weight_only with exactly qmm_weight_only_workspace_size(M, K) bytes, at both ends of every token tile's range."""
+  from xla_b200 import _capi
+  L = _capi.lib()
+  g = qc.gen(5)
+  N, K = 640, 4096
+  w = (qc.int4_weight if wbits == 4 else qc.int8_weight)(g, N, K).to(DEV)
+  wk = xla_b200.pack_int4(w) if wbits == 4 else w
+  s = (qc.per_channel_scale(g, N) if bs == -1 else qc.blockwise_scale(g, K // bs, N)).to(DEV)
+  xs = qc.activations(g, 200, K).to(DEV)
+  for M in (1, 5, 6, 10, 11, 16, 17, 29, 32, 33, 40, 42, 43, 60, 64, 65, 200):
+    x = xs[:M].contiguous()
+    nbytes = L.qmm_weight_only_workspace_size(M, K)
+    ws = torch.zeros(nbytes + 256, dtype=torch.uint8, device=DEV)
+    ws[nbytes:] = 77
+    out = torch.empty(M, N, dtype=out_dtype, device=DEV)
+    with torch.cuda.device(0):
+      _capi.check(L.qmm_weight_only(wbits, x.data_ptr(), _capi.BF16, wk.data_ptr(), s.data_ptr(), None, out.data_ptr(),
+                                    _capi.dtype_code(out_dtype), M, N, K, bs, _capi.VARIANTS[variant], ws.data_ptr(), nbytes,
+                                    _capi.stream_ptr(DEV)))
+    assert (ws[nbytes:] == 77).all()
+    with xla_b200.force_variant(variant):
+      ref = torch.ops.xla_b200.quantized_matmul_packed(x, wk, s, block_size=bs, int4_weight=wbits == 4, weight_is_packed=wbits == 4,
+                                                       out_dtype=out_dtype)
+    assert torch.equal(out, ref), M

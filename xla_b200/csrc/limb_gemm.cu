@@ -1365,8 +1365,10 @@ void limb_tc_set_limbs(int limbs) { g_limb_policy.store(limbs == 3 ? 3 : 0, std:
 size_t limb_tc_workspace_bytes(int64_t M, int64_t K) {
   if (M < 1 || K < 1) return 0;
   // Enough for either limb form (the output type is not known here) and for every batch up to M: the limbs of the
-  // longest chunk, and the partial tiles of the widest stream-K batch that is not longer than M.
-  return carve(nullptr, std::min(M, max_rows(3)), K, 3, (int)std::min<int64_t>(M, 64), kLimbMaxCtas).bytes;
+  // longest chunk, and partial tiles as wide as plan_for makes them for any batch up to M (they are whole tiles, wider
+  // than the batch itself).
+  const int tile_tokens = M <= 16 ? 16 : 64;
+  return carve(nullptr, std::min(M, max_rows(3)), K, 3, tile_tokens, kLimbMaxCtas).bytes;
 }
 
 bool limb_tc_shape_ok(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_size, int x_dt, bool has_zp) {
