@@ -392,8 +392,9 @@ QMM_API int qmm_host_pipeline_sync(void* pipeline);
 QMM_API int qmm_host_pipeline_destroy(void* pipeline);
 
 /*
- * Device-side error word of the current device.  Kernels that wait on hardware barriers give up
- * after a bounded number of polls and record a non-zero code here instead of hanging.
+ * Device-side error word of the current device.  Kernels that wait on hardware barriers, or for the partial sums of
+ * another CTA, give up after a while, store NaN (int32 accumulators: what is there) and record a non-zero code here
+ * instead of hanging.
  * Reads the word back (this call synchronises `stream`), stores it in *flag (HOST pointer) and
  * clears it.  Returns QMM_ERR_TIMEOUT if it was non-zero.
  */
@@ -413,10 +414,11 @@ QMM_API int qmm_device_error_flag(uint32_t* flag, void* stream);
 QMM_API int qmm_set_activation_limbs(int limbs);
 
 /*
- * How long the kernels that wait for another GPU (qmm_allreduce_oneshot, qmm_rowparallel_decode) keep waiting
- * before they give up: `seconds` of SM clock at about 2 GHz, in (0, 60]; the default is about one second.  On
- * expiry the kernel sets the device error word (code 7: all-reduce kernel, 8: fused decode exchange; the peer's
- * rank in bits 8 and up), fills its result with NaN and returns; the context stays usable.  Process-wide; applies
+ * How long the kernels that wait for another GPU (qmm_allreduce_oneshot, qmm_rowparallel_decode), or for the partial
+ * sums of another CTA of the same launch (QMM_VARIANT_I8TC, QMM_VARIANT_TMEM), keep waiting before they give up:
+ * `seconds` of SM clock at about 2 GHz, in (0, 60]; the default is about one second.  On expiry the kernel sets the
+ * device error word (code 7: all-reduce kernel, 8: fused decode exchange, with the peer's rank in bits 8 and up; 9 and
+ * 10: partial sums in I8TC and TMEM, with the CTA), fills its result with NaN and returns; the context stays usable.  Process-wide; applies
  * to launches made after the call.  Stands in for the reference's collective timeouts, which live in the PJRT
  * runtime (torch_xla/csrc/runtime/), not in this operator.
  */

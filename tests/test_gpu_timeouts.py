@@ -2,7 +2,8 @@
 sets and a wait limit of a few milliseconds.  The kernel must return, fill its result with NaN, leave the code of the
 wait in the device error word, and the context must stay usable.  Nothing here faults or hangs a GPU.
 
-The waits are the ones of the two kernels that wait for another GPU (one-shot all-reduce over peer memory, row-parallel
+The waits are the ones for the partial sums of another CTA (the flag words of the scratch hold a value that no CTA
+writes), and of the two kernels that wait for another GPU (one-shot all-reduce over peer memory, row-parallel
 decode with the exchange in its epilogue); on one GPU the "peer" is a second buffer of the same device whose flag
 stays zero.
 """
@@ -86,3 +87,37 @@ def test_fused_rowparallel_decode_gives_up_when_a_peer_never_signals(short_wait)
   # the library still works on this device
   y = torch.ops.xla.quantized_matmul(x, w, s)
   assert torch.isfinite(y).all()
+
+
+@pytest.mark.parametrize("variant,code", [("i8tc", 9), ("tmem", 10)])
+@pytest.mark.parametrize("wbits,bs,M", [(4, 128, 40), (8, -1, 29), (4, 128, 200)])
+def test_partial_sums_that_never_come(short_wait, variant, code, wbits, bs, M):
+  """Weight tiles split along K over several CTAs; the flags of their partial tiles are in a state that no CTA leaves."""
+  L = short_wait
+  g = qc.gen(M)
+  N, K = 3840, 8192
+  x = qc.activations(g, M, K).to(DEV)
+  w = (qc.int4_weight if wbits == 4 else qc.int8_weight)(g, N, K).to(DEV)
+  w = xla_b200.pack_int4(w) if wbits == 4 else w
+  s = (qc.per_channel_scale(g, N) if bs == -1 else qc.blockwise_scale(g, K // bs, N)).to(DEV)
+  nbytes = L.qmm_weight_only_workspace_size(M, K)
+  ws = torch.zeros(nbytes, dtype=torch.uint8, device=DEV)
+
+  def run():
+    out = torch.zeros(M, N, device=DEV)
+    with torch.cuda.device(0):
+      _capi.check(L.qmm_weight_only(wbits, x.data_ptr(), _capi.BF16, w.data_ptr(), s.data_ptr(), None, out.data_ptr(), _capi.F32, M, N, K,
+                                    bs, _capi.VARIANTS[variant], ws.data_ptr(), nbytes, _capi.stream_ptr(DEV)))
+    torch.cuda.synchronize()
+    return out
+
+  want = run()
+  assert _capi.device_error(DEV) == 0 and torch.isfinite(want).all()
+  assert not ws[:2048].any()  # the flags are idle again
+  ws[:2048].view(torch.int32).fill_(7)
+  lost = run()
+  assert _capi.device_error(DEV) & 0xff == code
+  assert torch.isnan(lost).any()
+  assert torch.equal(lost[~torch.isnan(lost)], want[~torch.isnan(lost)])
+  ws[:2048].zero_()
+  assert torch.equal(run(), want) and _capi.device_error(DEV) == 0

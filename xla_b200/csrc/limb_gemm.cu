@@ -121,6 +121,7 @@ struct Params {
   float* partial;   // [grid][MT][128] fp32
   uint32_t* flags;  // [grid], zero between launches
   uint32_t* err_word;
+  long long wait_cycles;  // for a partial tile
   int gate_up;
   int ytiles;    // token tiles per weight tile (1 up to one tile's tokens); a work item is a (weight tile, token tile) pair
   // The schedule: the first `items1` items go to the CTAs whole (CTA c takes items c, c + G, ...); the K units of
@@ -226,14 +227,6 @@ __device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, ui
 }
 __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void st_release_gpu(uint32_t* p, uint32_t v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-__device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
-  uint32_t v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
 }
 
 __device__ __forceinline__ float silu_mul(float gate, float up) { return gate / (1.f + expf(-gate)) * up; }
@@ -802,8 +795,11 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
           for (int t = 0; t < MTD; ++t)
             if (t < mcount) total[t] += __ldcg(src + j * kTile + t * BMW);
         }
-        drain_bar();
-        for (int j = dt; j < np; j += kDT) p.flags[blockIdx.x + 1 + j] = 0u;  // clean for the next launch
+      };
+      auto lost = [&]() {  // a wait ran out: NaN, not what is there
+        if (*abort_flag == 0) return;
+#pragma unroll
+        for (int t = 0; t < MTD; ++t) total[t] = __uint_as_float(0x7fc00000u);
       };
       if (first && !last) {
         if (dt == 0) {
@@ -949,17 +945,15 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
         // a later K range of a tile that another CTA started: leave the partial sums for that CTA
         float* dst = p.partial + ((size_t)blockIdx.x * MT + half * MTD) * BMW + rl;
         if (warp == kDrainWarp0) { DBG_STAMP1(18); }
+        lost();
 #pragma unroll
         for (int t = 0; t < MTD; ++t)
           if (t < mcount) __stcg(dst + t * BMW, total[t]);
         if (warp == kDrainWarp0) { DBG_STAMP1(19); }
-        // the barrier orders every drain thread's stores before thread 0's release, which is cumulative at GPU scope
+        // the barrier orders every drain thread's stores before thread 0's fence, which is cumulative
         drain_bar();
         if (warp == kDrainWarp0) { DBG_STAMP1(20); }
-        if (dt == 0) {
-          __threadfence();
-          st_release_gpu(p.flags + blockIdx.x, 1u);
-        }
+        if (dt == 0) ptx::partial_publish(p.flags + blockIdx.x);
         if (warp == kDrainWarp0) { DBG_STAMP1(21); }
         DBG_END(2);
         continue;
@@ -968,16 +962,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
       if (!last) {
         // add the partial sums of the CTAs that continue the tile, in CTA order
         for (int j = dt; j < np; j += kDT) {
-          const uint32_t* f = p.flags + blockIdx.x + 1 + j;
-          const long long t0 = clock64();
-          uint32_t spins = 0;
-          while (ld_acquire_gpu(f) == 0u) {
-            if ((++spins & 0xff) == 0 && (*abort_flag || clock64() - t0 > ptx::kWaitLimitCycles)) {
-              *abort_flag = kErrPartialWait;
-              if (p.err_word) atomicCAS(p.err_word, 0u, kErrPartialWait | (blockIdx.x << 8));
-              break;
-            }
-          }
+          ptx::partial_wait(p.flags + blockIdx.x + 1 + j, p.wait_cycles, abort_flag, p.err_word, kErrPartialWait);
         }
         drain_bar();
         if (warp == kDrainWarp0) { DBG_STAMP(15); }
@@ -985,6 +970,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
         if (warp == kDrainWarp0) { DBG_STAMP(16); }
       }
       drain_bar();  // the factors written at the top of the fragment are visible
+      lost();
       float psv = own_scale ? scale_value(ps_bits, p.s_dt) : 1.f;
       if constexpr (ZP) {
         // the zero points' term, once per tile: minus sum_b zp[b,n] * xs[b,m], in units of the fixed point; every lane
@@ -1522,6 +1508,7 @@ int launch_limb_impl(int wbits, const void* x, int x_dt, const void* w, const Sc
   p.partial = sc.partial;
   p.flags = sc.flags;
   p.err_word = device_error_word();
+  p.wait_cycles = peer_wait_cycles();
   p.gate_up = gate_up;
   p.ytiles = pl.items ? (int)ceil_div(M, pl.tile_tokens) : 1;
   p.m0 = 0;

@@ -448,6 +448,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(&acc_empty[buf]);
       }
+      if (*abort_flag) {  // a wait ran out: NaN, not what is there
+#pragma unroll
+        for (int j = 0; j < MP; ++j) acc[j] = __uint_as_float(0x7fc00000u);
+      }
       if constexpr (KSPLIT) {
         // (1) every CTA of the cluster is past its main loop: the leader's rings may be overwritten
         __syncwarp();
@@ -476,10 +480,11 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     } else {
       // large token tiles: one scale block only (per-channel); scale and store straight from TMEM
-      const float s = n_ok ? __ldg(p.scale + n) : 0.f;
+      float s = n_ok ? __ldg(p.scale + n) : 0.f;
       if (my_tiles > 0) {
         ptx::mbar_wait_warp(&acc_full[0], 0, abort_flag, p.err_word, ptx::kErrWaitTmemFull);
         ptx::tcgen05_fence_after();
+        if (*abort_flag) s = __uint_as_float(0x7fc00000u);
 #pragma unroll 1
         for (int c = 0; c < MP / 32; ++c) {
           uint32_t rr[32];

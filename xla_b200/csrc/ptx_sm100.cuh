@@ -4,7 +4,8 @@
 //
 // Every wait is bounded: a wait that does not complete within kWaitLimitCycles records a code in the
 // library's device error word and in a CTA-local abort flag; once that flag is set all later
-// waits return at once, so a kernel with a broken pipeline drains and exits instead of hanging.
+// waits return at once, so a kernel with a broken pipeline drains and exits instead of hanging.  Whoever stores results
+// looks at the flag first and stores NaN when it is set.
 #pragma once
 
 #include <cuda.h>
@@ -136,6 +137,35 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity,
   if ((threadIdx.x & 31) == 0) ok = mbar_wait<SLEEP_NS>(bar, parity, abort_flag, err_word, code);
   __syncwarp();
   return ok;
+}
+
+// ---- partial tiles between the CTAs of a launch ------------------------------------------------
+// A CTA that works on a later K range of a tile leaves its sums in global scratch for the tile's first CTA.  The flag word
+// beside them: 0 idle, 1 written, 2 given up by the reader; 0 again after every launch, also after one that gave up.
+// Both are called by one thread, the writer's behind a barrier that its CTA's stores precede.
+__device__ __forceinline__ void partial_publish(uint32_t* flag) {
+  __threadfence();
+  if (atomicCAS(flag, 0u, 1u) == 2u) atomicExch(flag, 0u);  // nobody waits for it any more
+}
+__device__ __forceinline__ bool partial_wait(uint32_t* flag, long long limit_cycles, volatile uint32_t* abort_flag, uint32_t* err_word,
+                                             uint32_t code) {
+  const long long t0 = clock64();
+  uint32_t spins = 0, v;
+  while (true) {
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
+    if (v == 1u) break;
+    if ((++spins & 0xff) == 0 && (*abort_flag || clock64() - t0 > limit_cycles)) {
+      if (atomicCAS(flag, 0u, 2u) == 1u) {  // there after all
+        __threadfence();
+        break;
+      }
+      *abort_flag = code;
+      if (err_word) atomicCAS(err_word, 0u, code | (blockIdx.x << 8));
+      return false;
+    }
+  }
+  atomicExch(flag, 0u);
+  return true;
 }
 
 // ---- proxies / fences ---------------------------------------------------------------------

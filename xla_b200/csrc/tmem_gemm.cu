@@ -74,6 +74,7 @@ struct Params {
   float* partial;   // [g2][th][128]
   uint32_t* flags;  // [g2], zero between launches
   uint32_t* err_word;
+  long long wait_cycles;  // for a partial tile
 };
 
 // KS: k values per step (64 for scale blocks of 64, else 128); NC: accumulator columns (tokens).
@@ -136,14 +137,6 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
 }
 __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void st_release_gpu(uint32_t* p, uint32_t v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-__device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
-  uint32_t v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
 }
 
 template <typename XT>
@@ -526,25 +519,21 @@ __global__ void __launch_bounds__(kThreads, 1)
         drain_bar();
         np = s_npart;
         for (int j = dt; j < np; j += 256) {
-          const uint32_t* f = p.flags + blockIdx.x + 1 + j;
-          const long long t0 = clock64();
-          uint32_t spins = 0;
-          while (ld_acquire_gpu(f) == 0u) {
-            if ((++spins & 0xff) == 0 && (*abort_flag || clock64() - t0 > ptx::kWaitLimitCycles)) {
-              *abort_flag = kErrPartial;
-              if (p.err_word) atomicCAS(p.err_word, 0u, kErrPartial | (blockIdx.x << 8));
-              break;
-            }
-          }
+          ptx::partial_wait(p.flags + blockIdx.x + 1 + j, p.wait_cycles, abort_flag, p.err_word, kErrPartial);
         }
         drain_bar();
       }
+      const bool lost = *abort_flag != 0;  // a wait ran out: NaN, not what is there
       const float ps = p.blocked || !n_ok ? 1.f : scale_value(load_scale_bits(p.scale, n, p.s_dt), p.s_dt);
       const float z1 = !p.blocked && p.zp && n_ok ? -scale_value(load_scale_bits(p.zp, n, p.s_dt), p.s_dt) : 0.f;
 #pragma unroll 1
       for (int c = 0; c < DT / 16; ++c) {
         const int l0 = grp * DT + 16 * c;  // token inside the item
         const int count = min(16, mcount - 16 * c);
+        if (lost) {
+#pragma unroll
+          for (int t = 0; t < 16; ++t) total[t] = __uint_as_float(0x7fc00000u);
+        }
         if (!first) {
           // a later K range of an item that another CTA started: leave the sums for that CTA
           float* dst = p.partial + ((size_t)blockIdx.x * p.th + l0) * BMW + rl;
@@ -586,14 +575,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int t = 0; t + 16 < DT; ++t) total[t] = total[t + 16];
       }
       if (!first) {
-        drain_bar();  // orders every drain thread's stores before thread 0's release, which is cumulative at GPU scope
-        if (dt == 0) {
-          __threadfence();
-          st_release_gpu(p.flags + blockIdx.x, 1u);
-        }
-      } else if (np > 0) {
-        drain_bar();
-        for (int j = dt; j < np; j += 256) p.flags[blockIdx.x + 1 + j] = 0u;  // clean for the next launch
+        drain_bar();  // orders every drain thread's stores before thread 0's fence, which is cumulative
+        if (dt == 0) ptx::partial_publish(p.flags + blockIdx.x);
       }
       asm volatile("cp.async.wait_group 0;" ::: "memory");  // the ring is refilled from its start
     }
@@ -791,6 +774,7 @@ int launch_tmem_gemm(int wbits, const void* x, int x_dt, const void* w, const Sc
   p.partial = sc.partial;
   p.flags = sc.flags;
   p.err_word = device_error_word();
+  p.wait_cycles = peer_wait_cycles();
 
   // ---- schedule ----
   const int tiles = (int)ceil_div(N, BMW), items = tiles * pl.ytiles, ctas = std::min(sm_count(), kMaxCtas);

@@ -181,7 +181,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       ptx::tcgen05_fence_after();
       const int64_t m = (int64_t)tm * BM + quad * 32 + lane;
       const bool row_ok = m < p.M;
-      const float xs = (row_ok && p.out) ? p.x_scale[m] : 0.f;
+      // (a wait that ran out makes every result of the tile NaN; int32 accumulators have no such value, see the error word)
+      const float xs = *abort_flag ? __uint_as_float(0x7fc00000u) : (row_ok && p.out) ? p.x_scale[m] : 0.f;
       const int32_t rs = (row_ok && p.rowsum) ? p.rowsum[m] : 0;
       const uint32_t taddr = tmem_base + ab * BN + ((uint32_t)(quad * 32) << 16);
       if (p.tma_store) {
