@@ -71,3 +71,34 @@ def test_weights_packed_directly_in_front(M):
   torch.cuda.synchronize()
   got = [run(w, False) for w in ws]
   assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+def test_two_streams_at_once():
+  """Launches whose CTAs wait for one another's partial sums, on two streams that share the SMs: nobody waits for a CTA that
+  has not started."""
+  from xla_b200 import _capi
+  assert _capi.device_error(DEV) == 0
+  g = qc.gen(3)
+  cases = []
+  for variant, wbits, bs, N, K, M in (("tmem", 4, 128, 2560, 8192, 29), ("i8tc", 4, 128, 5120, 8192, 40), ("i8tc", 8, -1, 2560, 8192, 16)):
+    w = (qc.int4_weight if wbits == 4 else qc.int8_weight)(g, N, K).to(DEV)
+    s = (qc.per_channel_scale(g, N) if bs == -1 else qc.blockwise_scale(g, K // bs, N)).to(DEV)
+    cases.append((variant, qc.activations(g, M, K).to(DEV), xla_b200.pack_int4(w) if wbits == 4 else w, s, bs, wbits == 4))
+
+  def run(c):
+    variant, x, w, s, bs, int4 = c
+    with xla_b200.force_variant(variant):
+      return torch.ops.xla_b200.quantized_matmul_packed(x, w, s, block_size=bs, int4_weight=int4, weight_is_packed=int4,
+                                                        out_dtype=torch.float32)
+
+  want = [run(c) for c in cases]
+  torch.cuda.synchronize()
+  streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+  outs = []
+  for i in range(60):
+    for j, st in enumerate(streams):
+      with torch.cuda.stream(st):
+        outs.append(((i + j) % 3, run(cases[(i + j) % 3])))
+  torch.cuda.synchronize()
+  assert _capi.device_error(DEV) == 0
+  assert all(torch.equal(y, want[k]) for k, y in outs)

@@ -118,14 +118,15 @@ struct Params {
   int scale_ring;  // block scales through the ring in shared memory (instances that have one)
   int S;       // scale blocks
   long long units;
-  float* partial;   // [grid][MT][128] fp32
-  uint32_t* flags;  // [grid], zero between launches
+  float* partial;   // [place of the deal][MT][128] fp32
+  uint32_t* flags;  // [place of the deal], zero between launches
   uint32_t* err_word;
   long long wait_cycles;  // for a partial tile
   int gate_up;
   int ytiles;    // token tiles per weight tile (1 up to one tile's tokens); a work item is a (weight tile, token tile) pair
   // The schedule: the first `items1` items go to the CTAs whole (CTA c takes items c, c + G, ...); the K units of
-  // the remaining items (`units` of them) are dealt in equal contiguous shares to the first `g2` CTAs (stream-K: an
+  // the remaining items (`units` of them) are dealt in equal contiguous shares to the first `g2` CTAs, from the last of
+  // them down (stream-K: an
   // item that spans CTAs is summed through the partial tiles).  One token tile: items1 = 0, g2 = the grid.
   long long items1;
   int g2;
@@ -185,6 +186,14 @@ struct Cfg {
 // The (item, unit range) fragments of this CTA's share of the schedule, in order.  Item i = (weight tile i / ytiles,
 // token tile i % ytiles): the token tiles of one weight tile are neighbours in the order, run on neighbouring CTAs at
 // the same time and share the tile's bytes in L2.
+//
+// The dealt units go to the CTAs from the last one down: place 0 of the deal is CTA g2 - 1.  A tile's first place waits for
+// the partial tiles of the places behind it, which are CTAs with lower indices.  CTAs start in the order of their indices,
+// so those run already or are done, and none of them waits before its partial tile is written; dealt the other way round,
+// two launches that share the GPU (two streams) could each hold the SMs that the other's missing CTAs needed, until the
+// waits ran out.
+__device__ __forceinline__ int deal_place(const Params& p) { return p.g2 - 1 - (int)blockIdx.x; }
+
 struct FragIter {
   long long u, hi;        // this CTA's range of the dealt units (counted from the first dealt item)
   int ut;
@@ -192,9 +201,9 @@ struct FragIter {
   long long item;         // the current fragment's item once next() returned true
   long long nxt, items1;  // whole items: the next one of this CTA, their number
   __device__ FragIter(const Params& p) : ut(p.ut), ytiles(p.ytiles), y(0), item(0), nxt(blockIdx.x), items1(p.items1) {
-    const long long c = blockIdx.x;
-    u = c < p.g2 ? c * p.units / p.g2 : 0;
-    hi = c < p.g2 ? (c + 1) * p.units / p.g2 : 0;
+    const long long c = deal_place(p);
+    u = c >= 0 ? c * p.units / p.g2 : 0;
+    hi = c >= 0 ? (c + 1) * p.units / p.g2 : 0;
   }
   __device__ bool next(int& tile, int& u0, int& u1) {
     if (nxt < items1) {
@@ -733,6 +742,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
     __shared__ float s_pw[2][64];
     static_assert(MT <= 64, "per-token factors of a tile");
     int frag = 0;
+    const int place = deal_place(p);
     // a fetched scale's value: the fp32 bits, or a 16-bit value's
     auto value = [&](uint32_t w) { return W16 ? scale_value(w, p.s_dt) : __uint_as_float(w); };
     // A scale fetched one hand-over ahead, at the end of the current one.  The permutation is one that the compiler does not
@@ -777,7 +787,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
       int np = 0;
       auto add_partials = [&]() {
         // two partial tiles in flight at a time (an L2 round trip each), added in CTA order
-        const float* src = p.partial + ((size_t)(blockIdx.x + 1) * MT + half * MTD) * BMW + rl;
+        const float* src = p.partial + ((size_t)(place + 1) * MT + half * MTD) * BMW + rl;
         constexpr size_t kTile = (size_t)MT * BMW;
         int j = 0;
         for (; C::kThreads <= 512 && j + 1 < np; j += 2) {  // (where the register budget allows)
@@ -804,7 +814,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
       if (first && !last) {
         if (dt == 0) {
           int cnt = 0;
-          for (long long c2 = blockIdx.x + 1; c2 < p.g2; ++c2) {
+          for (long long c2 = place + 1; c2 < p.g2; ++c2) {
             if (c2 * p.units / p.g2 >= (it.item - p.items1 + 1) * p.ut) break;
             ++cnt;
           }
@@ -943,7 +953,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
       // ---- end of the fragment ----
       if (!first) {
         // a later K range of a tile that another CTA started: leave the partial sums for that CTA
-        float* dst = p.partial + ((size_t)blockIdx.x * MT + half * MTD) * BMW + rl;
+        float* dst = p.partial + ((size_t)place * MT + half * MTD) * BMW + rl;
         if (warp == kDrainWarp0) { DBG_STAMP1(18); }
         lost();
 #pragma unroll
@@ -953,7 +963,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
         // the barrier orders every drain thread's stores before thread 0's fence, which is cumulative
         drain_bar();
         if (warp == kDrainWarp0) { DBG_STAMP1(20); }
-        if (dt == 0) ptx::partial_publish(p.flags + blockIdx.x);
+        if (dt == 0) ptx::partial_publish(p.flags + place);
         if (warp == kDrainWarp0) { DBG_STAMP1(21); }
         DBG_END(2);
         continue;
@@ -962,7 +972,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
       if (!last) {
         // add the partial sums of the CTAs that continue the tile, in CTA order
         for (int j = dt; j < np; j += kDT) {
-          ptx::partial_wait(p.flags + blockIdx.x + 1 + j, p.wait_cycles, abort_flag, p.err_word, kErrPartialWait);
+          ptx::partial_wait(p.flags + place + 1 + j, p.wait_cycles, abort_flag, p.err_word, kErrPartialWait);
         }
         drain_bar();
         if (warp == kDrainWarp0) { DBG_STAMP(15); }

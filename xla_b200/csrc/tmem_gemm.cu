@@ -98,14 +98,18 @@ struct Cfg {
   static_assert((2 * kRaw + kB + kASlots + 2 * kAcc + kDone) * 8 + 8 <= 512, "barrier space");
 };
 
-// The (item, unit range) fragments of this CTA, in order: whole items first, then its share of the dealt units.
+// The (item, unit range) fragments of this CTA, in order: whole items first, then its share of the dealt units.  These go to
+// the CTAs from the last one down, so that a CTA waits only for partial tiles of CTAs with lower indices: CTAs start in the
+// order of their indices, so those run already or are done, also when another launch holds a part of the SMs.
+__device__ __forceinline__ int deal_place(const Params& p) { return p.g2 - 1 - (int)blockIdx.x; }
+
 struct FragIter {
   const Params& p;
   int u, hi, nxt, item, tile, y, u0, u1;
   __device__ explicit FragIter(const Params& p) : p(p), nxt(blockIdx.x), item(0), tile(0), y(0), u0(0), u1(0) {
-    const int c = blockIdx.x;
-    u = c < p.g2 ? share(c) : 0;
-    hi = c < p.g2 ? share(c + 1) : 0;
+    const int c = deal_place(p);
+    u = c >= 0 ? share(c) : 0;
+    hi = c >= 0 ? share(c + 1) : 0;
   }
   __device__ int share(int c) const { return (int)((long long)c * p.units / p.g2); }
   __device__ bool next() {
@@ -414,6 +418,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const uint32_t* my_scale = s_scale + dt;
     const uint32_t my_scale_u32 = ptx::smem_u32(my_scale);
     auto value = [&](int i) { return scale_in<W16, XT>(my_scale + i * kDrain, rl, p.s_dt); };
+    const int place = deal_place(p);
     bool waited = false;
     FragIter it(p);
     int buf = 0;
@@ -510,7 +515,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         // the sums of the CTAs that continue the item are added in CTA order, once they are all there
         if (dt == 0) {
           int cnt = 0;
-          for (int c2 = blockIdx.x + 1; c2 < p.g2; ++c2) {
+          for (int c2 = place + 1; c2 < p.g2; ++c2) {
             if (it.share(c2) >= (it.item - p.items1 + 1) * p.ut) break;
             ++cnt;
           }
@@ -519,7 +524,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         drain_bar();
         np = s_npart;
         for (int j = dt; j < np; j += 256) {
-          ptx::partial_wait(p.flags + blockIdx.x + 1 + j, p.wait_cycles, abort_flag, p.err_word, kErrPartial);
+          ptx::partial_wait(p.flags + place + 1 + j, p.wait_cycles, abort_flag, p.err_word, kErrPartial);
         }
         drain_bar();
       }
@@ -536,14 +541,14 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         if (!first) {
           // a later K range of an item that another CTA started: leave the sums for that CTA
-          float* dst = p.partial + ((size_t)blockIdx.x * p.th + l0) * BMW + rl;
+          float* dst = p.partial + ((size_t)place * p.th + l0) * BMW + rl;
 #pragma unroll
           for (int t = 0; t < 16; ++t)
             if (t < count) __stcg(dst + t * BMW, total[t]);
         } else {
 #pragma unroll 1
           for (int j = 0; j < np; ++j) {
-            const float* src = p.partial + ((size_t)(blockIdx.x + 1 + j) * p.th + l0) * BMW + rl;
+            const float* src = p.partial + ((size_t)(place + 1 + j) * p.th + l0) * BMW + rl;
             float v[16];
 #pragma unroll
             for (int t = 0; t < 16; ++t) v[t] = t < count ? __ldcg(src + t * BMW) : 0.f;
@@ -576,7 +581,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       if (!first) {
         drain_bar();  // orders every drain thread's stores before thread 0's fence, which is cumulative
-        if (dt == 0) ptx::partial_publish(p.flags + blockIdx.x);
+        if (dt == 0) ptx::partial_publish(p.flags + place);
       }
       asm volatile("cp.async.wait_group 0;" ::: "memory");  // the ring is refilled from its start
     }
