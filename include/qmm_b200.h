@@ -174,8 +174,8 @@ QMM_API size_t qmm_weight_only_workspace_size_for(int wbits, int64_t max_M, int6
  * Replaces: get_tuned_block_sizes (torch_xla/experimental/pallas_kernels/quantized_matmul_kernel.py:537-555).
  */
 QMM_API int qmm_tuned_variant(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_size);
-/* Name of the kernel family qmm_weight_only's AUTO picks for a shape among those the measured table knows, given a
- * sufficient workspace (static string).  The few-token calls that QMM_VARIANT_I8MMA takes are decided before it. */
+/* Name of the kernel family that qmm_weight_only's AUTO picks for a shape with bf16 activations and results, aligned
+ * operands and a sufficient workspace on the current device (static string; the choice of the call itself). */
 QMM_API const char* qmm_weight_only_variant_for(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_size, int has_zp);
 /*
  * Whether qmm_weight_only's AUTO has a fast kernel that applies zero points itself for this shape (given a sufficient
@@ -431,7 +431,8 @@ QMM_API int qmm_set_peer_wait_limit(double seconds);
  */
 QMM_API int qmm_stream_read(const void* p, size_t bytes, void* sink, void* stream);
 
-/* Name of the kernel family the AUTO heuristic picks (static string, for logs and tests). */
+/* Name of the kernel family that AUTO picks in the entry point of that op, which has no workspace (static string, for logs
+ * and tests; qmm_weight_only: see qmm_weight_only_variant_for). */
 QMM_API const char* qmm_variant_for(int op, int64_t M, int64_t N, int64_t K, int64_t block_size,
                             int has_zp);
 

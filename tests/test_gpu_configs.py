@@ -113,3 +113,46 @@ def test_quantized_matmul_int8_without_activation_quantization(dtype, tol, bs, n
   assert out.dtype == dtype and tuple(out.shape) == (bs, n_out)
   exact = qo.quantized_matmul(x.float(), w, s, dot_round=None)
   assert qo.max_abs_rel(out, exact) < tol
+
+
+_ASK_AND_CALL = """
+import torch, xla_b200
+from xla_b200 import _capi
+L = _capi.lib()
+for wbits, bs, N, K in ((4, 128, 14336, 4096), (4, 128, 28672, 8192), (8, -1, 4096, 4096), (8, 128, 300, 1280), (4, 64, 512, 1024),
+                        (8, -1, 301, 72), (4, -1, 2048, 4096)):
+  for M in (1, 2, 4, 8, 9, 16, 29, 33, 64, 65, 200, 512):
+    for zp in (False, True):
+      s = torch.ones((N,) if bs == -1 else (K // bs, N), device="cuda")
+      w = torch.zeros((N, K * wbits // 8), dtype=torch.uint8 if wbits == 4 else torch.int8, device="cuda")
+      x = torch.zeros((M, K), dtype=torch.bfloat16, device="cuda")
+      if zp and not L.qmm_zero_point_in_kernel(wbits, M, N, K, bs, _capi.BF16):
+        continue
+      print("ask", M, N, K, L.qmm_weight_only_variant_for(wbits, M, N, K, bs, int(zp)).decode(), flush=True)
+      torch.ops.xla_b200.quantized_matmul_packed(x, w, s, s if zp else None, block_size=bs, int4_weight=wbits == 4,
+                                                 weight_is_packed=wbits == 4, out_dtype=torch.bfloat16)
+w8 = torch.zeros((300, 512), dtype=torch.int8, device="cuda")
+for M in (1, 8, 9, 12, 13, 15, 16, 64):
+  print("ask", M, 300, 512, L.qmm_variant_for(_capi.OP_W8A8_PERCHANNEL, M, 300, 512, 0, 0).decode(), flush=True)
+  torch.ops.xla.quantized_matmul(torch.ones((M, 512), dtype=torch.bfloat16, device="cuda"), w8, torch.ones(300, device="cuda"), quantize_activation=True)
+"""
+
+
+def test_the_named_kernel_is_the_one_that_runs():
+  """qmm_weight_only_variant_for and qmm_variant_for against the choice that the call logs."""
+  import os
+  import subprocess
+  import sys
+  r = subprocess.run([sys.executable, "-c", _ASK_AND_CALL], env=dict(os.environ, QMM_B200_LOG="1"), stdout=subprocess.PIPE,
+                     stderr=subprocess.STDOUT, text=True, timeout=300, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+  assert r.returncode == 0, r.stdout[-2000:]
+  asked, seen = None, 0
+  for line in r.stdout.splitlines():
+    if line.startswith("ask "):
+      assert asked is None, f"no call after {asked}"
+      asked = line.split()[1:]
+    elif line.startswith("[qmm_b200]") and asked:
+      _, _, m, n, k, _, name = line.split()
+      assert [m[2:], n[2:], k[2:]] == asked[:3] and name == asked[3], (asked, line)
+      asked, seen = None, seen + 1
+  assert asked is None and seen > 100

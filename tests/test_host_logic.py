@@ -148,11 +148,15 @@ def test_tuned_table_lookup_and_auto_choice():
   # the committed table and the tuner agree on the row format
   rows = [l for l in open(tune.__file__.replace("tune.py", "csrc/tuned_table.inc")) if l.startswith("{")]
   assert len(rows) >= 100 and all(re.match(r"\{[48], \d+, \d+, \d+, \{(\d, ){6}\d\}\},", r) for r in rows)
-  # AUTO: table first, shape rule on a miss; zero points rule the split-activation kernel out
-  assert L.qmm_weight_only_variant_for(4, 1, 28672, 8192, 128, 0) == b"i8tc"
-  assert L.qmm_weight_only_variant_for(4, 1, 14336, 4096, 128, 0) == b"mma"
+  # AUTO, asked as the call asks: the integer decode kernel at one token, then the table, the shape rule on a miss; zero
+  # points on few tokens rule the split-activation kernel out
+  assert L.qmm_weight_only_variant_for(4, 1, 28672, 8192, 128, 0) == b"i8mma"
+  assert L.qmm_weight_only_variant_for(4, 1, 14336, 4096, 128, 0) == b"i8mma"
+  assert L.qmm_weight_only_variant_for(4, 8, 28672, 8192, 128, 0) == b"i8tc"      # table
+  assert L.qmm_weight_only_variant_for(4, 8, 14336, 4096, 128, 0) == b"mma"       # table
   assert L.qmm_weight_only_variant_for(8, 512, 4097 * 2, 4096, 0, 0) == b"i8tc"   # shape rule: above 64 tokens
-  assert L.qmm_weight_only_variant_for(8, 1, 4097 * 2, 4096, 0, 0) == b"mma"      # shape rule: a small weight at M = 1
+  assert L.qmm_weight_only_variant_for(8, 16, 4097 * 2, 4096, 0, 0) == b"i8tc"    # shape rule: 32 MB from nine tokens on
+  assert L.qmm_weight_only_variant_for(8, 16, 4097, 4096, 0, 0) == b"mma"         # shape rule: a smaller weight
   assert L.qmm_weight_only_variant_for(8, 1, 28672, 8192, 0, 1) != b"i8tc"
 
 

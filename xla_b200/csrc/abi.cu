@@ -184,9 +184,9 @@ const char* qmm_last_error_string(void) { return g_last_error; }
 // batches, the tcgen05 kernel above that, the CUDA-core GEMV where those cannot go (zero points, f32
 // activations), the any-shape kernel for everything else.
 static int pick_weight_only(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, const void* x, int x_dt,
-                            const void* w, bool has_zp) {
+                            const void* w, bool has_zp, bool sm100) {
   if (decode_mma_supported(wbits, M, N, K, bs, x, x_dt, w, has_zp)) return QMM_VARIANT_MMA;
-  if (mixed_tc_supported(wbits, M, N, K, bs, x, x_dt, w, has_zp)) return QMM_VARIANT_TCGEN05;
+  if (sm100 && mixed_tc_shape_ok(wbits, M, N, K, bs, x_dt, has_zp) && aligned(x, 16) && aligned(w, 16)) return QMM_VARIANT_TCGEN05;
   if (gemv_nk_supported(wbits, M, N, K, bs, x, x_dt, w)) return QMM_VARIANT_GEMV;
   return QMM_VARIANT_GENERIC;
 }
@@ -234,7 +234,7 @@ int qmm_w8a16_perchannel(const void* x, int x_dtype, const int8_t* w, const floa
   int rc = check_common(x, x_dtype, w, scale, out, out_dtype, M, N, K);
   if (rc != QMM_OK || M * N == 0) return rc;
   cudaStream_t st = as_stream(stream);
-  if (variant == QMM_VARIANT_AUTO) variant = pick_weight_only(8, M, N, K, 0, x, x_dtype, w, zp != nullptr);
+  if (variant == QMM_VARIANT_AUTO) variant = pick_weight_only(8, M, N, K, 0, x, x_dtype, w, zp != nullptr, device_is_sm100());
   switch (variant) {
     case QMM_VARIANT_GENERIC:
       log_choice("w8a16_perchannel", "generic", M, N, K);
@@ -284,7 +284,7 @@ int qmm_w4a16_blockwise_packed(const void* x, int x_dtype, const uint8_t* wp, co
                 (long long)K, (long long)block_size);
   if (M * N == 0) return QMM_OK;
   cudaStream_t st = as_stream(stream);
-  if (variant == QMM_VARIANT_AUTO) variant = pick_weight_only(4, M, N, K, block_size, x, x_dtype, wp, zp != nullptr);
+  if (variant == QMM_VARIANT_AUTO) variant = pick_weight_only(4, M, N, K, block_size, x, x_dtype, wp, zp != nullptr, device_is_sm100());
   switch (variant) {
     case QMM_VARIANT_GENERIC:
       log_choice("w4a16_blockwise_packed", "generic", M, N, K);
@@ -314,7 +314,7 @@ int qmm_w8a16_blockwise(const void* x, int x_dtype, const int8_t* w, const float
                 (long long)K, (long long)block_size);
   if (M * N == 0) return QMM_OK;
   cudaStream_t st = as_stream(stream);
-  if (variant == QMM_VARIANT_AUTO) variant = pick_weight_only(8, M, N, K, block_size, x, x_dtype, w, zp != nullptr);
+  if (variant == QMM_VARIANT_AUTO) variant = pick_weight_only(8, M, N, K, block_size, x, x_dtype, w, zp != nullptr, device_is_sm100());
   switch (variant) {
     case QMM_VARIANT_GENERIC:
       log_choice("w8a16_blockwise", "generic", M, N, K);
@@ -370,22 +370,46 @@ int qmm_zero_point_in_kernel(int wbits, int64_t M, int64_t N, int64_t K, int64_t
          decode_i8_supported(wbits, M, N, K, block_size, ok, x_dtype, ok, true);
 }
 
+// qmm_weight_only's AUTO.  `room`: bytes of usable scratch.
+static int choose_weight_only(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, const void* x, int x_dt, int out_dt, const void* w,
+                              bool has_zp, size_t room, bool sm100) {
+  if (use_decode_i8(wbits, M, N, K, bs, x, x_dt, w, has_zp)) return QMM_VARIANT_I8MMA;
+  const bool tma = sm100 && aligned(x, 16) && aligned(w, 16);
+  if (tma && use_tmem(wbits, M, N, K, bs, x_dt, out_dt, has_zp) && room >= tmem_gemm_workspace_bytes(M, K)) return QMM_VARIANT_TMEM;
+  // the measured table first, the shape rule where the table has no entry for this shape
+  const int tuned = tuned_variant(wbits, bs, M, N, K);
+  if (tma && limb_tc_shape_ok(wbits, M, N, K, bs, x_dt, has_zp) && room >= limb_tc_workspace_bytes(M, K)) {
+    bool use = tuned ? tuned == QMM_VARIANT_I8TC : limb_tc_preferred(wbits, M, N, K, bs);
+    // Zero points and fp32 activations: the other kernels for more than a few tokens take neither, and the any-shape
+    // kernel is a hundred times slower (333 tokens of fp32 on [5120,6912] int8 with zero points: 12.2 ms, here 52 us).
+    // Up to eight tokens the register-dequant GEMV takes both.
+    if (has_zp || x_dt == QMM_F32) use = M > 8;
+    if (use) return QMM_VARIANT_I8TC;
+  }
+  if (!has_zp && tuned == QMM_VARIANT_MMA && decode_mma_supported(wbits, M, N, K, bs, x, x_dt, w, false)) return QMM_VARIANT_MMA;
+  if (!has_zp && tuned == QMM_VARIANT_TCGEN05 && tma && mixed_tc_shape_ok(wbits, M, N, K, bs, x_dt, false)) return QMM_VARIANT_TCGEN05;
+  return pick_weight_only(wbits, M, N, K, bs, x, x_dt, w, has_zp, sm100);
+}
+
+static const char* variant_name(int variant) {
+  switch (variant) {
+    case QMM_VARIANT_GEMV: return "gemv";
+    case QMM_VARIANT_TCGEN05: return "tcgen05";
+    case QMM_VARIANT_MMA: return "mma";
+    case QMM_VARIANT_I8TC: return "i8tc";
+    case QMM_VARIANT_I8MMA: return "i8mma";
+    case QMM_VARIANT_TMEM: return "tmem";
+    default: return "generic";
+  }
+}
+
+// a 256-byte aligned address, for questions about a shape
+static const void* any_pointer() { return reinterpret_cast<const void*>(uintptr_t(256)); }
+
 const char* qmm_weight_only_variant_for(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_size, int has_zp) {
-  // Shape-only view of qmm_weight_only's AUTO choice, for a caller that passes a sufficient workspace and aligned pointers.
-  if (block_size < 0) block_size = 0;
-  const void* ok = reinterpret_cast<const void*>(uintptr_t(256));
-  if (use_tmem(wbits, M, N, K, block_size, QMM_BF16, QMM_BF16, has_zp != 0)) return "tmem";
-  const bool can = limb_tc_shape_ok(wbits, M, N, K, block_size, QMM_BF16, has_zp != 0);
-  const int tuned = tuned_variant(wbits, block_size, M, N, K);
-  if (can && has_zp) {
-    if (M > 8) return "i8tc";
-  } else if (can && (tuned ? tuned == QMM_VARIANT_I8TC : limb_tc_preferred(wbits, M, N, K, block_size))) return "i8tc";
-  if (!has_zp && tuned == QMM_VARIANT_MMA && decode_mma_supported(wbits, M, N, K, block_size, ok, QMM_BF16, ok, false)) return "mma";
-  if (!has_zp && tuned == QMM_VARIANT_TCGEN05 && mixed_tc_shape_ok(wbits, M, N, K, block_size, QMM_BF16, false)) return "tcgen05";
-  if (decode_mma_supported(wbits, M, N, K, block_size, ok, QMM_BF16, ok, has_zp != 0)) return "mma";
-  if (mixed_tc_shape_ok(wbits, M, N, K, block_size, QMM_BF16, has_zp != 0)) return "tcgen05";
-  if (gemv_nk_supported(wbits, M, N, K, block_size, ok, QMM_BF16, ok)) return "gemv";
-  return "generic";
+  const void* ok = any_pointer();
+  return variant_name(choose_weight_only(wbits, M, N, K, std::max<int64_t>(block_size, 0), ok, QMM_BF16, QMM_BF16, ok, has_zp != 0,
+                                         SIZE_MAX, true));
 }
 
 size_t qmm_weight_only_workspace_size(int64_t max_M, int64_t K) {
@@ -418,30 +442,10 @@ int qmm_weight_only_typed(int wbits, const void* x, int x_dtype, const void* w, 
     if (block_size > 0 && K % block_size != 0)
       return fail(QMM_ERR_BAD_SHAPE, "input_dim should be divisible by block_size, got input_dim: %lld, block_size: %lld",
                   (long long)K, (long long)block_size);
-    if (variant == QMM_VARIANT_AUTO && use_decode_i8(wbits, M, N, K, block_size, x, x_dtype, w, zp != nullptr)) variant = QMM_VARIANT_I8MMA;
-    if (variant == QMM_VARIANT_AUTO && use_tmem(wbits, M, N, K, block_size, x_dtype, out_dtype, zp != nullptr) && aligned(x, 16) && aligned(w, 16) &&
-        device_is_sm100() && workspace && aligned(workspace, 256) && workspace_bytes >= tmem_gemm_workspace_bytes(M, K))
-      variant = QMM_VARIANT_TMEM;
-    const bool can = limb_tc_supported(wbits, M, N, K, block_size, x, x_dtype, w, zp != nullptr) && workspace &&
-                     workspace_bytes >= limb_tc_workspace_bytes(M, K) && aligned(workspace, 256);
-    // AUTO: the measured table first, the shape rule where the table has no entry for this shape
-    const int tuned = variant == QMM_VARIANT_AUTO ? tuned_variant(wbits, block_size, M, N, K) : 0;
-    bool use = variant == QMM_VARIANT_I8TC;
-    if (variant == QMM_VARIANT_AUTO && can) {
-      use = tuned ? tuned == QMM_VARIANT_I8TC : limb_tc_preferred(wbits, M, N, K, block_size);
-      // Zero points and fp32 activations: the other kernels for more than a few tokens take neither, and the any-shape
-      // kernel is a hundred times slower (333 tokens of fp32 on [5120,6912] int8 with zero points: 12.2 ms, here 56 us).
-      // Up to eight tokens the register-dequant GEMV takes both.
-      if (zp || x_dtype == QMM_F32) use = M > 8;
-    }
-    if (!use && tuned && tuned != QMM_VARIANT_I8TC && !zp) {
-      // the table names one of the kernels behind the entry points below; they refuse what they cannot run, and AUTO
-      // then decides there
-      const bool ok = tuned == QMM_VARIANT_MMA ? decode_mma_supported(wbits, M, N, K, block_size, x, x_dtype, w, false)
-                                               : (tuned == QMM_VARIANT_TCGEN05 && mixed_tc_supported(wbits, M, N, K, block_size, x, x_dtype, w, false));
-      if (ok) variant = tuned;
-    }
-    if (use) {
+    if (variant == QMM_VARIANT_AUTO)
+      variant = choose_weight_only(wbits, M, N, K, block_size, x, x_dtype, out_dtype, w, zp != nullptr,
+                                   workspace && aligned(workspace, 256) ? workspace_bytes : 0, device_is_sm100());
+    if (variant == QMM_VARIANT_I8TC) {
       log_choice("weight_only", "i8tc", M, N, K);
       return launch_limb_tc(wbits, x, x_dtype, w, sc, out, out_dtype, M, N, K, block_size, 0, workspace, workspace_bytes,
                             as_stream(stream));
@@ -465,7 +469,6 @@ int qmm_weight_only_typed(int wbits, const void* x, int x_dtype, const void* w, 
     int rc = check_common(x, x_dtype, w, scale, out, out_dtype, M, N, K);
     if (rc != QMM_OK || M * N == 0) return rc;
     if (block_size > 0 && K % block_size != 0) return fail(QMM_ERR_BAD_SHAPE, "weight_only: block_size must divide K");
-    if (variant == QMM_VARIANT_AUTO) variant = pick_weight_only(wbits, M, N, K, block_size, x, x_dtype, w, zp != nullptr);
     if (variant != QMM_VARIANT_MMA || zp) return fail(QMM_ERR_UNSUPPORTED, "weight_only: variant %d reads fp32 scales only", variant);
     log_choice("weight_only", "mma", M, N, K);
     return launch_decode_mma(wbits, x, x_dtype, w, scale, scale_dtype, out, out_dtype, M, N, K, block_size, as_stream(stream));
@@ -534,7 +537,7 @@ int qmm_w4a16_perchannel_packed(const void* x, int x_dtype, const uint8_t* wp, c
   if (K % 2 != 0) return fail(QMM_ERR_BAD_SHAPE, "packed int4 needs an even K, got %lld", (long long)K);
   if (M * N == 0) return QMM_OK;
   cudaStream_t st = as_stream(stream);
-  if (variant == QMM_VARIANT_AUTO) variant = pick_weight_only(4, M, N, K, 0, x, x_dtype, wp, zp != nullptr);
+  if (variant == QMM_VARIANT_AUTO) variant = pick_weight_only(4, M, N, K, 0, x, x_dtype, wp, zp != nullptr, device_is_sm100());
   switch (variant) {
     case QMM_VARIANT_GENERIC:
       log_choice("w4a16_perchannel_packed", "generic", M, N, K);
@@ -599,6 +602,16 @@ int qmm_w8a8_gemm(const int8_t* xq, const int8_t* w, const float* w_scale, const
 // against 20.5; 14336 x 4096: 14 to 27 against 23).
 constexpr int64_t kW8A8DecodeTokens = 12;
 
+// qmm_w8a8_perchannel's AUTO: I8MMA is the decode kernel, the others stand for the quantizer and that GEMM.
+static int choose_w8a8(int64_t M, int64_t N, int64_t K, const void* x, int x_dt, const void* w, bool has_zp, bool sm100) {
+  const int gemm = sm100 && K >= 16 && K % 16 == 0 && aligned(w, 16) ? QMM_VARIANT_TCGEN05 : QMM_VARIANT_GENERIC;
+  // Nine to fifteen tokens on a small weight with short rows: the any-shape GEMM is done in the 8 us that the others need
+  // to start ([300,512] at 15 tokens 8.2 us, tcgen05 17; at 10 fp16 tokens 8.8, decode kernel 11).
+  if (M > 8 && M < 16 && K <= 512 && N * K <= (1 << 20)) return QMM_VARIANT_GENERIC;
+  if (M <= kW8A8DecodeTokens && decode_w8a8_supported(M, N, K, x, x_dt, w, has_zp)) return QMM_VARIANT_I8MMA;
+  return gemm;
+}
+
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 size_t qmm_workspace_size(int op, int64_t M, int64_t N, int64_t K) {
@@ -626,11 +639,9 @@ int qmm_w8a8_perchannel_typed(const void* x, int x_dtype, const int8_t* w, const
   const Scales sc{w_scale, zp, scale_dtype};
   int rc = check_common(x, x_dtype, w, w_scale, out, out_dtype, M, N, K);
   if (rc != QMM_OK || M * N == 0) return rc;
-  // decode batches: one kernel quantizes and multiplies, no scratch
-  // Nine to fifteen tokens on a small weight with short rows: the any-shape GEMM is done in the 8 us that the others need
-  // to start ([300,512] at 15 tokens 8.2 us, tcgen05 17; at 10 fp16 tokens 8.8, decode kernel 11).
-  if (variant == QMM_VARIANT_AUTO && M > 8 && M < 16 && K <= 512 && N * K <= (1 << 20)) variant = QMM_VARIANT_GENERIC;
-  if (variant == QMM_VARIANT_AUTO && M <= kW8A8DecodeTokens && decode_w8a8_supported(M, N, K, x, x_dtype, w, zp != nullptr)) {
+  if (variant == QMM_VARIANT_AUTO) variant = choose_w8a8(M, N, K, x, x_dtype, w, zp != nullptr, device_is_sm100());
+  if (variant == QMM_VARIANT_I8MMA) {
+    // one kernel quantizes and multiplies, no scratch
     log_choice("w8a8_perchannel", "i8mma", M, N, K);
     return launch_decode_w8a8(x, x_dtype, w, sc, out, out_dtype, M, N, K, saturate, as_stream(stream));
   }
@@ -790,23 +801,19 @@ int qmm_set_peer_wait_limit(double seconds) {
 
 const char* qmm_variant_for(int op, int64_t M, int64_t N, int64_t K, int64_t block_size, int has_zp) {
   // Shape-only view of the AUTO heuristic (pointer alignment is assumed to be fine).
-  const void* ok = reinterpret_cast<const void*>(uintptr_t(256));
+  const void* ok = any_pointer();
   switch (op) {
     case QMM_OP_W8A16_PERCHANNEL:
     case QMM_OP_W4A16_BLOCKWISE_PACKED:
     case QMM_OP_W4A16_PERCHANNEL_PACKED: {
       const int wbits = op == QMM_OP_W8A16_PERCHANNEL ? 8 : 4;
       const int64_t bs = op == QMM_OP_W4A16_BLOCKWISE_PACKED ? block_size : 0;
-      if (decode_mma_supported(wbits, M, N, K, bs, ok, QMM_BF16, ok, has_zp != 0)) return "mma";
-      if (mixed_tc_shape_ok(wbits, M, N, K, bs, QMM_BF16, has_zp != 0)) return "tcgen05";
-      if (gemv_nk_supported(wbits, M, N, K, bs, ok, QMM_BF16, ok)) return "gemv";
-      return "generic";
+      return variant_name(pick_weight_only(wbits, M, N, K, bs, ok, QMM_BF16, ok, has_zp != 0, true));
     }
     case QMM_OP_BLOCKWISE_SBN:
       return "generic";
     case QMM_OP_W8A8_PERCHANNEL:
-      if (K % 16 != 0 || K < 64) return (K % 16 == 0 && K >= 16) ? "tcgen05" : "generic";
-      return M <= kW8A8DecodeTokens && decode_w8a8_supported(M, N, K, ok, QMM_BF16, ok, has_zp != 0) ? "i8mma" : "tcgen05";
+      return variant_name(choose_w8a8(M, N, K, ok, QMM_BF16, ok, has_zp != 0, true));
     default:
       return "generic";
   }
