@@ -35,9 +35,14 @@ def test_against_the_oracle(dtype, with_zp, wbits, bs, N, K, M):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("with_zp", [False, True])
-@pytest.mark.parametrize("M,N,K", [(1, 16, 64), (3, 261, 1072), (8, 4099, 512), (9, 130, 2048), (17, 77, 144), (32, 300, 256)])
-def test_w8a8_equals_the_two_kernel_path(dtype, with_zp, M, N, K):
-  """Quantization inside the decode kernel: the same bits as the quantizer kernel followed by the any-shape GEMM."""
+@pytest.mark.parametrize("M,N,K,kernel", [(1, 16, 64, b"i8mma"), (3, 261, 1072, b"i8mma"), (8, 4099, 512, b"i8mma"), (9, 130, 2048, b"i8mma"),
+                                          (12, 77, 1040, b"i8mma"), (13, 300, 1040, b"tcgen05"), (17, 77, 144, b"tcgen05"),
+                                          (32, 300, 256, b"tcgen05")])
+def test_w8a8_equals_the_two_kernel_path(dtype, with_zp, M, N, K, kernel):
+  """Quantization inside the decode kernel, up to twelve tokens, and the quantizer with the tensor-core GEMM from there on:
+  the same bits as the quantizer kernel followed by the any-shape GEMM."""
+  L = xla_b200._capi.lib()
+  assert L.qmm_variant_for(xla_b200._capi.OP_W8A8_PERCHANNEL, M, N, K, 0, int(with_zp)) == kernel
   g = qc.gen(M + N + K)
   x = qc.activations(g, M, K, dtype, outliers=True).to(DEV)
   w, s = qc.int8_weight(g, N, K).to(DEV), qc.per_channel_scale(g, N).to(DEV)

@@ -45,3 +45,27 @@ def test_gate_up(M):
   out = torch.ops.xla_b200.quantized_gate_up(x.to(DEV), w, s, block_size=bs, int4_weight=True, weight_is_packed=True,
                                              out_dtype=torch.float32)
   assert qo.max_abs_rel(out[rows.to(DEV)], torch.nn.functional.silu(torch.as_tensor(gate)) * torch.as_tensor(up)) < 1e-4
+
+
+@pytest.mark.parametrize("wbits,M", [(4, 16), (8, 29), (4, 65), (8, 200)])
+def test_gate_up_with_blocks_of_64(wbits, M):
+  """The C ABI's fused form with scale blocks of 64 (the operator runs two steps there): up to 32 tokens on the split-activation
+  kernel, above on the tensor-memory kernel."""
+  from xla_b200 import _capi
+  L = _capi.lib()
+  g = qc.gen(M)
+  N, K, bs = 640, 1024, 64
+  weight = qc.int4_weight if wbits == 4 else qc.int8_weight
+  x, wg, wu = qc.activations(g, M, K), weight(g, N, K), weight(g, N, K)
+  sg, su = qc.blockwise_scale(g, K // bs, N) / 16, qc.blockwise_scale(g, K // bs, N)
+  to_device = lambda w: xla_b200.pack_int4(w.to(DEV)) if wbits == 4 else w.to(DEV)  # noqa: E731
+  w, s = xla_b200.interleave_gate_up(to_device(wg), to_device(wu), sg.to(DEV), su.to(DEV), bs)
+  xd, out = x.to(DEV), torch.empty(M, N, device=DEV)
+  nbytes = L.qmm_weight_only_workspace_size(M, K)
+  ws = torch.zeros(nbytes, dtype=torch.uint8, device=DEV)
+  with torch.cuda.device(0):
+    _capi.check(L.qmm_gate_up(wbits, xd.data_ptr(), _capi.BF16, w.data_ptr(), s.data_ptr(), out.data_ptr(), _capi.F32, M, 2 * N, K, bs,
+                              ws.data_ptr(), nbytes, _capi.stream_ptr(DEV)))
+  gate = torch.as_tensor(qo.quantized_matmul(x.float(), qc.to_sbn(wg, bs), sg, block_size=bs, dot_round=None))
+  up = torch.as_tensor(qo.quantized_matmul(x.float(), qc.to_sbn(wu, bs), su, block_size=bs, dot_round=None))
+  assert qo.max_abs_rel(out, torch.nn.functional.silu(gate) * up) < 1e-4

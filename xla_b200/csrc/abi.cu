@@ -598,17 +598,13 @@ int qmm_w8a8_gemm(const int8_t* xq, const int8_t* w, const float* w_scale, const
   return w8a8_gemm(xq, w, Scales{w_scale, zp, QMM_F32}, x_scale, xq_rowsum, acc_out, out, out_dtype, M, N, K, variant, as_stream(stream));
 }
 
-// Up to here the decode kernel beats the quantizer and the tcgen05 GEMM (4096 x 4096: 6.4 to 19.5 us at 1 to 12 tokens
-// against 20.5; 14336 x 4096: 14 to 27 against 23).
-constexpr int64_t kW8A8DecodeTokens = 12;
-
 // qmm_w8a8_perchannel's AUTO: I8MMA is the decode kernel, the others stand for the quantizer and that GEMM.
 static int choose_w8a8(int64_t M, int64_t N, int64_t K, const void* x, int x_dt, const void* w, bool has_zp, bool sm100) {
   const int gemm = sm100 && K >= 16 && K % 16 == 0 && aligned(w, 16) ? QMM_VARIANT_TCGEN05 : QMM_VARIANT_GENERIC;
   // Nine to fifteen tokens on a small weight with short rows: the any-shape GEMM is done in the 8 us that the others need
   // to start ([300,512] at 15 tokens 8.2 us, tcgen05 17; at 10 fp16 tokens 8.8, decode kernel 11).
   if (M > 8 && M < 16 && K <= 512 && N * K <= (1 << 20)) return QMM_VARIANT_GENERIC;
-  if (M <= kW8A8DecodeTokens && decode_w8a8_supported(M, N, K, x, x_dt, w, has_zp)) return QMM_VARIANT_I8MMA;
+  if (decode_w8a8_supported(M, N, K, x, x_dt, w, has_zp)) return QMM_VARIANT_I8MMA;
   return gemm;
 }
 
@@ -639,8 +635,9 @@ int qmm_w8a8_perchannel_typed(const void* x, int x_dtype, const int8_t* w, const
   const Scales sc{w_scale, zp, scale_dtype};
   int rc = check_common(x, x_dtype, w, w_scale, out, out_dtype, M, N, K);
   if (rc != QMM_OK || M * N == 0) return rc;
-  if (variant == QMM_VARIANT_AUTO) variant = choose_w8a8(M, N, K, x, x_dtype, w, zp != nullptr, device_is_sm100());
-  if (variant == QMM_VARIANT_I8MMA) {
+  const bool any = variant == QMM_VARIANT_AUTO;
+  if (any) variant = choose_w8a8(M, N, K, x, x_dtype, w, zp != nullptr, device_is_sm100());
+  if (any && variant == QMM_VARIANT_I8MMA) {
     // one kernel quantizes and multiplies, no scratch
     log_choice("w8a8_perchannel", "i8mma", M, N, K);
     return launch_decode_w8a8(x, x_dtype, w, sc, out, out_dtype, M, N, K, saturate, as_stream(stream));

@@ -42,6 +42,7 @@ namespace {
 constexpr int kRows = 16;       // weight rows per tile = MMA rows
 constexpr int kMaxTiles = 16;   // tiles per CTA
 constexpr int kMaxTokens = 16;
+static_assert(kW8A8DecodeTokens <= kMaxTokens, "per-token words in shared memory");
 constexpr size_t kSmemMax = 227 * 1024 - 512;  // static shared memory beside it
 
 struct Args {
@@ -200,8 +201,8 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 2 : 1) decode_i8_kernel(const
   constexpr int NA = NT <= 2 ? 2 : 1;  // accumulator sets: shorter MMA chains where a step has few of them
   constexpr int kSlot = slot_bytes(BLOCKED, NB);
   extern __shared__ __align__(128) uint8_t smem[];
-  __shared__ uint32_t s_max[kMaxTokens * 2];
-  __shared__ float s_pw[kMaxTokens * 2];
+  __shared__ uint32_t s_max[kMaxTokens];
+  __shared__ float s_pw[kMaxTokens];
   __shared__ uint8_t s_first[kMaxTiles];  // first warp whose piece reaches into a tile
   uint8_t* xs = smem;
   int* s_xs = reinterpret_cast<int*>(smem + p.xs_off);
@@ -311,7 +312,7 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 2 : 1) decode_i8_kernel(const
     // the first steps' scales, behind the weights under way, are waited for when the activations have been split
     if constexpr (BLOCKED) first_scales(copy_scales);
     asm volatile("cp.async.commit_group;" ::: "memory");
-    if (threadIdx.x < kMaxTokens * 2) s_max[threadIdx.x] = 0;
+    if (threadIdx.x < kMaxTokens) s_max[threadIdx.x] = 0;
     if (ZP)
       for (int i = threadIdx.x; i < p.S * cols; i += kThreads) s_xs[i] = 0;
     // groups complete in order: the activations' with the weights' first steps
@@ -592,12 +593,15 @@ int launch_nt(int nt, const Args& a, const Layout& l, cudaStream_t st) {
   switch (nt) {
     case 1: QMM_CASE(1);
     case 2: QMM_CASE(2);
-    case 3: QMM_CASE(3);
-    case 4: QMM_CASE(4);
-    default:
-      if constexpr (NL == 3) QMM_CASE(6);
-      return fail(QMM_ERR_UNSUPPORTED, "decode kernel: too many tokens");
   }
+  if constexpr (NL == 3) {
+    switch (nt) {
+      case 3: QMM_CASE(3);
+      case 4: QMM_CASE(4);
+      default: QMM_CASE(6);
+    }
+  }
+  return fail(QMM_ERR_UNSUPPORTED, "decode kernel: too many tokens");
 #undef QMM_CASE
 }
 
@@ -681,7 +685,7 @@ int launch_decode_i8(int wbits, const void* x, int x_dt, const void* w, const Sc
 }
 
 bool decode_w8a8_supported(int64_t M, int64_t N, int64_t K, const void* x, int x_dt, const void* w, bool has_zp) {
-  if (M > 2 * kMaxTokens || !shape_ok(8, 1, (int)dtype_size(x_dt), M, N, K, 0, has_zp)) return false;
+  if (M > kW8A8DecodeTokens || !shape_ok(8, 1, (int)dtype_size(x_dt), M, N, K, 0, has_zp)) return false;
   return aligned(x, 16) && aligned(w, 16);
 }
 

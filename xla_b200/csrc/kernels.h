@@ -60,7 +60,11 @@ int launch_decode_mma_allreduce(int wbits, const void* x, int x_dt, const void* 
 
 // ---- decode_i8.cu -------------------------------------------------------------------------
 // Decode kernels on the warp-level integer MMAs.  Weight-only: M <= 16, bf16/f16 activations, zero points allowed, the
-// limbs of all tokens have to fit shared memory.  W8A8: M <= 32, activations of any type quantized in the kernel.
+// limbs of all tokens have to fit shared memory.  W8A8: M <= 12, activations of any type quantized in the kernel.
+//
+// Up to twelve tokens the W8A8 form beats the quantizer and the tcgen05 GEMM (4096 x 4096: 6.4 to 19.5 us at 1 to 12 tokens
+// against 20.5; 14336 x 4096: 14 to 27 against 23).
+constexpr int64_t kW8A8DecodeTokens = 12;
 bool decode_i8_supported(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_size, const void* x, int x_dt, const void* w,
                          bool has_zp);
 int launch_decode_i8(int wbits, const void* x, int x_dt, const void* w, const Scales& sc, void* out, int out_dt, int64_t M, int64_t N,
