@@ -177,6 +177,25 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int tm = tile % p.tiles_m, tn = tile / p.tiles_m;
       const int ab = tcount % kAccBufs;
       const uint32_t aph = (tcount / kAccBufs) & 1;
+      const int e = threadIdx.x - 64;  // 0..127 among the epilogue threads
+      if (p.out) {
+        // the scales and zero points of the tile's columns, in fp32, under the MMAs
+        if (p.tma_store && e == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // staging free again
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        uint32_t sb[BN / 128], zb[BN / 128];  // all loads under way together
+#pragma unroll
+        for (int i = 0; i < BN / 128; ++i) {
+          const int64_t n = (int64_t)tn * BN + e + 128 * i;
+          sb[i] = n < p.N ? load_scale_bits(p.w_scale, n, p.s_dt) : 0u;
+          zb[i] = p.zp && n < p.N ? load_scale_bits(p.zp, n, p.s_dt) : 0u;
+        }
+#pragma unroll
+        for (int i = 0; i < BN / 128; ++i) {
+          s_ws[e + 128 * i] = scale_value(sb[i], p.s_dt);
+          s_zp[e + 128 * i] = scale_value(zb[i], p.s_dt);
+        }
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+      }
       ptx::mbar_wait(&tmem_full[ab], aph, abort_flag, p.err_word, ptx::kErrWaitTmemFull);
       ptx::tcgen05_fence_after();
       const int64_t m = (int64_t)tm * BM + quad * 32 + lane;
@@ -187,15 +206,6 @@ __global__ void __launch_bounds__(kThreads, 1)
       const uint32_t taddr = tmem_base + ab * BN + ((uint32_t)(quad * 32) << 16);
       if (p.tma_store) {
         // ---- 16-bit output: dequantise into a swizzled shared-memory tile, one TMA store per 64 columns ----
-        const int e = threadIdx.x - 64;  // 0..127 among the epilogue threads
-        if (e == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // staging free again
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        for (int j = e; j < BN; j += 128) {
-          const int64_t n = (int64_t)tn * BN + j;
-          s_ws[j] = n < p.N ? load_as_f32(p.w_scale, n, p.s_dt) : 0.f;
-          s_zp[j] = (p.zp && n < p.N) ? load_as_f32(p.zp, n, p.s_dt) : 0.f;
-        }
-        asm volatile("bar.sync 1, 128;" ::: "memory");
         const int rl = quad * 32 + lane;  // row inside the tile
         const uint32_t row_base = ptx::smem_u32(staging) + rl * 128;
         const uint32_t sw = (uint32_t)(rl & 7);
@@ -267,11 +277,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (live && p.out) {
           float v[32];
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const int64_t n = (n0 + j < p.N) ? n0 + j : p.N - 1;
-            const float z = p.zp ? load_as_f32(p.zp, n, p.s_dt) : 0.f;
-            v[j] = w8a8_dequant((int32_t)r[j], load_as_f32(p.w_scale, n, p.s_dt), p.zp ? &z : nullptr, rs, xs);
-          }
+          for (int j = 0; j < 32; ++j)
+            v[j] = w8a8_dequant((int32_t)r[j], s_ws[c * 32 + j], p.zp ? &s_zp[c * 32 + j] : nullptr, rs, xs);
           if (p.out_dt == QMM_F32)
             store_row_chunk<float>(reinterpret_cast<float*>(p.out) + m * p.N + n0, v, ncols, p.out_vec != 0);
           else if (p.out_dt == QMM_BF16)
