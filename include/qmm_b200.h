@@ -189,8 +189,9 @@ QMM_API int qmm_weight_only(int wbits, const void* x, int x_dtype, const void* w
 /*
  * The same with scales and zero points of type scale_dtype (one type for both): what the buffers of a quantized 16-bit
  * model hold, read as they are.  Results are those of the fp32 call with the same values.  QMM_ERR_UNSUPPORTED, before
- * anything is launched, where the kernel that `variant` stands for at this shape reads fp32 only: the any-shape, GEMV
- * and TCGEN05 kernels; MMA, and TMEM with scale blocks, unless scale_dtype is x_dtype; blockwise scales with an odd N or not 4-byte aligned.  Callers
+ * anything is launched, where the kernel that `variant` stands for at this shape reads fp32 only: the any-shape and GEMV
+ * kernels; MMA, and TMEM with scale blocks, unless scale_dtype is x_dtype; blockwise scales that do not start on
+ * 4 bytes, and in TMEM an odd number of them.  Callers
  * then convert the scales and call qmm_weight_only.
  */
 QMM_API int qmm_weight_only_typed(int wbits, const void* x, int x_dtype, const void* w, const void* scale, const void* zp,

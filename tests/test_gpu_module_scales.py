@@ -1,6 +1,6 @@
 """A module's scales and zero points are read on every call, in the type they are held in: 16-bit ones give the bits of the
 fp32 call with the same values in every kernel that a module reaches, and a write to the buffers shows in the next call
-however it was made.  (N odd or a buffer at an odd element: the calls that convert the scales first.)"""
+however it was made.  (Scale blocks in a buffer at an odd element, and in the tensor-memory kernel an odd number of them, are converted first.)"""
 import pytest
 import torch
 
@@ -19,6 +19,15 @@ CASES = [
     (8, 128, False, False, 1000, 2048, 70, False), (8, -1, False, False, 1025, 2048, 300, True), (8, 256, True, False, 2048, 1024, 9, False),
     (4, 256, False, False, 4096, 2048, 520, False), (8, -1, False, True, 514, 1024, 4, False), (8, -1, True, True, 300, 1024, 40, True),
     (8, -1, True, True, 300, 512, 10, False), (4, 128, True, False, 301, 1024, 29, False), (8, 64, True, False, 300, 832, 9, True),
+    # odd row counts: 16-bit pairs that span two blocks; with an odd number of blocks a last value that has no partner
+    (4, 128, False, False, 1027, 128 * 33, 1, False), (8, 64, True, False, 33, 192, 2, False), (4, 64, True, False, 131, 320, 5, False),
+    (4, 128, True, False, 257, 128 * 9, 40, False), (8, 64, True, False, 385, 64 * 15, 33, False), (4, 128, False, False, 129, 128 * 31, 16, False),
+    (4, 128, False, False, 4097, 128 * 63, 24, False), (4, 256, False, False, 3841, 256 * 17, 12, False), (8, 128, False, False, 513, 128 * 21, 100, False),
+    (4, 128, True, False, 1023, 128 * 17, 16, False), (4, 128, True, False, 1023, 128 * 16, 29, False),
+    (4, 128, True, False, 257, 128 * 10, 3, False), (4, 64, True, False, 131, 384, 5, False), (4, 128, False, False, 4097, 128 * 64, 24, False),
+    (8, 64, True, False, 385, 64 * 16, 33, False), (4, 256, False, False, 3841, 256 * 16, 12, False),
+    # small weights above 32 tokens: the conversion kernel
+    (4, -1, False, False, 1976, 1504, 45, True), (8, -1, False, False, 269, 1536, 300, False), (8, 128, False, False, 301, 1024, 45, True),
 ]
 
 

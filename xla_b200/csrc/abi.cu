@@ -249,7 +249,7 @@ int qmm_w8a16_perchannel(const void* x, int x_dtype, const int8_t* w, const floa
     case QMM_VARIANT_TCGEN05:
       log_choice("w8a16_perchannel", "tcgen05", M, N, K);
       if (zp) return fail(QMM_ERR_UNSUPPORTED, "tcgen05 weight-only kernel does not take a zero point");
-      return launch_mixed_tc(8, x, x_dtype, w, scale, out, out_dtype, M, N, K, 0, st);
+      return launch_mixed_tc(8, x, x_dtype, w, scale, QMM_F32, out, out_dtype, M, N, K, 0, st);
     default:
       return fail(QMM_ERR_UNSUPPORTED, "unknown variant %d", variant);
   }
@@ -299,7 +299,7 @@ int qmm_w4a16_blockwise_packed(const void* x, int x_dtype, const uint8_t* wp, co
     case QMM_VARIANT_TCGEN05:
       log_choice("w4a16_blockwise_packed", "tcgen05", M, N, K);
       if (zp) return fail(QMM_ERR_UNSUPPORTED, "tcgen05 weight-only kernel does not take a zero point");
-      return launch_mixed_tc(4, x, x_dtype, wp, scale, out, out_dtype, M, N, K, block_size, st);
+      return launch_mixed_tc(4, x, x_dtype, wp, scale, QMM_F32, out, out_dtype, M, N, K, block_size, st);
     default:
       return fail(QMM_ERR_UNSUPPORTED, "unknown variant %d", variant);
   }
@@ -329,7 +329,7 @@ int qmm_w8a16_blockwise(const void* x, int x_dtype, const int8_t* w, const float
     case QMM_VARIANT_TCGEN05:
       log_choice("w8a16_blockwise", "tcgen05", M, N, K);
       if (zp) return fail(QMM_ERR_UNSUPPORTED, "tcgen05 weight-only kernel does not take a zero point");
-      return launch_mixed_tc(8, x, x_dtype, w, scale, out, out_dtype, M, N, K, block_size, st);
+      return launch_mixed_tc(8, x, x_dtype, w, scale, QMM_F32, out, out_dtype, M, N, K, block_size, st);
     default:
       return fail(QMM_ERR_UNSUPPORTED, "unknown variant %d", variant);
   }
@@ -465,11 +465,16 @@ int qmm_weight_only_typed(int wbits, const void* x, int x_dtype, const void* w, 
                             as_stream(stream));
   }
   if (scale_dtype != QMM_F32) {
-    // the entry points below read fp32 scales; the one kernel behind them that also takes others is called here
+    // the entry points below read fp32 scales; the two kernels behind them that also take others are called here
     int rc = check_common(x, x_dtype, w, scale, out, out_dtype, M, N, K);
     if (rc != QMM_OK || M * N == 0) return rc;
     if (block_size > 0 && K % block_size != 0) return fail(QMM_ERR_BAD_SHAPE, "weight_only: block_size must divide K");
-    if (variant != QMM_VARIANT_MMA || zp) return fail(QMM_ERR_UNSUPPORTED, "weight_only: variant %d reads fp32 scales only", variant);
+    if ((variant != QMM_VARIANT_MMA && variant != QMM_VARIANT_TCGEN05) || zp)
+      return fail(QMM_ERR_UNSUPPORTED, "weight_only: variant %d reads fp32 scales only", variant);
+    if (variant == QMM_VARIANT_TCGEN05) {
+      log_choice("weight_only", "tcgen05", M, N, K);
+      return launch_mixed_tc(wbits, x, x_dtype, w, scale, scale_dtype, out, out_dtype, M, N, K, block_size, as_stream(stream));
+    }
     log_choice("weight_only", "mma", M, N, K);
     return launch_decode_mma(wbits, x, x_dtype, w, scale, scale_dtype, out, out_dtype, M, N, K, block_size, as_stream(stream));
   }
@@ -552,7 +557,7 @@ int qmm_w4a16_perchannel_packed(const void* x, int x_dtype, const uint8_t* wp, c
     case QMM_VARIANT_TCGEN05:
       log_choice("w4a16_perchannel_packed", "tcgen05", M, N, K);
       if (zp) return fail(QMM_ERR_UNSUPPORTED, "tcgen05 weight-only kernel does not take a zero point");
-      return launch_mixed_tc(4, x, x_dtype, wp, scale, out, out_dtype, M, N, K, 0, st);
+      return launch_mixed_tc(4, x, x_dtype, wp, scale, QMM_F32, out, out_dtype, M, N, K, 0, st);
     default:
       return fail(QMM_ERR_UNSUPPORTED, "unknown variant %d", variant);
   }

@@ -111,24 +111,33 @@ inline const void* elements_from(const void* p, int64_t n, int dt) {
 }
 
 // Kernels that stream block scales copy them in 32-bit words: one fp32 value, or the pair of 16-bit values that holds the
-// wanted one.  For that every row of a 16-bit [S,N] tensor has to start on a word.  (Per channel they are read one by one.)
-inline bool scale_words_ok(const Scales& s, int64_t N, int64_t block_size) {
-  return s.dt == QMM_F32 || block_size <= 0 || (N % 2 == 0 && aligned(s.scale, 4) && aligned(s.zp, 4));
+// wanted one.  For that a 16-bit tensor has to start on a word.  (Per channel the scales are read one by one.)
+inline bool scale_words_ok(const Scales& s, int64_t block_size) {
+  return s.dt == QMM_F32 || block_size <= 0 || (aligned(s.scale, 4) && aligned(s.zp, 4));
 }
+// An odd number of 16-bit scales: the last one's word would reach beyond the tensor, so it is copied by itself.
+inline int scale_tail(const Scales& s, int64_t blocks, int64_t N) { return s.dt != QMM_F32 && blocks * N % 2 != 0; }
 
-// Byte offset of the word that holds element n
+// Copies the word that holds the scale at `src` to shared memory.  W16: 16-bit scales; a template parameter of the kernels,
+// because their loops have no register to spare for the conversion (decided at run time it cost fp32 scales 2 to 25 %: int4
+// block 128, [57344,8192] and [8192,28672] at 64 tokens 182 us, up to 228).
 template <bool W16>
-__device__ __forceinline__ int64_t scale_word_offset(int64_t n) {
-  return W16 ? (n & ~1ll) * 2 : n * 4;
+__device__ __forceinline__ void copy_scale_word(uint32_t dst, const uint8_t* src) {
+  const uintptr_t at = reinterpret_cast<uintptr_t>(src);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(W16 ? at & ~(uintptr_t)3 : at) : "memory");
 }
 
-// The scale of element n in the word that was copied for it.  W16: 16-bit scales, of type T if that is given.  A template
-// parameter of the kernels, because their loops have no register to spare for the conversion (decided at run time it cost
-// fp32 scales 2 to 25 %: int4 block 128, [57344,8192] and [8192,28672] at 64 tokens 182 us, up to 228).
+__device__ __forceinline__ void copy_last_scale(uint32_t dst, const uint8_t* src) {
+  asm volatile("st.shared.u16 [%0], %1;" ::"r"(dst), "h"(ld_ordered(reinterpret_cast<const unsigned short*>(src))) : "memory");
+}
+
+// The scale in a copied word: of row n (counted from an even one) and block b of a weight with N rows; T: its type, if known.
+// The odd rows, and with an odd N those of the other parity in every second block, are the second value of a pair.
 template <bool W16, typename T = void>
-__device__ __forceinline__ float scale_in(const uint32_t* word, int n, int dt) {
+__device__ __forceinline__ float scale_in(const uint32_t* word, int n, int b, int N, int dt) {
   if (!W16) return __uint_as_float(*word);
-  const unsigned short h = reinterpret_cast<const unsigned short*>(word)[n & 1];
+  const uint32_t at = ((uint32_t)n & 1u) ^ ((uint32_t)b & (uint32_t)N & 1u);
+  const unsigned short h = reinterpret_cast<const unsigned short*>(word)[at];
   if (std::is_same<T, __half>::value || (std::is_void<T>::value && dt == QMM_F16)) return __half2float(__ushort_as_half(h));
   return __uint_as_float((uint32_t)h << 16);
 }

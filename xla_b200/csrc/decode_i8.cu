@@ -59,6 +59,7 @@ struct Args {
   int fold_steps;      // steps per scale block (0: per channel)
   int fold_shift;      // log2(fold_steps), or -1
   int S;               // scale blocks (1: per channel)
+  int scale_tail;      // an odd number of 16-bit block scales
   int gate_up;
   int saturate;        // W8A8: clamp (1) or wrap (0) +128
   int xpitch;          // bytes between limb rows in shared memory
@@ -232,17 +233,21 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 2 : 1) decode_i8_kernel(const
   const uint8_t *lp0, *lp1;
   const uint8_t* lsc = nullptr;  // this lane's row of the scales (lanes 0..15) or zero points (lanes 16..31)
   auto scale_row = [&](int tile) {
-    return static_cast<const uint8_t*>(ZP && lane >= 16 ? p.zp : p.scale) + scale_word_offset<W16>(min(tile * kRows + (lane & 15), n_last));
+    return static_cast<const uint8_t*>(ZP && lane >= 16 ? p.zp : p.scale) + min(tile * kRows + (lane & 15), n_last) * (int64_t)(W16 ? 2 : 4);
   };
   // the block scales and zero points of a step, into its ring slot
   auto copy_scales = [&](uint32_t slot, const uint8_t* row, int step) {
     if (!ZP && lane >= 16) return;
+    auto copy = [&](uint32_t dst, int b) {
+      const uint8_t* src = row + b * p.sc_pitch;
+      if (W16 && p.scale_tail && b + 1 == p.S && row == scale_row(n_last / kRows + 1)) copy_last_scale(dst, src);
+      else copy_scale_word<W16>(dst, src);
+    };
     if constexpr (HALF) {
-      cp_async_small<4>(slot + 1024 + lane * 4, row + (2 * step) * p.sc_pitch);
-      if (2 * step + 1 < p.S) cp_async_small<4>(slot + 1152 + lane * 4, row + (2 * step + 1) * p.sc_pitch);
+      copy(slot + 1024 + lane * 4, 2 * step);
+      if (2 * step + 1 < p.S) copy(slot + 1152 + lane * 4, 2 * step + 1);
     } else {
-      const int b = p.fold_shift >= 0 ? step >> p.fold_shift : step / p.fold_steps;
-      cp_async_small<4>(slot + 1024 + lane * 4, row + b * p.sc_pitch);
+      copy(slot + 1024 + lane * 4, p.fold_shift >= 0 ? step >> p.fold_shift : step / p.fold_steps);
     }
   };
   auto set_tile = [&]() {
@@ -371,7 +376,8 @@ __global__ void __launch_bounds__(W * 32, W == 8 ? 2 : 1) decode_i8_kernel(const
   // zero-point term
   auto fold = [&](const uint32_t* sc, int b, bool zp_too) {
     if constexpr (BLOCKED) {
-      auto value = [&](int i) { return scale_in<W16>(sc + i, g, p.s_dt); };  // (rows g and g + 8; tiles start at even rows)
+      // (rows g and g + 8 of a tile, which starts at an even row)
+      auto value = [&](int i) { return scale_in<W16>(sc + i, g, b, (int)p.N, p.s_dt); };
       const float s0 = value(g), s1 = value(g + 8);
 #pragma unroll
       for (int i = 0; i < NT; ++i) {
@@ -644,6 +650,7 @@ Args make_args(int wbits, const void* x, int x_dt, const void* w, const Scales& 
   a.tiles_lo = tiles / l.grid;
   a.tiles_extra = tiles % l.grid;
   a.S = block_size > 0 ? (int)(K / block_size) : 1;
+  a.scale_tail = scale_tail(sc, a.S, N);
   a.fold_steps = block_size > 0 ? std::max(1, (int)(block_size / vps)) : 0;
   a.fold_shift = -1;
   for (int s = 0; s < 16; ++s)
@@ -670,7 +677,7 @@ int launch_decode_i8(int wbits, const void* x, int x_dt, const void* w, const Sc
   const bool zp = sc.zp != nullptr;
   if (gate_up && N % 16 != 0)
     return fail(QMM_ERR_BAD_SHAPE, "fused gate/up epilogue: the interleaved weight needs a multiple of 16 rows, got %lld", (long long)N);
-  if (!decode_i8_supported(wbits, M, N, K, block_size, x, x_dt, w, zp) || !scale_words_ok(sc, N, block_size))
+  if (!decode_i8_supported(wbits, M, N, K, block_size, x, x_dt, w, zp) || !scale_words_ok(sc, block_size))
     return fail(QMM_ERR_UNSUPPORTED, "integer decode kernel: M=%lld N=%lld K=%lld bs=%lld not supported", (long long)M, (long long)N,
                 (long long)K, (long long)block_size);
   const bool half = half_blocks(wbits, block_size);

@@ -652,11 +652,6 @@ __global__ void __launch_bounds__(kStagedWarps * 32, 1)
     if (active && wk < steps) {
       fetch_w(wk, qa);
       fetch_w(wk + WK, qb);
-      if (first && blockwise) {
-        const int b = spb_shift >= 0 ? (wk >> spb_shift) : (wk / steps_per_block);
-#pragma unroll
-        for (int r = 0; r < 2; ++r) prefetch_l2(srow[r] + (int64_t)b * N);
-      }
     }
     if (first) {
       // weights are static: their first loads may overlap the previous kernel of the stream; the scales, the

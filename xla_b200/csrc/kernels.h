@@ -124,7 +124,7 @@ int launch_w8a8_tc(const int8_t* xq, const int8_t* w, const Scales& sc, const fl
 bool mixed_tc_shape_ok(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_size, int x_dt, bool has_zp);
 bool mixed_tc_supported(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_size, const void* x,
                         int x_dt, const void* w, bool has_zp);
-int launch_mixed_tc(int wbits, const void* x, int x_dt, const void* w, const float* scale,
+int launch_mixed_tc(int wbits, const void* x, int x_dt, const void* w, const void* scale, int scale_dt,
                     void* out, int out_dt, int64_t M, int64_t N, int64_t K, int64_t block_size,
                     cudaStream_t st);
 

@@ -99,6 +99,7 @@ struct Params {
   const void* zp;      // like scale, or null
   int s_dt;
   int64_t sc_pitch;    // bytes from one scale block to the next
+  int scale_tail;      // an odd number of 16-bit block scales
   uint32_t as_is;      // the byte permutation that changes nothing
   const float* xs;     // with zp: [S][xs_pitch] sums of the fixed-point activations over each scale block
   int xs_pitch;
@@ -233,9 +234,6 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
 }
 __device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 
 __device__ __forceinline__ float silu_mul(float gate, float up) { return gate / (1.f + expf(-gate)) * up; }
@@ -839,11 +837,16 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
         const int b0 = p.mode == kBlockSlots ? u0 : s0 * per_slot, b1 = p.mode == kBlockSlots ? u1 : s1 * per_slot;
         const uint32_t* ring = scale_base + rl;
         const uint32_t ring_u32 = ptx::smem_u32(ring);
-        const uint8_t* word_n = static_cast<const uint8_t*>(p.scale) + scale_word_offset<W16>(nc);
-        auto copied = [&](int i) { return scale_in<W16>(ring + i * 128, rl, p.s_dt); };
+        // (a tile starts at an even row)
+        auto copied = [&](int b) { return scale_in<W16>(ring + (b % R) * 128, rl, min(b, p.S - 1), (int)p.ld, p.s_dt); };
         auto fetch = [&](int b) {
           // (a last slot may hold fewer blocks than the others: their sums are zero, but the factor has to be a number)
-          if (b < b1) cp_async4(ring_u32 + (uint32_t)(b % R) * 512, word_n + min(b, p.S - 1) * p.sc_pitch);
+          if (b < b1) {
+            const uint32_t dst = ring_u32 + (uint32_t)(b % R) * 512;
+            const uint8_t* src = scale_n + min(b, p.S - 1) * p.sc_pitch;
+            if (W16 && p.scale_tail && b + 1 >= p.S && n >= p.N - 1) copy_last_scale(dst, src);
+            else copy_scale_word<W16>(dst, src);
+          }
           asm volatile("cp.async.commit_group;" ::: "memory");
         };
 #pragma unroll 1
@@ -853,7 +856,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
           for (int b = b0; b < b1; b += 2) {
             wait_acc();
             asm volatile("cp.async.wait_group %0;" ::"n"(R - 2) : "memory");
-            const float sc0 = copied(b % R), sc1 = copied((b + 1) % R);
+            const float sc0 = copied(b), sc1 = copied(b + 1);
             const uint32_t a = lane_addr + buf * (2 * NCOLS) + col0;
             fold_region<DC, MTD, NL, true>(a, sc0, total, false, release);
             fold_region<DC, MTD, NL, true>(a + NCOLS, sc1, total, true, release);
@@ -866,7 +869,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
           for (int b = b0; b < b1; ++b) {
             wait_acc();
             asm volatile("cp.async.wait_group %0;" ::"n"(R - 1) : "memory");
-            const float sc = copied(b % R);
+            const float sc = copied(b);
             if (small) fold_region<DC, MTD, NL, true>(lane_addr + buf * NCOLS + col0, sc, total, true, release);
             else fold_region<DC, MTD, NL, false>(lane_addr + buf * NCOLS + col0, sc, total, true, release);
             next_acc();
@@ -1422,7 +1425,7 @@ int launch_limb_impl(int wbits, const void* x, int x_dt, const void* w, const Sc
                      int64_t K, int64_t block_size, int gate_up, void* workspace, size_t workspace_bytes, float pw_mul, int w_dep,
                      cudaStream_t st) {
   const bool zp = scales.zp != nullptr;
-  if (!limb_tc_supported(wbits, M, N, K, block_size, x, x_dt, w, zp) || !scale_words_ok(scales, N, block_size))
+  if (!limb_tc_supported(wbits, M, N, K, block_size, x, x_dt, w, zp) || !scale_words_ok(scales, block_size))
     return fail(QMM_ERR_UNSUPPORTED,
                 "split-activation tensor-core kernel: needs an sm_100 device, K >= 128 and a multiple of %d, "
                 "block_size 64, 128 or a multiple of 256, 16-byte aligned x/w (M=%lld N=%lld K=%lld bs=%lld)",
@@ -1513,6 +1516,7 @@ int launch_limb_impl(int wbits, const void* x, int x_dt, const void* w, const Sc
   p.slots = (int)ceil_div(K, kSlotK);
   p.mode = block_size <= 0 ? kPerChannel : (block_size == kTileK ? kBlock128 : block_size == 64 ? kBlock64 : kBlockSlots);
   p.S = block_size > 0 ? (int)(K / block_size) : 1;
+  p.scale_tail = scale_tail(scales, p.S, N);
   p.spu = p.mode == kBlockSlots ? (int)(block_size / kSlotK) : 1;
   p.ut = (int)ceil_div(p.slots, p.spu);
   p.partial = sc.partial;

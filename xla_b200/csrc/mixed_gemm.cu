@@ -43,7 +43,8 @@ constexpr int kABytes = BMW * BK * 2;
 constexpr int kThreads = 512;
 
 struct Params {
-  const float* scale;
+  const void* scale;  // of type s_dt
+  int s_dt;
   void* out;
   int out_dt;
   int64_t M, N, K;
@@ -433,9 +434,10 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int j = 0; j < MP; ++j) acc[j] = 0.f;
       for (int b = 0; b < n_blocks; ++b) {
         const int buf = b & 1;
-        const float s = n_ok ? (p.blockwise ? __ldg(p.scale + (int64_t)(block0 + b) * p.N + n) : 1.f) : 0.f;
+        const uint32_t sb = p.blockwise && n_ok ? load_scale_bits(p.scale, (int64_t)(block0 + b) * p.N + n, p.s_dt) : 0u;
         ptx::mbar_wait_warp<32>(&acc_full[buf], (b >> 1) & 1, abort_flag, p.err_word, ptx::kErrWaitTmemFull);
         ptx::tcgen05_fence_after();
+        const float s = p.blockwise ? scale_value(sb, p.s_dt) : n_ok ? 1.f : 0.f;
 #pragma unroll
         for (int c = 0; c < MP / 16; ++c) {
           uint32_t rr[16];
@@ -473,14 +475,14 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       }
       if (n_ok && krank == 0) {
-        const float ps = p.blockwise ? 1.f : __ldg(p.scale + n);
+        const float ps = p.blockwise ? 1.f : load_as_f32(p.scale, n, p.s_dt);
 #pragma unroll
         for (int j = 0; j < MP; ++j)
           if (m0 + j < p.M) store_from_f32(p.out, (m0 + j) * p.N + n, p.out_dt, acc[j] * ps);
       }
     } else {
       // large token tiles: one scale block only (per-channel); scale and store straight from TMEM
-      float s = n_ok ? __ldg(p.scale + n) : 0.f;
+      float s = n_ok ? load_as_f32(p.scale, n, p.s_dt) : 0.f;
       if (my_tiles > 0) {
         ptx::mbar_wait_warp(&acc_full[0], 0, abort_flag, p.err_word, ptx::kErrWaitTmemFull);
         ptx::tcgen05_fence_after();
@@ -592,7 +594,7 @@ bool mixed_tc_supported(int wbits, int64_t M, int64_t N, int64_t K, int64_t bloc
   return device_is_sm100();
 }
 
-int launch_mixed_tc(int wbits, const void* x, int x_dt, const void* w, const float* scale, void* out,
+int launch_mixed_tc(int wbits, const void* x, int x_dt, const void* w, const void* scale, int scale_dt, void* out,
                     int out_dt, int64_t M, int64_t N, int64_t K, int64_t block_size, cudaStream_t st) {
   if (!mixed_tc_supported(wbits, M, N, K, block_size, x, x_dt, w, false))
     return fail(QMM_ERR_UNSUPPORTED,
@@ -614,6 +616,7 @@ int launch_mixed_tc(int wbits, const void* x, int x_dt, const void* w, const flo
   if (rc != QMM_OK) return rc;
   Params p;
   p.scale = scale;
+  p.s_dt = scale_dt;
   p.out = out;
   p.out_dt = out_dt;
   p.M = M;

@@ -276,9 +276,13 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         if (live && p.out) {
           float v[32];
+          if (p.zp) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
-            v[j] = w8a8_dequant((int32_t)r[j], s_ws[c * 32 + j], p.zp ? &s_zp[c * 32 + j] : nullptr, rs, xs);
+            for (int j = 0; j < 32; ++j) v[j] = w8a8_dequant((int32_t)r[j], s_ws[c * 32 + j], &s_zp[c * 32 + j], rs, xs);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = w8a8_dequant((int32_t)r[j], s_ws[c * 32 + j], nullptr, rs, xs);
+          }
           if (p.out_dt == QMM_F32)
             store_row_chunk<float>(reinterpret_cast<float*>(p.out) + m * p.N + n0, v, ncols, p.out_vec != 0);
           else if (p.out_dt == QMM_BF16)
