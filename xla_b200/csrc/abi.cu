@@ -191,11 +191,16 @@ static int pick_weight_only(int wbits, int64_t M, int64_t N, int64_t K, int64_t 
   return QMM_VARIANT_GENERIC;
 }
 
-// AUTO's choice between the two warp-level decode kernels.  The integer one streams weights 1.5 times faster, but every
+// AUTO's choice between the two warp-level decode kernels (asked before the measured table, which knows neither this kernel
+// nor tmem_gemm.cu).  The integer one streams weights 1.5 times faster, but every
 // CTA of it first splits all activations into limbs, about 0.6 us per token at K = 4096, in proportion to M * K; the
 // gain is proportional to the weight bytes.  K cancels: it wins at one token, and up to one token per 1850 bytes of
 // weight column (14336 int8 outputs: 7 tokens; measured 15.1 against 16.7 us at 4, equal at 8; 4096 outputs: 2).
 // Zero points, scale blocks of 64 and ragged K are beyond the other kernel.
+// The line was drawn against decode_mma.cu.  limb_gemm.cu, which the table names on the largest weights, is the faster one
+// there from three tokens on, and at every batch on int8: int4 block 128 [28672,8192] 25.1 us here and 28.0 there at one
+// token, 27.6 and 28.5 at two, 34.5 and 29.0 at five; [57344,8192] 48.9 and 45.7 at one, 65.0 and 47.1 at five; int8
+// [28672,8192] 43.0 and 39.6 at one, 52.2 and 40.6 at five; [14336,4096] 11.8 and 13.7 at one, 15.6 and 13.8 at four.
 static bool use_decode_i8(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, const void* x, int x_dt, const void* w, bool has_zp) {
   if (!decode_i8_supported(wbits, M, N, K, bs, x, x_dt, w, has_zp)) return false;
   return M == 1 || M * 1850 <= N * wbits / 8 || !decode_mma_supported(wbits, M, N, K, bs, x, x_dt, w, has_zp);
@@ -211,7 +216,7 @@ static bool use_decode_i8(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs
 //                  512 tokens 135 us against 232).
 //   int4           above 64 tokens, when the (128-row, up to 192-token) items fill two thirds of the SMs: fewer leave it
 //                  to the split-activation kernel's narrower ones ([4096,4096] at 128 tokens 23 us against 19;
-//                  [14336,4096] at 96 tokens 27 against 35, [28672,8192] at 512 tokens 284 against 340).  Per channel up
+//                  [14336,4096] at 96 tokens 27 against 35, [28672,8192] at 512 tokens 266 against 337).  Per channel up
 //                  to 384 tokens, from where that kernel expands the weights once.
 //   fp32 results   above 64 tokens, when the items fill half of the SMs: the other kernel needs a third limb per token
 //                  there (int8 [28672,8192] at 512 tokens 257 us against 312, [2432,9248] at 763 tokens 49 against 74).
@@ -606,10 +611,12 @@ int qmm_w8a8_gemm(const int8_t* xq, const int8_t* w, const float* w_scale, const
 // qmm_w8a8_perchannel's AUTO: I8MMA is the decode kernel, the others stand for the quantizer and that GEMM.
 static int choose_w8a8(int64_t M, int64_t N, int64_t K, const void* x, int x_dt, const void* w, bool has_zp, bool sm100) {
   const int gemm = sm100 && K >= 16 && K % 16 == 0 && aligned(w, 16) ? QMM_VARIANT_TCGEN05 : QMM_VARIANT_GENERIC;
-  // Nine to fifteen tokens on a small weight with short rows: the any-shape GEMM is done in the 8 us that the others need
-  // to start ([300,512] at 15 tokens 8.2 us, tcgen05 17; at 10 fp16 tokens 8.8, decode kernel 11).
-  if (M > 8 && M < 16 && K <= 512 && N * K <= (1 << 20)) return QMM_VARIANT_GENERIC;
   if (decode_w8a8_supported(M, N, K, x, x_dt, w, has_zp)) return QMM_VARIANT_I8MMA;
+  // Thirteen to fifteen tokens on a small weight with short rows and a row count that rules the GEMM's TMA stores out: the
+  // any-shape kernel ([300,512] at 15 tokens 12.3 us, the GEMM 16.4).  Where N is a multiple of eight the GEMM is the faster
+  // one ([512,512] 10.2 against 12.3, [2048,512] 10.2 against 16.4, [4096,256] 10.2 against 18.4), and up to twelve tokens
+  // the decode kernel (9 tokens on [300,512] 8.5 against 12.3, on [2048,512] 10.6 against 14.3).
+  if (M > 8 && M < 16 && N % 8 != 0 && K <= 512 && N * K <= (1 << 20)) return QMM_VARIANT_GENERIC;
   return gemm;
 }
 
