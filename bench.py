@@ -362,7 +362,7 @@ def _variant_name(wbits, M, N, K, bs):
   from xla_b200 import _capi
   L = _capi.lib()
   name = L.qmm_weight_only_variant_for(wbits, M, N, K, bs, 0).decode()
-  return name + (" (tuned table)" if L.qmm_tuned_variant(wbits, M, N, K, bs) else " (shape rule)")
+  return name + (" (tuned table)" if L.qmm_tuned_variant(wbits, M, N, K, bs) == _capi.VARIANTS[name] else " (shape rule)")
 
 
 def other_configs(dev, stream, peaks, seed):

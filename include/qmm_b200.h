@@ -66,7 +66,7 @@ typedef enum qmm_variant {
   QMM_VARIANT_MMA = 4,     /* decode: weights dequantised in registers into warp-level MMAs, M <= 32 */
   /* 5 was a tensor-memory decode variant that lost to QMM_VARIANT_MMA on every shape; the value is not reused */
   QMM_VARIANT_I8TC = 6,    /* activations split into int8 limbs, unconverted weights into tcgen05.mma.kind::i8, stream-K
-                              over all SMs, 1 <= M <= 64; only through qmm_weight_only (needs workspace) */
+                              over all SMs, any M (long batches in chunks); only through qmm_weight_only (needs workspace) */
   QMM_VARIANT_I8MMA = 7,   /* decode: activations split into int8 limbs, unconverted weights into warp-level int8 MMAs,
                               M <= 16, zero points allowed; only through qmm_weight_only (no workspace) */
   QMM_VARIANT_TMEM = 8,    /* weights converted into tensor memory as the A operand of tcgen05.mma.kind::f16, any M, bf16/f16
@@ -213,9 +213,11 @@ QMM_API int qmm_weight_only_typed(int wbits, const void* x, int x_dtype, const v
 QMM_API int qmm_gate_up_decode(int wbits, const void* x, int x_dtype, const void* w, const float* scale, void* out,
                        int out_dtype, int64_t M, int64_t N2, int64_t K, int64_t block_size, void* stream);
 /*
- * The same fused operation for any batch up to 1008 tokens on the split-activation kernel (QMM_VARIANT_I8TC), whose
- * drain warps apply silu(gate) * up before the one store: bf16 / f16 / f32 activations, K >= 128 and a multiple of
- * 16 (int8) or 32 (int4), block_size 0, 64, 128 or a multiple of 256.  workspace: as for qmm_weight_only
+ * The same fused operation for batches on the tensor cores, whose drain warps apply silu(gate) * up before the one store:
+ * any batch where the tensor-memory kernel (QMM_VARIANT_TMEM) is the choice for [N2,K], else the split-activation kernel
+ * (QMM_VARIANT_I8TC) up to 1024 tokens with 16-bit results and 1008 with fp32: bf16 / f16 / f32 activations, K >= 128 and
+ * a multiple of 16 (int8) or 32 (int4), block_size 0, 64, 128 or a multiple of 256.  (The operator above this ABI comes
+ * here above 32 tokens, and not with blocks of 64.)  workspace: as for qmm_weight_only
  * (qmm_weight_only_workspace_size(M, K) bytes, 256-byte aligned, first 2048 bytes zero before the first use).
  * Returns QMM_ERR_UNSUPPORTED outside that range.  No counterpart in the reference (see qmm_gate_up_decode).
  */

@@ -62,3 +62,30 @@ def test_module_follows_its_scales(dtype, wbits, bs, zp, qact, N, K, M, odd):
     mod.zero_point.data.copy_(z)
   y = mod(x)
   assert y.dtype == dtype and torch.equal(y, in_f32(s, z))
+
+
+@pytest.mark.parametrize("wbits,bs", [(4, 128), (4, -1), (8, 128), (8, -1)])
+def test_module_follows_its_weight(wbits, bs):
+  """The K-minor weight that a module keeps is made again when the buffer is written in place or replaced; other scales in
+  another type need nothing."""
+  g = qc.gen(11)
+  N, K, M = 256, 1024, 3
+  x = qc.activations(g, M, K).to(DEV)
+  layout = lambda w: (w if bs == -1 else qc.to_sbn(w, bs)).to(DEV)  # noqa: E731
+  weights = [(qc.int4_weight if wbits == 4 else qc.int8_weight)(g, N, K) for _ in range(3)]
+  s = (qc.per_channel_scale(g, N) if bs == -1 else qc.blockwise_scale(g, K // bs, N)).to(DEV)
+
+  def fresh(w, scale):
+    m = xla_b200.XlaQuantizedLinear(K, N, is_symmetric=True, block_size=bs, int4_weight=wbits == 4)
+    m.load_quantized_weight(layout(w), scale)
+    return m
+
+  mod = fresh(weights[0], s)
+  assert torch.equal(mod(x), fresh(weights[0], s)(x))
+  mod.weight.copy_(layout(weights[1]))
+  assert torch.equal(mod(x), fresh(weights[1], s)(x))
+  mod.weight = layout(weights[2])
+  assert torch.equal(mod(x), fresh(weights[2], s)(x))
+  mod.weight_scaler = s.bfloat16()
+  y = mod(x)
+  assert y.dtype == torch.bfloat16 and torch.equal(y, fresh(weights[2], s.bfloat16())(x))

@@ -75,7 +75,7 @@ int launch_decode_w8a8(const void* x, int x_dt, const int8_t* w, const Scales& s
 
 // ---- limb_gemm.cu (tcgen05 kind::i8 on unconverted weights; activations split into int8 limbs) ----------
 // Weight-only linear (bf16/f16/f32 activations): stream-K over all SMs, needs
-// limb_tc_workspace_bytes(M, K) bytes of caller scratch whose first 1024 bytes are zero before the first use (the
+// limb_tc_workspace_bytes(M, K) bytes of caller scratch whose first 2048 bytes are zero before the first use (the
 // kernel leaves them zero).  gate_up as in launch_decode_mma.
 constexpr int kLimbMaxCtas = 320;  // two CTAs per SM on up to 160 SMs
 size_t limb_tc_workspace_bytes(int64_t M, int64_t K);

@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(1024) split_rows_kernel(const XT* x, int8_t* _
       // Eight neighbouring groups (64 values) are inside one scale block and add to it together, in two 32-bit halves:
       // at most 1024 times, so neither overflows.  (The machine adds 32-bit words in shared memory by itself; 64-bit ones
       // are retried until no other lane was faster: 333 rows of 6912 fp32 values in one block each 52.1 us with the GEMM
-      // and sixteen groups to an add, now 47.4.)
+      // and sixteen groups to an add, 47.4 so.)
       auto sum = [](const uint32_t* l) { return __dp4a((int)l[1], 0x01010101, __dp4a((int)l[0], 0x01010101, 0)); };
       int t = sum(l0) + 256 * sum(l1) + (NL == 3 ? 65536 * sum(l2) : 0);
 #pragma unroll
@@ -823,7 +823,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
       }
       // Block scales are fetched one hand-over ahead, from clamped addresses, and change registers at its end.  (A longer
       // register queue does not fetch further ahead: its shift waits for the youngest load, and shifting twice per
-      // hand-over put a whole memory round trip into each: int4 block 128 [28672,8192] at 512 tokens 363 us, now 337.)
+      // hand-over put a whole memory round trip into each: int4 block 128 [28672,8192] at 512 tokens 363 us, 337 so.)
       using SBits = typename std::conditional<W16, unsigned short, uint32_t>::type;
       const int64_t nc = min(n, p.N - 1);
       const uint8_t* scale_n = static_cast<const uint8_t*>(p.scale) + nc * sizeof(SBits);
@@ -831,7 +831,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
       if (C::kScaleRing > 0 && p.scale_ring) {
         // A hand-over here is shorter than a round trip to HBM, so the scales come eight blocks ahead, into a ring of the
         // thread's own (one hand-over ahead, in registers: int4 block 128 [57344,8192] 53.9 us at 4 tokens and 82.0 at 16,
-        // now 46.4 and 74.3).
+        // 46.4 and 74.3 so).
         constexpr int R = C::kScaleRing > 0 ? C::kScaleRing : 1;
         const int per_slot = p.mode == kBlock128 ? 2 : p.mode == kBlock64 ? 4 : 1;  // blocks
         const int b0 = p.mode == kBlockSlots ? u0 : s0 * per_slot, b1 = p.mode == kBlockSlots ? u1 : s1 * per_slot;

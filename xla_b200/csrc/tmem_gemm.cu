@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const uint32_t idesc = ptx::make_idesc(/*f32*/ 1, fmt, fmt, BMW, (uint32_t)p.th);
       // Operands of the MMA live in uniform registers.  What the compiler cannot see to be the same in all lanes (a value
       // from shared memory, a branch on a predicate computed earlier) is moved there again for every MMA: int4 block 128
-      // [28672,8192] at 512 tokens 285 us, now 266.
+      // [28672,8192] at 512 tokens 285 us moved every time, 266 so.
       const uint32_t tb = __reduce_or_sync(0xffffffffu, tmem_base);
       const uint32_t desc_hi = (uint32_t)(ptx::make_sw128_kmajor_desc(0) >> 32);
       const uint32_t b_lo0 = (uint32_t)ptx::make_sw128_kmajor_desc(ptx::smem_u32(b_base));

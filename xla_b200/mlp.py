@@ -8,8 +8,10 @@ operand sharing to XLA's fusion passes.  Here the two projections become ONE wei
                            then the eight up rows of the same outputs) so that one output tile of the decode
                            kernels holds both halves of eight outputs.
   ``quantized_gate_up``    ``torch.ops.xla_b200.quantized_gate_up``: silu(x @ Wgate^T) * (x @ Wup^T) in one
-                           kernel for decode batches (M <= 32), computed in fp32 from the fp32 accumulators;
-                           larger batches run the stacked weight as one linear and apply the activation after.
+                           kernel, computed in fp32 from the fp32 accumulators: the decode kernels up to 32
+                           tokens, the tensor-core kernels above (up to 1008 tokens, any number where the
+                           tensor-memory kernel takes the shape); other calls run the stacked weight as one
+                           linear and apply the activation after.
   ``concat_projections``   row-concatenates K-minor weights (and their scales) of projections that read the
                            same activations; one call then produces all outputs, split by ``split_outputs``.
 
@@ -86,7 +88,8 @@ def quantized_gate_up(x, w, scaler, block_size=-1, int4_weight=False, weight_is_
     out = None
     if (32 < M <= 1008 and x2.dtype in (torch.bfloat16, torch.float16, torch.float32) and K >= 128 and K % (128 // wbits) == 0 and
         (block_size == -1 or block_size == 128 or block_size % 256 == 0) and _qm.current_variant() in ("auto", "i8tc")):
-      # larger batches: the split-activation tensor-core kernel applies silu(gate) * up in its drain
+      # larger batches: the tensor-core kernels apply silu(gate) * up in their drain (the operator's C++ form comes first and
+      # also takes longer batches, where the library does)
       expect = (N2,) if block_size == -1 else (K // block_size, N2)
       assert tuple(s32.shape) == expect, f"weight scaler shape is expect to be {list(expect)}, got {list(s32.shape)}."
       wc = w if w.is_contiguous() else _capi.settled(w.contiguous())
