@@ -26,6 +26,9 @@ CASES = [
     (4, 128, True, False, 1023, 128 * 17, 16, False), (4, 128, True, False, 1023, 128 * 16, 29, False),
     (4, 128, True, False, 257, 128 * 10, 3, False), (4, 64, True, False, 131, 384, 5, False), (4, 128, False, False, 4097, 128 * 64, 24, False),
     (8, 64, True, False, 385, 64 * 16, 33, False), (4, 256, False, False, 3841, 256 * 16, 12, False),
+    # shapes that only the any-shape and the GEMV kernel take, which read fp32 scales
+    (8, -1, True, False, 40, 72, 5, False), (8, -1, True, False, 40, 48, 5, True), (8, 4, False, False, 12, 20, 3, False),
+    (8, -1, True, True, 40, 72, 5, False),
     # small weights above 32 tokens: the conversion kernel
     (4, -1, False, False, 1976, 1504, 45, True), (8, -1, False, False, 269, 1536, 300, False), (8, 128, False, False, 301, 1024, 45, True),
 ]

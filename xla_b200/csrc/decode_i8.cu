@@ -21,9 +21,9 @@
 // once, at the end, to add their pieces of each tile in warp order.  8 warps while two CTAs fit an SM (for small weights
 // the second place is the next linear's, whose first weights are then in flight while this one drains), else 16.
 //
-// Measured (B200, launches back to back over weights larger than L2, against decode_mma.cu or limb_gemm.cu):
-//   int4 block 128, one token   [14336,4096] 9.1 us (13.9)   [28672,8192] 25.6 (36)   [8192,28672] 29.2 (33)
-//   int8 per channel, one token [14336,4096] 11.5 us = 5.1 TB/s (16.7)   [28672,8192] 41 us = 5.7 TB/s (43)
+// Measured (B200, launches back to back over weights larger than L2; decode_mma.cu and limb_gemm.cu in brackets):
+//   int4 block 128, one token   [14336,4096] 9.5 us (13.9, 13.5)   [28672,8192] 25.1 (41.9, 28.0)   [8192,28672] 30.0 (55.5, 32.6)
+//   int8 per channel, one token [14336,4096] 11.8 us = 5.0 TB/s (16.9, 13.7)   [28672,8192] 43.0 us = 5.5 TB/s (56.9, 39.6)
 //   W8A8 [14336,4096]           13.1 us at 1 token, 14.4 at 4, 22 at 12 (any-shape kernel: 113; quantizer + GEMM: 23)
 //
 // Semantics: torch_xla/experimental/xla_quantized_matmul.py:152-170 (weight-only), :107-114, :134-135 (W8A8).
