@@ -69,3 +69,49 @@ def test_gate_up_with_blocks_of_64(wbits, M):
   gate = torch.as_tensor(qo.quantized_matmul(x.float(), qc.to_sbn(wg, bs), sg, block_size=bs, dot_round=None))
   up = torch.as_tensor(qo.quantized_matmul(x.float(), qc.to_sbn(wu, bs), su, block_size=bs, dot_round=None))
   assert qo.max_abs_rel(out, torch.nn.functional.silu(gate) * up) < 1e-4
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("wbits,bs,N,K,M", [
+    (4, -1, 256, 512, 20), (8, -1, 256, 640, 20), (4, 128, 256, 384, 33), (8, 128, 256, 640, 64), (4, 64, 256, 192, 7),
+    (8, 64, 256, 448, 64), (4, 128, 256, 896, 70), (8, 128, 256, 640, 150),
+])
+def test_every_weight_value_is_converted_exactly(dtype, wbits, bs, N, K, M):
+  """Small whole activations and scales of one: the fp32 result is a whole number, equal to the integer product."""
+  g = qc.gen(K + M)
+  lo, hi = (-8, 8) if wbits == 4 else (-128, 128)
+  w = (torch.arange(N * K, dtype=torch.int32).reshape(N, K) * 7 % (hi - lo) + lo).to(torch.int8)
+  x = torch.randint(-2, 3, (M, K), generator=g)
+  s = torch.ones((N,) if bs == -1 else (K // bs, N))
+  wd = xla_b200.pack_int4(w.to(DEV)) if wbits == 4 else w.to(DEV)
+  with xla_b200.force_variant("tmem"):
+    out = torch.ops.xla_b200.quantized_matmul_packed(x.to(dtype).to(DEV), wd, s.to(DEV), block_size=bs, int4_weight=wbits == 4,
+                                                     weight_is_packed=wbits == 4, out_dtype=torch.float32)
+  assert torch.equal(out.cpu().long(), x.long() @ w.long().T)
+
+
+@pytest.mark.parametrize("scales", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("zp", [False, True])
+@pytest.mark.parametrize("wbits,bs,N,K,M", [
+    (4, 128, 128 * 150 + 2, 640, 2), (4, 128, 1026, 1152, 32), (4, 128, 1026, 2176, 64), (8, 128, 514, 896, 31),
+    (8, 128, 1026, 1408, 63), (4, 64, 514, 320, 32), (8, 64, 514, 832, 61), (4, 256, 514, 2304, 48), (8, 384, 514, 1152, 30),
+    (4, 128, 514, 1920, 100), (4, 128, 514, 1920, 190), (8, -1, 514, 1136, 40), (4, -1, 514, 2592, 25),
+])
+def test_steps_that_the_blocks_do_not_fill(wbits, bs, N, K, M, zp, scales):
+  """Odd numbers of scale blocks in steps of two, more tiles than CTAs, ragged rows; zero points; scales in the activations' type."""
+  g = qc.gen(N + K + M)
+  x = qc.activations(g, M, K, torch.bfloat16, outliers=True)
+  w = qc.int4_weight(g, N, K) if wbits == 4 else qc.int8_weight(g, N, K)
+  s = (qc.per_channel_scale(g, N) if bs == -1 else qc.blockwise_scale(g, K // bs, N)).to(scales)
+  z = (torch.randint(-2, 3, s.shape, generator=g) * s).to(scales) if zp else None
+  wd = xla_b200.pack_int4(w.to(DEV)) if wbits == 4 else w.to(DEV)
+  with xla_b200.force_variant("tmem"):
+    out = torch.ops.xla_b200.quantized_matmul_packed(x.to(DEV), wd, s.to(DEV), None if z is None else z.to(DEV), block_size=bs,
+                                                     int4_weight=wbits == 4, weight_is_packed=wbits == 4, out_dtype=torch.float32)
+  S = 1 if bs == -1 else K // bs
+  xb, wb = x.double().to(DEV).view(M, S, K // S), w.double().to(DEV).view(N, S, K // S)
+  exact = torch.einsum("msk,nsk,sn->mn", xb, wb, s.double().to(DEV).view(S, N))
+  if zp:
+    exact -= torch.einsum("ms,sn->mn", xb.sum(-1), z.double().to(DEV).view(S, N))
+  # exact products, at most K / 128 + 3 roundings of the running sum: far below 1e-5 of the largest result
+  assert qo.max_abs_rel(out, exact) < 1e-5

@@ -142,6 +142,15 @@ __device__ __forceinline__ float scale_in(const uint32_t* word, int n, int b, in
   return __uint_as_float((uint32_t)h << 16);
 }
 
+// The same for a word in a register; T: the type of 16-bit scales.
+template <bool W16, typename T>
+__device__ __forceinline__ float scale_of_word(uint32_t word, int n, int b, int N) {
+  if (!W16) return __uint_as_float(word);
+  const uint32_t at = ((uint32_t)n & 1u) ^ ((uint32_t)b & (uint32_t)N & 1u);
+  const uint32_t h = __byte_perm(word, 0u, at ? 0x3244u : 0x1044u);  // the value in the upper half
+  return std::is_same<T, __half>::value ? __half2float(__ushort_as_half((unsigned short)(h >> 16))) : __uint_as_float(h);
+}
+
 // A single scale as its bits, and their value: apart, because the conversion waits for the load
 __device__ __forceinline__ uint32_t load_scale_bits(const void* p, int64_t n, int dt) {
   return dt == QMM_F32 ? ld_ordered(static_cast<const uint32_t*>(p) + n) : (uint32_t)ld_ordered(static_cast<const unsigned short*>(p) + n);

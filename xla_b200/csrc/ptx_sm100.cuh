@@ -139,6 +139,43 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity,
   return ok;
 }
 
+// The same by address, for loops in which every instruction counts (a lone warp issues a dependent one every 4 to 6 cycles,
+// and a generic pointer costs several to turn into an address).  All lanes look; a wait costs about 57 cycles when the phase
+// is complete.
+__device__ __forceinline__ bool bar_try_wait(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return __all_sync(0xffffffffu, ok != 0);
+}
+__device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t* err_word, uint32_t code) {
+  if (__builtin_expect(bar_try_wait(bar, parity), 1)) return;
+  uint32_t spins = 0;
+  long long t0 = 0;
+  while (!bar_try_wait(bar, parity)) {
+    if ((++spins & 0xfff) == 0) {
+      if (__any_sync(0xffffffffu, *abort_flag != 0)) return;
+      const long long now = clock64();
+      if (t0 == 0) t0 = now;
+      if (__any_sync(0xffffffffu, now - t0 > kWaitLimitCycles)) {
+        *abort_flag = code;
+        if (err_word) atomicCAS(err_word, 0u, code | (blockIdx.x << 8));
+        return;
+      }
+    }
+  }
+}
+__device__ __forceinline__ void mbar_arrive_a(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
 // ---- partial tiles between the CTAs of a launch ------------------------------------------------
 // A CTA that works on a later K range of a tile leaves its sums in global scratch for the tile's first CTA.  The flag word
 // beside them: 0 idle, 1 written, 2 given up by the reader; 0 again after every launch, also after one that gave up.
@@ -279,6 +316,10 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
                : "memory");
 }
 
+__device__ __forceinline__ void mma_commit_a(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+
 // ---- TMEM -> registers --------------------------------------------------------------------
 // Each thread of the warp reads 32 consecutive 32-bit columns of its own TMEM lane
 // (lane = 32 * (warp_id % 4) + lane_id; the lane quadrant goes into bits [16,32) of taddr).
@@ -307,6 +348,13 @@ __device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t* r) 
       : "memory");
 }
 
+__device__ __forceinline__ void tmem_ld_32x32b_x8(uint32_t taddr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
+
 __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
@@ -320,6 +368,10 @@ __device__ __forceinline__ void tmem_ld_landed16(uint32_t* r) {
                : "memory");
 }
 
+__device__ __forceinline__ void tmem_ld_landed8(uint32_t* r) {
+  asm volatile("" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]) : : "memory");
+}
+
 // ---- registers -> TMEM --------------------------------------------------------------------
 // Each thread of the warp writes 16 consecutive 32-bit columns of its own TMEM lane.
 __device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_t* r) {
@@ -328,6 +380,14 @@ __device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_
       "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
       "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
       "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+
+__device__ __forceinline__ void tmem_st_32x32b_x32(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
       : "memory");
 }
 

@@ -7,20 +7,26 @@
 // registers.  (The integer form, limb_gemm.cu, needs two limb columns per token for 16-bit outputs: the same tensor-core
 // cycles, but twice the accumulator columns to read back and convert at every scale block.)
 //
-// What bounds this shape of kernel is the shared-memory port, 128 bytes a cycle for everything TMA writes and the MMA
-// reads (limb_gemm.cu at 512 tokens, per channel: 1035 cycles per slot of 64 KB written and 64 KB read, exactly that).
-// So the weights never go back to shared memory: converting warps read the raw bytes and write the bf16/f16 operand to
-// tensor memory, where the MMA takes its A side from, and token tiles are as wide as two accumulators allow (192 columns:
-// 96 KB of port traffic for the activations of a K step of 128, and 16 or 32 KB for the weights, against 768 cycles of
-// MMAs).
+// The shared-memory port carries 128 bytes a cycle for everything TMA writes and the MMA reads, so the weights never go back to
+// shared memory: converting warps read the raw bytes and write the bf16/f16 operand to tensor memory, where the MMA takes its
+// A side from, and token tiles are as wide as two accumulators allow (192 columns).
 //
 //   warp 0        TMA: raw weight tiles, 128 rows x 128 bytes
-//   warp 1        MMA issuer: per K step 8 (KS = 64: 4) x tcgen05.mma.kind::f16 (M128 x N<=192 x K16, A in tensor memory)
-//                 and ONE commit, which everybody who needs the step's completion waits for; the next step's barriers are
-//                 looked at before the current step is issued
 //   warp 2        TMA: activation tiles, one K step x up to 192 tokens
-//   warps 4..11   converters: two groups of four warps that take alternate K steps; lane = weight row
-//   warps 12..19  drain: thread = weight row, half of the tokens in fp32 registers: tcgen05.ld, scale, add; epilogue
+//   warps 1, 3    MMA issuers, alternate folds: per K step 16, 8 or 4 x tcgen05.mma.kind::f16 (M128 x N<=192 x K16, A in
+//                 tensor memory), a commit for the step's operands and one for the accumulators
+//   converters    four groups of four warps (two for tiles above 128 tokens); lane = weight row.  A step of 256 values (up to
+//                 64 tokens) is shared by two groups, one of 128 is a group's own; the groups take the steps in turn
+//   drain         eight warps: thread = weight row, half of the tokens in fp32 registers: tcgen05.ld, scale, add; epilogue
+//
+// What bounds it.  Up to 64 tokens the instructions of the converters and of the hand-overs: about 440 a scheduler and 128
+// values (ten for eight int4 weights, 160 of them), issued in two thirds of the cycles.  A wait for a complete barrier costs a
+// warp about 57 cycles and a dependent instruction 4 to 6, so a lone warp's loop of three waits, sixteen MMAs and a commit takes
+// 1000 cycles: hence two issuers, steps of 256 values with two scale blocks under one hand-over, barriers by address, four
+// groups of converters that wait side by side, and scales a batch at a time.  int4 block 128 [57344,8192]: 29 tokens 121 us
+// with one issuer and steps of 128 values, 74 now; 64 tokens 134 and 87.  Above 128 tokens a step of 128 values takes 1300
+// cycles for 704 of MMAs: instructions again (790 a scheduler: 96 sums a thread), at 1.65 GHz under load.  512 tokens 511 us
+// and 460.
 //
 // Schedule: (weight tile, token tile) items walk the CTAs whole; the items of a partly filled last round (all of them
 // when there are fewer items than SMs) are split along K over several CTAs and summed, in CTA order, from fp32 partial
@@ -41,12 +47,8 @@ namespace {
 
 constexpr int BMW = 128;                  // weight rows per tile (UMMA M)
 constexpr uint32_t kRawBytes = BMW * 128; // one raw tile: 128 rows x 128 bytes
-constexpr int kACols = 64;                // tensor-memory columns per operand step (32 are used for steps of 64 values)
 constexpr int kDone = 8;                  // step-complete barriers
-constexpr int kThreads = 640;
 constexpr int kDrain = 256;               // drain threads
-constexpr int kScaleRing = 8;             // folds whose scales (and zero points) are on their way
-constexpr int kMiscRegs = 40, kConvRegs = 64, kDrainRegs = 152;  // x 128, 256, 256 threads: within 640 x 96
 constexpr uint32_t kErrPartial = 10;      // owner CTA never saw a partial tile arrive
 
 struct Params {
@@ -60,41 +62,64 @@ struct Params {
   int out_dt;
   int M;
   int64_t N;
-  int stages;     // K steps per tile
   int fu;         // steps per fold (accumulation in the tensor core), >= 1
   int blocked;    // scale blocks (0: per channel; folds are then plain additions)
   int S;
-  int ut;         // scheduling units (folds of fu steps) per tile
+  int unit;       // steps per scheduling unit: whole folds and whole raw tiles
+  int fpu;        // folds per unit
+  int ut;         // units per tile (steps beyond K multiply zeros)
   int th;         // tokens per item (a multiple of 16)
   int ytiles;
   int items1;     // items handed out whole: CTA c takes c, c + G, ...
   int units;      // units of the remaining items, dealt in equal contiguous shares to the first g2 CTAs
   int g2;
   int gate_up;
-  float* partial;   // [g2][th][128]
+  float* partial;   // [g2][th / 4][128][4]
   uint32_t* flags;  // [g2], zero between launches
   uint32_t* err_word;
   long long wait_cycles;  // for a partial tile
 };
 
-// KS: k values per step (64 for scale blocks of 64, else 128); NC: accumulator columns (tokens).
-template <int WBITS, int NC, int KS>
+// NC: accumulator columns (tokens); KS: k values per step; SUB: scale blocks per step that have an accumulator each (a fold is
+// then one step), or 1 (a fold is one or more steps).
+template <int WBITS, int NC, int KS, int SUB>
 struct Cfg {
-  static constexpr int kAcc = NC <= 64 ? 4 : 2;
-  static constexpr int kASlots = NC == 192 ? 2 : 4;
+  static constexpr int kAccCols = SUB * NC;
+  static constexpr int kAcc = 2;
+  static constexpr int kACols = KS / 2;  // tensor-memory columns per operand step
+  static constexpr int kASlots = std::min(4, (512 - kAcc * kAccCols) / kACols / 2 * 2);
   static constexpr int kACol0 = 512 - kASlots * kACols;
+  // Groups of four converting warps.  Teams of one group (steps of up to 128 values) or two (half of 256 each) take the steps
+  // in turn.
+  static constexpr int kGroups = NC == 192 ? 2 : 4, kTeamGroups = NC <= 64 ? 2 : 1, kTeams = kGroups / kTeamGroups;
+  static constexpr int kThreads = 128 + 128 * kGroups + kDrain;
+  // setmaxnreg: within threads x registers at launch
+  static constexpr int kMiscRegs = NC == 192 ? 32 : 40;
+  static constexpr int kConvRegs = 56;
+  static constexpr int kDrainRegs = NC == 192 ? 168 : 120;
+  static constexpr int kLaunchRegs = kThreads == 640 ? 96 : 72;
+  static_assert(128 * kMiscRegs + 128 * kGroups * kConvRegs + kDrain * kDrainRegs <= kThreads * kLaunchRegs, "register split");
   static constexpr uint32_t kBStage = NC * KS * 2;
-  static constexpr int kB = std::min(kDone, (NC == 192 ? 3 : NC == 128 ? 4 : NC == 64 ? 6 : 8) * (128 / KS));
-  static constexpr int kRaw = NC == 192 ? 4 : NC == 128 ? 5 : NC == 64 ? 6 : 8;
-  static constexpr int kSPR = 1024 / (WBITS * KS);  // K steps per raw tile
+  static constexpr int kRaw = NC >= 64 ? 4 : 8;
+  static constexpr int kB = std::min(kDone, (NC == 192 ? 144 : NC >= 64 ? 128 : 64) * 1024 / (int)kBStage);
+  static constexpr int kTV = 1024 / WBITS;          // values of a row per raw tile
+  static constexpr int kVV = KS / kTeamGroups;      // values per step and converting group
   static constexpr int kDT = NC / 2;                // tokens per drain thread
-  static constexpr size_t kScaleBytes = 2 * kScaleRing * kDrain * 4;
-  static constexpr size_t kSmem = 1024 + (size_t)kRaw * kRawBytes + (size_t)kB * kBStage + kScaleBytes + 512;
-  static_assert(kAcc * NC <= kACol0, "tensor memory");
+  // columns per tensor-memory load of the drain, and sets of registers for them
+  static constexpr int kCh = kDT == 96 || kDT == 16 ? 16 : 32, kChBufs = kDT == 96 || SUB > 1 ? 2 : 1;
+  // block scales, zero points and block sums of the activations (per group of drain warps) on their way, in two batches
+  static constexpr int kScaleRing = NC == 32 ? 12 : NC == 192 ? 6 : 8, kBatch = kScaleRing / 2;
+  static constexpr size_t kScaleBytes = 2 * kScaleRing * kDrain * 4, kSumBytes = 2 * kScaleRing * kDT * 4;
+  static constexpr size_t kSmem = 1024 + (size_t)kRaw * kRawBytes + (size_t)kB * kBStage + kScaleBytes + kSumBytes + 512;
+  static_assert(kAcc * kAccCols <= kACol0 && kASlots >= 2, "tensor memory");
   static_assert(kSmem <= 227 * 1024, "shared memory budget");
   // A parity wait is right only while the barrier is at most one phase away: whoever waits for step i - d does so for every
-  // step in turn, and step i - d + kDone cannot complete before it has gone on.
-  static_assert(kB <= kDone && kASlots <= kDone && kAcc <= kDone, "step-complete barriers");
+  // step in turn (the converters: for every step of their team), and step i - d + kDone cannot complete before it has gone on.
+  static_assert(kB <= kDone && kASlots <= kB && kAcc <= kDone, "turns of the rings");
+  static_assert(kASlots % kTeams == 0 && kDone % kTeams == 0 && kVV <= kTV, "slots of a team");
+  static_assert(kRaw % std::max(1, kTeams * KS / kTV) == 0, "a group comes back to the raw slots it has waited for");
+  static_assert(kBatch % SUB == 0 && kBatch * kDT / 4 <= kDrain / 2, "batches of scales and block sums");
+  static_assert(SUB == 1 || (kDT <= 32 && SUB == 2), "a load per accumulator");
   static_assert((2 * kRaw + kB + kASlots + 2 * kAcc + kDone) * 8 + 8 <= 512, "barrier space");
 };
 
@@ -130,8 +155,10 @@ struct FragIter {
     y = item - tile * p.ytiles;
     return true;
   }
-  __device__ int s0() const { return u0 * p.fu; }
-  __device__ int s1() const { return min(p.stages, u1 * p.fu); }
+  __device__ int s0() const { return u0 * p.unit; }
+  __device__ int s1() const { return u1 * p.unit; }
+  // steps of all fragments, before the first next()
+  __device__ int steps() const { return ((nxt < p.items1 ? (p.items1 - 1 - nxt) / (int)gridDim.x + 1 : 0) * p.ut + (hi - u)) * p.unit; }
 };
 
 __device__ __forceinline__ uint4 lds128(uint32_t addr) {
@@ -140,58 +167,70 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
   return v;
 }
 
+// a * m + c on pairs
 template <typename XT>
-__device__ __forceinline__ uint32_t sub2(uint32_t a, uint32_t b) {
-  if constexpr (std::is_same<XT, __half>::value) {
-    const __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
-    return *reinterpret_cast<const uint32_t*>(&r);
-  } else {
-    const __nv_bfloat162 r = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&b));
-    return *reinterpret_cast<const uint32_t*>(&r);
-  }
+__device__ __forceinline__ uint32_t pair_fma(uint32_t a, uint32_t m, uint32_t c) {
+  uint32_t r;
+  if constexpr (std::is_same<XT, __half>::value) asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(m), "r"(c));
+  else asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(m), "r"(c));
+  return r;
 }
 
-// Eight nibbles -> four pairs in k order.  Offset-binary nibbles are spread to bytes, put under the exponent byte of 128
-// (bf16) or 1024 (f16), and the offset is subtracted (exact).
+// Byte permutation with the selectors' sign bit: 8 + i is the sign of byte i, eight times
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+  uint32_t r;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
+  return r;
+}
+
+// Integers to 16-bit floats.  A 16-bit float with a zero in its upper byte is its lower byte u times the type's smallest
+// subnormal, 2^-133 (bf16) or 2^-24 (f16), for every u: subnormals and the first normal numbers are evenly spaced.  So the
+// offset-binary value only has to be put beside a zero byte, wherever it lies in the byte, and one multiply-add takes the
+// offset off and brings the value to 2^-6 (bf16) or 2^-9 (f16) of itself; all of it is exact.  The factor is the most that the
+// types' largest power of two leaves, and comes back in at the end (Unit).  (Integer instructions run at half rate and bound
+// the batches up to 64 tokens: nine for eight nibbles and six for four bytes when the bytes go under an exponent, six and
+// three this way.)
+template <typename XT>
+struct Unit {
+  static constexpr bool kHalf = std::is_same<XT, __half>::value;
+  static constexpr float kBack = kHalf ? 512.f : 64.f;
+  static constexpr uint32_t kLow = kHalf ? 0x7800u : 0x7F00u, kHigh = kHalf ? 0x6800u : 0x7D00u;  // 2^15, 2^11; 2^127, 2^123
+  static constexpr uint32_t kEight = kHalf ? 0xA400u : 0xBE00u, k128 = kHalf ? 0xB400u : 0xC000u;  // -8 and -128 of these units
+};
+
+// Eight nibbles -> four pairs in k order: the low nibble of a byte, then the high one (sixteen times itself in its byte).
 template <typename XT>
 __device__ __forceinline__ void cvt_s4x8(uint32_t w, uint32_t* p) {
-  constexpr bool kHalf = std::is_same<XT, __half>::value;
-  constexpr uint32_t expo = kHalf ? 0x64646464u : 0x43434343u, bias = kHalf ? 0x64086408u : 0x43084308u;
-  const uint32_t lo = (w & 0x0F0F0F0Fu) ^ 0x08080808u, hi = ((w >> 4) & 0x0F0F0F0Fu) ^ 0x08080808u;
-  const uint32_t q0 = __byte_perm(lo, hi, 0x5140), q1 = __byte_perm(lo, hi, 0x7362);
-  p[0] = sub2<XT>(__byte_perm(q0, expo, 0x4140), bias);
-  p[1] = sub2<XT>(__byte_perm(q0, expo, 0x4342), bias);
-  p[2] = sub2<XT>(__byte_perm(q1, expo, 0x4140), bias);
-  p[3] = sub2<XT>(__byte_perm(q1, expo, 0x4342), bias);
+  using U = Unit<XT>;
+  const uint32_t lo = (w & 0x0F0F0F0Fu) ^ 0x08080808u, hi = (w & 0xF0F0F0F0u) ^ 0x80808080u;
+  // selector 8 + i: the sign of byte i of `lo`, a zero
+  p[0] = pair_fma<XT>(prmt(lo, hi, 0x8480), U::kHigh << 16 | U::kLow, U::kEight * 0x10001u);
+  p[1] = pair_fma<XT>(prmt(lo, hi, 0x8581), U::kHigh << 16 | U::kLow, U::kEight * 0x10001u);
+  p[2] = pair_fma<XT>(prmt(lo, hi, 0x8682), U::kHigh << 16 | U::kLow, U::kEight * 0x10001u);
+  p[3] = pair_fma<XT>(prmt(lo, hi, 0x8783), U::kHigh << 16 | U::kLow, U::kEight * 0x10001u);
 }
 
-// Four bytes -> two pairs in k order.  f16: the offset-binary byte under the exponent of 1024, minus 1152.  bf16 holds
-// seven bits under an exponent: the low seven go under 128, and the sign bit, which is the lowest exponent bit, makes
-// the subtrahend 128 or 256.
+// Four bytes -> two pairs in k order
 template <typename XT>
 __device__ __forceinline__ void cvt_s8x4(uint32_t w, uint32_t* p) {
-  if constexpr (std::is_same<XT, __half>::value) {
-    const uint32_t u = w ^ 0x80808080u;
-    p[0] = sub2<XT>(__byte_perm(u, 0x64646464u, 0x4140), 0x64806480u);
-    p[1] = sub2<XT>(__byte_perm(u, 0x64646464u, 0x4342), 0x64806480u);
-  } else {
-    const uint32_t t0 = __byte_perm(w, 0u, 0x4140), t1 = __byte_perm(w, 0u, 0x4342);
-    p[0] = sub2<XT>((t0 & 0x007F007Fu) | 0x43004300u, (t0 & 0x00800080u) | 0x43004300u);
-    p[1] = sub2<XT>((t1 & 0x007F007Fu) | 0x43004300u, (t1 & 0x00800080u) | 0x43004300u);
-  }
+  using U = Unit<XT>;
+  const uint32_t u = w ^ 0x80808080u;
+  p[0] = pair_fma<XT>(__byte_perm(u, 0u, 0x4140), U::kLow * 0x10001u, U::k128 * 0x10001u);
+  p[1] = pair_fma<XT>(__byte_perm(u, 0u, 0x4342), U::kLow * 0x10001u, U::k128 * 0x10001u);
 }
 
-// Sixteen tokens of one output column, `pitch` elements apart
-template <typename OT>
-__device__ __forceinline__ void store16_as(OT* o, int64_t pitch, const float* v, int count) {
+// C tokens of one output column, `pitch` elements apart
+template <int C, typename OT>
+__device__ __forceinline__ void store_tokens_as(OT* o, int64_t pitch, const float* v, int count) {
 #pragma unroll
-  for (int t = 0; t < 16; ++t)
-    if (t < count) o[t * pitch] = from_f32<OT>(v[t]);
+  for (int t = 0; t < C; ++t, o += pitch)
+    if (t < count) *o = from_f32<OT>(v[t]);
 }
-__device__ __forceinline__ void store16(void* out, int dt, int64_t at, int64_t pitch, const float* v, int count) {
-  if (dt == QMM_BF16) store16_as(reinterpret_cast<__nv_bfloat16*>(out) + at, pitch, v, count);
-  else if (dt == QMM_F16) store16_as(reinterpret_cast<__half*>(out) + at, pitch, v, count);
-  else store16_as(reinterpret_cast<float*>(out) + at, pitch, v, count);
+template <int C>
+__device__ __forceinline__ void store_tokens(void* out, int dt, int64_t at, int64_t pitch, const float* v, int count) {
+  if (dt == QMM_BF16) store_tokens_as<C>(reinterpret_cast<__nv_bfloat16*>(out) + at, pitch, v, count);
+  else if (dt == QMM_F16) store_tokens_as<C>(reinterpret_cast<__half*>(out) + at, pitch, v, count);
+  else store_tokens_as<C>(reinterpret_cast<float*>(out) + at, pitch, v, count);
 }
 
 template <int REGS>
@@ -203,24 +242,25 @@ __device__ __forceinline__ void reg_dec() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS));
 }
 
-template <int WBITS, typename XT, int NC, int KS, bool W16>
-__global__ void __launch_bounds__(kThreads, 1)
+template <int WBITS, typename XT, int NC, int KS, int SUB, bool W16>
+__global__ void __launch_bounds__(Cfg<WBITS, NC, KS, SUB>::kThreads, 1)
     tmem_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const Params p) {
-  using C = Cfg<WBITS, NC, KS>;
-  constexpr int kRaw = C::kRaw, kB = C::kB, kAcc = C::kAcc, DT = C::kDT, kASlots = C::kASlots, kSPR = C::kSPR;
+  using C = Cfg<WBITS, NC, KS, SUB>;
+  constexpr int kRaw = C::kRaw, kB = C::kB, kAcc = C::kAcc, DT = C::kDT, kASlots = C::kASlots, kACols = C::kACols, kGroups = C::kGroups,
+                kScaleRing = C::kScaleRing;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* raw_base = smem;
   uint8_t* b_base = raw_base + (size_t)kRaw * kRawBytes;
   uint32_t* s_scale = reinterpret_cast<uint32_t*>(b_base + (size_t)kB * C::kBStage);  // [scale, zero point][kScaleRing][kDrain]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(s_scale) + C::kScaleBytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(s_scale) + C::kScaleBytes + C::kSumBytes);
   uint64_t* raw_full = bars;                 // [kRaw]    TMA bytes
-  uint64_t* raw_empty = raw_full + kRaw;     // [kRaw]    the converting warps that share the tile
+  uint64_t* raw_empty = raw_full + kRaw;     // [kRaw]    the converting warps that read the tile
   uint64_t* b_full = raw_empty + kRaw;       // [kB]      TMA bytes
-  uint64_t* a_full = b_full + kB;            // [kASlots] the four converting warps of the step's group
+  uint64_t* a_full = b_full + kB;            // [kASlots] the converting warps of the step
   uint64_t* acc_empty = a_full + kASlots;    // [kAcc]    eight drain warps
-  uint64_t* acc_full = acc_empty + kAcc;     // [kAcc]    tcgen05.commit, folds of several steps only
+  uint64_t* acc_full = acc_empty + kAcc;     // [kAcc]    tcgen05.commit: the fold is complete
   uint64_t* done = acc_full + kAcc;          // [kDone]   tcgen05.commit: the MMAs of step i are complete
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + kDone);
   volatile uint32_t* abort_flag = tmem_slot + 1;
@@ -229,10 +269,10 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (threadIdx.x == 0) {
     for (int s = 0; s < kRaw; ++s) {
       ptx::mbar_init(&raw_full[s], 1);
-      ptx::mbar_init(&raw_empty[s], kSPR == 1 ? 4 : 8);
+      ptx::mbar_init(&raw_empty[s], 4 * C::kTV / C::kVV);
     }
     for (int s = 0; s < kB; ++s) ptx::mbar_init(&b_full[s], 1);
-    for (int s = 0; s < kASlots; ++s) ptx::mbar_init(&a_full[s], 4);
+    for (int s = 0; s < kASlots; ++s) ptx::mbar_init(&a_full[s], 4 * C::kTeamGroups);
     for (int s = 0; s < kAcc; ++s) {
       ptx::mbar_init(&acc_empty[s], 8);
       ptx::mbar_init(&acc_full[s], 1);
@@ -254,7 +294,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (warp < 4) {
-    reg_dec<kMiscRegs>();
+    reg_dec<C::kMiscRegs>();
     FragIter it(p);
     if (warp == 0) {
       // ---------------- raw weight producer: static data, no wait for earlier kernels ----------------
@@ -263,10 +303,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         uint32_t ph = 0;
         while (it.next()) {
           const int s0 = it.s0(), s1 = it.s1();
-          for (int s = s0; s < s1; s += kSPR) {
+          for (int b = s0 * (KS * WBITS / 8); b < s1 * (KS * WBITS / 8); b += 128) {
             ptx::mbar_wait(&raw_empty[slot], ph ^ 1, abort_flag, p.err_word, ptx::kErrWaitEmpty);
             ptx::mbar_expect_tx(&raw_full[slot], kRawBytes);
-            ptx::tma_load_2d(raw_base + (size_t)slot * kRawBytes, &map_w, &raw_full[slot], s * (KS * WBITS / 8), it.tile * BMW);
+            ptx::tma_load_2d(raw_base + (size_t)slot * kRawBytes, &map_w, &raw_full[slot], b, it.tile * BMW);
             if (++slot == kRaw) { slot = 0; ph ^= 1; }
           }
         }
@@ -291,8 +331,9 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
         }
       }
-    } else if (warp == 1) {
-      // ---------------- MMA issuer: the whole warp walks the loop, one elected thread issues ----------------
+    } else {
+      // ---------------- MMA issuers, warps 1 and 3: the folds alternate between them ----------------
+      // A whole warp walks the loop, one elected thread issues.
       constexpr uint32_t fmt = std::is_same<XT, __half>::value ? 0u : 1u;
       const uint32_t idesc = ptx::make_idesc(/*f32*/ 1, fmt, fmt, BMW, (uint32_t)p.th);
       // Operands of the MMA live in uniform registers.  What the compiler cannot see to be the same in all lanes (a value
@@ -301,213 +342,324 @@ __global__ void __launch_bounds__(kThreads, 1)
       const uint32_t tb = __reduce_or_sync(0xffffffffu, tmem_base);
       const uint32_t desc_hi = (uint32_t)(ptx::make_sw128_kmajor_desc(0) >> 32);
       const uint32_t b_lo0 = (uint32_t)ptx::make_sw128_kmajor_desc(ptx::smem_u32(b_base));
-      int sa = 0, sb = 0, buf = 0, dn = 0;
-      uint32_t pa = 0, pb = 0, pacc = 1;
-      bool ready = false;  // the barriers of the coming step were seen complete
-      while (it.next()) {
-        const int s0 = it.s0(), s1 = it.s1();
-        int in_fold = 0;
-        for (int s = s0; s < s1; ++s) {
-          if (!__all_sync(0xffffffffu, ready)) {
-            if (in_fold == 0) ptx::mbar_wait(&acc_empty[buf], pacc, abort_flag, p.err_word, ptx::kErrWaitTmemEmpty);
-            ptx::mbar_wait(&b_full[sb], pb, abort_flag, p.err_word, ptx::kErrWaitFull);
-            ptx::mbar_wait(&a_full[sa], pa, abort_flag, p.err_word, ptx::kErrWaitConv);
-          }
+      const uint32_t b_full_a = ptx::smem_u32(b_full), a_full_a = ptx::smem_u32(a_full), acc_empty_a = ptx::smem_u32(acc_empty),
+                     acc_full_a = ptx::smem_u32(acc_full), done_a = ptx::smem_u32(done);
+      // Alternating only while the rings are long enough: a wait for step i may not find its barrier a whole turn behind.
+      // The accumulator that the fold needs was drained, and with it (the drain goes in order) all folds up to kAcc before;
+      // step i - kASlots has to be among those.
+      const bool alternate = (kAcc - 1) * p.fu < kASlots;
+      const uint32_t me = (uint32_t)warp >> 1;
+      const uint32_t total = (uint32_t)it.steps(), fu = (uint32_t)p.fu;
+      const uint32_t jump = alternate ? fu : 0u;  // steps of the other issuer between two folds
+      uint32_t j = me * fu, buf = me, pacc = 1, sb = j % kB, pb = 0;
+      const uint32_t buf_inc = alternate ? 2 : 1;
+      if (!alternate && me) j = total;
+      // The accumulator is what is waited for longest, so its barrier comes last where the turns of the other rings are this
+      // issuer's own steps (and first where they are not, see above).
+      constexpr bool kAccLast = kB % 2 == 0 && kASlots % 2 == 0;
+      while (j < total) {
+        if (!kAccLast) ptx::bar_wait(acc_empty_a + buf * 8, pacc, abort_flag, p.err_word, ptx::kErrWaitTmemEmpty);
+        const uint32_t d = tb + buf * C::kAccCols;
+        for (uint32_t q = 0; q < fu; ++q, ++j) {
+          const uint32_t sa = j % kASlots;
+          ptx::bar_wait(b_full_a + sb * 8, pb, abort_flag, p.err_word, ptx::kErrWaitFull);
+          ptx::bar_wait(a_full_a + sa * 8, (j / kASlots) & 1, abort_flag, p.err_word, ptx::kErrWaitConv);
+          if (kAccLast && q == 0) ptx::bar_wait(acc_empty_a + buf * 8, pacc, abort_flag, p.err_word, ptx::kErrWaitTmemEmpty);
           ptx::tcgen05_fence_after();
-          const uint32_t d = tb + buf * NC, a = tb + C::kACol0 + sa * kACols;
-          const uint32_t lo = b_lo0 + (uint32_t)sb * (C::kBStage >> 4);
-          const uint32_t acc0 = in_fold != 0 ? 1u : 0u;
-          const int buf_now = buf, dn_now = dn;
-          const bool last = ++in_fold == p.fu || s + 1 == s1;
-          if (++sa == kASlots) { sa = 0; pa ^= 1; }
-          if (++sb == kB) { sb = 0; pb ^= 1; }
-          if (++dn == kDone) dn = 0;
-          if (last) {
-            in_fold = 0;
-            if (++buf == kAcc) { buf = 0; pacc ^= 1; }
-          }
-          ready = ptx::mbar_test_wait(&a_full[sa], pa) & ptx::mbar_test_wait(&b_full[sb], pb) &
-                  (!last | ptx::mbar_test_wait(&acc_empty[buf], pacc));
+          const uint32_t a = tb + C::kACol0 + sa * kACols;
+          const uint32_t lo = b_lo0 + sb * (C::kBStage >> 4);
           if (ptx::elect_one()) {
 #pragma unroll
-            for (int k = 0; k < KS / 16; ++k)
-              ptx::mma_f16_ts(d, a + k * 8, ((uint64_t)desc_hi << 32) | (uint64_t)(lo + (k >> 2) * (NC * 128 >> 4) + (k & 3) * 2), idesc,
-                              acc0 | (uint32_t)k);
-            ptx::mma_commit(&done[dn_now]);
-            if (last && p.fu > 1) ptx::mma_commit(&acc_full[buf_now]);
+            for (int k = 0; k < KS / 16; ++k) {
+              constexpr int kPerAcc = KS / 16 / SUB;
+              ptx::mma_f16_ts(d + k / kPerAcc * NC, a + k * 8, ((uint64_t)desc_hi << 32) | (uint64_t)(lo + (k >> 2) * (NC * 128 >> 4) + (k & 3) * 2),
+                              idesc, q | (uint32_t)(k % kPerAcc));
+            }
+            ptx::mma_commit_a(done_a + (j % kDone) * 8);
+            if (q + 1 == fu) ptx::mma_commit_a(acc_full_a + buf * 8);
           }
+          if (++sb == kB) { sb = 0; pb ^= 1; }
         }
+        j += jump;
+        sb += jump;
+        if (sb >= kB) { sb -= kB; pb ^= 1; }
+        buf += buf_inc;
+        if (buf >= kAcc) { buf -= kAcc; pacc ^= 1; }
       }
     }
     __syncwarp();
-  } else if (warp < 12) {
-    // ---------------- converters: lane = weight row; group g takes the steps of its parity ----------------
-    reg_dec<kConvRegs>();
+  } else if (warp < 4 + 4 * kGroups) {
+    // ---------------- converters: lane = weight row; two groups take half of a step's values each ----------------
+    reg_dec<C::kConvRegs>();
     const int quad = warp & 3, grp = (warp - 4) >> 2;
-    const int r = quad * 32 + lane;
-    const uint32_t sw = (uint32_t)(r & 7);
-    const uint32_t raw_row = ptx::smem_u32(raw_base) + r * 128;
-    const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16) + C::kACol0;
-    constexpr int kPieces = KS * WBITS / 8 / 16;  // 16-byte pieces of a row per step: 2, 4 or 8
-    FragIter it(p);
-    int rs = 0;
-    uint32_t rph = 0, i = 0;
-    while (it.next()) {
-      const int s0 = it.s0(), s1 = it.s1();
-      for (int s = s0; s < s1; s += kSPR) {
-        if (kSPR > 1 || (int)(i & 1) == grp) {
-          ptx::mbar_wait_warp(&raw_full[rs], rph, abort_flag, p.err_word, ptx::kErrWaitRaw);
-          const uint32_t row = raw_row + rs * kRawBytes;
-#pragma unroll 1
-          for (int q = 0; q < kSPR; ++q) {
-            const uint32_t j = i + q;
-            if (s + q >= s1 || (int)(j & 1) != grp) continue;
-            auto piece = [&](int c) { return lds128(row + (((uint32_t)(q * kPieces + c) ^ sw) << 4)); };
-            uint4 v = piece(0);
-            // the MMAs that read this operand slot last are complete
-            if (j >= (uint32_t)kASlots)
-              ptx::mbar_wait_warp(&done[(j - kASlots) % kDone], ((j - kASlots) / kDone) & 1, abort_flag, p.err_word, ptx::kErrWaitEmpty);
-            ptx::tcgen05_fence_after();
-            uint32_t t = t_row + (j % kASlots) * kACols;
-            // Rolled: the three kinds of warps of a scheduler share its instruction cache, and this body is the longest.
-#pragma unroll 1
-            for (int c = 0; c < kPieces; ++c) {
-              const uint4 nx = piece(min(c + 1, kPieces - 1));
-              uint32_t o[16];
-              if constexpr (WBITS == 4) {
-                cvt_s4x8<XT>(v.x, o);
-                cvt_s4x8<XT>(v.y, o + 4);
-                cvt_s4x8<XT>(v.z, o + 8);
-                cvt_s4x8<XT>(v.w, o + 12);
-                ptx::tmem_st_32x32b_x16(t, o);
-                t += 16;
-              } else {
-                cvt_s8x4<XT>(v.x, o);
-                cvt_s8x4<XT>(v.y, o + 2);
-                cvt_s8x4<XT>(v.z, o + 4);
-                cvt_s8x4<XT>(v.w, o + 6);
-                ptx::tmem_st_32x32b_x8(t, o);
-                t += 8;
-              }
-              v = nx;
-            }
-            ptx::tmem_st_wait();
-            ptx::tcgen05_fence_before();
-            __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&a_full[j % kASlots]);
+    const uint32_t r = quad * 32 + lane;
+    constexpr int kTeams = C::kTeams, kTV = C::kTV, kVV = C::kVV;
+    constexpr int kWords = kVV / 2 < 32 ? kVV / 2 : 32; // words of converted pairs per tensor-memory store
+    constexpr int kPieces = kWords * 2 * WBITS / 128;   // the 16-byte pieces of a row that make them
+    const uint32_t done_a = ptx::smem_u32(done), a_full_a = ptx::smem_u32(a_full);
+    const int team = grp / C::kTeamGroups, part = grp % C::kTeamGroups;
+    const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16) + C::kACol0 + part * (kVV / 2);
+    const uint32_t steps = (uint32_t)FragIter(p).steps();
+    uint32_t s = team;
+    uint32_t off = s * KS + part * kVV;  // of this group's values in the raw tile
+    uint32_t rs = off / kTV * 8;         // eight times the raw slot
+    off = off % kTV * WBITS / 8;
+    uint32_t rph = 0;
+    const uint32_t raw_full_a = ptx::smem_u32(raw_full), raw_empty_a = ptx::smem_u32(raw_empty);
+    // the row in the first raw tile, with the swizzle: piece c is at row0 ^ (c << 4)
+    const uint32_t row0 = ptx::smem_u32(raw_base) + r * 128 + ((r & 7) << 4);
+    for (; s < steps; s += kTeams) {
+      ptx::bar_wait(raw_full_a + rs, rph, abort_flag, p.err_word, ptx::kErrWaitRaw);
+      const uint32_t row = (row0 + rs * (kRawBytes / 8)) ^ off;
+      const uint32_t sa = kASlots == kTeams ? (uint32_t)team : s % kASlots, ts = t_row + sa * kACols;
+#pragma unroll
+      for (int h = 0; h < kVV / 2 / kWords; ++h) {
+        uint32_t o[kWords];
+#pragma unroll
+        for (int c = 0; c < kPieces; ++c) {
+          const uint4 w = lds128(row ^ ((h * kPieces + c) << 4));
+          if constexpr (WBITS == 4) {
+            cvt_s4x8<XT>(w.x, o + 16 * c);
+            cvt_s4x8<XT>(w.y, o + 16 * c + 4);
+            cvt_s4x8<XT>(w.z, o + 16 * c + 8);
+            cvt_s4x8<XT>(w.w, o + 16 * c + 12);
+          } else {
+            cvt_s8x4<XT>(w.x, o + 8 * c);
+            cvt_s8x4<XT>(w.y, o + 8 * c + 2);
+            cvt_s8x4<XT>(w.z, o + 8 * c + 4);
+            cvt_s8x4<XT>(w.w, o + 8 * c + 6);
           }
-          __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(&raw_empty[rs]);
         }
-        i += min(kSPR, s1 - s);
-        if (++rs == kRaw) { rs = 0; rph ^= 1; }
+        if (h == 0) {
+          // the MMAs that read this operand slot last are complete
+          if (s >= (uint32_t)kASlots)
+            ptx::bar_wait(done_a + (s - kASlots) % kDone * 8, (s - kASlots) / kDone & 1, abort_flag, p.err_word, ptx::kErrWaitEmpty);
+          ptx::tcgen05_fence_after();
+        }
+        if constexpr (kWords == 32) ptx::tmem_st_32x32b_x32(ts + 32 * h, o);
+        else ptx::tmem_st_32x32b_x16(ts, o);
       }
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive_a(raw_empty_a + rs);
+      ptx::tmem_st_wait();
+      ptx::tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive_a(a_full_a + sa * 8);
+      if constexpr (kTeams * KS >= kTV) {
+        rs += kTeams * KS / kTV * 8;
+      } else {
+        off += kTeams * KS * WBITS / 8;
+        if (off >= 128) {
+          off -= 128;
+          rs += 8;
+        }
+      }
+      if (rs >= kRaw * 8) { rs -= kRaw * 8; rph ^= 1; }
     }
   } else {
     // ---------------- drain: thread = weight row (its TMEM lane), half of the item's tokens ----------------
-    reg_inc<kDrainRegs>();
-    const int quad = warp & 3, grp = (warp - 12) >> 2;
+    reg_inc<C::kDrainRegs>();
+    const int quad = warp & 3, grp = (warp - 4 - 4 * kGroups) >> 2;
     const int rl = quad * 32 + lane;
-    const int dt = (int)threadIdx.x - 12 * 32;  // 0..255
+    const int dt = (int)threadIdx.x - (4 + 4 * kGroups) * 32;  // 0..255
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + grp * DT;
     auto drain_bar = [&]() { asm volatile("bar.sync 1, 256;" ::: "memory"); };
     __shared__ int s_npart;
-    const uint32_t* my_scale = s_scale + dt;
-    const uint32_t my_scale_u32 = ptx::smem_u32(my_scale);
-    // (a tile starts at an even row)
-    auto value = [&](int i, int f) { return scale_in<W16, XT>(my_scale + i * kDrain, rl, f, (int)p.N, p.s_dt); };
+    const uint32_t my_scale_a = ptx::smem_u32(s_scale + dt), acc_empty_a = ptx::smem_u32(acc_empty);
+    // the scale of block f at place i of the ring
+    auto value = [&](uint32_t i, int f) {
+      uint32_t w;
+      asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w) : "r"(my_scale_a + i * (kDrain * 4)) : "memory");
+      return scale_of_word<W16, XT>(w, rl, f, (int)p.N);  // (a tile starts at an even row)
+    };
+    const uint32_t acc_full_a = ptx::smem_u32(acc_full);
+    if (!p.blocked) {
+#pragma unroll 1
+      for (int e = 0; e < kScaleRing; ++e) asm volatile("st.shared.f32 [%0], 0f3f800000;" ::"r"(my_scale_a + e * (kDrain * 4)) : "memory");
+    }
+    const bool block_zp = p.blocked && p.zp;
+    const int gt = dt % (kDrain / 2);
+    const uint32_t sums_a = ptx::smem_u32(reinterpret_cast<uint8_t*>(s_scale) + C::kScaleBytes) + grp * (kScaleRing * DT * 4);
+    // the drain group's threads have all come here
+    auto group_bar = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(2 + grp), "n"(kDrain / 2) : "memory"); };
     const int place = deal_place(p);
-    bool waited = false;
     FragIter it(p);
-    int buf = 0;
-    uint32_t i = 0, pacc = 0;
-    while (it.next()) {
+    uint32_t i = 0;  // folds of this CTA
+    // Block scales and zero points are a stream of their own (a round trip to HBM each): every thread copies its own row's, one
+    // to two batches of folds ahead, into a ring of its own; the first two of a fragment ahead of the epilogue of the fragment
+    // before it.  (Held in registers that shift from fold to fold, the shift waits for the load of the fold before, whatever
+    // the nominal distance.)
+    const uint8_t *scp = nullptr, *zpp = nullptr;
+    int to_fetch = 0, xs_at = 0, xs_end = 0;  // blocks of the fragment that are left; the next whose sums are fetched, and their end
+    const float* xs_m = nullptr;              // block sums of the thread's piece of the group's tokens
+    const int xs_e = gt / (DT / 4), xs_piece = gt % (DT / 4);
+    auto fetch_batch = [&](uint32_t at) {
+      const uint32_t dst = my_scale_a + at * (kDrain * 4);
+      if (to_fetch >= C::kBatch) {
+#pragma unroll
+        for (int e = 0; e < C::kBatch; ++e) {
+          copy_scale_word<W16>(dst + e * (kDrain * 4), scp);
+          scp += p.sc_pitch;
+        }
+        if (p.zp) {
+#pragma unroll
+          for (int e = 0; e < C::kBatch; ++e) {
+            copy_scale_word<W16>(dst + (kScaleRing + e) * (kDrain * 4), zpp);
+            zpp += p.sc_pitch;
+          }
+        }
+      } else if (p.blocked) {
+#pragma unroll 1
+        for (int e = 0; e < C::kBatch; ++e) {
+          const uint32_t d = dst + e * (kDrain * 4);
+          if (e < to_fetch) {
+            copy_scale_word<W16>(d, scp);
+            scp += p.sc_pitch;
+            if (p.zp) {
+              copy_scale_word<W16>(d + kScaleRing * (kDrain * 4), zpp);
+              zpp += p.sc_pitch;
+            }
+          } else {
+            // beyond the last block: its sums are zero, and the factor has to be a number
+            asm volatile("st.shared.u32 [%0], 0;" ::"r"(d) : "memory");
+            asm volatile("st.shared.u32 [%0], 0;" ::"r"(d + kScaleRing * (kDrain * 4)) : "memory");
+          }
+        }
+      }
+      if (block_zp) {
+        // the sums of the batch's blocks for the group's tokens, 16 bytes by a thread
+        if (xs_e < C::kBatch && xs_at + xs_e < xs_end)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sums_a + (at + xs_e) * (DT * 4) + xs_piece * 16),
+                       "l"(xs_m + (int64_t)min(xs_at + xs_e, p.S - 1) * p.xs_pitch)
+                       : "memory");
+        xs_at += C::kBatch;
+      }
+      to_fetch -= C::kBatch;
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // the scales of the fragment that `it` has come to
+    auto fetch_first = [&]() {
+      const int b0 = it.u0 * p.fpu * SUB, b1 = it.u1 * p.fpu * SUB;
+      const int64_t off = min((int64_t)it.tile * BMW + rl, p.N - 1) * (W16 ? 2 : 4) + b0 * p.sc_pitch;
+      scp = static_cast<const uint8_t*>(p.scale) + off;
+      zpp = static_cast<const uint8_t*>(p.zp) + off;
+      to_fetch = p.blocked ? min(b1, p.S) - b0 : 0;
+      xs_at = b0;
+      xs_end = b1;
+      xs_m = p.xs + it.y * p.th + grp * DT + xs_piece * 4;
+      fetch_batch(0);
+      fetch_batch(C::kBatch);
+    };
+    bool more = it.next();
+    if (more) {
+      // scales (a conversion may be the kernel in front), block sums, scratch and `out` belong to earlier kernels until here
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      fetch_first();
+    }
+    while (more) {
       const int64_t n = (int64_t)it.tile * BMW + rl;
       const bool n_ok = n < p.N;
+      const int item = it.item, f0 = it.u0 * p.fpu, f1 = it.u1 * p.fpu;  // folds
       const bool first = it.u0 == 0, last = it.u1 == p.ut;
       const int m0 = it.y * p.th + grp * DT;                      // first token of this thread
       const int mcount = min(p.M - m0, min(DT, p.th - grp * DT)); // its tokens
       float total[DT];
 #pragma unroll
       for (int t = 0; t < DT; ++t) total[t] = 0.f;
-      // Block scales and zero points are a stream of their own (a round trip to HBM each): every thread copies its own
-      // row's, seven folds ahead, into a ring of its own.  (Held in registers that shift from fold to fold, the shift
-      // waits for the load of the fold before, whatever the nominal distance.)
-      const int64_t sc_off = min(n, p.N - 1) * (W16 ? 2 : 4);
-      const uint8_t* scp = static_cast<const uint8_t*>(p.scale) + sc_off;
-      const uint8_t* zpp = static_cast<const uint8_t*>(p.zp) + sc_off;
-      auto fetch = [&](int f) {
-        if (p.blocked && f < it.u1) {
-          const uint32_t dst = my_scale_u32 + (uint32_t)(f % kScaleRing) * (kDrain * 4);
-          copy_scale_word<W16>(dst, scp + f * p.sc_pitch);
-          if (p.zp) copy_scale_word<W16>(dst + kScaleRing * kDrain * 4, zpp + f * p.sc_pitch);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-      };
-      if (!waited) {
-        // scales (a conversion may be the kernel in front), block sums, scratch and `out` belong to earlier kernels until here
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-        waited = true;
-      }
+      uint32_t half = 0;  // batch of the ring
 #pragma unroll 1
-      for (int f = 0; f < kScaleRing - 1; ++f) fetch(it.u0 + f);
-      for (int f = it.u0; f < it.u1; ++f) {
-        fetch(f + kScaleRing - 1);
-        if (p.fu == 1) {
-          ptx::mbar_wait_warp(&done[i % kDone], (i / kDone) & 1, abort_flag, p.err_word, ptx::kErrWaitTmemFull);
-          ++i;
-        } else {
-          ptx::mbar_wait_warp(&acc_full[buf], pacc, abort_flag, p.err_word, ptx::kErrWaitTmemFull);
-        }
-        ptx::tcgen05_fence_after();
-        const uint32_t a = lane_addr + buf * NC;
-        // the next sixteen columns are on their way while the current ones are added
-        uint32_t r[2][16];
-        ptx::tmem_ld_32x32b_x16(a, r[0]);
-        asm volatile("cp.async.wait_group %0;" ::"n"(kScaleRing - 1) : "memory");
-        const float sc = p.blocked ? value(f % kScaleRing, f) : 1.f;
+      for (int f = f0; f < f1;) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        if (block_zp) group_bar();  // the block sums of the batch have landed
+        const int fe = min(f1, f + C::kBatch / SUB);
+        uint32_t at = half;
+#pragma unroll 1
+        for (; f < fe; ++f, ++i, at += SUB) {
+          float sc[SUB];
 #pragma unroll
-        for (int c = 0; c < DT / 16; ++c) {
-          uint32_t* cur = r[c & 1];
-          ptx::tmem_ld_wait();
-          ptx::tmem_ld_landed16(cur);
-          if (c + 1 < DT / 16) {
-            ptx::tmem_ld_32x32b_x16(a + 16 * (c + 1), r[(c + 1) & 1]);
-          } else {
+          for (int h = 0; h < SUB; ++h) sc[h] = value(at + h, f * SUB + h);
+          if (block_zp) {
+            // the zero points' share first, while the fold's MMAs run: it needs the block sums only
+#pragma unroll
+            for (int h = 0; h < SUB; ++h) {
+              const float z = value(kScaleRing + at + h, f * SUB + h) * (-1.f / Unit<XT>::kBack);  // (zero beyond the last block)
+#pragma unroll
+              for (int t = 0; t < DT; t += 4) {
+                const uint4 v = lds128(sums_a + (at + h) * (DT * 4) + t * 4);
+                total[t] = fmaf(z, __uint_as_float(v.x), total[t]);
+                total[t + 1] = fmaf(z, __uint_as_float(v.y), total[t + 1]);
+                total[t + 2] = fmaf(z, __uint_as_float(v.z), total[t + 2]);
+                total[t + 3] = fmaf(z, __uint_as_float(v.w), total[t + 3]);
+              }
+            }
+          }
+          static_assert(kAcc == 2, "turns of the accumulators");
+          const uint32_t buf = i % kAcc;
+          ptx::bar_wait(acc_full_a + buf * 8, (i >> 1) & 1, abort_flag, p.err_word, ptx::kErrWaitTmemFull);
+          ptx::tcgen05_fence_after();
+          const uint32_t a = lane_addr + buf * C::kAccCols;
+          auto release = [&]() {
             ptx::tcgen05_fence_before();
             __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&acc_empty[buf]);
-          }
+            if (lane == 0) ptx::mbar_arrive_a(acc_empty_a + buf * 8);
+          };
+          constexpr int CH = C::kCh, NB = C::kChBufs, kChunks = DT / CH;
+          uint32_t r[NB][CH];
+          auto load = [&](uint32_t at, uint32_t* to) {
+            if constexpr (CH == 16) ptx::tmem_ld_32x32b_x16(at, to);
+            else if constexpr (CH == 32) ptx::tmem_ld_32x32b_x32(at, to);
+            else {
+              ptx::tmem_ld_32x32b_x16(at, to);
+              ptx::tmem_ld_32x32b_x8(at + 16, to + 16);
+            }
+          };
+          auto add = [&](const uint32_t* from, float s, float* to) {
 #pragma unroll
-          for (int t = 0; t < 16; ++t) total[16 * c + t] = fmaf(sc, __uint_as_float(cur[t]), total[16 * c + t]);
-        }
-        if (++buf == kAcc) {
-          buf = 0;
-          pacc ^= 1;
-        }
-        if (p.blocked && p.zp) {
-          const float z = -value(kScaleRing + f % kScaleRing, f);
-          const float* xs = p.xs + (int64_t)f * p.xs_pitch + m0;  // the same for all lanes; the pitch covers whole tiles
+            for (int t = 0; t < CH; ++t) to[t] = fmaf(s, __uint_as_float(from[t]), to[t]);
+          };
+          if constexpr (SUB > 1) {
 #pragma unroll
-          for (int t = 0; t < DT; t += 4) {
-            const float4 v = ld_ordered(reinterpret_cast<const float4*>(xs + t));
-            total[t] = fmaf(z, v.x, total[t]);
-            total[t + 1] = fmaf(z, v.y, total[t + 1]);
-            total[t + 2] = fmaf(z, v.z, total[t + 2]);
-            total[t + 3] = fmaf(z, v.w, total[t + 3]);
+            for (int h = 0; h < SUB; ++h) load(a + h * NC, r[h]);
+            ptx::tmem_ld_wait();
+#pragma unroll
+            for (int h = 0; h < SUB; ++h)
+#pragma unroll
+              for (int t = 0; t < CH; t += 8) ptx::tmem_ld_landed8(r[h] + t);
+            release();
+#pragma unroll
+            for (int h = 0; h < SUB; ++h) add(r[h], sc[h], total);
+          } else {
+            load(a, r[0]);
+#pragma unroll
+            for (int c = 0; c < kChunks; ++c) {
+              uint32_t* cur = r[c % NB];
+              ptx::tmem_ld_wait();
+#pragma unroll
+              for (int t = 0; t < CH; t += 8) ptx::tmem_ld_landed8(cur + t);
+              if (NB > 1 && c + 1 < kChunks) load(a + (c + 1) * CH, r[(c + 1) % NB]);
+              if (c + 1 == kChunks) release();
+              add(cur, sc[0], total + CH * c);
+              if (NB == 1 && c + 1 < kChunks) load(a + (c + 1) * CH, r[0]);
+            }
           }
         }
+        if (block_zp) group_bar();
+        fetch_batch(half);  // the batch that was used up
+        half = C::kBatch - half;
       }
       // ---- end of the fragment ----
-      // Sixteen tokens at a time in a rolled loop that rotates the sums through the first sixteen registers: unrolled over
-      // all tokens this part is tens of kilobytes of code that runs once per item, and fetching it took 10 to 30 us.
+      more = it.next();
+      if (more) fetch_first();
+      // Up to 32 tokens at a time in a rolled loop that rotates the sums through the first registers: unrolled over all tokens
+      // this part is tens of kilobytes of code that runs once per item, and fetching it took 10 to 30 us.
+      constexpr int EC = DT <= 32 ? DT : 16;
       int np = 0;
       if (first && !last) {
         // the sums of the CTAs that continue the item are added in CTA order, once they are all there
         if (dt == 0) {
           int cnt = 0;
           for (int c2 = place + 1; c2 < p.g2; ++c2) {
-            if (it.share(c2) >= (it.item - p.items1 + 1) * p.ut) break;
+            if (it.share(c2) >= (item - p.items1 + 1) * p.ut) break;
             ++cnt;
           }
           s_npart = cnt;
@@ -523,58 +675,79 @@ __global__ void __launch_bounds__(kThreads, 1)
       const float ps = p.blocked || !n_ok ? 1.f : scale_value(load_scale_bits(p.scale, n, p.s_dt), p.s_dt);
       const float z1 = !p.blocked && p.zp && n_ok ? -scale_value(load_scale_bits(p.zp, n, p.s_dt), p.s_dt) : 0.f;
 #pragma unroll 1
-      for (int c = 0; c < DT / 16; ++c) {
-        const int l0 = grp * DT + 16 * c;  // token inside the item
-        const int count = min(16, mcount - 16 * c);
+      for (int c = 0; c < DT / EC; ++c) {
+        const int l0 = grp * DT + EC * c;  // token inside the item
+        const int count = min(EC, mcount - EC * c);
         if (lost) {
 #pragma unroll
-          for (int t = 0; t < 16; ++t) total[t] = __uint_as_float(0x7fc00000u);
+          for (int t = 0; t < EC; ++t) total[t] = __uint_as_float(0x7fc00000u);
         }
         if (!first) {
           // a later K range of an item that another CTA started: leave the sums for that CTA
-          float* dst = p.partial + ((size_t)place * p.th + l0) * BMW + rl;
+          float4* dst = reinterpret_cast<float4*>(p.partial + ((size_t)place * p.th + l0) * BMW) + rl;
 #pragma unroll
-          for (int t = 0; t < 16; ++t)
-            if (t < count) __stcg(dst + t * BMW, total[t]);
+          for (int t = 0; t < EC; t += 4)
+            if (t < count) __stcg(dst + t / 4 * BMW, make_float4(total[t], total[t + 1], total[t + 2], total[t + 3]));
         } else {
+          // added in CTA order; two partial tiles on their way at a time where the registers allow (a round trip to L2 each)
+          constexpr int kAhead = DT <= 32 ? 2 : 1;
+          const float4* src = reinterpret_cast<const float4*>(p.partial + ((size_t)(place + 1) * p.th + l0) * BMW) + rl;
+          const size_t pitch = (size_t)p.th * (BMW / 4);
 #pragma unroll 1
-          for (int j = 0; j < np; ++j) {
-            const float* src = p.partial + ((size_t)(place + 1 + j) * p.th + l0) * BMW + rl;
-            float v[16];
+          for (int j = 0; j < np; j += kAhead, src += kAhead * pitch) {
 #pragma unroll
-            for (int t = 0; t < 16; ++t) v[t] = t < count ? __ldcg(src + t * BMW) : 0.f;
+            for (int t0 = 0; t0 < EC; t0 += 16) {
+              float4 v[kAhead][4];
 #pragma unroll
-            for (int t = 0; t < 16; ++t) total[t] += v[t];
+              for (int a = 0; a < kAhead; ++a)
+#pragma unroll
+                for (int t = 0; t < 4; ++t)
+                  v[a][t] = t0 + 4 * t < count && j + a < np ? __ldcg(src + a * pitch + (t0 / 4 + t) * BMW) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+              for (int a = 0; a < kAhead; ++a)
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                  total[t0 + 4 * t] += v[a][t].x;
+                  total[t0 + 4 * t + 1] += v[a][t].y;
+                  total[t0 + 4 * t + 2] += v[a][t].z;
+                  total[t0 + 4 * t + 3] += v[a][t].w;
+                }
+            }
           }
+#pragma unroll
+          for (int t = 0; t < EC; ++t) total[t] *= Unit<XT>::kBack;
           if (!p.blocked) {
 #pragma unroll
-            for (int t = 0; t < 16; ++t) {
+            for (int t = 0; t < EC; ++t) {
               total[t] *= ps;
-              if (p.zp && t < count) total[t] = fmaf(z1, ld_ordered(p.xs + m0 + 16 * c + t), total[t]);
+              if (p.zp && t < count) total[t] = fmaf(z1, ld_ordered(p.xs + m0 + EC * c + t), total[t]);
             }
           }
-          const int64_t row_out = m0 + 16 * c;
+          const int64_t row_out = m0 + EC * c;
           if (!p.gate_up) {
-            store16(p.out, p.out_dt, row_out * p.N + n, p.N, total, n_ok ? count : 0);
+            store_tokens<EC>(p.out, p.out_dt, row_out * p.N + n, p.N, total, n_ok ? count : 0);
           } else {
-            // rows come in groups of 16: eight gate rows, then the eight up rows of the same outputs
-            float v[16];
+            // Rows come in groups of 16: eight gate rows, then the eight up rows of the same outputs.  The thread of the gate
+            // row does the first half of the tokens, that of the up row the second.
+            const bool up_row = (rl & 8) != 0;
+            float v[EC / 2];
 #pragma unroll
-            for (int t = 0; t < 16; ++t) {
-              const float u = __shfl_down_sync(0xffffffffu, total[t], 8);
-              v[t] = total[t] / (1.f + expf(-total[t])) * u;
+            for (int t = 0; t < EC / 2; ++t) {
+              const float got = __shfl_xor_sync(0xffffffffu, up_row ? total[t] : total[t + EC / 2], 8);
+              const float g = up_row ? got : total[t], u = up_row ? total[t + EC / 2] : got;
+              v[t] = g / (1.f + expf(-g)) * u;
             }
-            store16(p.out, p.out_dt, row_out * (p.N >> 1) + ((n >> 4) << 3) + (n & 7), p.N >> 1, v, n_ok && (rl & 8) == 0 ? count : 0);
+            const int t0 = up_row ? EC / 2 : 0;
+            store_tokens<EC / 2>(p.out, p.out_dt, (row_out + t0) * (p.N >> 1) + ((n >> 4) << 3) + (n & 7), p.N >> 1, v, n_ok ? count - t0 : 0);
           }
         }
 #pragma unroll
-        for (int t = 0; t + 16 < DT; ++t) total[t] = total[t + 16];
+        for (int t = 0; t + EC < DT; ++t) total[t] = total[t + EC];
       }
       if (!first) {
         drain_bar();  // orders every drain thread's stores before thread 0's fence, which is cumulative
         if (dt == 0) ptx::partial_publish(p.flags + place);
       }
-      asm volatile("cp.async.wait_group 0;" ::: "memory");  // the ring is refilled from its start
     }
   }
 
@@ -586,28 +759,34 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
-// Sums of the activations over each scale block, for the zero points: xs[b * pitch + m], one warp per (token, block);
-// tokens from M up to the pitch get zeros.
+// Sums of the activations over each scale block, for the zero points: xs[b * pitch + m]; tokens from M up to the pitch get
+// zeros.  A warp takes 256 values of a row, or a whole larger block, at a time; a block shorter than that is summed by the
+// lanes that hold it. 
+constexpr int kSumsThreads = 512;
 template <typename XT>
-__global__ void __launch_bounds__(256) block_sums_kernel(const XT* x, float* __restrict__ xs, int pitch, int M, int K, int S) {
+__global__ void __launch_bounds__(kSumsThreads) block_sums_kernel(const XT* x, float* __restrict__ xs, int pitch, int M, int K, int S) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  const int lane = threadIdx.x & 31;
-  const int64_t i = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (i >= (int64_t)pitch * S) return;
-  const int m = (int)(i / S), b = (int)(i - (int64_t)m * S), len = K / S;
-  float s = 0.f;
-  if (m < M) {
-    const uint4* row = reinterpret_cast<const uint4*>(x + (int64_t)m * K + (int64_t)b * len);
-    for (int k = lane; k < len / 8; k += 32) {
-      const uint4 v = row[k];
-      const XT* e = reinterpret_cast<const XT*>(&v);
+  const int lane = threadIdx.x & 31, len = K / S;
+  const int per = max(len, 256), pieces = (K + per - 1) / per;
+  const int group = min(32, len / 8);  // lanes that hold a block
+  const int warps = gridDim.x * (kSumsThreads / 32);
+  for (int64_t i = (int64_t)blockIdx.x * (kSumsThreads / 32) + (threadIdx.x >> 5); i < (int64_t)pitch * pieces; i += warps) {
+    const int m = (int)(i / pieces), k0 = (int)(i - (int64_t)m * pieces) * per;
+    float s = 0.f;
+    if (m < M) {
+      const XT* row = x + (int64_t)m * K;
+      for (int k = k0 + lane * 8; k < min(K, k0 + per); k += 256) {
+        const uint4 v = *reinterpret_cast<const uint4*>(row + k);
+        const XT* e = reinterpret_cast<const XT*>(&v);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) s += to_f32(e[j]);
+        for (int j = 0; j < 8; ++j) s += to_f32(e[j]);
+      }
+      for (int o = group >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     }
-    s = warp_sum(s);
+    const int b = (k0 + lane * 8) / len;
+    if (lane % group == 0 && b < S && (group == 32 ? lane == 0 : true)) xs[(int64_t)b * pitch + m] = s;
   }
-  if (lane == 0) xs[(int64_t)b * pitch + m] = s;
 }
 
 template <typename Kernel, typename... Args>
@@ -625,19 +804,24 @@ cudaError_t launch_pdl(Kernel kern, unsigned grid, unsigned block, size_t smem, 
   return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
-template <int WBITS, typename XT, int NC, int KS, bool W16>
+template <int WBITS, typename XT, int NC, int KS, int SUB, bool W16>
 int launch_with(const CUtensorMap& map_w, const CUtensorMap& map_x, const Params& p, int grid, cudaStream_t st) {
-  using C = Cfg<WBITS, NC, KS>;
-  auto kern = tmem_gemm_kernel<WBITS, XT, NC, KS, W16>;
+  using C = Cfg<WBITS, NC, KS, SUB>;
+  auto kern = tmem_gemm_kernel<WBITS, XT, NC, KS, SUB, W16>;
   static bool attr_set[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || !attr_set[dev]) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmem);
     if (e != cudaSuccess) return fail(QMM_ERR_LAUNCH, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    // the warps' shares of the registers add up to this
+    cudaFuncAttributes at;
+    e = cudaFuncGetAttributes(&at, kern);
+    if (e != cudaSuccess || at.numRegs != C::kLaunchRegs)
+      return fail(QMM_ERR_LAUNCH, "tmem_gemm_kernel: built with %d registers per thread, not %d", e == cudaSuccess ? at.numRegs : -1, C::kLaunchRegs);
     if (dev >= 0 && dev < 64) attr_set[dev] = true;
   }
-  cudaError_t e = launch_pdl(kern, (unsigned)grid, kThreads, C::kSmem, st, map_w, map_x, p);
+  cudaError_t e = launch_pdl(kern, (unsigned)grid, C::kThreads, C::kSmem, st, map_w, map_x, p);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(QMM_ERR_LAUNCH, "tmem_gemm_kernel launch: %s", cudaGetErrorString(e));
@@ -645,25 +829,40 @@ int launch_with(const CUtensorMap& map_w, const CUtensorMap& map_x, const Params
   return QMM_OK;
 }
 
-template <int WBITS, typename XT, int NC, int KS>
+template <int WBITS, typename XT, int NC, int KS, int SUB>
 int launch_cfg(const CUtensorMap& map_w, const CUtensorMap& map_x, const Params& p, int grid, cudaStream_t st) {
-  return p.blocked && p.s_dt != QMM_F32 ? launch_with<WBITS, XT, NC, KS, true>(map_w, map_x, p, grid, st)
-                                        : launch_with<WBITS, XT, NC, KS, false>(map_w, map_x, p, grid, st);
+  return p.blocked && p.s_dt != QMM_F32 ? launch_with<WBITS, XT, NC, KS, SUB, true>(map_w, map_x, p, grid, st)
+                                        : launch_with<WBITS, XT, NC, KS, SUB, false>(map_w, map_x, p, grid, st);
+}
+
+// Values per step, and scale blocks per step with an accumulator each
+struct Step {
+  int ks, sub;
+};
+Step step_for(int nc, int64_t block_size) {
+  if (nc <= 64)
+    return block_size == 64 ? Step{128, 2} : block_size == 128 ? Step{256, 2} : block_size > 0 && block_size % 256 != 0 ? Step{128, 1} : Step{256, 1};
+  return block_size == 64 ? Step{64, 1} : Step{128, 1};
 }
 
 template <int WBITS, typename XT>
-int launch_shape(int nc, int ks, const CUtensorMap& map_w, const CUtensorMap& map_x, const Params& p, int grid, cudaStream_t st) {
-#define QMM_CASE(NC)                                                           \
-  case NC:                                                                     \
-    return ks == 64 ? launch_cfg<WBITS, XT, NC, 64>(map_w, map_x, p, grid, st) \
-                    : launch_cfg<WBITS, XT, NC, 128>(map_w, map_x, p, grid, st)
-  switch (nc) {
-    QMM_CASE(32);
-    QMM_CASE(64);
-    QMM_CASE(128);
-    default: QMM_CASE(192);
-  }
+int launch_shape(int nc, const Step& sp, const CUtensorMap& map_w, const CUtensorMap& map_x, const Params& p, int grid, cudaStream_t st) {
+#define QMM_CASE(NC, KS, SUB) \
+  if (nc == NC && sp.ks == KS && sp.sub == SUB) return launch_cfg<WBITS, XT, NC, KS, SUB>(map_w, map_x, p, grid, st)
+  QMM_CASE(32, 128, 2);
+  QMM_CASE(32, 256, 2);
+  QMM_CASE(32, 256, 1);
+  QMM_CASE(64, 128, 2);
+  QMM_CASE(64, 256, 2);
+  QMM_CASE(64, 256, 1);
+  QMM_CASE(32, 128, 1);
+  QMM_CASE(64, 128, 1);
+  QMM_CASE(128, 64, 1);
+  QMM_CASE(128, 128, 1);
+  QMM_CASE(192, 64, 1);
+  QMM_CASE(192, 128, 1);
 #undef QMM_CASE
+  return fail(QMM_ERR_UNSUPPORTED, "tensor-memory kernel: no instance for %d tokens, steps of %d", nc, sp.ks);
 }
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
@@ -697,7 +896,8 @@ Scratch carve(void* base, int64_t M, int64_t K) {
   size_t off = 2048;
   s.flags = reinterpret_cast<uint32_t*>(b);
   s.xs = reinterpret_cast<float*>(b + off);
-  s.xs_pitch = (int)align_up((size_t)M, 4) + 192;  // a drain thread reads whole groups of columns
+  const Plan pl = plan_for(M);
+  s.xs_pitch = (pl.ytiles - 1) * pl.th + pl.nc;  // a drain thread reads all of its columns
   off += align_up((size_t)ceil_div(K, 64) * s.xs_pitch * 4, 256);
   s.partial = reinterpret_cast<float*>(b + off);
   off += (size_t)kMaxCtas * plan_for(M).th * BMW * 4;
@@ -758,14 +958,24 @@ int launch_tmem_gemm(int wbits, const void* x, int x_dt, const void* w, const Sc
   p.out_dt = out_dt;
   p.M = (int)M;
   p.N = N;
-  const int ks = block_size == 64 ? 64 : 128;
-  p.stages = (int)ceil_div(K, ks);
+  const Step sp = step_for(pl.nc, block_size);
+  const int ks = sp.ks;
+  const int stages = (int)ceil_div(K, ks);
   p.blocked = block_size > 0;
   p.S = block_size > 0 ? (int)(K / block_size) : 1;
-  // Per channel the sums leave the tensor core every 512 values all the same: the additions across them are then single
+  // Per channel the sums leave the tensor core about every 512 values all the same: the additions across them are then single
   // fp32 additions in registers, and the drain stays well under the MMAs.
-  p.fu = block_size > 0 ? std::max<int>(1, (int)(block_size / ks)) : 4;
-  p.ut = (int)ceil_div(p.stages, p.fu);
+  const int spr = std::max(1, 1024 / (wbits * ks));  // steps per raw tile
+  if (block_size > 0) {
+    p.fu = (int)std::max<int64_t>(1, block_size / ks);
+    p.unit = p.fu;
+    while (p.unit % spr != 0) p.unit += p.fu;
+  } else {
+    const int folds = (int)ceil_div(stages, 512 / ks);
+    p.fu = p.unit = (int)align_up((size_t)ceil_div(stages, folds), spr);
+  }
+  p.fpu = p.unit / p.fu;
+  p.ut = (int)ceil_div(stages, p.unit);
   p.th = pl.th;
   p.ytiles = pl.ytiles;
   p.gate_up = gate_up;
@@ -782,8 +992,8 @@ int launch_tmem_gemm(int wbits, const void* x, int x_dt, const void* w, const Sc
   if (left != 0) {
     // Splitting the left-over items over s CTAs each: item / s plus an exchange that grows with s (one partial tile per
     // CTA, written, and read by the item's first CTA).
-    const double stage_us = std::max(wbits == 4 ? 0.2 : 0.38, 0.06 + 0.0024 * pl.th) * (ks == 64 ? 0.6 : 1.0);
-    const double item_us = p.stages * stage_us, partial_us = 0.25 + 1.1 * pl.th / 256;
+    const double stage_us = (wbits == 4 ? 0.27 + 0.003 * pl.th : 0.32 + 0.0038 * pl.th) * (ks / 128.0);
+    const double item_us = p.ut * p.unit * stage_us, partial_us = 0.25 + 1.1 * pl.th / 256;
     double s = std::sqrt(item_us / partial_us);
     s = std::min(s, std::min((double)ctas / (double)left, (double)p.ut));
     if (s >= 1.2 && item_us / s + 2.0 + partial_us * s < 0.85 * item_us) {
@@ -795,10 +1005,12 @@ int launch_tmem_gemm(int wbits, const void* x, int x_dt, const void* w, const Sc
   }
 
   if (zp) {
-    const unsigned g = (unsigned)ceil_div((int64_t)sc.xs_pitch * p.S, 8);
-    cudaError_t e = x_dt == QMM_BF16
-                        ? launch_pdl(block_sums_kernel<__nv_bfloat16>, g, 256, 0, st, reinterpret_cast<const __nv_bfloat16*>(x), sc.xs, sc.xs_pitch, (int)M, (int)K, p.S)
-                        : launch_pdl(block_sums_kernel<__half>, g, 256, 0, st, reinterpret_cast<const __half*>(x), sc.xs, sc.xs_pitch, (int)M, (int)K, p.S);
+    const int64_t pieces = ceil_div(K, std::max<int64_t>(K / p.S, 256));
+    const unsigned g = (unsigned)std::min<int64_t>(sm_count(), ceil_div(sc.xs_pitch * pieces, kSumsThreads / 32));
+    cudaError_t e = x_dt == QMM_BF16 ? launch_pdl(block_sums_kernel<__nv_bfloat16>, g, kSumsThreads, 0, st, reinterpret_cast<const __nv_bfloat16*>(x),
+                                                  sc.xs, sc.xs_pitch, (int)M, (int)K, p.S)
+                                     : launch_pdl(block_sums_kernel<__half>, g, kSumsThreads, 0, st, reinterpret_cast<const __half*>(x), sc.xs,
+                                                  sc.xs_pitch, (int)M, (int)K, p.S);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return fail(QMM_ERR_LAUNCH, "block_sums_kernel launch: %s", cudaGetErrorString(e));
@@ -810,10 +1022,10 @@ int launch_tmem_gemm(int wbits, const void* x, int x_dt, const void* w, const Sc
   rc = encode_tmap_2d(&map_x, x, 2, true, (uint64_t)M, (uint64_t)K, (uint32_t)pl.th, 64);
   if (rc != QMM_OK) return rc;
   if (wbits == 4)
-    return x_dt == QMM_BF16 ? launch_shape<4, __nv_bfloat16>(pl.nc, ks, map_w, map_x, p, grid, st)
-                            : launch_shape<4, __half>(pl.nc, ks, map_w, map_x, p, grid, st);
-  return x_dt == QMM_BF16 ? launch_shape<8, __nv_bfloat16>(pl.nc, ks, map_w, map_x, p, grid, st)
-                          : launch_shape<8, __half>(pl.nc, ks, map_w, map_x, p, grid, st);
+    return x_dt == QMM_BF16 ? launch_shape<4, __nv_bfloat16>(pl.nc, sp, map_w, map_x, p, grid, st)
+                            : launch_shape<4, __half>(pl.nc, sp, map_w, map_x, p, grid, st);
+  return x_dt == QMM_BF16 ? launch_shape<8, __nv_bfloat16>(pl.nc, sp, map_w, map_x, p, grid, st)
+                          : launch_shape<8, __half>(pl.nc, sp, map_w, map_x, p, grid, st);
 }
 
 }  // namespace qmm
