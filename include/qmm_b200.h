@@ -217,12 +217,18 @@ QMM_API int qmm_gate_up_decode(int wbits, const void* x, int x_dtype, const void
  * any batch where the tensor-memory kernel (QMM_VARIANT_TMEM) is the choice for [N2,K], else the split-activation kernel
  * (QMM_VARIANT_I8TC) up to 1024 tokens with 16-bit results and 1008 with fp32: bf16 / f16 / f32 activations, K >= 128 and
  * a multiple of 16 (int8) or 32 (int4), block_size 0, 64, 128 or a multiple of 256.  (The operator above this ABI comes
- * here above 32 tokens, and not with blocks of 64.)  workspace: as for qmm_weight_only
+ * here where qmm_gate_up_on_tensor_cores says so, and above 32 tokens not with blocks of 64.)  workspace: as for qmm_weight_only
  * (qmm_weight_only_workspace_size(M, K) bytes, 256-byte aligned, first 2048 bytes zero before the first use).
  * Returns QMM_ERR_UNSUPPORTED outside that range.  No counterpart in the reference (see qmm_gate_up_decode).
  */
 QMM_API int qmm_gate_up(int wbits, const void* x, int x_dtype, const void* w, const float* scale, void* out, int out_dtype,
                 int64_t M, int64_t N2, int64_t K, int64_t block_size, void* workspace, size_t workspace_bytes, void* stream);
+
+/*
+ * Whether qmm_gate_up is the faster of the two for this shape (1) or qmm_gate_up_decode, where that takes it (0): always
+ * above 32 tokens, and from two on by the size of the weight.  Asks no device.
+ */
+QMM_API int qmm_gate_up_on_tensor_cores(int wbits, int x_dtype, int out_dtype, int64_t M, int64_t N2, int64_t K, int64_t block_size);
 
 /*
  * Per-token dynamic activation quantizer:

@@ -115,3 +115,21 @@ def test_steps_that_the_blocks_do_not_fill(wbits, bs, N, K, M, zp, scales):
     exact -= torch.einsum("ms,sn->mn", xb.sum(-1), z.double().to(DEV).view(S, N))
   # exact products, at most K / 128 + 3 roundings of the running sum: far below 1e-5 of the largest result
   assert qo.max_abs_rel(out, exact) < 1e-5
+
+
+@pytest.mark.parametrize("wbits,bs,M", [(4, 128, 9), (4, 128, 32), (8, 128, 4), (4, 64, 20), (8, -1, 17)])
+def test_gate_up_of_small_batches_on_large_weights(wbits, bs, M):
+  """Where the operator takes the tensor-core form at up to 32 tokens: against the two projections and the activation."""
+  from xla_b200 import _capi
+  g = torch.Generator(device=DEV).manual_seed(M)
+  N2, K = 9216, 4096
+  assert _capi.lib().qmm_gate_up_on_tensor_cores(wbits, _capi.BF16, _capi.BF16, M, N2, K, max(bs, 0))
+  w = torch.randint(0, 256, (N2, K * wbits // 8), generator=g, device=DEV, dtype=torch.uint8)
+  w = w if wbits == 4 else w.view(torch.int8)
+  s = (torch.rand((N2,) if bs == -1 else (K // bs, N2), generator=g, device=DEV) + 0.5) / (4.6 if wbits == 4 else 73.) / K**0.5
+  x = torch.randn(M, K, generator=g, device=DEV).bfloat16()
+  kw = dict(block_size=bs, int4_weight=wbits == 4, weight_is_packed=wbits == 4)
+  out = torch.ops.xla_b200.quantized_gate_up(x, w, s, out_dtype=torch.bfloat16, **kw)
+  y = torch.ops.xla_b200.quantized_matmul_packed(x, w, s, None, out_dtype=torch.float32, **kw).view(M, N2 // 16, 2, 8).double()
+  ref = (torch.nn.functional.silu(y[:, :, 0]) * y[:, :, 1]).reshape(M, N2 // 2)
+  assert qo.max_abs_rel(out, ref) < 1e-2  # one rounding to bf16

@@ -63,6 +63,7 @@ SIGNATURES = {
     "qmm_pack_int4_sbn": (_i, [_p, _p, _i64, _i64, _i64, _p]),
     "qmm_unpack_int4_nk": (_i, [_p, _p, _i64, _i64, _p]),
     "qmm_device_error_flag": (_i, [_p, _p]),
+    "qmm_gate_up_on_tensor_cores": (_i, [_i, _i, _i, _i64, _i64, _i64, _i64]),
     "qmm_gate_up": (_i, [ctypes.c_int, _p, ctypes.c_int, _p, _p, _p, ctypes.c_int, _i64, _i64, _i64, _i64, _p, _sz, _p]),
     "qmm_set_peer_wait_limit": (_i, [ctypes.c_double]),
     "qmm_set_activation_limbs": (_i, [ctypes.c_int]),

@@ -191,46 +191,92 @@ static int pick_weight_only(int wbits, int64_t M, int64_t N, int64_t K, int64_t 
   return QMM_VARIANT_GENERIC;
 }
 
-// AUTO's choice between the two warp-level decode kernels (asked before the measured table, which knows neither this kernel
-// nor tmem_gemm.cu).  The integer one streams weights 1.5 times faster, but every
+// AUTO's choice between the two warp-level decode kernels (where the tensor-core kernels below were not taken).  The integer
+// one streams weights 1.5 times faster, but every
 // CTA of it first splits all activations into limbs, about 0.6 us per token at K = 4096, in proportion to M * K; the
 // gain is proportional to the weight bytes.  K cancels: it wins at one token, and up to one token per 1850 bytes of
 // weight column (14336 int8 outputs: 7 tokens; measured 15.1 against 16.7 us at 4, equal at 8; 4096 outputs: 2).
 // Zero points, scale blocks of 64 and ragged K are beyond the other kernel.
-// The line was drawn against decode_mma.cu.  limb_gemm.cu, which the table names on the largest weights, is the faster one
-// there from three tokens on, and at every batch on int8: int4 block 128 [28672,8192] 25.1 us here and 28.0 there at one
-// token, 27.6 and 28.5 at two, 34.5 and 29.0 at five; [57344,8192] 48.9 and 45.7 at one, 65.0 and 47.1 at five; int8
-// [28672,8192] 43.0 and 39.6 at one, 52.2 and 40.6 at five; [14336,4096] 11.8 and 13.7 at one, 15.6 and 13.8 at four.
 static bool use_decode_i8(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, const void* x, int x_dt, const void* w, bool has_zp) {
   if (!decode_i8_supported(wbits, M, N, K, bs, x, x_dt, w, has_zp)) return false;
   return M == 1 || M * 1850 <= N * wbits / 8 || !decode_mma_supported(wbits, M, N, K, bs, x, x_dt, w, has_zp);
 }
 
+// Batches of two tokens and more of which a tensor-core kernel (tmem or i8tc: both take about as long for one token as for
+// 32) beats the decode kernels, whose time grows with the tokens.  `decode`: the integer decode kernel takes the call.
+//   zero points  The other decode kernel is the GEMV, four tokens at a time: int4 block 128 [8192,28672] 70 us at two tokens and
+//                188 at eight, 49 on tmem; [28672,8192] 31 at two, 43 at five on the integer kernel, 49 on tmem, 185 on the GEMV
+//                from six on.  int8: [14336,4096] 15 us at two and 18 at four, 16 on i8tc.
+static bool zp_decode_on_tc(int wbits, int64_t M, int64_t N, int64_t K, bool decode) {
+  const int64_t E = N * K;
+  if (M < 2) return false;
+  if (M > 8) return true;
+  if (!decode) return E >= 1 << 24;
+  return E >= 1 << 25 && (wbits == 8 ? M * E >= 175000000 : M >= 6);
+}
+
 // Where AUTO takes the tensor-memory kernel (16-bit activations).
-//   zero points    above eight tokens: it applies them in the drain it runs anyway (int4 block 128
-//                  [37888,3584] at 29 tokens 42 us against 59 on the split-activation kernel, [14336,4096] at 512: 147
-//                  against 211).  Not per channel with int8 weights, or with larger int4 weights up to the 42 tokens of one
-//                  tile of the other kernel, which hands over once per tile then (20 tokens on [14336,4096]: int8 17.7 us
-//                  against 23.0, int4 14.1 against 20.1; int4 [4096,4096] 12.8 against 11.8; 64 tokens 28 against 22).
-//   blocks of 64   above 32 tokens: the split-activation kernel hands over four times per slot there (int4 [14336,4096] at
-//                  512 tokens 135 us against 232).
-//   int4           above 64 tokens, when the (128-row, up to 192-token) items fill two thirds of the SMs: fewer leave it
-//                  to the split-activation kernel's narrower ones ([4096,4096] at 128 tokens 23 us against 19;
-//                  [14336,4096] at 96 tokens 27 against 35, [28672,8192] at 512 tokens 266 against 337).  Per channel up
-//                  to 384 tokens, from where that kernel expands the weights once.
-//   fp32 results   above 64 tokens, when the items fill half of the SMs: the other kernel needs a third limb per token
-//                  there (int8 [28672,8192] at 512 tokens 257 us against 312, [2432,9248] at 763 tokens 49 against 74).
+//   zero points    with scale blocks wherever a tensor-core kernel is taken: it applies them in the drain it runs anyway (int4
+//                  block 128 [37888,3584] at 29 tokens 32 us against 59 on the split-activation kernel, [14336,4096] at 512: 106
+//                  against 211).  Per channel the other kernel hands over once per tile: int8 up to 64 tokens on fewer
+//                  than 12288 outputs from 33 tokens ([4096,4096] at 64 tokens 20 us, 16 there; [14336,4096] 21, 25 there), large
+//                  int4 weights up to its 42 tokens ([28672,8192] at 16 tokens 37 us, 31 there), all up to eight tokens
+//                  ([8192,28672] 50, 37 there), and above 64 tokens with fewer than 64 items of 128 rows and 192 tokens.
+//   fp32 results   per channel only where the other kernels need as many roundings: above 64 tokens, when the items fill
+//                  half of the SMs (the other kernel needs a third limb per token there; int8 [28672,8192] at 512 tokens 219 us
+//                  against 312, [2432,9248] at 763 tokens 49 against 74).
+//   2..8 tokens    int8 on large weights: block 128 [28672,8192] at two tokens 44 us against 50, [14336,4096] at four 15 against
+//                  17 (per channel 14 against 16).
+//   9..32 tokens   weights of 34 million values, 2^24 from 17 tokens, any for int8 from 17: int4 block 128 [14336,4096] at 16 tokens
+//                  14.3 us against 18.4, [4096,4096] at 24 11.4 against 12.2 (at 16 11.6 against 10.3); int8 per channel
+//                  [1024,4096] at 32 8.8 against 11.  Not per channel from 2^27 values, where i8tc streams faster (int4
+//                  [28672,8192] 34 against 30), nor int4 blocks there up to ten tokens (40 against 31).
+//   33..64 tokens  int4, int8 blocks, int8 per channel below 2^26.5 values: int4 block 128 [57344,8192] at 64 tokens 87 us
+//                  against 104, [4096,4096] 15 against 16.5; int8 [5120,6912] 17 against 22, [28672,8192] 55 against 51.
+//   above 64       int4 and int8 blocks, when the items fill half of the SMs, or 64 of them on weights of 2^25 values: fewer
+//                  leave it to i8tc's narrower ones ([4096,4096] at 128 tokens 26 us against 19; [14336,4096] at 96 25
+//                  against 34, [5120,6912] at 256 33 against 51, [28672,8192] at 512 230 against 337).  int4 per channel from 384
+//                  tokens, where i8tc expands the weights once, on 2^25 values ([4096,4096] at 1024 53 us against 46, [28672,8192]
+//                  400 against 492).
 //   narrow int8    up to 2048 outputs and above the 1024 tokens of one launch of the other kernel, whose launches are then
 //                  a round or two of items each ([1536,14592] at 4178 tokens 189 us against 313).
-static bool use_tmem(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, int x_dt, int out_dt, bool has_zp) {
+static bool use_tmem(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, int x_dt, int out_dt, bool has_zp, bool decode_i8) {
   if (!tmem_gemm_shape_ok(wbits, M, N, K, bs, x_dt)) return false;
-  if (has_zp && bs <= 0 && (wbits == 8 || (M <= 42 && N * K >= 1 << 25)) && limb_tc_shape_ok(wbits, M, N, K, bs, x_dt, true)) return false;
-  if (has_zp) return M > 8;
-  if (bs == 64) return M > 32;
-  const int64_t items = ceil_div(N, 128) * ceil_div(M, 192);
-  if (out_dt == QMM_F32 && M > 64 && 2 * items >= sm_count() && (wbits == 8 || bs > 0 || M < 384)) return true;
-  if (wbits == 8) return M > 1024 && N <= 2048;
-  return M > 64 && 3 * items >= 2 * sm_count() && (bs > 0 || M < 384);
+  const bool blocked = bs > 0;
+  const int64_t E = N * K, items = ceil_div(N, 128) * ceil_div(M, 192);
+  if (has_zp) {
+    if (blocked) return zp_decode_on_tc(wbits, M, N, K, decode_i8);
+    if (!limb_tc_shape_ok(wbits, M, N, K, bs, x_dt, true)) return zp_decode_on_tc(wbits, M, N, K, decode_i8);
+    if (M <= 8) return false;
+    if (M > 64) return items >= 64;
+    return wbits == 4 ? M > 42 || E < 1 << 25 : M <= 32 || N >= 12288;
+  }
+  if (M == 1) return false;
+  if (M <= 64) {
+    if (out_dt == QMM_F32 && !blocked) return false;
+    if (M > 32) return E >= 1 << 22 && (wbits == 4 || blocked || E < 95000000);
+    if (E >= 1 << 27) {
+      if (blocked) return wbits == 8 || M > 10;
+      return wbits == 8 && E < 1 << 28;
+    }
+    if (M > 16) return E >= (wbits == 8 ? 1 << 22 : 1 << 24);
+    if (M > 8) return E >= (wbits == 8 && blocked ? 1 << 24 : 34000000);
+    return wbits == 8 && E >= 34000000 && M >= (blocked ? 3 : 4);
+  }
+  const bool filled = 2 * items >= sm_count();
+  if (out_dt == QMM_F32 && filled && (wbits == 8 || blocked || M < 384)) return true;
+  if (wbits == 8 && !blocked) return M > 1024 && N <= 2048;
+  if (!blocked && M >= 384 && E < 1 << 25) return false;
+  return filled || (items >= 64 && E >= 1 << 25);
+}
+
+// Where AUTO takes the split-activation kernel ahead of the decode kernels, at two to eight tokens: zero points per channel (see
+// above), and weights of 100 MB without (int4 block 128 [57344,8192] at two tokens 46 us against 54, at five 47 against 65;
+// int8 [28672,8192] 41 against 48).
+static bool use_limb_decode(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, int x_dt, bool has_zp, bool decode_i8) {
+  if (M < 2 || M > 16 || x_dt == QMM_F32 || bs == 64 || !limb_tc_shape_ok(wbits, M, N, K, bs, x_dt, has_zp)) return false;
+  if (has_zp) return M <= 8 && bs <= 0 && zp_decode_on_tc(wbits, M, N, K, decode_i8);
+  return N * K * wbits / 8 >= 100000000;
 }
 
 int qmm_w8a16_perchannel(const void* x, int x_dtype, const int8_t* w, const float* scale,
@@ -371,16 +417,19 @@ int qmm_tuned_variant(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_
 int qmm_zero_point_in_kernel(int wbits, int64_t M, int64_t N, int64_t K, int64_t block_size, int x_dtype) {
   if (block_size < 0) block_size = 0;
   const void* ok = reinterpret_cast<const void*>(uintptr_t(256));
-  return M <= 8 || use_tmem(wbits, M, N, K, block_size, x_dtype, QMM_F32, true) || limb_tc_shape_ok(wbits, M, N, K, block_size, x_dtype, true) ||
+  return M <= 8 || use_tmem(wbits, M, N, K, block_size, x_dtype, QMM_F32, true, false) || limb_tc_shape_ok(wbits, M, N, K, block_size, x_dtype, true) ||
          decode_i8_supported(wbits, M, N, K, block_size, ok, x_dtype, ok, true);
 }
 
 // qmm_weight_only's AUTO.  `room`: bytes of usable scratch.
 static int choose_weight_only(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, const void* x, int x_dt, int out_dt, const void* w,
                               bool has_zp, size_t room, bool sm100) {
-  if (use_decode_i8(wbits, M, N, K, bs, x, x_dt, w, has_zp)) return QMM_VARIANT_I8MMA;
+  if (M == 1 && use_decode_i8(wbits, M, N, K, bs, x, x_dt, w, has_zp)) return QMM_VARIANT_I8MMA;
   const bool tma = sm100 && aligned(x, 16) && aligned(w, 16);
-  if (tma && use_tmem(wbits, M, N, K, bs, x_dt, out_dt, has_zp) && room >= tmem_gemm_workspace_bytes(M, K)) return QMM_VARIANT_TMEM;
+  const bool decode_i8 = decode_i8_supported(wbits, M, N, K, bs, x, x_dt, w, has_zp);
+  if (tma && use_tmem(wbits, M, N, K, bs, x_dt, out_dt, has_zp, decode_i8) && room >= tmem_gemm_workspace_bytes(M, K)) return QMM_VARIANT_TMEM;
+  if (tma && use_limb_decode(wbits, M, N, K, bs, x_dt, has_zp, decode_i8) && room >= limb_tc_workspace_bytes(M, K)) return QMM_VARIANT_I8TC;
+  if (use_decode_i8(wbits, M, N, K, bs, x, x_dt, w, has_zp)) return QMM_VARIANT_I8MMA;
   // the measured table first, the shape rule where the table has no entry for this shape
   const int tuned = tuned_variant(wbits, bs, M, N, K);
   if (tma && limb_tc_shape_ok(wbits, M, N, K, bs, x_dt, has_zp) && room >= limb_tc_workspace_bytes(M, K)) {
@@ -519,6 +568,13 @@ int qmm_gate_up_decode(int wbits, const void* x, int x_dtype, const void* w, con
   return launch_decode_mma(wbits, x, x_dtype, w, scale, QMM_F32, out, out_dtype, M, N2, K, block_size, st, 1);
 }
 
+int qmm_gate_up_on_tensor_cores(int wbits, int x_dtype, int out_dtype, int64_t M, int64_t N2, int64_t K, int64_t block_size) {
+  if (M > 32) return 1;
+  if (wbits != 4 && wbits != 8) return 0;
+  block_size = std::max<int64_t>(block_size, 0);
+  return use_tmem(wbits, M, N2, K, block_size, x_dtype, out_dtype, false, false) || use_limb_decode(wbits, M, N2, K, block_size, x_dtype, false, false);
+}
+
 int qmm_gate_up(int wbits, const void* x, int x_dtype, const void* w, const float* scale, void* out, int out_dtype, int64_t M,
                 int64_t N2, int64_t K, int64_t block_size, void* workspace, size_t workspace_bytes, void* stream) {
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
@@ -530,7 +586,7 @@ int qmm_gate_up(int wbits, const void* x, int x_dtype, const void* w, const floa
     return fail(QMM_ERR_BAD_SHAPE, "gate_up: K (%lld) must be a multiple of block_size (%lld)", (long long)K, (long long)block_size);
   if (M == 0 || N2 == 0) return QMM_OK;
   const Scales sc{scale, nullptr, QMM_F32};
-  if (use_tmem(wbits, M, N2, K, block_size, x_dtype, out_dtype, false) && aligned(x, 16) && aligned(w, 16) && workspace &&
+  if (use_tmem(wbits, M, N2, K, block_size, x_dtype, out_dtype, false, false) && aligned(x, 16) && aligned(w, 16) && workspace &&
       workspace_bytes >= tmem_gemm_workspace_bytes(M, K)) {
     log_choice("gate_up", "tmem", M, N2, K);
     return launch_tmem_gemm(wbits, x, x_dtype, w, sc, out, out_dtype, M, N2, K, block_size, 1, workspace, workspace_bytes, st);

@@ -261,12 +261,15 @@ Tensor quantized_gate_up(const Tensor& x, const Tensor& w, const Tensor& scale, 
     const int64_t K = x.size(-1), M = x.numel() / K;
     const int wbits = weight_is_packed ? 4 : 8;
     const bool half = x.scalar_type() != at::kFloat;
-    const bool decode = M <= 32 && half && K % (512 / wbits) == 0 && (block_size == -1 || block_size % (512 / wbits) == 0) &&
-                        (tl_variant == QMM_VARIANT_AUTO || tl_variant == QMM_VARIANT_MMA);
-    const bool batch = !decode && M > 32 && K >= 128 && K % (128 / wbits) == 0 &&
-                       (block_size == -1 || block_size == 128 || block_size % 256 == 0) &&
-                       (tl_variant == QMM_VARIANT_AUTO || tl_variant == QMM_VARIANT_I8TC);
     const at::ScalarType dt = out_dtype.has_value() ? *out_dtype : promote(x, scale, {});
+    const bool tc = M > 32 || (tl_variant == QMM_VARIANT_AUTO && half && dtype_code(dt) >= 0 &&
+                               qmm_gate_up_on_tensor_cores(wbits, dtype_code(x.scalar_type()), dtype_code(dt), M, w.size(0), K,
+                                                           block_size == -1 ? 0 : block_size));
+    const bool decode = !tc && half && K % (512 / wbits) == 0 && (block_size == -1 || block_size % (512 / wbits) == 0) &&
+                        (tl_variant == QMM_VARIANT_AUTO || tl_variant == QMM_VARIANT_MMA);
+    const bool batch = tc && K >= 128 && K % (128 / wbits) == 0 &&
+                       (block_size == -1 || block_size == 128 || block_size % 256 == 0 || (M <= 32 && block_size == 64)) &&
+                       (tl_variant == QMM_VARIANT_AUTO || tl_variant == QMM_VARIANT_I8TC);
     if (dtype_code(dt) >= 0 && (decode || batch)) {
       c10::cuda::OptionalCUDAGuard guard(x.device());
       Call c = make_call(x, w, scale, {}, block_size, weight_is_packed);
@@ -283,6 +286,7 @@ Tensor quantized_gate_up(const Tensor& x, const Tensor& w, const Tensor& scale, 
         void* ws;
         size_t ws_bytes;
         scratch(dev, st, qmm_weight_only_workspace_size(M, K), &ws, &ws_bytes);
+        // (short of scratch, the Python form takes the decode kernel up to 32 tokens)
         rc = qmm_gate_up(wbits, x.data_ptr(), dtype_code(x.scalar_type()), w.data_ptr(), (const float*)c.scale.data_ptr(),
                          out.data_ptr(), dtype_code(dt), M, c.N, K, c.block, ws, ws_bytes, st);
       }

@@ -69,6 +69,8 @@ def quantized_gate_up(x, w, scaler, block_size=-1, int4_weight=False, weight_is_
   M, N2 = x2.shape[0], w.shape[0]
   s32 = _qm._f32(scaler)
   wbits = 4 if weight_is_packed else 8
+  # (up to 32 tokens the operator's C++ form takes the tensor-core kernels on large weights; this one is for the calls that it
+  # leaves: other layouts, a capture without scratch)
   fused = (1 <= M <= 32 and x2.dtype in (torch.bfloat16, torch.float16) and K % (512 // wbits) == 0 and
            (block_size == -1 or block_size % (512 // wbits) == 0) and _qm.current_variant() in ("auto", "mma"))
   if fused:
