@@ -236,8 +236,8 @@ static bool zp_decode_on_tc(int wbits, int64_t M, int64_t N, int64_t K, bool dec
 //   above 64       int4 and int8 blocks, when the items fill half of the SMs, or 64 of them on weights of 2^25 values: fewer
 //                  leave it to i8tc's narrower ones ([4096,4096] at 128 tokens 26 us against 19; [14336,4096] at 96 25
 //                  against 34, [5120,6912] at 256 33 against 51, [28672,8192] at 512 230 against 337).  int4 per channel from 384
-//                  tokens, where i8tc expands the weights once, on 2^25 values ([4096,4096] at 1024 53 us against 46, [28672,8192]
-//                  400 against 492).
+//                  tokens, where i8tc expands the weights once, on 2^25 values ([4096,4096] at 1024 50 us against 38; [5120,6912] at
+//                  512 39 against 54), from 512 on fewer than 12288 outputs ([14336,4096] at 1024 117 against 94).
 //   narrow int8    up to 2048 outputs and above the 1024 tokens of one launch of the other kernel, whose launches are then
 //                  a round or two of items each ([1536,14592] at 4178 tokens 189 us against 313).
 static bool use_tmem(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, int x_dt, int out_dt, bool has_zp, bool decode_i8) {
@@ -266,7 +266,7 @@ static bool use_tmem(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, int
   const bool filled = 2 * items >= sm_count();
   if (out_dt == QMM_F32 && filled && (wbits == 8 || blocked || M < 384)) return true;
   if (wbits == 8 && !blocked) return M > 1024 && N <= 2048;
-  if (!blocked && M >= 384 && E < 1 << 25) return false;
+  if (!blocked && M >= 384 && (E < 1 << 25 || (M >= 512 && N >= 12288))) return false;
   return filled || (items >= 64 && E >= 1 << 25);
 }
 
@@ -645,6 +645,8 @@ static int w8a8_gemm(const int8_t* xq, const int8_t* w, const Scales& sc, const 
                                  out, out_dtype, M, N, K, st);
     case QMM_VARIANT_TCGEN05:
       log_choice("w8a8_gemm", "tcgen05", M, N, K);
+      if (!acc_out && w8a8_tc_supported(M, N, K, xq, w) && pair_gemm_preferred_w8a8(M, N, K, out_dtype))
+        return launch_pair_gemm(1, w, xq, sc, x_scale, xq_rowsum, 1.f, out, out_dtype, M, N, K, N, 0, nullptr, nullptr, st);
       return launch_w8a8_tc(xq, w, sc, x_scale, xq_rowsum, acc_out, out, out_dtype, M, N, K, st);
     default:
       return fail(QMM_ERR_UNSUPPORTED, "w8a8_gemm: variant %d is not available", variant);

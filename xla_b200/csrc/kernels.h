@@ -90,6 +90,18 @@ bool limb_tc_preferred(int wbits, int64_t M, int64_t N, int64_t K, int64_t block
 int launch_limb_tc(int wbits, const void* x, int x_dt, const void* w, const Scales& sc, void* out, int out_dt, int64_t M, int64_t N,
                    int64_t K, int64_t block_size, int gate_up, void* workspace, size_t workspace_bytes, cudaStream_t st);
 
+// ---- pair_gemm.cu (tcgen05 kind::i8 on pairs of CTAs) -------------------------------------------------
+// [N,K] int8 weights with scales per output times nl rows per token of b [nl * M, K]: nl = 1 W8A8 (tok: x_scale, sums: int32 row
+// sums), 2 or 3 limbs (tok: the powers of two, sums: fp32, zp_mul: the factor in the weight bytes).  ld: row pitch of `out`;
+// w_dep: the weights come from the kernel before.  partial (nl > 1; may be null): 160 partial tiles of 128 rows x
+// pair_gemm_tokens(nl) floats, flags: as many words that are zero between launches.  K a multiple of 16, w and b 16-byte aligned.
+int pair_gemm_tokens(int nl);  // per tile
+bool pair_gemm_preferred(int nl, int64_t M, int64_t N, int64_t K);
+bool pair_gemm_preferred_w8a8(int64_t M, int64_t N, int64_t K, int out_dt);
+int launch_pair_gemm(int nl, const int8_t* w, const int8_t* b, const Scales& scales, const float* tok, const void* sums, float zp_mul,
+                     void* out, int out_dt, int64_t M, int64_t N, int64_t K, int64_t ld, int w_dep, float* partial, uint32_t* flags,
+                     cudaStream_t st);
+
 // ---- tmem_gemm.cu (tcgen05 kind::f16, weights converted into tensor memory) -------------------------------------------
 // Weight-only linear for batches of bf16/f16 activations, zero points allowed; scratch as limb_gemm.cu's (its first 2 KB
 // are flag words that are zero between launches).

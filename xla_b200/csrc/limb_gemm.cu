@@ -1526,6 +1526,10 @@ int launch_limb_impl(int wbits, const void* x, int x_dt, const void* w, const Sc
   p.gate_up = gate_up;
   p.ytiles = pl.items ? (int)ceil_div(M, pl.tile_tokens) : 1;
   p.m0 = 0;
+  // int8 weights (or int4 expanded to them) with a scale per output: the same sums on pairs of CTAs, where the batch fills them
+  if (slice_rows == 0 && wbits == 8 && block_size <= 0 && !gate_up && pl.ncols == 128 && pair_gemm_preferred(nl, M, N, K))
+    return launch_pair_gemm(nl, static_cast<const int8_t*>(w), sc.limbs, scales, sc.pw, sc.xs, p.zp_mul, out, out_dt, M, N, K, N, w_dep,
+                            sc.partial, sc.flags, st);
   if (slice_rows == 0) {
     p.scale = scales.scale;
     p.zp = scales.zp;
