@@ -205,13 +205,14 @@ static bool use_decode_i8(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs
 // Batches of two tokens and more of which a tensor-core kernel (tmem or i8tc: both take about as long for one token as for
 // 32) beats the decode kernels, whose time grows with the tokens.  `decode`: the integer decode kernel takes the call.
 //   zero points  The other decode kernel is the GEMV, four tokens at a time: int4 block 128 [8192,28672] 70 us at two tokens and
-//                188 at eight, 49 on tmem; [28672,8192] 31 at two, 43 at five on the integer kernel, 49 on tmem, 185 on the GEMV
+//                188 at eight, 49 on tmem; int8 per channel [4096,4096] 8 at two, 13 at four, 18 at five, 14 on i8tc, [5120,6912]
+//                14 at two and 22 at three, 17 there; [28672,8192] 31 at two, 43 at five on the integer kernel, 49 on tmem, 185 on the GEMV
 //                from six on.  int8: [14336,4096] 15 us at two and 18 at four, 16 on i8tc.
 static bool zp_decode_on_tc(int wbits, int64_t M, int64_t N, int64_t K, bool decode) {
   const int64_t E = N * K;
   if (M < 2) return false;
   if (M > 8) return true;
-  if (!decode) return E >= 1 << 24;
+  if (!decode) return E >= (M == 2 ? 50000000 : M <= 4 ? 1 << 25 : 1 << 24);
   return E >= 1 << 25 && (wbits == 8 ? M * E >= 175000000 : M >= 6);
 }
 

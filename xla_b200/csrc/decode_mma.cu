@@ -14,8 +14,7 @@
 // k slots in whatever order the conversion produces; the lane loads the matching activations of
 // token g (B operand, column g) from global memory through L1 (x is a few KB and shared by all CTAs).
 // After each scale block the 16x8 partial tile is folded into fp32 accumulators with scale[b,n].
-// The int4 conversion leaves a constant bias in the weights (see Bias below); it is taken out again at
-// every fold with bias * sum_k x, which an extra MMA against an all-ones operand supplies.
+// The converted weights are exact, in units of a power of two that comes back in with the sums (convert.cuh).
 //
 // Semantics: torch_xla/experimental/xla_quantized_matmul.py:152-159 (per channel), :165-170 (blockwise).
 #include <algorithm>
@@ -23,12 +22,12 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "convert.cuh"
 #include "kernels.h"
 
 namespace qmm {
 
 namespace {
-
 
 template <typename XT>
 __device__ __forceinline__ void mma_16816(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
@@ -54,68 +53,6 @@ __device__ __forceinline__ void mma_16816_nv(float* c, const uint32_t* a, uint32
     asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-  }
-}
-
-// Bias carried by the converted weights.  The conversion drops an offset-binary nibble (v + 8) or byte
-// (v + 128) under the exponent of a power of two and does NOT subtract it again; the kernel removes
-// bias * sum_k x[m,k] instead, which the tensor core computes for free from the same activation
-// registers (an MMA against an all-ones A operand).  Saves one packed subtract per two weights.
-template <typename XT, int WBITS>
-struct Bias;
-template <>
-struct Bias<__nv_bfloat16, 4> { static constexpr float value = 136.f; static constexpr uint32_t ones = 0x3F803F80u; };
-template <>
-struct Bias<__half, 4> { static constexpr float value = 1032.f; static constexpr uint32_t ones = 0x3C003C00u; };
-template <>
-struct Bias<__nv_bfloat16, 8> { static constexpr float value = 0.f; static constexpr uint32_t ones = 0x3F803F80u; };
-template <>
-struct Bias<__half, 8> { static constexpr float value = 1152.f; static constexpr uint32_t ones = 0x3C003C00u; };
-
-// 8 nibbles (nibble i = k offset i, two's complement) -> packed pairs (k0,k1)(k2,k3)(k4,k5)(k6,k7) of
-// (v + 8) + 128 in bf16 or (v + 8) + 1024 in fp16: 9 integer instructions per 8 weights.
-template <typename XT>
-__device__ __forceinline__ void cvt_s4x8_biased(uint32_t w, uint32_t* p) {
-  constexpr bool kBf16 = !std::is_same<XT, __half>::value;
-  const uint32_t lo = (w & 0x0F0F0F0Fu) ^ 0x08080808u;         // k0 k2 k4 k6, offset binary
-  const uint32_t hi = ((w >> 4) & 0x0F0F0F0Fu) ^ 0x08080808u;  // k1 k3 k5 k7
-  const uint32_t q0 = __byte_perm(lo, hi, 0x5140);             // k0 k1 k2 k3
-  const uint32_t q1 = __byte_perm(lo, hi, 0x7362);             // k4 k5 k6 k7
-  const uint32_t expo = kBf16 ? 0x43434343u : 0x64646464u;     // exponent byte of 128.0 (bf16) / 1024.0 (f16)
-  p[0] = __byte_perm(q0, expo, 0x4140);
-  p[1] = __byte_perm(q0, expo, 0x4342);
-  p[2] = __byte_perm(q1, expo, 0x4140);
-  p[3] = __byte_perm(q1, expo, 0x4342);
-}
-
-// 4 int8 -> packed pairs (k0,k1)(k2,k3).  fp16: (v + 128) + 1024, bias left in (3 instructions);
-// bf16 cannot hold a byte under an exponent, so it goes through fp32 and is exact (bias 0).
-template <typename XT>
-__device__ __forceinline__ void cvt_s8x4_biased(uint32_t w, uint32_t* p) {
-  const uint32_t u = w ^ 0x80808080u;
-  if constexpr (std::is_same<XT, __half>::value) {
-    p[0] = __byte_perm(u, 0x64646464u, 0x4140);
-    p[1] = __byte_perm(u, 0x64646464u, 0x4342);
-  } else {
-    const float f0 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7540)) - 8388736.f;
-    const float f1 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7541)) - 8388736.f;
-    const float f2 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7542)) - 8388736.f;
-    const float f3 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7543)) - 8388736.f;
-    __nv_bfloat162 a = __floats2bfloat162_rn(f0, f1), b = __floats2bfloat162_rn(f2, f3);
-    p[0] = *reinterpret_cast<uint32_t*>(&a);
-    p[1] = *reinterpret_cast<uint32_t*>(&b);
-  }
-}
-
-// packed pair minus (bias, bias): exact, the operands are small integers
-template <typename XT>
-__device__ __forceinline__ uint32_t sub_bias(uint32_t p, float bias) {
-  if constexpr (std::is_same<XT, __half>::value) {
-    const __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&p), __float2half2_rn(bias));
-    return *reinterpret_cast<const uint32_t*>(&r);
-  } else {
-    const __nv_bfloat162 r = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&p), __float2bfloat162_rn(bias));
-    return *reinterpret_cast<const uint32_t*>(&r);
   }
 }
 
@@ -162,8 +99,8 @@ __device__ __forceinline__ float ar_ld_peer(const float* p) {
 
 // NT = number of 8-token tiles (M <= 8*NT); RG = 16-row groups per CTA (each warp converts RG groups per
 // step and reuses its activation registers for all of them); WARPS = warps splitting K.
-// One "fold" = the end of a scale block (blockwise) or of a single step (per-channel): the partial tile,
-// minus bias * sum(x), is added into the totals.
+// One "fold" = the end of a scale block (blockwise) or of a single step (per-channel): the partial tile is added
+// into the totals.
 template <int WBITS, typename XT, typename ST, int NT, int RG, int WARPS, bool AR = false>
 __global__ void __launch_bounds__(WARPS * 32)
     decode_mma_kernel(const XT* x, const uint8_t* __restrict__ w, const ST* scale,
@@ -174,13 +111,6 @@ __global__ void __launch_bounds__(WARPS * 32)
   constexpr int VPL = VPS / 4;          // values per lane per row per step: 32 or 16
   constexpr int XREGS = VPL / 2;        // packed activation pairs per lane per token tile: 16 or 8
   constexpr int ROWS = 16 * RG;         // output rows per CTA
-  // With one token tile the bias stays in and a ones-MMA removes it (the integer pipe is the limiter
-  // there); with more tiles the tensor pipe matters more, so the bias is subtracted in the conversion
-  // (a packed subtract on the otherwise idle FMA pipe) and the extra MMAs disappear.
-  constexpr float kBias = Bias<XT, WBITS>::value;
-  constexpr bool kHasBias = kBias != 0.f && NT == 1;
-  constexpr bool kSubBias = kBias != 0.f && NT != 1;
-  constexpr uint32_t kOnes = Bias<XT, WBITS>::ones;
   __shared__ float s_part[WARPS][ROWS][NT * 8];
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -208,16 +138,14 @@ __global__ void __launch_bounds__(WARPS * 32)
     xrow[i] = x + (int64_t)(tok < M ? tok : 0) * K + t * VPL;
   }
 
-  float total[RG][NT][4], part[RG][NT][4], xsum[NT][4];
+  float total[RG][NT][4], part[RG][NT][4];
 #pragma unroll
   for (int i = 0; i < NT; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      xsum[i][j] = 0.f;
 #pragma unroll
       for (int r = 0; r < RG; ++r) total[r][i][j] = part[r][i][j] = 0.f;
     }
-  const uint32_t ones[4] = {kOnes, kOnes, kOnes, kOnes};
 
   // Software pipeline, one step deep: the weights of this warp's next step are in flight while the
   // current step is converted and multiplied.  (Prefetching the activations as well costs 24 registers
@@ -290,15 +218,8 @@ __global__ void __launch_bounds__(WARPS * 32)
 #pragma unroll
         for (int r = 0; r < RG; ++r) {
           uint32_t pa[4], pb[4];
-          cvt_s4x8_biased<XT>(reinterpret_cast<const uint32_t*>(&wc[2 * r])[wi], pa);
-          cvt_s4x8_biased<XT>(reinterpret_cast<const uint32_t*>(&wc[2 * r + 1])[wi], pb);
-          if constexpr (kSubBias) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              pa[q] = sub_bias<XT>(pa[q], kBias);
-              pb[q] = sub_bias<XT>(pb[q], kBias);
-            }
-          }
+          cvt_s4x8<XT>(reinterpret_cast<const uint32_t*>(&wc[2 * r])[wi], pa);
+          cvt_s4x8<XT>(reinterpret_cast<const uint32_t*>(&wc[2 * r + 1])[wi], pb);
           const uint32_t a_lo[4] = {pa[0], pb[0], pa[1], pb[1]};
           const uint32_t a_hi[4] = {pa[2], pb[2], pa[3], pb[3]};
 #pragma unroll
@@ -307,33 +228,15 @@ __global__ void __launch_bounds__(WARPS * 32)
             mma_16816_nv<XT>(part[r][i], a_hi, xr[i][4 * wi + 2], xr[i][4 * wi + 3]);
           }
         }
-        if constexpr (kHasBias) {
-#pragma unroll
-          for (int i = 0; i < NT; ++i) {
-            mma_16816_nv<XT>(xsum[i], ones, xr[i][4 * wi], xr[i][4 * wi + 1]);
-            mma_16816_nv<XT>(xsum[i], ones, xr[i][4 * wi + 2], xr[i][4 * wi + 3]);
-          }
-        }
       } else {
 #pragma unroll
         for (int r = 0; r < RG; ++r) {
           uint32_t pa[2], pb[2];
-          cvt_s8x4_biased<XT>(reinterpret_cast<const uint32_t*>(&wc[2 * r])[wi], pa);
-          cvt_s8x4_biased<XT>(reinterpret_cast<const uint32_t*>(&wc[2 * r + 1])[wi], pb);
-          if constexpr (kSubBias) {
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-              pa[q] = sub_bias<XT>(pa[q], kBias);
-              pb[q] = sub_bias<XT>(pb[q], kBias);
-            }
-          }
+          cvt_s8x4<XT>(reinterpret_cast<const uint32_t*>(&wc[2 * r])[wi], pa);
+          cvt_s8x4<XT>(reinterpret_cast<const uint32_t*>(&wc[2 * r + 1])[wi], pb);
           const uint32_t a[4] = {pa[0], pb[0], pa[1], pb[1]};
 #pragma unroll
           for (int i = 0; i < NT; ++i) mma_16816_nv<XT>(part[r][i], a, xr[i][2 * wi], xr[i][2 * wi + 1]);
-        }
-        if constexpr (kHasBias) {
-#pragma unroll
-          for (int i = 0; i < NT; ++i) mma_16816_nv<XT>(xsum[i], ones, xr[i][2 * wi], xr[i][2 * wi + 1]);
         }
       }
     }
@@ -342,20 +245,13 @@ __global__ void __launch_bounds__(WARPS * 32)
       for (int i = 0; i < NT; ++i) {
 #pragma unroll
         for (int r = 0; r < RG; ++r) {
-          // xsum rows are all equal: c0,c1 (tokens 2t, 2t+1) serve both row g and row g+8
-          const float p0 = kHasBias ? fmaf(-kBias, xsum[i][0], part[r][i][0]) : part[r][i][0];
-          const float p1 = kHasBias ? fmaf(-kBias, xsum[i][1], part[r][i][1]) : part[r][i][1];
-          const float p2 = kHasBias ? fmaf(-kBias, xsum[i][0], part[r][i][2]) : part[r][i][2];
-          const float p3 = kHasBias ? fmaf(-kBias, xsum[i][1], part[r][i][3]) : part[r][i][3];
-          total[r][i][0] = fmaf(sc[2 * r], p0, total[r][i][0]);
-          total[r][i][1] = fmaf(sc[2 * r], p1, total[r][i][1]);
-          total[r][i][2] = fmaf(sc[2 * r + 1], p2, total[r][i][2]);
-          total[r][i][3] = fmaf(sc[2 * r + 1], p3, total[r][i][3]);
+          total[r][i][0] = fmaf(sc[2 * r], part[r][i][0], total[r][i][0]);
+          total[r][i][1] = fmaf(sc[2 * r], part[r][i][1], total[r][i][1]);
+          total[r][i][2] = fmaf(sc[2 * r + 1], part[r][i][2], total[r][i][2]);
+          total[r][i][3] = fmaf(sc[2 * r + 1], part[r][i][3], total[r][i][3]);
 #pragma unroll
           for (int j = 0; j < 4; ++j) part[r][i][j] = 0.f;
         }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) xsum[i][j] = 0.f;
       }
     }
   }
@@ -365,10 +261,10 @@ __global__ void __launch_bounds__(WARPS * 32)
   for (int r = 0; r < RG; ++r)
 #pragma unroll
     for (int i = 0; i < NT; ++i) {
-      s_part[warp][16 * r + g][8 * i + 2 * t] = total[r][i][0];
-      s_part[warp][16 * r + g][8 * i + 2 * t + 1] = total[r][i][1];
-      s_part[warp][16 * r + g + 8][8 * i + 2 * t] = total[r][i][2];
-      s_part[warp][16 * r + g + 8][8 * i + 2 * t + 1] = total[r][i][3];
+      s_part[warp][16 * r + g][8 * i + 2 * t] = total[r][i][0] * Unit<XT>::kBack;
+      s_part[warp][16 * r + g][8 * i + 2 * t + 1] = total[r][i][1] * Unit<XT>::kBack;
+      s_part[warp][16 * r + g + 8][8 * i + 2 * t] = total[r][i][2] * Unit<XT>::kBack;
+      s_part[warp][16 * r + g + 8][8 * i + 2 * t + 1] = total[r][i][3] * Unit<XT>::kBack;
     }
   __syncthreads();
   if constexpr (AR) {
@@ -521,7 +417,6 @@ __global__ void __launch_bounds__(kStagedWarps * 32, 1)
   constexpr int PITCH = CHUNK_UNITS * 16 + 16;
   constexpr int STAGE_BYTES = ROWS_X * PITCH;
   constexpr int THREADS = kStagedWarps * 32;
-  constexpr float kBias = Bias<XT, WBITS>::value;
   constexpr int kRedPitch = 17;
   constexpr bool kLateFetch = NT == 4;
   static_assert(kStagedWarps * kRedPitch * ROWS_X * 4 <= 2 * STAGE_BYTES, "the reduction buffer reuses the ring");
@@ -692,13 +587,8 @@ __global__ void __launch_bounds__(kStagedWarps * 32, 1)
 #pragma unroll
         for (int wi = 0; wi < 4; ++wi) {
           uint32_t pa[4], pb[4];
-          cvt_s4x8_biased<XT>(reinterpret_cast<const uint32_t*>(&w0)[wi], pa);
-          cvt_s4x8_biased<XT>(reinterpret_cast<const uint32_t*>(&w1)[wi], pb);
-#pragma unroll
-          for (int qd = 0; qd < 4; ++qd) {
-            pa[qd] = sub_bias<XT>(pa[qd], kBias);
-            pb[qd] = sub_bias<XT>(pb[qd], kBias);
-          }
+          cvt_s4x8<XT>(reinterpret_cast<const uint32_t*>(&w0)[wi], pa);
+          cvt_s4x8<XT>(reinterpret_cast<const uint32_t*>(&w1)[wi], pb);
           const uint32_t a_lo[4] = {pa[0], pb[0], pa[1], pb[1]};
           const uint32_t a_hi[4] = {pa[2], pb[2], pa[3], pb[3]};
           const unsigned char* xp = (wi < 2 ? xa : xb) + (wi & 1) * 16;
@@ -723,15 +613,8 @@ __global__ void __launch_bounds__(kStagedWarps * 32, 1)
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             uint32_t pa[2], pb[2];
-            cvt_s8x4_biased<XT>(reinterpret_cast<const uint32_t*>(&w0)[2 * wp + h], pa);
-            cvt_s8x4_biased<XT>(reinterpret_cast<const uint32_t*>(&w1)[2 * wp + h], pb);
-            if constexpr (kBias != 0.f) {
-#pragma unroll
-              for (int qd = 0; qd < 2; ++qd) {
-                pa[qd] = sub_bias<XT>(pa[qd], kBias);
-                pb[qd] = sub_bias<XT>(pb[qd], kBias);
-              }
-            }
+            cvt_s8x4<XT>(reinterpret_cast<const uint32_t*>(&w0)[2 * wp + h], pa);
+            cvt_s8x4<XT>(reinterpret_cast<const uint32_t*>(&w1)[2 * wp + h], pb);
             a[h][0] = pa[0];
             a[h][1] = pb[0];
             a[h][2] = pa[1];
@@ -803,10 +686,10 @@ __global__ void __launch_bounds__(kStagedWarps * 32, 1)
       for (int i = 0; i < NT; ++i) {
         // token-major with a pitch of 17 floats: rows g, g+8 of tokens 2t, 2t+1 land on distinct banks
         float* r0 = red + (warp * ROWS_X + 8 * i + 2 * t) * kRedPitch + g;
-        r0[0] = total[i][0];
-        r0[kRedPitch] = total[i][1];
-        r0[8] = total[i][2];
-        r0[kRedPitch + 8] = total[i][3];
+        r0[0] = total[i][0] * Unit<XT>::kBack;
+        r0[kRedPitch] = total[i][1] * Unit<XT>::kBack;
+        r0[8] = total[i][2] * Unit<XT>::kBack;
+        r0[kRedPitch + 8] = total[i][3] * Unit<XT>::kBack;
       }
     }
     __syncthreads();
