@@ -14,7 +14,10 @@
 // k slots in whatever order the conversion produces; the lane loads the matching activations of
 // token g (B operand, column g) from global memory through L1 (x is a few KB and shared by all CTAs).
 // After each scale block the 16x8 partial tile is folded into fp32 accumulators with scale[b,n].
-// The converted weights are exact, in units of a power of two that comes back in with the sums (convert.cuh).
+// The converted weights are exact, in units of a power of two that comes back in with the sums (convert.cuh): six integer
+// instructions for eight int4 weights, three for four int8 ones, where a form with a bias has nine and six or seven.  Eight tokens
+// of int4 block 128 with sixteen warps per tile: [4096,4096] 7.5 -> 5.4 us, [4096,14336] 17.7 -> 12.1; of int8 [4096,4096] at
+// sixteen 9.5 -> 8.8.  Where the bias stays: Bias below.
 //
 // Semantics: torch_xla/experimental/xla_quantized_matmul.py:152-159 (per channel), :165-170 (blockwise).
 #include <algorithm>
@@ -54,6 +57,28 @@ __device__ __forceinline__ void mma_16816_nv(float* c, const uint32_t* a, uint32
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
   }
+}
+
+// The other conversion of int4, which leaves a bias in: an offset-binary nibble under the exponent of a power of two, 136 (bf16)
+// or 1032 (f16) more than the value: nine integer instructions for eight weights, but no multiply-adds.  The kernel takes bias *
+// sum_k x[m,k] off at every fold; an MMA against ones gives those sums.  It is the faster form for five to eight tokens with four
+// warps per tile ([14336,4096] block 128 through the operator at eight tokens 13.4 us, 14.0 with the exact one; in a graph at one
+// token 14.4 and 13.4, at four 14.6 and 13.6, and on [28672,4096] 22.8 and 19.3, 23.1 and 21.1): see launch_nt.
+template <typename XT>
+struct Bias {
+  static constexpr bool kHalf = std::is_same<XT, __half>::value;
+  static constexpr float value = kHalf ? 1032.f : 136.f;
+  static constexpr uint32_t ones = kHalf ? 0x3C003C00u : 0x3F803F80u;
+};
+template <typename XT>
+__device__ __forceinline__ void cvt_s4x8_biased(uint32_t w, uint32_t* p) {
+  const uint32_t lo = (w & 0x0F0F0F0Fu) ^ 0x08080808u, hi = ((w >> 4) & 0x0F0F0F0Fu) ^ 0x08080808u;
+  const uint32_t q0 = __byte_perm(lo, hi, 0x5140), q1 = __byte_perm(lo, hi, 0x7362);  // k0 k1 k2 k3, k4 k5 k6 k7
+  constexpr uint32_t expo = Bias<XT>::kHalf ? 0x64646464u : 0x43434343u;
+  p[0] = __byte_perm(q0, expo, 0x4140);
+  p[1] = __byte_perm(q0, expo, 0x4342);
+  p[2] = __byte_perm(q1, expo, 0x4140);
+  p[3] = __byte_perm(q1, expo, 0x4342);
 }
 
 // Fused MLP epilogue: the weight rows are stored in groups of 16, eight rows of the gate projection followed
@@ -101,7 +126,8 @@ __device__ __forceinline__ float ar_ld_peer(const float* p) {
 // step and reuses its activation registers for all of them); WARPS = warps splitting K.
 // One "fold" = the end of a scale block (blockwise) or of a single step (per-channel): the partial tile is added
 // into the totals.
-template <int WBITS, typename XT, typename ST, int NT, int RG, int WARPS, bool AR = false>
+// BIASED: int4 through the conversion above.
+template <int WBITS, typename XT, typename ST, int NT, int RG, int WARPS, bool AR = false, bool BIASED = false>
 __global__ void __launch_bounds__(WARPS * 32)
     decode_mma_kernel(const XT* x, const uint8_t* __restrict__ w, const ST* scale,
                       void* __restrict__ out, int out_dt, int M, int64_t N, int64_t K, int steps_per_block,
@@ -111,6 +137,8 @@ __global__ void __launch_bounds__(WARPS * 32)
   constexpr int VPL = VPS / 4;          // values per lane per row per step: 32 or 16
   constexpr int XREGS = VPL / 2;        // packed activation pairs per lane per token tile: 16 or 8
   constexpr int ROWS = 16 * RG;         // output rows per CTA
+  static_assert(!BIASED || (WBITS == 4 && NT == 1), "one token tile of int4");
+  constexpr float kBack = BIASED ? 1.f : Unit<XT>::kBack;
   __shared__ float s_part[WARPS][ROWS][NT * 8];
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -138,7 +166,8 @@ __global__ void __launch_bounds__(WARPS * 32)
     xrow[i] = x + (int64_t)(tok < M ? tok : 0) * K + t * VPL;
   }
 
-  float total[RG][NT][4], part[RG][NT][4];
+  float total[RG][NT][4], part[RG][NT][4], xsum[4] = {0.f, 0.f, 0.f, 0.f};
+  const uint32_t ones[4] = {Bias<XT>::ones, Bias<XT>::ones, Bias<XT>::ones, Bias<XT>::ones};
 #pragma unroll
   for (int i = 0; i < NT; ++i)
 #pragma unroll
@@ -218,8 +247,13 @@ __global__ void __launch_bounds__(WARPS * 32)
 #pragma unroll
         for (int r = 0; r < RG; ++r) {
           uint32_t pa[4], pb[4];
-          cvt_s4x8<XT>(reinterpret_cast<const uint32_t*>(&wc[2 * r])[wi], pa);
-          cvt_s4x8<XT>(reinterpret_cast<const uint32_t*>(&wc[2 * r + 1])[wi], pb);
+          if constexpr (BIASED) {
+            cvt_s4x8_biased<XT>(reinterpret_cast<const uint32_t*>(&wc[2 * r])[wi], pa);
+            cvt_s4x8_biased<XT>(reinterpret_cast<const uint32_t*>(&wc[2 * r + 1])[wi], pb);
+          } else {
+            cvt_s4x8<XT>(reinterpret_cast<const uint32_t*>(&wc[2 * r])[wi], pa);
+            cvt_s4x8<XT>(reinterpret_cast<const uint32_t*>(&wc[2 * r + 1])[wi], pb);
+          }
           const uint32_t a_lo[4] = {pa[0], pb[0], pa[1], pb[1]};
           const uint32_t a_hi[4] = {pa[2], pb[2], pa[3], pb[3]};
 #pragma unroll
@@ -227,6 +261,10 @@ __global__ void __launch_bounds__(WARPS * 32)
             mma_16816_nv<XT>(part[r][i], a_lo, xr[i][4 * wi], xr[i][4 * wi + 1]);
             mma_16816_nv<XT>(part[r][i], a_hi, xr[i][4 * wi + 2], xr[i][4 * wi + 3]);
           }
+        }
+        if constexpr (BIASED) {
+          mma_16816_nv<XT>(xsum, ones, xr[0][4 * wi], xr[0][4 * wi + 1]);
+          mma_16816_nv<XT>(xsum, ones, xr[0][4 * wi + 2], xr[0][4 * wi + 3]);
         }
       } else {
 #pragma unroll
@@ -245,6 +283,11 @@ __global__ void __launch_bounds__(WARPS * 32)
       for (int i = 0; i < NT; ++i) {
 #pragma unroll
         for (int r = 0; r < RG; ++r) {
+          if constexpr (BIASED) {
+            // the sums' rows are all equal: tokens 2t and 2t + 1 for row g and row g + 8
+#pragma unroll
+            for (int j = 0; j < 4; ++j) part[r][i][j] = fmaf(-Bias<XT>::value, xsum[j & 1], part[r][i][j]);
+          }
           total[r][i][0] = fmaf(sc[2 * r], part[r][i][0], total[r][i][0]);
           total[r][i][1] = fmaf(sc[2 * r], part[r][i][1], total[r][i][1]);
           total[r][i][2] = fmaf(sc[2 * r + 1], part[r][i][2], total[r][i][2]);
@@ -253,6 +296,8 @@ __global__ void __launch_bounds__(WARPS * 32)
           for (int j = 0; j < 4; ++j) part[r][i][j] = 0.f;
         }
       }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) xsum[j] = 0.f;
     }
   }
 
@@ -261,10 +306,10 @@ __global__ void __launch_bounds__(WARPS * 32)
   for (int r = 0; r < RG; ++r)
 #pragma unroll
     for (int i = 0; i < NT; ++i) {
-      s_part[warp][16 * r + g][8 * i + 2 * t] = total[r][i][0] * Unit<XT>::kBack;
-      s_part[warp][16 * r + g][8 * i + 2 * t + 1] = total[r][i][1] * Unit<XT>::kBack;
-      s_part[warp][16 * r + g + 8][8 * i + 2 * t] = total[r][i][2] * Unit<XT>::kBack;
-      s_part[warp][16 * r + g + 8][8 * i + 2 * t + 1] = total[r][i][3] * Unit<XT>::kBack;
+      s_part[warp][16 * r + g][8 * i + 2 * t] = total[r][i][0] * kBack;
+      s_part[warp][16 * r + g][8 * i + 2 * t + 1] = total[r][i][1] * kBack;
+      s_part[warp][16 * r + g + 8][8 * i + 2 * t] = total[r][i][2] * kBack;
+      s_part[warp][16 * r + g + 8][8 * i + 2 * t + 1] = total[r][i][3] * kBack;
     }
   __syncthreads();
   if constexpr (AR) {
@@ -810,6 +855,9 @@ int launch_nt(const void* x, const void* w, const ST* scale, void* out, int out_
       err = QMM_DECODE_LAUNCH(1, 1, 16);
     else if (warps >= 8)
       err = QMM_DECODE_LAUNCH(1, 1, 8);
+    else if (WBITS == 4 && M > 4)  // the conversion with a bias: figures at Bias
+      err = launch_pdl(decode_mma_kernel<WBITS, XT, ST, 1, 1, 4, false, WBITS == 4>, (unsigned)tiles, 128, 0, st, xp, wp, scale, out, out_dt,
+                       (int)M, N, K, spb, shift, bw, gate_up, ArParams{}, (uint32_t*)nullptr);
     else
       err = QMM_DECODE_LAUNCH(1, 1, 4);
   }
