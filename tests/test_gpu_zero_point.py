@@ -30,3 +30,24 @@ def test_zero_points_above_eight_tokens(wbits, bs, N, K, M, dtype):
     out = torch.ops.xla_b200.quantized_matmul_packed(x.to(DEV), wd, s.to(DEV), zp.to(DEV), block_size=bs, int4_weight=wbits == 4,
                                                      weight_is_packed=wbits == 4, out_dtype=out_dtype)
     assert qo.max_abs_rel(out, exact) < tol, out_dtype
+
+
+@pytest.mark.parametrize("variant", ["auto", "tmem"])
+@pytest.mark.parametrize("M", [9, 32, 70])
+@pytest.mark.parametrize("wbits,K", [(8, k) for k in (64, 80, 96, 112, 128, 144, 160, 176, 192, 208, 224, 240, 256, 272)] +
+                         [(4, k) for k in (64, 96, 128, 160, 192, 224, 256, 288)])
+def test_zero_points_per_channel_on_few_inputs(wbits, K, M, variant):
+  """The sum over all of a row, from eight lanes' worth of values to more than a warp's.  AUTO on both sides of its lines (1030
+  outputs, and enough items for the tensor-memory kernel above 64 tokens)."""
+  for N in ((1030, 12290) if variant == "auto" else (130,)):
+    g = qc.gen(N + K + M)
+    x = (torch.rand(M, K, generator=g) + 0.5).bfloat16().to(DEV)  # a sum in which a value left out shows
+    w = (qc.int4_weight if wbits == 4 else qc.int8_weight)(g, N, K).to(DEV)
+    s = qc.per_channel_scale(g, N).to(DEV)
+    z = torch.randint(-20, 21, (N,), generator=g).to(DEV) * s
+    with xla_b200.force_variant(variant):
+      out = torch.ops.xla_b200.quantized_matmul_packed(x, xla_b200.pack_int4(w) if wbits == 4 else w, s, z, int4_weight=wbits == 4,
+                                                       weight_is_packed=wbits == 4, out_dtype=torch.float32)
+    exact = (x.double() @ w.double().T) * s.double() - x.double().sum(1, keepdim=True) * z.double()
+    # exact products (or 2^-22 of the row's largest activation); K additions in fp32 at most: K 2^-24 < 2e-5 of the largest result
+    assert qo.max_abs_rel(out, exact) < 2e-5

@@ -709,8 +709,9 @@ __global__ void __launch_bounds__(Cfg<WBITS, NC, KS, SUB>::kThreads, 1)
 }
 
 // Sums of the activations over each scale block, for the zero points: xs[b * pitch + m]; tokens from M up to the pitch get
-// zeros.  A warp takes 256 values of a row, or a whole larger block, at a time; a block shorter than that is summed by the
-// lanes that hold it. 
+// zeros.  A warp takes 256 values of a row, or a whole larger block, at a time.  Several shorter blocks of a row (of 64 or 128
+// values) are summed by the lanes that hold them, 8 or 16; one that is alone in its row (per channel, any multiple of eight values)
+// by all lanes, of which those beyond it hold zeros.
 constexpr int kSumsThreads = 512;
 template <typename XT>
 __global__ void __launch_bounds__(kSumsThreads) block_sums_kernel(const XT* x, float* __restrict__ xs, int pitch, int M, int K, int S) {
@@ -718,7 +719,7 @@ __global__ void __launch_bounds__(kSumsThreads) block_sums_kernel(const XT* x, f
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const int lane = threadIdx.x & 31, len = K / S;
   const int per = max(len, 256), pieces = (K + per - 1) / per;
-  const int group = min(32, len / 8);  // lanes that hold a block
+  const int group = S > 1 && len < 256 ? len / 8 : 32;  // lanes that sum a block, a power of two
   const int warps = gridDim.x * (kSumsThreads / 32);
   for (int64_t i = (int64_t)blockIdx.x * (kSumsThreads / 32) + (threadIdx.x >> 5); i < (int64_t)pitch * pieces; i += warps) {
     const int m = (int)(i / pieces), k0 = (int)(i - (int64_t)m * pieces) * per;
@@ -734,7 +735,7 @@ __global__ void __launch_bounds__(kSumsThreads) block_sums_kernel(const XT* x, f
       for (int o = group >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     }
     const int b = (k0 + lane * 8) / len;
-    if (lane % group == 0 && b < S && (group == 32 ? lane == 0 : true)) xs[(int64_t)b * pitch + m] = s;
+    if (lane % group == 0 && b < S) xs[(int64_t)b * pitch + m] = s;
   }
 }
 
