@@ -133,3 +133,24 @@ def test_gate_up_of_small_batches_on_large_weights(wbits, bs, M):
   y = torch.ops.xla_b200.quantized_matmul_packed(x, w, s, None, out_dtype=torch.float32, **kw).view(M, N2 // 16, 2, 8).double()
   ref = (torch.nn.functional.silu(y[:, :, 0]) * y[:, :, 1]).reshape(M, N2 // 2)
   assert qo.max_abs_rel(out, ref) < 1e-2  # one rounding to bf16
+
+
+@pytest.mark.parametrize("wbits,bs,N,K,M", [
+    (4, 384, 1030, 3840, 20), (8, 384, 1030, 3840, 64), (4, 384, 20000, 1536, 33), (8, 384, 514, 4224, 100), (4, 384, 514, 4224, 128),
+    (8, -1, 514, 384, 100), (8, -1, 514, 704, 128), (8, -1, 514, 1152, 65), (8, 640, 514, 3840, 50), (4, 256, 514, 4096, 100),
+])
+def test_folds_of_several_steps(wbits, bs, N, K, M):
+  """Three and five steps per fold, which one issuer has to itself, and two, which alternate: the same bits each time."""
+  g = qc.gen(N + K + M)
+  x = qc.activations(g, M, K, torch.bfloat16, outliers=True).to(DEV)
+  w = (qc.int4_weight if wbits == 4 else qc.int8_weight)(g, N, K).to(DEV)
+  s = (qc.per_channel_scale(g, N) if bs == -1 else qc.blockwise_scale(g, K // bs, N)).to(DEV)
+  wd = xla_b200.pack_int4(w) if wbits == 4 else w
+  with xla_b200.force_variant("tmem"):
+    run = lambda: torch.ops.xla_b200.quantized_matmul_packed(x, wd, s, block_size=bs, int4_weight=wbits == 4,  # noqa: E731
+                                                             weight_is_packed=wbits == 4, out_dtype=torch.float32)
+    out = run()
+    assert all(torch.equal(run(), out) for _ in range(5))
+  S = 1 if bs == -1 else K // bs
+  exact = torch.einsum("msk,nsk,sn->mn", x.double().view(M, S, -1), w.double().view(N, S, -1), s.double().view(S, N))
+  assert qo.max_abs_rel(out, exact) < 1e-5  # exact products, a rounding per block and per 512 values

@@ -39,6 +39,7 @@
 
 #include "common.cuh"
 #include "convert.cuh"
+#include "issue_order.h"
 #include "kernels.h"
 #include "ptx_sm100.cuh"
 
@@ -64,6 +65,7 @@ struct Params {
   int M;
   int64_t N;
   int fu;         // steps per fold (accumulation in the tensor core), >= 1
+  int alternate;  // the folds alternate between the two issuers (else the first one has them all)
   int blocked;    // scale blocks (0: per channel; folds are then plain additions)
   int S;
   int unit;       // steps per scheduling unit: whole folds and whole raw tiles
@@ -103,6 +105,9 @@ struct Cfg {
   static constexpr uint32_t kBStage = NC * KS * 2;
   static constexpr int kRaw = NC >= 64 ? 4 : 8;
   static constexpr int kB = std::min(kDone, (NC == 192 ? 144 : NC >= 64 ? 128 : 64) * 1024 / (int)kBStage);
+  // The accumulator is what an issuer waits for longest, so its barrier comes last where the turns of the other rings are the
+  // issuer's own steps, and first where they are not.
+  static constexpr bool kAccLast = kB % 2 == 0 && kASlots % 2 == 0;
   static constexpr int kTV = 1024 / WBITS;          // values of a row per raw tile
   static constexpr int kVV = KS / kTeamGroups;      // values per step and converting group
   static constexpr int kDT = NC / 2;                // tokens per drain thread
@@ -117,6 +122,7 @@ struct Cfg {
   // A parity wait is right only while the barrier is at most one phase away: whoever waits for step i - d does so for every
   // step in turn (the converters: for every step of their team), and step i - d + kDone cannot complete before it has gone on.
   static_assert(kB <= kDone && kASlots <= kB && kAcc <= kDone, "turns of the rings");
+  static_assert(issuers_may_alternate(1, kASlots, kB, kAccLast), "folds of one step alternate");
   static_assert(kASlots % kTeams == 0 && kDone % kTeams == 0 && kVV <= kTV, "slots of a team");
   static_assert(kRaw % std::max(1, kTeams * KS / kTV) == 0, "a group comes back to the raw slots it has waited for");
   static_assert(kBatch % SUB == 0 && kBatch * kDT / 4 <= kDrain / 2, "batches of scales and block sums");
@@ -293,19 +299,14 @@ __global__ void __launch_bounds__(Cfg<WBITS, NC, KS, SUB>::kThreads, 1)
       const uint32_t b_lo0 = (uint32_t)ptx::make_sw128_kmajor_desc(ptx::smem_u32(b_base));
       const uint32_t b_full_a = ptx::smem_u32(b_full), a_full_a = ptx::smem_u32(a_full), acc_empty_a = ptx::smem_u32(acc_empty),
                      acc_full_a = ptx::smem_u32(acc_full), done_a = ptx::smem_u32(done);
-      // Alternating only while the rings are long enough: a wait for step i may not find its barrier a whole turn behind.
-      // The accumulator that the fold needs was drained, and with it (the drain goes in order) all folds up to kAcc before;
-      // step i - kASlots has to be among those.
-      const bool alternate = (kAcc - 1) * p.fu < kASlots;
+      const bool alternate = p.alternate != 0;
       const uint32_t me = (uint32_t)warp >> 1;
       const uint32_t total = (uint32_t)it.steps(), fu = (uint32_t)p.fu;
       const uint32_t jump = alternate ? fu : 0u;  // steps of the other issuer between two folds
       uint32_t j = me * fu, buf = me, pacc = 1, sb = j % kB, pb = 0;
       const uint32_t buf_inc = alternate ? 2 : 1;
       if (!alternate && me) j = total;
-      // The accumulator is what is waited for longest, so its barrier comes last where the turns of the other rings are this
-      // issuer's own steps (and first where they are not, see above).
-      constexpr bool kAccLast = kB % 2 == 0 && kASlots % 2 == 0;
+      constexpr bool kAccLast = C::kAccLast;
       while (j < total) {
         if (!kAccLast) ptx::bar_wait(acc_empty_a + buf * 8, pacc, abort_flag, p.err_word, ptx::kErrWaitTmemEmpty);
         const uint32_t d = tb + buf * C::kAccCols;
@@ -755,8 +756,9 @@ cudaError_t launch_pdl(Kernel kern, unsigned grid, unsigned block, size_t smem, 
 }
 
 template <int WBITS, typename XT, int NC, int KS, int SUB, bool W16>
-int launch_with(const CUtensorMap& map_w, const CUtensorMap& map_x, const Params& p, int grid, cudaStream_t st) {
+int launch_with(const CUtensorMap& map_w, const CUtensorMap& map_x, Params p, int grid, cudaStream_t st) {
   using C = Cfg<WBITS, NC, KS, SUB>;
+  p.alternate = issuers_may_alternate(p.fu, C::kASlots, C::kB, C::kAccLast);
   auto kern = tmem_gemm_kernel<WBITS, XT, NC, KS, SUB, W16>;
   static bool attr_set[64] = {};
   int dev = 0;
