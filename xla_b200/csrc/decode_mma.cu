@@ -126,8 +126,8 @@ __device__ __forceinline__ float ar_ld_peer(const float* p) {
 // step and reuses its activation registers for all of them); WARPS = warps splitting K.
 // One "fold" = the end of a scale block (blockwise) or of a single step (per-channel): the partial tile is added
 // into the totals.
-// BIASED: int4 through the conversion above.
-template <int WBITS, typename XT, typename ST, int NT, int RG, int WARPS, bool AR = false, bool BIASED = false>
+// BIASED: int4 through the conversion above.  AHEAD: a step's activations are loaded a step ahead too.
+template <int WBITS, typename XT, typename ST, int NT, int RG, int WARPS, bool AR = false, bool BIASED = false, bool AHEAD = false>
 __global__ void __launch_bounds__(WARPS * 32)
     decode_mma_kernel(const XT* x, const uint8_t* __restrict__ w, const ST* scale,
                       void* __restrict__ out, int out_dt, int M, int64_t N, int64_t K, int steps_per_block,
@@ -177,9 +177,8 @@ __global__ void __launch_bounds__(WARPS * 32)
     }
 
   // Software pipeline, one step deep: the weights of this warp's next step are in flight while the
-  // current step is converted and multiplied.  (Prefetching the activations as well costs 24 registers
-  // and measured slower: they come from L1.)
-  constexpr bool kPrefetchX = false;
+  // current step is converted and multiplied.  (Prefetching the activations as well costs 22 registers, and
+  // is slower where those are another CTA's: they come from L1.  See launch_nt for where it is not.)
   auto load_x = [&](int step, uint32_t (&dst)[NT][XREGS]) {
 #pragma unroll
     for (int i = 0; i < NT; ++i) {
@@ -207,13 +206,13 @@ __global__ void __launch_bounds__(WARPS * 32)
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   uint32_t xn[NT][XREGS];
-  if (kPrefetchX && s < steps) load_x(s, xn);
+  if (AHEAD && s < steps) load_x(s, xn);
   for (; s < steps; s += WARPS) {
     uint4 wc[2 * RG];
 #pragma unroll
     for (int r = 0; r < 2 * RG; ++r) wc[r] = wn[r];
     uint32_t xr[NT][XREGS];
-    if (kPrefetchX) {
+    if (AHEAD) {
 #pragma unroll
       for (int i = 0; i < NT; ++i)
 #pragma unroll
@@ -223,7 +222,7 @@ __global__ void __launch_bounds__(WARPS * 32)
     if (sn < steps) {
 #pragma unroll
       for (int r = 0; r < 2 * RG; ++r) wn[r] = ld_stream_u4(wrow[r] + (int64_t)sn * 64);
-      if (kPrefetchX) load_x(sn, xn);
+      if (AHEAD) load_x(sn, xn);
     }
     // fold after this step?  (blockwise: this warp's next step belongs to another block)
     bool fold = true;
@@ -239,7 +238,7 @@ __global__ void __launch_bounds__(WARPS * 32)
         for (int r = 0; r < 2 * RG; ++r) sc[r] = to_f32(ld_ordered(srow[r] + (int64_t)b * N));
       }
     }
-    if (!kPrefetchX) load_x(s, xr);
+    if (!AHEAD) load_x(s, xr);
 #pragma unroll
     for (int wi = 0; wi < 4; ++wi) {
       if constexpr (WBITS == 4) {
@@ -851,7 +850,15 @@ int launch_nt(const void* x, const void* w, const ST* scale, void* out, int out_
                        (int)M, N, K, spb, shift, bw, 0, a, device_error_word());
     }
   } else if (M <= 8) {
-    if (warps >= 16)
+    // int4, a row tile per SM at most, more than a step per warp: the activations a step ahead.  There are registers to spare, and
+    // those keep the next launch's CTAs off the SMs that are in use: with 60 a thread two fit, and as the launch has fewer CTAs than
+    // there are places, some SMs get two of it.  M = 7, [2048,4480] block 128: 5.8 us a launch back to back without, 4.0 with it (4.4
+    // with the 70 registers of the conversion with a bias); [2048,10240] at one 8.1, 6.4; [1280,27392] at eight 21.4, 15.0.  With
+    // another kernel between the launches it is 3 % at 100 steps and even at 20.
+    if (WBITS == 4 && warps >= 16 && tiles <= sms && K / VPS > 16)
+      err = launch_pdl(decode_mma_kernel<WBITS, XT, ST, 1, 1, 16, false, false, WBITS == 4>, (unsigned)tiles, 512, 0, st, xp, wp, scale, out, out_dt,
+                       (int)M, N, K, spb, shift, bw, gate_up, ArParams{}, (uint32_t*)nullptr);
+    else if (warps >= 16)
       err = QMM_DECODE_LAUNCH(1, 1, 16);
     else if (warps >= 8)
       err = QMM_DECODE_LAUNCH(1, 1, 8);
