@@ -51,3 +51,23 @@ def test_zero_points_per_channel_on_few_inputs(wbits, K, M, variant):
     exact = (x.double() @ w.double().T) * s.double() - x.double().sum(1, keepdim=True) * z.double()
     # exact products (or 2^-22 of the row's largest activation); K additions in fp32 at most: K 2^-24 < 2e-5 of the largest result
     assert qo.max_abs_rel(out, exact) < 2e-5
+
+
+@pytest.mark.parametrize("wbits,bs,K,M", [(8, -1, 2032, 20), (8, -1, 2048, 20), (8, -1, 2064, 9), (4, -1, 4128, 70), (8, -1, 12304, 33),
+                                          (4, 384, 7680, 300), (8, 256, 4096, 513), (4, 2048, 8192, 40)])
+def test_sums_of_long_rows_and_many_blocks(wbits, bs, K, M):
+  """A row per warp and per CTA, on both sides of the line; more pieces than a few CTAs have warps."""
+  g = qc.gen(K + M)
+  N = 130
+  x = (torch.rand(M, K, generator=g) + 0.5).bfloat16().to(DEV)
+  w = (qc.int4_weight if wbits == 4 else qc.int8_weight)(g, N, K).to(DEV)
+  s = (qc.per_channel_scale(g, N) if bs == -1 else qc.blockwise_scale(g, K // bs, N)).to(DEV)
+  z = torch.randint(-20, 21, s.shape, generator=g).to(DEV) * s
+  with xla_b200.force_variant("tmem"):
+    out = torch.ops.xla_b200.quantized_matmul_packed(x, xla_b200.pack_int4(w) if wbits == 4 else w, s, z, block_size=bs,
+                                                     int4_weight=wbits == 4, weight_is_packed=wbits == 4, out_dtype=torch.float32)
+  S = 1 if bs == -1 else K // bs
+  xb, wb = x.double().view(M, S, -1), w.double().view(N, S, -1)
+  exact = torch.einsum("msk,nsk,sn->mn", xb, wb, s.double().view(S, N)) - torch.einsum("ms,sn->mn", xb.sum(-1), z.double().view(S, N))
+  # the sums of positive activations: a lane adds K / 32 of them at most in fp32, the products' sums fewer in a row
+  assert qo.max_abs_rel(out, exact) < 2e-5

@@ -712,31 +712,58 @@ __global__ void __launch_bounds__(Cfg<WBITS, NC, KS, SUB>::kThreads, 1)
 // Sums of the activations over each scale block, for the zero points: xs[b * pitch + m]; tokens from M up to the pitch get
 // zeros.  A warp takes 256 values of a row, or a whole larger block, at a time.  Several shorter blocks of a row (of 64 or 128
 // values) are summed by the lanes that hold them, 8 or 16; one that is alone in its row (per channel, any multiple of eight values)
-// by all lanes, of which those beyond it hold zeros.
-constexpr int kSumsThreads = 512;
-template <typename XT>
+// by all lanes, of which those beyond it hold zeros.  ROW: a CTA takes a row, for long rows per channel.
+// Bound by the latency of its loads, so a warp has one piece, as many loads at a time as that needs: with one CTA per SM walking the pieces,
+// 2044 tokens of [735,14592] block 384 took 154 us with the GEMM, 81 so.  A long row has a CTA for the same reason ([588,27456] int4 per
+// channel at 120 tokens 58 us with a warp, 41 so).
+constexpr int kSumsThreads = 256;
+constexpr int kLongRow = 2048;  // values
+template <typename XT, bool ROW>
 __global__ void __launch_bounds__(kSumsThreads) block_sums_kernel(const XT* x, float* __restrict__ xs, int pitch, int M, int K, int S) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  const int lane = threadIdx.x & 31, len = K / S;
-  const int per = max(len, 256), pieces = (K + per - 1) / per;
-  const int group = S > 1 && len < 256 ? len / 8 : 32;  // lanes that sum a block, a power of two
-  const int warps = gridDim.x * (kSumsThreads / 32);
-  for (int64_t i = (int64_t)blockIdx.x * (kSumsThreads / 32) + (threadIdx.x >> 5); i < (int64_t)pitch * pieces; i += warps) {
-    const int m = (int)(i / pieces), k0 = (int)(i - (int64_t)m * pieces) * per;
+  const int lane = threadIdx.x & 31;
+  // 256 values by the lanes of the warp, eight each
+  auto add = [](float s, const XT* at) {
+    const uint4 v = *reinterpret_cast<const uint4*>(at);
+    const XT* e = reinterpret_cast<const XT*>(&v);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s += to_f32(e[j]);
+    return s;
+  };
+  if constexpr (ROW) {
+    __shared__ float s_warp[kSumsThreads / 32];
+    const int m = blockIdx.x;
     float s = 0.f;
     if (m < M) {
       const XT* row = x + (int64_t)m * K;
-      for (int k = k0 + lane * 8; k < min(K, k0 + per); k += 256) {
-        const uint4 v = *reinterpret_cast<const uint4*>(row + k);
-        const XT* e = reinterpret_cast<const XT*>(&v);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) s += to_f32(e[j]);
-      }
-      for (int o = group >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+#pragma unroll 4
+      for (int k = threadIdx.x * 8; k < K; k += kSumsThreads * 8) s = add(s, row + k);
     }
-    const int b = (k0 + lane * 8) / len;
-    if (lane % group == 0 && b < S) xs[(int64_t)b * pitch + m] = s;
+    s = warp_sum(s);
+    if (lane == 0) s_warp[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+      for (int i = 1; i < kSumsThreads / 32; ++i) s += s_warp[i];
+      xs[m] = s;
+    }
+  } else {
+    const int len = K / S, per = max(len, 256), pieces = (K + per - 1) / per;
+    const int group = S > 1 && len < 256 ? len / 8 : 32;  // lanes that sum a block, a power of two
+    const int64_t warps = (int64_t)gridDim.x * (kSumsThreads / 32);
+    for (int64_t i = (int64_t)blockIdx.x * (kSumsThreads / 32) + (threadIdx.x >> 5); i < (int64_t)pitch * pieces; i += warps) {
+      const int m = (int)(i / pieces), k0 = (int)(i - (int64_t)m * pieces) * per, k1 = min(K, k0 + per);
+      float s = 0.f;
+      if (m < M) {
+        const XT* row = x + (int64_t)m * K;
+#pragma unroll 4
+        for (int k = k0 + lane * 8; k < k1; k += 256) s = add(s, row + k);
+        for (int o = group >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      }
+      const int b = (k0 + lane * 8) / len;
+      if (lane % group == 0 && b < S) xs[(int64_t)b * pitch + m] = s;
+    }
   }
 }
 
@@ -957,12 +984,18 @@ int launch_tmem_gemm(int wbits, const void* x, int x_dt, const void* w, const Sc
   }
 
   if (zp) {
+    const bool row = p.S == 1 && K >= kLongRow;
     const int64_t pieces = ceil_div(K, std::max<int64_t>(K / p.S, 256));
-    const unsigned g = (unsigned)std::min<int64_t>(sm_count(), ceil_div(sc.xs_pitch * pieces, kSumsThreads / 32));
-    cudaError_t e = x_dt == QMM_BF16 ? launch_pdl(block_sums_kernel<__nv_bfloat16>, g, kSumsThreads, 0, st, reinterpret_cast<const __nv_bfloat16*>(x),
-                                                  sc.xs, sc.xs_pitch, (int)M, (int)K, p.S)
-                                     : launch_pdl(block_sums_kernel<__half>, g, kSumsThreads, 0, st, reinterpret_cast<const __half*>(x), sc.xs,
-                                                  sc.xs_pitch, (int)M, (int)K, p.S);
+    const unsigned g = row ? (unsigned)sc.xs_pitch : (unsigned)std::min<int64_t>(1 << 20, ceil_div(sc.xs_pitch * pieces, kSumsThreads / 32));
+    auto sums = [&](auto kern, auto* from) { return launch_pdl(kern, g, kSumsThreads, 0, st, from, sc.xs, sc.xs_pitch, (int)M, (int)K, p.S); };
+    cudaError_t e;
+    if (x_dt == QMM_BF16) {
+      auto* from = reinterpret_cast<const __nv_bfloat16*>(x);
+      e = row ? sums(block_sums_kernel<__nv_bfloat16, true>, from) : sums(block_sums_kernel<__nv_bfloat16, false>, from);
+    } else {
+      auto* from = reinterpret_cast<const __half*>(x);
+      e = row ? sums(block_sums_kernel<__half, true>, from) : sums(block_sums_kernel<__half, false>, from);
+    }
     if (e != cudaSuccess) {
       cudaGetLastError();
       return fail(QMM_ERR_LAUNCH, "block_sums_kernel launch: %s", cudaGetErrorString(e));
