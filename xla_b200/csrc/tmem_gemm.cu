@@ -969,16 +969,31 @@ int launch_tmem_gemm(int wbits, const void* x, int x_dt, const void* w, const Sc
   p.items1 = items;
   int grid = std::min(items, ctas);
   if (left != 0) {
-    // Splitting the left-over items over s CTAs each: item / s plus an exchange that grows with s (one partial tile per
-    // CTA, written, and read by the item's first CTA).
-    const double stage_us = (wbits == 4 ? 0.27 + 0.003 * pl.th : 0.32 + 0.0038 * pl.th) * (ks / 128.0);
-    const double item_us = p.ut * p.unit * stage_us, partial_us = 0.25 + 1.1 * pl.th / 256;
-    double s = std::sqrt(item_us / partial_us);
-    s = std::min(s, std::min((double)ctas / (double)left, (double)p.ut));
-    if (s >= 1.2 && item_us / s + 2.0 + partial_us * s < 0.85 * item_us) {
+    // The left-over items are split over s CTAs each where that is sooner done.  A step's time is what its 128 or 256 values take and a
+    // share per fold; the exchange (one partial tile per CTA, written, and read by the item's first CTA) about 2 us and a share per
+    // CTA.  Where s is not whole, CTAs have parts of two items and the exchanges come one behind the other, 1.75 times as long: int4
+    // block 128 [5120,3072] at 96 tokens, 40 items, 17.7 us whole, 16.8 and 16.6 over two and three CTAs, 21.8 over 3.7 (and 33.6
+    // against 29.9 whole over 1.3 with 6144 inputs).  Times read off 1036 shapes of five to 260 tiles with s forced; [5120,1536] int8
+    // block 384 at 127 tokens 19.6 us by a step's time as of longer folds, 11.7 so.
+    const int64_t nc = pl.nc;
+    const double per_fold = nc <= 64 ? 0.12 : nc <= 128 ? 0.27 : 0.33, per_zp = !zp || !p.blocked ? 0.0 : nc <= 32 ? 0.06 : nc <= 64 ? 0.12 : 0.3;
+    const double per_128 = nc <= 32 ? 0.21 : nc <= 64 ? (wbits == 4 ? 0.25 : 0.36) : nc <= 128 ? 0.3 : 0.38;
+    const double step_us = (per_128 + (per_fold + per_zp) * 128.0 / (block_size > 0 ? (double)block_size : 512.0)) * (ks / 128.0);
+    const double share = nc <= 32 ? 0.25 : nc <= 64 ? 0.5 : 0.011 * pl.th, more_ctas = 0.011;
+    const double whole_us = p.ut * p.unit * step_us, most = std::min((double)ctas / left, (double)p.ut);
+    double best = 0.95 * whole_us, s = 1.0;
+    for (int k = 2; k <= (int)std::min(most, 24.0); ++k) {
+      const double us = (double)ceil_div(p.ut, k) * p.unit * step_us + 2.0 + share * k + more_ctas * left * (k - 1);
+      if (us < best) {
+        best = us;
+        s = k;
+      }
+    }
+    if (most > (int)most && whole_us / most + 1.75 * (2.0 + share * most) + more_ctas * (ctas - left) < best) s = most;
+    if (s > 1.0) {
       p.items1 = items - left;
       p.units = left * p.ut;
-      p.g2 = std::min(ctas, std::max(left, (int)((double)left * s)));
+      p.g2 = std::min(ctas, std::max(left, (int)(left * s)));
       grid = std::max(std::min(p.items1, ctas), p.g2);
     }
   }
