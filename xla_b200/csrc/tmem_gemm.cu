@@ -952,6 +952,21 @@ int launch_tmem_gemm(int wbits, const void* x, int x_dt, const void* w, const Sc
   } else {
     const int folds = (int)ceil_div(stages, 512 / ks);
     p.fu = p.unit = (int)align_up((size_t)ceil_div(stages, folds), spr);
+    // Up to 128 columns shorter folds where that means fewer steps beyond K: a fold takes a fifth of a step up to 64 tokens, near a half
+    // above (int4 [674,768] at 11 tokens, three steps for four, 4.2 us -> 3.8).  int4 with 128 columns: two steps, which both issuers take
+    // in turn (0.37 us for 128 values, 0.42 with four on one issuer; [6205,2304] at 92 tokens 15.8 us -> 14.4).  With 192 columns the
+    // accumulators ahead are what the epilogue hides under, so folds stay long ([14336,768] at 268 tokens 22.3 us, 23.0 with two steps).
+    if (pl.nc <= 128) {
+      const double fold = pl.nc <= 64 ? 0.2 : 0.45;
+      double best = 1e30;
+      for (int fu = spr; fu <= (pl.nc == 128 && wbits == 4 ? 2 : 512 / ks); fu += spr) {
+        const double t = (double)align_up((size_t)stages, (size_t)fu) * (1.0 + fold / fu);
+        if (t < best) {
+          best = t;
+          p.fu = p.unit = fu;
+        }
+      }
+    }
   }
   p.fpu = p.unit / p.fu;
   p.ut = (int)ceil_div(stages, p.unit);
@@ -978,7 +993,7 @@ int launch_tmem_gemm(int wbits, const void* x, int x_dt, const void* w, const Sc
     const int64_t nc = pl.nc;
     const double per_fold = nc <= 64 ? 0.12 : nc <= 128 ? 0.27 : 0.33, per_zp = !zp || !p.blocked ? 0.0 : nc <= 32 ? 0.06 : nc <= 64 ? 0.12 : 0.3;
     const double per_128 = nc <= 32 ? 0.21 : nc <= 64 ? (wbits == 4 ? 0.25 : 0.36) : nc <= 128 ? 0.3 : 0.38;
-    const double step_us = (per_128 + (per_fold + per_zp) * 128.0 / (block_size > 0 ? (double)block_size : 512.0)) * (ks / 128.0);
+    const double step_us = (per_128 + (per_fold + per_zp) * 128.0 / (block_size > 0 ? (double)block_size : (double)(p.fu * ks))) * (ks / 128.0);
     const double share = nc <= 32 ? 0.25 : nc <= 64 ? 0.5 : 0.011 * pl.th, more_ctas = 0.011;
     const double whole_us = p.ut * p.unit * step_us, most = std::min((double)ctas / left, (double)p.ut);
     double best = 0.95 * whole_us, s = 1.0;
