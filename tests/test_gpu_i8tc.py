@@ -306,3 +306,37 @@ def test_a_workspace_of_the_stated_size_suffices(variant, out_dtype, wbits, bs):
       ref = torch.ops.xla_b200.quantized_matmul_packed(x, wk, s, block_size=bs, int4_weight=wbits == 4, weight_is_packed=wbits == 4,
                                                        out_dtype=out_dtype)
     assert torch.equal(out, ref), M
+
+
+@pytest.mark.parametrize("wbits,bs,M,zp", [(8, -1, 7, True), (8, 128, 28, False), (4, -1, 6, True), (8, -1, 20, False)])
+def test_a_prime_number_of_weight_tiles(wbits, bs, M, zp):
+  """167 tiles divide among no grid but one CTA: the same result as 166 tiles have in the rows they share, in about the time."""
+  K, N = 2048, 167 * 128
+  g = torch.Generator(device=DEV).manual_seed(M)
+  x = torch.randn(M, K, generator=g, device=DEV).bfloat16()
+  w = torch.randint(-8, 8, (N, K), generator=g, device=DEV, dtype=torch.int8)
+  s = (torch.rand((N,) if bs == -1 else (K // bs, N), generator=g, device=DEV) + 0.5) / 200
+  z = torch.randint(-2, 3, s.shape, generator=g, device=DEV) * s if zp else None
+
+  def run(rows):
+    cut = lambda t: None if t is None else (t[:rows] if bs == -1 else t[:, :rows].contiguous())  # noqa: E731
+    wd, sd, zd = w[:rows].contiguous(), cut(s), cut(z)
+    wd = xla_b200.pack_int4(wd) if wbits == 4 else wd
+    call = lambda: torch.ops.xla_b200.quantized_matmul_packed(x, wd, sd, zd, block_size=bs, int4_weight=wbits == 4,  # noqa: E731
+                                                              weight_is_packed=wbits == 4, out_dtype=torch.float32)
+    start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    with xla_b200.force_variant("i8tc"):
+      out = call()
+      times = []
+      for _ in range(5):
+        start.record()
+        for _ in range(10):
+          call()
+        end.record()
+        torch.cuda.synchronize()
+        times.append(start.elapsed_time(end))
+    return out, min(times)
+
+  (few, t_few), (all_rows, t_all) = run(166 * 128), run(N)
+  assert qo.max_abs_rel(all_rows[:, :166 * 128], few) < 1e-6  # the K ranges of the CTAs differ, by a few roundings of fp32 sums
+  assert t_all < 4 * t_few  # one CTA took thirty times as long

@@ -1290,22 +1290,22 @@ Split split_one_tile(int wbits, const Plan& pl, long long tiles, long long slots
   sp.grid = (int)std::min<long long>(ctas_max, std::max<long long>(1, units / min_units));
   const long long sk_slots = ceil_div(units, sp.grid) * spu;                  // slots per CTA, stream-K
   const long long per_sm = occ;                                               // CTAs that share an SM's bandwidth
-  const long long dp_rounds = ceil_div(tiles, ctas_max);
-  const long long dp_slots = dp_rounds * slots;                               // slots per CTA, whole tiles
+  // Whole tiles: the units must split at tile boundaries, so the grid divides the tile count.  (The largest such grid may be far below
+  // the CTAs there are: of 223 tiles it is one CTA, and int8 [28495,3328] at seven tokens took 903 us, 27 with the tiles split)
+  long long dp_ctas = std::min(tiles, ctas_max);
+  while (tiles % dp_ctas != 0) --dp_ctas;
+  const long long dp_slots = tiles / dp_ctas * slots;                         // slots per CTA, whole tiles
   // exchange cost in slots of streaming (measured: ~3 us for tiles of 5 tokens, ~13 us for 64); a partial tile is
   // 128 x tokens floats, so it grows with the tile
   // (a slot of the 128-column int4 instance takes three times as long as one of the narrow ones: fewer per exchange)
   const long long exchange = ((wbits == 4 && pl.ncols == 128) ? 3 : (wbits == 4 ? 8 : 4)) * (16 + pl.tile_tokens) / 16;
-  // compare per-SM streaming: with whole tiles only ceil(tiles / rounds) CTAs run, spread over the SMs
-  const long long dp_ctas = ceil_div(tiles, dp_rounds);
+  // compare per-SM streaming
   const long long dp_per_sm = ceil_div(dp_ctas, sm_count());
   const bool fills = occ == 1 || dp_ctas * 4 >= ctas_max * 3;  // two CTAs per SM only pay off when both slots are used
   sp.cost = sk_slots * per_sm + exchange;
-  if (fills && dp_slots * dp_per_sm <= sp.cost && tiles <= ctas_max * dp_rounds) {
+  if (fills && dp_slots * dp_per_sm <= sp.cost) {
     sp.cost = dp_slots * dp_per_sm;
-    sp.grid = (int)std::min<long long>(tiles, ctas_max);
-    // with several rounds the units must still split at tile boundaries: a grid that divides the tile count
-    while (tiles % sp.grid != 0) --sp.grid;
+    sp.grid = (int)dp_ctas;
   }
   return sp;
 }
