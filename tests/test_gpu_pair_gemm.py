@@ -48,3 +48,17 @@ def test_weight_only(M, N, K, zp, x_dt, out_dt):
   # three limbs: 2^-22 of the row's largest value per activation; two (16-bit results without zero points): 2^-15 of it, under
   # the rounding of the result
   assert qo.max_abs_rel(out, exact) < {torch.float32: 1e-5, torch.float16: 3e-3, torch.bfloat16: 1e-2}[out_dt]
+
+
+@pytest.mark.parametrize("M,N,K,zp", [(129, 11008, 384, False), (256, 11008, 384, False), (100, 4096, 12288, False), (92, 5120, 640, True), (128, 5120, 640, True)])
+def test_both_sides_of_the_line_between_pairs_and_single_ctas(M, N, K, zp):
+  """A round of tiles less on pairs than on single CTAs, and the same number; K long enough to be split."""
+  g = torch.Generator(device=DEV).manual_seed(M + N + K)
+  x = torch.randn(M, K, generator=g, device=DEV).bfloat16()
+  w = torch.randint(-127, 128, (N, K), generator=g, device=DEV, dtype=torch.int8)
+  s = (torch.rand(N, generator=g, device=DEV) + 0.5) / 73 / K**0.5
+  z = torch.randint(-20, 21, (N,), generator=g, device=DEV) * s if zp else None
+  with xla_b200.force_variant("i8tc"):
+    out = torch.ops.xla_b200.quantized_matmul_packed(x, w, s, z, out_dtype=torch.float32)
+  exact = (x.double() @ w.double().T) * s.double() - (x.double().sum(1, keepdim=True) * z.double() if zp else 0.)
+  assert qo.max_abs_rel(out, exact) < 1e-5  # three limbs: 2^-22 of the row's largest value per activation

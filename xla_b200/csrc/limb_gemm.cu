@@ -1291,7 +1291,7 @@ Split split_one_tile(int wbits, const Plan& pl, long long tiles, long long slots
   const long long sk_slots = ceil_div(units, sp.grid) * spu;                  // slots per CTA, stream-K
   const long long per_sm = occ;                                               // CTAs that share an SM's bandwidth
   // Whole tiles: the units must split at tile boundaries, so the grid divides the tile count.  (The largest such grid may be far below
-  // the CTAs there are: of 223 tiles it is one CTA, and int8 [28495,3328] at seven tokens took 903 us, 27 with the tiles split)
+  // the CTAs there are: of 223 tiles it is one CTA, and int8 [28495,3328] at seven tokens took 903 us, 25 with the tiles split)
   long long dp_ctas = std::min(tiles, ctas_max);
   while (tiles % dp_ctas != 0) --dp_ctas;
   const long long dp_slots = tiles / dp_ctas * slots;                         // slots per CTA, whole tiles

@@ -497,12 +497,17 @@ int launch_with(const CUtensorMap& map_w, const CUtensorMap& map_b, const Params
 
 int pair_gemm_tokens(int nl) { return nl == 3 ? Tile<3>::kTokens : kCols / nl; }
 
-// Weight-only: with 40 items, or 16 long ones, which are split ([4096,4096] int8 at 256 tokens, 32 items, 19 us against 17 on
-// limb_gemm.cu, at 333 20 against 24; [14336,4096] at 128 19 against 25, at 512 49 against 61; [28672,8192] at 512 158 against 208;
-// [4096,14336] at 96 30 against 39).  Three limbs: [14336,4096] with zero points at 64 tokens 20 against 25.
+// Weight-only, against limb_gemm.cu's 128 x 64 (42 with three limbs) tiles on single CTAs.  A round of tiles takes about as long there as
+// here, a little less, with half of the work in it.  So here where that saves a round: int8 [11008,5120] at 256 tokens, 86 items in two
+// rounds against 344 in three, 32 us, 36 there; at 129, 258 in two there as well, 31 and 27; [5120,5120] at 256 (40 items, 160)
+// 21 and 26, at 129 (40, 120) 19.5 and 17.7.  At equal rounds from 12288 inputs on, which are split over K here ([2560,28672] at 256 tokens
+// 46 and 65), and few items from 8192 ([2560,9472] at 128 22.6 and 25.2).  1832 shapes measured on both.
 bool pair_gemm_preferred(int nl, int64_t M, int64_t N, int64_t K) {
   const int64_t items = ceil_div(N, 2 * kRows) * ceil_div(M, pair_gemm_tokens(nl));
-  return M > (nl == 3 ? 42 : 64) && (items >= 40 || (items >= 16 && K >= 8192));
+  const int64_t there = ceil_div(N, kRows) * ceil_div(M, nl == 3 ? 42 : 64);  // limb_gemm.cu's items
+  const int sms = sm_count();
+  if (M <= (nl == 3 ? 42 : 64) || items < 16) return false;
+  return ceil_div(items, sms / 2) < ceil_div(there, sms) || K >= 12288 || (K >= 8192 && items < 24);
 }
 
 // W8A8, against w8a8_gemm.cu's 128 x 256 tiles on single CTAs: by rounds of tiles, at 0.31 us a stage here and 0.5 there, and a
