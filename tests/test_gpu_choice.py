@@ -1,0 +1,43 @@
+"""AUTO's choice of kernel on both sides of its lines, by name (16-bit results), with a result against 64 bits."""
+import pytest
+import torch
+
+import xla_b200
+from oracle import qmm_oracle as qo
+from xla_b200 import _capi
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def chosen(wbits, bs, zp, M, N, K):
+  return _capi.lib().qmm_weight_only_variant_for(wbits, M, N, K, max(bs, 0), int(zp)).decode()
+
+
+def call_and_exact(wbits, bs, zp, M, N, K, out_dtype, dtype=torch.bfloat16):
+  g = torch.Generator(device=DEV).manual_seed(M + N + K)
+  x = torch.randn(M, K, generator=g, device=DEV)
+  x = torch.where(torch.rand(M, K, generator=g, device=DEV) < 0.01, x * 20, x).to(dtype)
+  lo, hi = (-8, 8) if wbits == 4 else (-127, 128)
+  w = torch.randint(lo, hi, (N, K), generator=g, device=DEV, dtype=torch.int8)
+  S = 1 if bs == -1 else K // bs
+  s = (torch.rand((N,) if bs == -1 else (S, N), generator=g, device=DEV) + 0.5) / (4.6 if wbits == 4 else 73) / K**0.5
+  z = torch.randint(-2, 3, s.shape, generator=g, device=DEV) * s if zp else None
+  wd = xla_b200.pack_int4(w) if wbits == 4 else w
+  call = lambda: torch.ops.xla_b200.quantized_matmul_packed(x, wd, s, z, block_size=bs, int4_weight=wbits == 4,  # noqa: E731
+                                                            weight_is_packed=wbits == 4, out_dtype=out_dtype)
+  xb = x.double().view(M, S, -1)
+  exact = torch.einsum("msk,nsk,sn->mn", xb, w.double().view(N, S, -1), s.double().view(S, N))
+  if zp:
+    exact -= torch.einsum("ms,sn->mn", xb.sum(-1), z.double().view(S, N))
+  return call, exact
+
+
+@pytest.mark.parametrize("wbits,bs,zp,M,N,K,kernel", [
+    (4, 64, False, 33, 512, 960, "tmem"), (8, 64, False, 35, 512, 960, "tmem"), (4, 64, False, 126, 1280, 1472, "tmem"),
+    (8, 64, False, 1143, 640, 1344, "tmem"), (8, 64, False, 8, 8192, 7424, "mma"), (8, 64, False, 9, 8192, 4160, "tmem"),
+])
+def test_choice(wbits, bs, zp, M, N, K, kernel):
+  assert chosen(wbits, bs, zp, M, N, K) == kernel
+  call, exact = call_and_exact(wbits, bs, zp, M, N, K, torch.bfloat16)
+  assert qo.max_abs_rel(call(), exact) < 1e-2  # one rounding to bf16

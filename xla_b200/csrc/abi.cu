@@ -223,6 +223,9 @@ static bool zp_decode_on_tc(int wbits, int64_t M, int64_t N, int64_t K, bool dec
 //                  than 12288 outputs from 33 tokens ([4096,4096] at 64 tokens 20 us, 16 there; [14336,4096] 21, 25 there), large
 //                  int4 weights up to its 42 tokens ([28672,8192] at 16 tokens 37 us, 31 there), all up to eight tokens
 //                  ([8192,28672] 50, 37 there), and above 64 tokens with fewer than 64 items of 128 rows and 192 tokens.
+//   blocks of 64   above 32 tokens always: the other kernel that goes on with them there, tcgen05, has 64 tokens a pass (int4 [3584,20416] at
+//                  114 tokens 44 us against 104, int8 [1280,11328] at 1143 59 against 172, [512,960] at 35 7.3 against 10).  Not up to eight (int8
+//                  [8192,7424] at six tokens 19.5 us, 14.4 on the decode kernel).
 //   fp32 results   per channel only where the other kernels need as many roundings: above 64 tokens, when the items fill
 //                  half of the SMs (the other kernel needs a third limb per token there; int8 [28672,8192] at 512 tokens 219 us
 //                  against 312, [2432,9248] at 763 tokens 49 against 74).
@@ -253,6 +256,7 @@ static bool use_tmem(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, int
     return wbits == 4 ? M > 42 || E < 1 << 25 : M <= 32 || N >= 12288;
   }
   if (M == 1) return false;
+  if (bs == 64 && (M <= 8 || M > 32)) return M > 32;
   if (M <= 64) {
     if (out_dt == QMM_F32 && !blocked) return false;
     if (M > 32) return E >= 1 << 22 && (wbits == 4 || blocked || E < 95000000);
