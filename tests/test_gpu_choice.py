@@ -36,6 +36,8 @@ def call_and_exact(wbits, bs, zp, M, N, K, out_dtype, dtype=torch.bfloat16):
 @pytest.mark.parametrize("wbits,bs,zp,M,N,K,kernel", [
     (4, 64, False, 33, 512, 960, "tmem"), (8, 64, False, 35, 512, 960, "tmem"), (4, 64, False, 126, 1280, 1472, "tmem"),
     (8, 64, False, 1143, 640, 1344, "tmem"), (8, 64, False, 8, 8192, 7424, "mma"), (8, 64, False, 9, 8192, 4160, "tmem"),
+    (8, 128, False, 1100, 1024, 1152, "tmem"), (8, 256, False, 1100, 260, 1024, "tmem"), (8, 128, False, 1024, 1024, 1152, "i8tc"),
+    (8, -1, False, 1100, 1024, 1040, "tmem"),
 ])
 def test_choice(wbits, bs, zp, M, N, K, kernel):
   assert chosen(wbits, bs, zp, M, N, K) == kernel

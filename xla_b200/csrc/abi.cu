@@ -243,7 +243,8 @@ static bool zp_decode_on_tc(int wbits, int64_t M, int64_t N, int64_t K, bool dec
 //                  tokens, where i8tc expands the weights once, on 2^25 values ([4096,4096] at 1024 50 us against 38; [5120,6912] at
 //                  512 39 against 54), from 512 on fewer than 12288 outputs ([14336,4096] at 1024 117 against 94).
 //   narrow int8    up to 2048 outputs and above the 1024 tokens of one launch of the other kernel, whose launches are then
-//                  a round or two of items each ([1536,14592] at 4178 tokens 189 us against 313).
+//                  a round or two of items each (per channel [1536,14592] at 4178 tokens 189 us against 313, block 128 [1024,3968] at 1131 24
+//                  against 46; with two limbs there, exact products here).
 static bool use_tmem(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, int x_dt, int out_dt, bool has_zp, bool decode_i8) {
   if (!tmem_gemm_shape_ok(wbits, M, N, K, bs, x_dt)) return false;
   const bool blocked = bs > 0;
@@ -270,7 +271,8 @@ static bool use_tmem(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, int
   }
   const bool filled = 2 * items >= sm_count();
   if (out_dt == QMM_F32 && filled && (wbits == 8 || blocked || M < 384)) return true;
-  if (wbits == 8 && !blocked) return M > 1024 && N <= 2048;
+  if (wbits == 8 && M > 1024 && N <= 2048) return true;
+  if (wbits == 8 && !blocked) return false;
   if (!blocked && M >= 384 && (E < 1 << 25 || (M >= 512 && N >= 12288))) return false;
   return filled || (items >= 64 && E >= 1 << 25);
 }
