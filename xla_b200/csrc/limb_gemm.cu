@@ -35,7 +35,6 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
-#include <cstdio>
 #include <cstdlib>
 
 #include "common.cuh"
@@ -58,31 +57,6 @@ constexpr int kDrainWarp0 = 4;
 constexpr int kConvWarp0 = 8;
 constexpr int kMaxAcc = 8;
 constexpr uint32_t kSmemBudget = 227 * 1024 - 1024 /*alignment*/ - 1024 /*barriers*/;
-
-// Optional per-role cycle accounting of CTA 0 (compile with -DQMM_LIMB_DBG; never in the shipped build).
-#ifdef QMM_LIMB_DBG
-}  // namespace
-__device__ long long g_limb_dbg[64];
-__device__ long long g_limb_cta[4 * 512];  // per CTA: entry, first slot full, MMAs issued, exit (globaltimer ns)
-namespace {
-#define DBG_DECL long long dbg_t = 0, dbg_w[4] = {0, 0, 0, 0}; const long long dbg_t0 = clock64(); (void)dbg_t
-#define DBG_BEGIN() dbg_t = clock64()
-#define DBG_END(i) dbg_w[i] += clock64() - dbg_t
-#define DBG_STAMP(i) if (blockIdx.x == 0 && (threadIdx.x & 31) == 0) g_limb_dbg[42 + (i)] = (long long)ptx::globaltimer_ns()
-#define DBG_STAMP1(i) if (blockIdx.x == 1 && (threadIdx.x & 31) == 0) g_limb_dbg[42 + (i)] = (long long)ptx::globaltimer_ns()
-#define DBG_FLUSH(base)                                                  \
-  if (blockIdx.x == 0 && (threadIdx.x & 31) == 0) {                      \
-    for (int i_ = 0; i_ < 4; ++i_) g_limb_dbg[(base) + i_] = dbg_w[i_];  \
-    g_limb_dbg[(base) + 4] = clock64() - dbg_t0;                         \
-  }
-#else
-#define DBG_DECL
-#define DBG_BEGIN()
-#define DBG_END(i)
-#define DBG_STAMP(i)
-#define DBG_STAMP1(i)
-#define DBG_FLUSH(base)
-#endif
 
 enum LimbErr : uint32_t { kErrPartialWait = 9 };  // owner CTA never saw a partial tile arrive
 
@@ -255,10 +229,8 @@ __global__ void __launch_bounds__(1024) split_rows_kernel(const XT* x, int8_t* _
                                                           int block_groups) {
   __shared__ uint32_t s_max[32];
   __shared__ int s_lo[kMaxZpBlocks], s_hi[kMaxZpBlocks];
-  if (blockIdx.x == 0 && threadIdx.x == 0) { DBG_STAMP(10); }
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");  // x may come from the previous kernel of the stream
-  if (blockIdx.x == 0 && threadIdx.x == 0) { DBG_STAMP(11); }
   const int m = blockIdx.x;
   const XT* xr = x + (int64_t)m * K;
   const int64_t groups = K >> 3;
@@ -339,7 +311,6 @@ __global__ void __launch_bounds__(1024) split_rows_kernel(const XT* x, int8_t* _
     __syncthreads();
     for (int b = threadIdx.x; b < blocks; b += blockDim.x) xs[(int64_t)b * xs_pitch + m] = (float)((long long)s_hi[b] * 65536 + s_lo[b]);
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) { DBG_STAMP(12); }
 }
 
 // ---- int4 -> int8 once, for long batches ----
@@ -499,14 +470,6 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int warp = ptx::warp_index(), lane = threadIdx.x & 31;
-#ifdef QMM_LIMB_DBG
-  const long long dbg_k0 = clock64();
-  const unsigned long long dbg_g0 = ptx::globaltimer_ns();
-#endif
-  if (threadIdx.x == 0) { DBG_STAMP(0); }
-#ifdef QMM_LIMB_DBG
-  if (threadIdx.x == 0 && blockIdx.x < 512) g_limb_cta[4 * blockIdx.x] = (long long)ptx::globaltimer_ns();
-#endif
   // accumulators per hand-over and hand-over buffers in the TMEM ring
   const int gph = (p.mode == kBlock128 && C::kPair) ? 2 : 1;
   const int nacc = min(kMaxAcc, C::kRegions / gph);
@@ -539,7 +502,6 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
   __syncthreads();
   ptx::tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if (threadIdx.x == 0) { DBG_STAMP(1); }
   // The next kernel of the stream may start its own set-up now; it touches nothing of ours before its own wait.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
@@ -548,48 +510,38 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
     if (lane == 0) {
       if (p.w_dep) asm volatile("griddepcontrol.wait;" ::: "memory");
       FragIter it(p);
-      DBG_DECL;
       int tile, u0, u1, slot = 0;
       uint32_t ph = 0;
       while (it.next(tile, u0, u1)) {
         const int s0 = u0 * p.spu, s1 = min(p.slots, u1 * p.spu);
         for (int s = s0; s < s1; ++s) {
           if constexpr (WBITS == 8) {
-            DBG_BEGIN();
             ptx::mbar_wait<32>(&empty[slot], ph ^ 1, abort_flag, p.err_word, ptx::kErrWaitEmpty);
-            DBG_END(0);
             uint8_t* dst = slot_base + (size_t)slot * kSlot;
             ptx::mbar_expect_tx(&full[slot], kASlot);
             ptx::tma_load_2d(dst, &map_w, &full[slot], s * kSlotK, tile * BMW);
             ptx::tma_load_2d(dst + kATile, &map_w, &full[slot], s * kSlotK + kTileK, tile * BMW);
             if (++slot == kSlots) { slot = 0; ph ^= 1; }
           } else {
-            DBG_BEGIN();
             ptx::mbar_wait<32>(&raw_empty[slot], ph ^ 1, abort_flag, p.err_word, ptx::kErrWaitEmpty);
-            DBG_END(0);
             ptx::mbar_expect_tx(&raw_full[slot], kRawBytes);
             ptx::tma_load_2d(raw_base + (size_t)slot * kRawBytes, &map_w, &raw_full[slot], s * 128, tile * BMW);
             if (++slot == kRaw) { slot = 0; ph ^= 1; }
           }
         }
       }
-      DBG_FLUSH(0);
     }
   } else if (warp == 2) {
     // ---------------- limb tile producer ----------------
     if (lane == 0) {
       asm volatile("griddepcontrol.wait;" ::: "memory");  // the limbs are written by the kernel before this one
-      DBG_STAMP(2);
       FragIter it(p);
-      DBG_DECL;
       int tile, u0, u1, slot = 0;
       uint32_t ph = 0;
       while (it.next(tile, u0, u1)) {
         const int s0 = u0 * p.spu, s1 = min(p.slots, u1 * p.spu);
         for (int s = s0; s < s1; ++s) {
-          DBG_BEGIN();
           ptx::mbar_wait<32>(&empty[slot], ph ^ 1, abort_flag, p.err_word, ptx::kErrWaitEmpty);
-          DBG_END(0);
           uint8_t* dst = slot_base + (size_t)slot * kSlot + C::kAInSlot;
           ptx::mbar_expect_tx(&full[slot], 2 * kBTile);
           ptx::tma_load_2d(dst, &map_x, &full[slot], s * kSlotK, it.y * (NL * MT));
@@ -597,7 +549,6 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
           if (++slot == kSlots) { slot = 0; ph ^= 1; }
         }
       }
-      DBG_FLUSH(8);
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer: the whole warp walks the loop, one elected thread issues ----------------
@@ -606,7 +557,6 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
     const uint32_t desc_hi = (uint32_t)(ptx::make_sw128_kmajor_desc(0) >> 32);
     const uint32_t lo0 = (uint32_t)ptx::make_sw128_kmajor_desc(ptx::smem_u32(slot_base));
     FragIter it(p);
-    DBG_DECL;
     int tile, u0, u1;
     int slot = 0, buf = 0;
     uint32_t ph = 0, pacc = 0;
@@ -631,28 +581,15 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
     };
     auto issue_tile = [&](uint32_t d, int t, uint32_t accum) { issue_part(d, t, 0, kTileK / UMMA_K, accum); };
     auto wait_acc = [&]() {
-      DBG_BEGIN();
       ptx::mbar_wait(&acc_empty[buf], pacc ^ 1, abort_flag, p.err_word, ptx::kErrWaitTmemEmpty);
-      DBG_END(0);
       ptx::tcgen05_fence_after();
     };
     auto next_acc = [&]() {
       if (leader) ptx::mma_commit(&acc_full[buf]);
       if (++buf == nacc) { buf = 0; pacc ^= 1; }
     };
-    bool dbg_first = true;
-    (void)dbg_first;
     auto wait_slot = [&]() {
-      DBG_BEGIN();
       ptx::mbar_wait(&full[slot], ph, abort_flag, p.err_word, ptx::kErrWaitFull);
-      DBG_END(1);
-      if (dbg_first) {
-        DBG_STAMP(3);
-#ifdef QMM_LIMB_DBG
-        if (lane == 0 && blockIdx.x < 512) g_limb_cta[4 * blockIdx.x + 1] = (long long)ptx::globaltimer_ns();
-#endif
-        dbg_first = false;
-      }
       ptx::tcgen05_fence_after();
     };
     auto next_slot = [&]() {
@@ -712,11 +649,6 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
         }
       }
     }
-    DBG_STAMP(4);
-#ifdef QMM_LIMB_DBG
-    if (lane == 0 && blockIdx.x < 512) g_limb_cta[4 * blockIdx.x + 2] = (long long)ptx::globaltimer_ns();
-#endif
-    DBG_FLUSH(16);
   } else if ((warp >= kDrainWarp0 && warp < kDrainWarp0 + 4) || (C::kHalves == 2 && warp >= C::kXDrainWarp0)) {
     // ---------------- drain: thread = one weight row n (its TMEM lane), all or half of the tile's tokens ----------------
     constexpr int MTD = MT / C::kHalves;                      // tokens per drain thread
@@ -726,14 +658,12 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
     constexpr int kDT = 128 * C::kHalves;                     // drain threads
     const bool small = p.mode == kBlock128 || p.mode == kBlock64 || (p.mode == kBlockSlots && p.spu == 1);
     asm volatile("griddepcontrol.wait;" ::: "memory");  // pw, the scratch and `out` belong to earlier kernels until here
-    if (warp == kDrainWarp0) { DBG_STAMP(5); }
     const int quad = warp & 3;
     const int rl = quad * 32 + lane;  // row inside the tile
     const int dt = half ? 128 + (int)threadIdx.x - C::kXDrainWarp0 * 32 : (int)threadIdx.x - kDrainWarp0 * 32;  // 0..kDT-1
     auto drain_bar = [&]() { asm volatile("bar.sync 1, %0;" ::"n"(kDT) : "memory"); };
     const uint32_t lane_addr = tmem_base + ((uint32_t)(quad * 32) << 16);
     FragIter it(p);
-    DBG_DECL;
     int tile, u0, u1, buf = 0;
     uint32_t pacc = 0;
     __shared__ int s_npart;
@@ -749,9 +679,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
     // that way, 180 this way).
     auto arrived = [&](uint32_t w) { return W16 ? value(w) : __uint_as_float(__byte_perm(w, 0u, p.as_is)); };
     auto wait_acc = [&]() {
-      DBG_BEGIN();
       ptx::mbar_wait_warp<32>(&acc_full[buf], pacc, abort_flag, p.err_word, ptx::kErrWaitTmemFull);
-      DBG_END(0);
       ptx::tcgen05_fence_after();
     };
     auto release = [&]() {
@@ -899,7 +827,6 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
             const uint32_t nx0 = fetch_scale(2 * s + 2), nx1 = fetch_scale(2 * s + 3);
             if (C::kPair) {
               wait_acc();
-              DBG_BEGIN();
               const uint32_t a = lane_addr + buf * (2 * NCOLS) + col0;
               if constexpr (C::kPipeDrain) {
                 fold_regions_pipelined<DC, MTD, NL, true, 2>(a, NCOLS, sc2, total, release);
@@ -907,20 +834,17 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
                 fold_region<DC, MTD, NL, true>(a, sc2[0], total, false, release);
                 fold_region<DC, MTD, NL, true>(a + NCOLS, sc2[1], total, true, release);
               }
-              DBG_END(1);
               next_acc();
             } else {
 #pragma unroll 1
               for (int h = 0; h < 2; ++h) {
                 wait_acc();
-                DBG_BEGIN();
                 const float sc1[1] = {h ? sc2[1] : sc2[0]};
                 if constexpr (C::kPipeDrain) {
                   fold_regions_pipelined<DC, MTD, NL, true, 1>(lane_addr + buf * NCOLS + col0, 0, sc1, total, release);
                 } else {
                   fold_region<DC, MTD, NL, true>(lane_addr + buf * NCOLS + col0, sc1[0], total, true, release);
                 }
-                DBG_END(1);
                 next_acc();
               }
             }
@@ -937,7 +861,6 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
           const int g_end = s + per;
           const uint32_t nx = p.mode == kPerChannel ? 0u : fetch_scale(++b);
           wait_acc();
-          DBG_BEGIN();
           if constexpr (C::kPipeDrain) {
             const float sc1[1] = {sc};
             if (small) fold_regions_pipelined<DC, MTD, NL, true, 1>(lane_addr + buf * NCOLS + col0, 0, sc1, total, release);
@@ -946,41 +869,31 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
             if (small) fold_region<DC, MTD, NL, true>(lane_addr + buf * NCOLS + col0, sc, total, true, release);
             else fold_region<DC, MTD, NL, false>(lane_addr + buf * NCOLS + col0, sc, total, true, release);
           }
-          DBG_END(1);
           next_acc();
           s = g_end;
           if (p.mode != kPerChannel) sc = arrived(nx);
         }
       }
-      DBG_BEGIN();
       // ---- end of the fragment ----
       if (!first) {
         // a later K range of a tile that another CTA started: leave the partial sums for that CTA
         float* dst = p.partial + ((size_t)place * MT + half * MTD) * BMW + rl;
-        if (warp == kDrainWarp0) { DBG_STAMP1(18); }
         lost();
 #pragma unroll
         for (int t = 0; t < MTD; ++t)
           if (t < mcount) __stcg(dst + t * BMW, total[t]);
-        if (warp == kDrainWarp0) { DBG_STAMP1(19); }
         // the barrier orders every drain thread's stores before thread 0's fence, which is cumulative
         drain_bar();
-        if (warp == kDrainWarp0) { DBG_STAMP1(20); }
         if (dt == 0) ptx::partial_publish(p.flags + place);
-        if (warp == kDrainWarp0) { DBG_STAMP1(21); }
-        DBG_END(2);
         continue;
       }
-      if (warp == kDrainWarp0) { DBG_STAMP(14); }
       if (!last) {
         // add the partial sums of the CTAs that continue the tile, in CTA order
         for (int j = dt; j < np; j += kDT) {
           ptx::partial_wait(p.flags + place + 1 + j, p.wait_cycles, abort_flag, p.err_word, kErrPartialWait);
         }
         drain_bar();
-        if (warp == kDrainWarp0) { DBG_STAMP(15); }
         add_partials();
-        if (warp == kDrainWarp0) { DBG_STAMP(16); }
       }
       drain_bar();  // the factors written at the top of the fragment are visible
       lost();
@@ -1029,10 +942,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
             store_from_f32(p.out, (int64_t)(p.m0 + mt0 + t) * (p.ld >> 1) + gate_up_column(n), p.out_dt, silu_mul(v, u));
         }
       }
-      DBG_END(2);
     }
-    if (warp == kDrainWarp0) { DBG_STAMP(6); }
-    if (warp == kDrainWarp0) { DBG_FLUSH(24); }
   } else if (WBITS == 4 && warp >= kConvWarp0 && warp < kConvWarp0 + 4 * C::kGroups) {
     // ---------------- int4: nibble -> high half of a byte (value * 16 as int8); lane = row ----------------
     // Two groups of four warps; group g expands the slots g, g+2, ... of the CTA's sequence (ring depths are even,
@@ -1043,7 +953,6 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
     const uint32_t raw_row = ptx::smem_u32(raw_base) + r * 128;
     const uint32_t a_row = ptx::smem_u32(slot_base) + r * 128;
     FragIter it(p);
-    DBG_DECL;
     int tile, u0, u1;
     uint32_t i = 0;  // position in the CTA's slot sequence
     while (it.next(tile, u0, u1)) {
@@ -1051,15 +960,11 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
       for (int s = s0; s < s1; ++s, ++i) {
         if (C::kGroups == 2 && (int)(i & 1) != grp) continue;
         const uint32_t sr = i % kRaw, pr = (i / kRaw) & 1, sa = i % kSlots, pa = (i / kSlots) & 1;
-        DBG_BEGIN();
         ptx::mbar_wait_warp<32>(&raw_full[sr], pr, abort_flag, p.err_word, ptx::kErrWaitRaw);
-        DBG_END(0);
         uint4 v[8];
 #pragma unroll
         for (int c = 0; c < 8; ++c) v[c] = lds128(raw_row + sr * kRawBytes + (((uint32_t)c ^ sw) << 4));
-        DBG_BEGIN();
         ptx::mbar_wait_warp<32>(&empty[sa], pa ^ 1, abort_flag, p.err_word, ptx::kErrWaitEmpty);
-        DBG_END(1);
         if constexpr (C::kATmem) {
           ptx::tcgen05_fence_after();  // the MMAs that read this TMEM slot last have completed (their commit freed it)
           const uint32_t t_row = tmem_base + ((uint32_t)(cw * 32) << 16) + C::kATmemCol0 + sa * C::kATmemSlotCols;
@@ -1093,21 +998,10 @@ __global__ void __launch_bounds__(Cfg<WBITS, NCOLS, NL>::kThreads, Cfg<WBITS, NC
         }
       }
     }
-    if (warp == kConvWarp0) { DBG_FLUSH(32); }
   }
 
   ptx::tcgen05_fence_before();
   __syncthreads();
-#ifdef QMM_LIMB_DBG
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    g_limb_dbg[40] = clock64() - dbg_k0;
-    g_limb_dbg[41] = (long long)(ptx::globaltimer_ns() - dbg_g0);
-    DBG_STAMP(7);
-  }
-  if (threadIdx.x == 0 && blockIdx.x < 512) {
-    g_limb_cta[4 * blockIdx.x + 3] = (long long)ptx::globaltimer_ns();
-  }
-#endif
   if (warp == 1) {
     ptx::tcgen05_fence_after();
     ptx::tmem_dealloc(tmem_base, C::kTmemCols);
@@ -1568,37 +1462,3 @@ size_t limb_tc_wide_bytes(int wbits, int64_t M, int64_t N, int64_t K) {
 }
 
 }  // namespace qmm
-
-#ifdef QMM_LIMB_DBG
-extern "C" __attribute__((visibility("default"))) void qmm_debug_limb_dump() {
-  cudaDeviceSynchronize();
-  long long h[64];
-  cudaMemcpyFromSymbol(h, qmm::g_limb_dbg, sizeof(h));
-  const char* names[5] = {"wprod", "bprod", "mma", "drain", "conv"};
-  for (int r = 0; r < 5; ++r)
-    fprintf(stderr, "[dbg] %-6s w0=%lld w1=%lld w2=%lld w3=%lld total=%lld\n", names[r], h[8 * r], h[8 * r + 1], h[8 * r + 2],
-            h[8 * r + 3], h[8 * r + 4]);
-  fprintf(stderr, "[dbg] timeline (us after entry): setup %.2f | prev-kernel-done(B) %.2f | first slot full %.2f | MMAs issued %.2f | drain start %.2f | drain end %.2f | exit %.2f || split: entry %.2f wait-done %.2f end %.2f\n",
-          (h[43] - h[42]) * 1e-3, (h[44] - h[42]) * 1e-3, (h[45] - h[42]) * 1e-3, (h[46] - h[42]) * 1e-3, (h[47] - h[42]) * 1e-3,
-          (h[48] - h[42]) * 1e-3, (h[49] - h[42]) * 1e-3, (h[52] - h[42]) * 1e-3, (h[53] - h[42]) * 1e-3, (h[54] - h[42]) * 1e-3);
-  {
-    static long long c[4 * 512];
-    cudaMemcpyFromSymbol(c, qmm::g_limb_cta, sizeof(c));
-    long long t0 = 0;
-    int n = 0;
-    for (int i = 0; i < 512; ++i)
-      if (c[4 * i + 3] > 0) { ++n; if (t0 == 0 || c[4 * i] < t0) t0 = c[4 * i]; }
-    fprintf(stderr, "[dbg] per-CTA (us after the first entry): cta entry first-full mma-issued exit\n");
-    for (int i = 0; i < n; i += (n > 40 ? n / 20 : 1))
-      fprintf(stderr, "[dbg]   %3d %7.2f %7.2f %7.2f %7.2f\n", i, (c[4 * i] - t0) * 1e-3, (c[4 * i + 1] - t0) * 1e-3, (c[4 * i + 2] - t0) * 1e-3,
-              (c[4 * i + 3] - t0) * 1e-3);
-    double mx = 0, mxe = 0;
-    for (int i = 0; i < n; ++i) { mx = std::max(mx, (c[4 * i + 3] - t0) * 1e-3); mxe = std::max(mxe, (c[4 * i] - t0) * 1e-3); }
-    fprintf(stderr, "[dbg]   %d CTAs, last entry %.2f, last exit %.2f\n", n, mxe, mx);
-  }
-  fprintf(stderr, "[dbg] exchange (us after CTA 0's entry): owner CTA 0: K loop folded %.2f | flags seen %.2f | partials added %.2f | stored %.2f || CTA 1: partial ready %.2f | stored %.2f | fenced %.2f | flag set %.2f\n",
-          (h[56] - h[42]) * 1e-3, (h[57] - h[42]) * 1e-3, (h[58] - h[42]) * 1e-3, (h[48] - h[42]) * 1e-3, (h[60] - h[42]) * 1e-3,
-          (h[61] - h[42]) * 1e-3, (h[62] - h[42]) * 1e-3, (h[63] - h[42]) * 1e-3);
-  fprintf(stderr, "[dbg] kernel  cycles=%lld ns=%lld -> %.3f GHz\n", h[40], h[41], h[41] ? (double)h[40] / (double)h[41] : 0.0);
-}
-#endif
