@@ -344,7 +344,8 @@ __global__ void __launch_bounds__(Cfg<WBITS, NC, KS, SUB>::kThreads, 1)
     const int quad = warp & 3, grp = (warp - 4) >> 2;
     const uint32_t r = quad * 32 + lane;
     constexpr int kTeams = C::kTeams, kTV = C::kTV, kVV = C::kVV;
-    constexpr int kWords = kVV / 2 < 32 ? kVV / 2 : 32; // words of converted pairs per tensor-memory store
+    constexpr int kWords = 32;                          // words of converted pairs per tensor-memory store
+    static_assert(kVV / 2 % kWords == 0, "whole stores");
     constexpr int kPieces = kWords * 2 * WBITS / 128;   // the 16-byte pieces of a row that make them
     const uint32_t done_a = ptx::smem_u32(done), a_full_a = ptx::smem_u32(a_full);
     const int team = grp / C::kTeamGroups, part = grp % C::kTeamGroups;
@@ -386,8 +387,7 @@ __global__ void __launch_bounds__(Cfg<WBITS, NC, KS, SUB>::kThreads, 1)
             ptx::bar_wait(done_a + (s - kASlots) % kDone * 8, (s - kASlots) / kDone & 1, abort_flag, p.err_word, ptx::kErrWaitEmpty);
           ptx::tcgen05_fence_after();
         }
-        if constexpr (kWords == 32) ptx::tmem_st_32x32b_x32(ts + 32 * h, o);
-        else ptx::tmem_st_32x32b_x16(ts, o);
+        ptx::tmem_st_32x32b_x32(ts + 32 * h, o);
       }
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive_a(raw_empty_a + rs);
@@ -556,12 +556,9 @@ __global__ void __launch_bounds__(Cfg<WBITS, NC, KS, SUB>::kThreads, 1)
           constexpr int CH = C::kCh, NB = C::kChBufs, kChunks = DT / CH;
           uint32_t r[NB][CH];
           auto load = [&](uint32_t at, uint32_t* to) {
+            static_assert(CH == 16 || CH == 32, "columns of a load");
             if constexpr (CH == 16) ptx::tmem_ld_32x32b_x16(at, to);
-            else if constexpr (CH == 32) ptx::tmem_ld_32x32b_x32(at, to);
-            else {
-              ptx::tmem_ld_32x32b_x16(at, to);
-              ptx::tmem_ld_32x32b_x8(at + 16, to + 16);
-            }
+            else ptx::tmem_ld_32x32b_x32(at, to);
           };
           auto add = [&](const uint32_t* from, float s, float* to) {
 #pragma unroll
