@@ -43,3 +43,18 @@ def test_choice(wbits, bs, zp, M, N, K, kernel):
   assert chosen(wbits, bs, zp, M, N, K) == kernel
   call, exact = call_and_exact(wbits, bs, zp, M, N, K, torch.bfloat16)
   assert qo.max_abs_rel(call(), exact) < 1e-2  # one rounding to bf16
+
+
+@pytest.mark.parametrize("wbits,M,N,K,kernel", [
+    (4, 128, 1024, 4096, "i8tc"), (4, 128, 1024, 8192, "tmem"), (4, 1008, 256, 512, "i8tc"), (4, 1009, 256, 512, "tmem"),
+    (4, 84, 7168, 2048, "i8tc"), (4, 85, 7168, 2048, "tmem"), (4, 85, 7168, 1984, "i8tc"), (4, 200, 4096, 768, "tmem"),
+    (8, 445, 2970, 1792, "i8tc"), (8, 445, 2970, 4096, "tmem"), (8, 1009, 2970, 1792, "tmem"), (8, 1009, 4112, 512, "i8tc"),
+    (4, 8, 21601, 2208, "tmem"), (4, 5, 21601, 2208, "i8mma"), (8, 8, 21601, 2208, "tmem"), (8, 2, 14336, 4096, "i8mma"), (4, 8, 16384, 8192, "i8tc"),
+])
+def test_zero_points_per_channel(wbits, M, N, K, kernel):
+  """Each line from both sides: few tokens, few items, long rows, more tokens than a launch of the split-activation kernel."""
+  assert chosen(wbits, -1, True, M, N, K) == kernel
+  for out_dtype, tol in ((torch.bfloat16, 1e-2), (torch.float32, 1e-5)):
+    call, exact = call_and_exact(wbits, -1, True, M, N, K, out_dtype)
+    # fp32: exact products or 2^-22 of the row's largest activation; sums of at most 512 products, then of those
+    assert qo.max_abs_rel(call(), exact) < tol

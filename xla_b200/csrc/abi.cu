@@ -219,10 +219,17 @@ static bool zp_decode_on_tc(int wbits, int64_t M, int64_t N, int64_t K, bool dec
 // Where AUTO takes the tensor-memory kernel (16-bit activations).
 //   zero points    with scale blocks wherever a tensor-core kernel is taken: it applies them in the drain it runs anyway (int4
 //                  block 128 [37888,3584] at 29 tokens 32 us against 59 on the split-activation kernel, [14336,4096] at 512: 106
-//                  against 211).  Per channel the other kernel hands over once per tile: int8 up to 64 tokens on fewer
-//                  than 12288 outputs from 33 tokens ([4096,4096] at 64 tokens 20 us, 16 there; [14336,4096] 21, 25 there), large
-//                  int4 weights up to its 42 tokens ([28672,8192] at 16 tokens 37 us, 31 there), all up to eight tokens
-//                  ([8192,28672] 50, 37 there), and above 64 tokens with fewer than 64 items of 128 rows and 192 tokens.
+//                  against 211).  Per channel the other kernel hands over once per tile, and the products are exact here but fp32
+//                  sums of int8 ones are a little further off (2.5e-7 of the results against 1.2e-7; int4 8e-8 and 1.2e-7).  So
+//                  2..8     here, but int8 with fp32 results and int4 from 2^27 values there: int4 [21601,2208] at eight tokens 14.8 us,
+//                           18.4 there and 15.2 on the integer decode kernel, [8192,8192] at six 14.5, 18.9 there; [28672,8192] 33.6, 29.4
+//                  9..32    here, but int4 from 2^25 values (to 42 tokens, a tile there: [28672,8192] at 16 37 us, 31 there)
+//                  33..64   int4 here; int8 from 12288 outputs ([14336,4096] at 64 16 us, 18 there; [2970,1792] 10.4, 9.9 there)
+//                  above    from 64 items of 128 rows and 192 tokens on, int8 only with long rows or narrow beyond one launch there
+//                           ([8192,2048] at 445 36 us, 25 there, [28672,2048] 81, 62; [4096,14336] 62, 73; [2970,1792] at 1024 24, 31).  Fewer
+//                           items: int4 with long rows, more items than SMs there (of 42 tokens), or more than one launch: [4096,14336] at
+//                           128 32 us, 38 there, [8064,7168] 28, 38, [7168,2048] at 100 16, 19, [1024,512] at 1024 15, 21; else there where
+//                           the result has 16 bits ([1024,4096] at 128 20, 17 there, [4096,4096] 21, 18)
 //   blocks of 64   above 32 tokens always: the other kernel that goes on with them there, tcgen05, has 64 tokens a pass (int4 [3584,20416] at
 //                  114 tokens 44 us against 104, int8 [1280,11328] at 1143 59 against 172, [512,960] at 35 7.3 against 10).  Not up to eight (int8
 //                  [8192,7424] at six tokens 19.5 us, 14.4 on the decode kernel).
@@ -252,8 +259,10 @@ static bool use_tmem(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, int
   if (has_zp) {
     if (blocked) return zp_decode_on_tc(wbits, M, N, K, decode_i8);
     if (!limb_tc_shape_ok(wbits, M, N, K, bs, x_dt, true)) return zp_decode_on_tc(wbits, M, N, K, decode_i8);
-    if (M <= 8) return false;
-    if (M > 64) return items >= 64;
+    if (M <= 8) return (wbits == 4 ? E < 1 << 27 : out_dt != QMM_F32) && zp_decode_on_tc(wbits, M, N, K, decode_i8);
+    if (M > 64 && wbits == 8) return items >= 64 && (K >= 4096 || (M > 1008 && N <= 4096));
+    if (M > 64)
+      return items >= 64 || out_dt == QMM_F32 || K >= 8192 || M > 1008 || (K >= 2048 && ceil_div(N, 128) * ceil_div(M, 42) > sm_count());
     return wbits == 4 ? M > 42 || E < 1 << 25 : M <= 32 || N >= 12288;
   }
   if (M == 1) return false;
@@ -277,12 +286,13 @@ static bool use_tmem(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, int
   return filled || (items >= 64 && E >= 1 << 25);
 }
 
-// Where AUTO takes the split-activation kernel ahead of the decode kernels, at two to eight tokens: zero points per channel (see
-// above), and weights of 100 MB without (int4 block 128 [57344,8192] at two tokens 46 us against 54, at five 47 against 65;
-// int8 [28672,8192] 41 against 48).
+// Where AUTO takes the split-activation kernel ahead of the decode kernels: zero points per channel at two to eight tokens (see
+// above; not on short rows where the integer decode kernel goes: int8 [21601,2208] at eight 18.0 us, 16.0 there), and weights of 100 MB
+// without at two to sixteen (int4 block 128 [57344,8192] at two tokens 46 us against 54, at five 47 against 65; int8 [28672,8192] 41
+// against 48).
 static bool use_limb_decode(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, int x_dt, bool has_zp, bool decode_i8) {
   if (M < 2 || M > 16 || x_dt == QMM_F32 || bs == 64 || !limb_tc_shape_ok(wbits, M, N, K, bs, x_dt, has_zp)) return false;
-  if (has_zp) return M <= 8 && bs <= 0 && zp_decode_on_tc(wbits, M, N, K, decode_i8);
+  if (has_zp) return M <= 8 && bs <= 0 && (!decode_i8 || K >= 3072) && zp_decode_on_tc(wbits, M, N, K, decode_i8);
   return N * K * wbits / 8 >= 100000000;
 }
 
