@@ -238,13 +238,14 @@ static bool zp_decode_on_tc(int wbits, int64_t M, int64_t N, int64_t K, bool dec
 //                  against 312, [2432,9248] at 763 tokens 49 against 74).
 //   2..8 tokens    int8 on large weights: block 128 [28672,8192] at two tokens 44 us against 50, [14336,4096] at four 15 against
 //                  17 (per channel 14 against 16).
-//   9..32 tokens   weights of 34 million values, 2^24 from 17 tokens, any for int8 from 17: int4 block 128 [14336,4096] at 16 tokens
-//                  14.3 us against 18.4, [4096,4096] at 24 11.4 against 12.2 (at 16 11.6 against 10.3); int8 per channel
-//                  [1024,4096] at 32 8.8 against 11.  Not per channel from 2^27 values, where i8tc streams faster (int4
-//                  [28672,8192] 34 against 30), nor int4 blocks there up to ten tokens (40 against 31).
-//   33..64 tokens  int4, int8 blocks, int8 per channel below 2^26.5 values: int4 block 128 [57344,8192] at 64 tokens 87 us
+//   9..32 tokens   weights of 34 million values, 2^24 in int8 blocks and from 17 tokens, 2^22 for int8 from 17: int4 block 128
+//                  [14336,4096] at 16 tokens 14.3 us against 18.4, [4096,4096] at 24 11.4 against 12.2 (at 16 11.6 against 10.3); int8
+//                  per channel [1024,4096] at 32 8.8 against 11.  From 2^27 values not int4 per channel, nor int8 from 2^28, where i8tc
+//                  streams faster (int4 [28672,8192] 32 against 30), nor int4 blocks up to ten tokens (40 against 31).
+//   33..64 tokens  from 2^22 values int4, int8 blocks, and int8 per channel below 95 million: int4 block 128 [57344,8192] at 64 tokens 87 us
 //                  against 104, [4096,4096] 15 against 16.5; int8 [5120,6912] 17 against 22, [28672,8192] 55 against 51.
-//   above 64       int4 and int8 blocks, when the items fill half of the SMs, or 64 of them on weights of 2^25 values: fewer
+//   above 64       int4 and int8 blocks, when the items fill half of the SMs (also with short K: [9728,1024] block 128 at 128 tokens 11 us
+//                  against 15 for int8 and 17 for int4, [9728,512] 9 against 13 and 14), or 64 of them on weights of 2^25 values: fewer
 //                  leave it to i8tc's narrower ones ([4096,4096] at 128 tokens 26 us against 19; [14336,4096] at 96 25
 //                  against 34, [5120,6912] at 256 33 against 51, [28672,8192] at 512 230 against 337).  int4 per channel from 384
 //                  tokens, where i8tc expands the weights once, on 2^25 values ([4096,4096] at 1024 50 us against 38; [5120,6912] at
