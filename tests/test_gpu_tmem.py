@@ -154,3 +154,42 @@ def test_folds_of_several_steps(wbits, bs, N, K, M):
   S = 1 if bs == -1 else K // bs
   exact = torch.einsum("msk,nsk,sn->mn", x.double().view(M, S, -1), w.double().view(N, S, -1), s.double().view(S, N))
   assert qo.max_abs_rel(out, exact) < 1e-5  # exact products, a rounding per block and per 512 values
+
+
+GATE_UP_ROUTES = [
+    # from 100 MB at two to sixteen tokens: the split-activation kernel's narrow instances, of 16, 32 and 48 columns
+    (4, 128, 2, 57344, 4096, "i8tc"), (4, 128, 5, 57344, 4096, "i8tc"), (4, 128, 6, 57344, 4096, "i8tc"), (4, 128, 10, 57344, 4096, "i8tc"),
+    (8, -1, 16, 28672, 4096, "i8tc"), (4, -1, 13, 57344, 4096, "i8tc"),
+    # scale blocks that are a multiple of 128, but not of 256
+    (4, 384, 9, 14336, 4224, "tmem"), (8, 384, 4, 14336, 4224, "tmem"),
+]
+LARGE_GATE_UP = """
+import sys, torch, xla_b200
+from xla_b200 import _capi
+wbits, bs, M, N2, K = map(int, sys.argv[1:])
+g = torch.Generator(device="cuda:0").manual_seed(M)
+w = torch.randint(0, 256, (N2, K * wbits // 8), generator=g, device="cuda:0", dtype=torch.uint8)
+w = w if wbits == 4 else w.view(torch.int8)
+s = (torch.rand((N2,) if bs == -1 else (K // bs, N2), generator=g, device="cuda:0") + 0.5) / (4.6 if wbits == 4 else 73.) / K**0.5
+x = torch.randn(M, K, generator=g, device="cuda:0").bfloat16()
+kw = dict(block_size=bs, int4_weight=wbits == 4, weight_is_packed=wbits == 4)
+out = torch.ops.xla_b200.quantized_gate_up(x, w, s, out_dtype=torch.float32, **kw)
+with xla_b200.force_variant("generic"):
+  y = torch.ops.xla_b200.quantized_matmul_packed(x, w, s, None, out_dtype=torch.float32, **kw).view(M, N2 // 16, 2, 8).double()
+ref = (torch.nn.functional.silu(y[:, :, 0]) * y[:, :, 1]).reshape(M, N2 // 2)
+print("error", float((out - ref).abs().max() / ref.abs().max()))
+"""
+
+
+@pytest.mark.parametrize("wbits,bs,M,N2,K,kernel", GATE_UP_ROUTES)
+def test_gate_up_takes_the_kernel_it_asked_for(wbits, bs, M, N2, K, kernel):
+  """The kernel by the library's log, in a process of its own, and the result against the any-shape kernel's two projections."""
+  import os
+  import subprocess
+  import sys
+  r = subprocess.run([sys.executable, "-c", LARGE_GATE_UP] + [str(v) for v in (wbits, bs, M, N2, K)], text=True, capture_output=True,
+                     env=dict(os.environ, QMM_B200_LOG="1"), timeout=300, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+  assert r.returncode == 0, r.stderr[-2000:]
+  assert f"gate_up M={M} N={N2} K={K} -> {kernel}\n" in r.stderr, r.stderr[-500:]
+  # exact products or three limbs: a rounding per block and K ones of the fp32 sums on either side, 2^-24 each at random
+  assert float(r.stdout.split()[-1]) < 1e-5

@@ -265,10 +265,11 @@ Tensor quantized_gate_up(const Tensor& x, const Tensor& w, const Tensor& scale, 
     const bool tc = M > 32 || (tl_variant == QMM_VARIANT_AUTO && half && dtype_code(dt) >= 0 &&
                                qmm_gate_up_on_tensor_cores(wbits, dtype_code(x.scalar_type()), dtype_code(dt), M, w.size(0), K,
                                                            block_size == -1 ? 0 : block_size));
+    // (up to 32 tokens `tc` has asked for the shape, scale blocks of any multiple of 128 among them)
     const bool decode = !tc && half && K % (512 / wbits) == 0 && (block_size == -1 || block_size % (512 / wbits) == 0) &&
                         (tl_variant == QMM_VARIANT_AUTO || tl_variant == QMM_VARIANT_MMA);
     const bool batch = tc && K >= 128 && K % (128 / wbits) == 0 &&
-                       (block_size == -1 || block_size == 128 || block_size % 256 == 0 || (M <= 32 && block_size == 64)) &&
+                       (M <= 32 || block_size == -1 || block_size == 128 || block_size % 256 == 0) &&
                        (tl_variant == QMM_VARIANT_AUTO || tl_variant == QMM_VARIANT_I8TC);
     if (dtype_code(dt) >= 0 && (decode || batch)) {
       c10::cuda::OptionalCUDAGuard guard(x.device());
