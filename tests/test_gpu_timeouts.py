@@ -121,3 +121,35 @@ def test_partial_sums_that_never_come(short_wait, variant, code, wbits, bs, M):
   assert torch.equal(lost[~torch.isnan(lost)], want[~torch.isnan(lost)])
   ws[:2048].zero_()
   assert torch.equal(run(), want) and _capi.device_error(DEV) == 0
+
+
+@pytest.mark.parametrize("wbits,M,out_dt,dtype", [(8, 128, _capi.F32, torch.float32), (8, 200, _capi.BF16, torch.bfloat16)])
+def test_partial_sums_that_never_come_to_a_pair_of_ctas(short_wait, wbits, M, out_dt, dtype):
+  """The same of the kernel on pairs of CTAs (int8 per channel, long K): items split along K, three limbs and two."""
+  L = short_wait
+  g = torch.Generator(device=DEV).manual_seed(M)
+  N, K = 4096, 14336
+  x = torch.randn(M, K, generator=g, device=DEV).bfloat16()
+  w = torch.randint(-127, 128, (N, K), generator=g, device=DEV, dtype=torch.int8)
+  s = (torch.rand(N, generator=g, device=DEV) + 0.5) / 73 / K**0.5
+  nbytes = L.qmm_weight_only_workspace_size(M, K)
+  ws = torch.zeros(nbytes, dtype=torch.uint8, device=DEV)
+
+  def run():
+    out = torch.zeros(M, N, device=DEV, dtype=dtype)
+    with torch.cuda.device(0):
+      _capi.check(L.qmm_weight_only(wbits, x.data_ptr(), _capi.BF16, w.data_ptr(), s.data_ptr(), None, out.data_ptr(), out_dt, M, N, K,
+                                    0, _capi.VARIANTS["i8tc"], ws.data_ptr(), nbytes, _capi.stream_ptr(DEV)))
+    torch.cuda.synchronize()
+    return out
+
+  want = run()
+  assert _capi.device_error(DEV) == 0 and torch.isfinite(want).all()
+  assert not ws[:2048].any()  # the flags are idle again
+  ws[:2048].view(torch.int32).fill_(7)
+  lost = run()
+  assert _capi.device_error(DEV) & 0xff == 11
+  assert torch.isnan(lost).any()
+  assert torch.equal(lost[~torch.isnan(lost)], want[~torch.isnan(lost)])
+  ws[:2048].zero_()
+  assert torch.equal(run(), want) and _capi.device_error(DEV) == 0
