@@ -38,6 +38,11 @@ def call_and_exact(wbits, bs, zp, M, N, K, out_dtype, dtype=torch.bfloat16):
     (8, 64, False, 1143, 640, 1344, "tmem"), (8, 64, False, 8, 8192, 7424, "mma"), (8, 64, False, 9, 8192, 4160, "tmem"),
     (8, 128, False, 1100, 1024, 1152, "tmem"), (8, 256, False, 1100, 260, 1024, "tmem"), (8, 128, False, 1024, 1024, 1152, "i8tc"),
     (8, -1, False, 1100, 1024, 1040, "tmem"),
+    # int4 blocks of few tokens: from 80 million values, more weight tiles than SMs (18944 outputs), long blocks, and blocks that i8tc leaves
+    (4, 128, False, 9, 11008, 8192, "i8tc"), (4, 128, False, 10, 8448, 8192, "tmem"), (4, 128, False, 11, 11008, 8192, "tmem"),
+    (4, 128, False, 10, 18945, 3584, "i8tc"), (4, 128, False, 10, 18944, 3584, "tmem"), (4, 256, False, 16, 22016, 3584, "i8tc"),
+    (4, 128, False, 16, 22016, 3584, "tmem"), (4, 256, False, 17, 22016, 3584, "tmem"), (4, 64, False, 9, 33024, 4160, "tmem"),
+    (4, 384, False, 10, 33024, 4224, "tmem"), (4, 64, False, 8, 14336, 4224, "i8mma"),
 ])
 def test_choice(wbits, bs, zp, M, N, K, kernel):
   assert chosen(wbits, bs, zp, M, N, K) == kernel

@@ -160,6 +160,7 @@ GATE_UP_ROUTES = [
     # from 100 MB at two to sixteen tokens: the split-activation kernel's narrow instances, of 16, 32 and 48 columns
     (4, 128, 2, 57344, 4096, "i8tc"), (4, 128, 5, 57344, 4096, "i8tc"), (4, 128, 6, 57344, 4096, "i8tc"), (4, 128, 10, 57344, 4096, "i8tc"),
     (8, -1, 16, 28672, 4096, "i8tc"), (4, -1, 13, 57344, 4096, "i8tc"),
+    (4, 128, 10, 28672, 3072, "i8tc"), (4, 128, 11, 28672, 3072, "tmem"),
     # scale blocks that are a multiple of 128, but not of 256
     (4, 384, 9, 14336, 4224, "tmem"), (8, 384, 4, 14336, 4224, "tmem"),
 ]

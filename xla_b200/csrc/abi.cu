@@ -216,6 +216,15 @@ static bool zp_decode_on_tc(int wbits, int64_t M, int64_t N, int64_t K, bool dec
   return E >= 1 << 25 && (wbits == 8 ? M * E >= 175000000 : M >= 6);
 }
 
+// Batches of nine to sixteen tokens, int4 with scale blocks, that the split-activation kernel has ahead of the tensor-memory one (figures
+// there, under 9..32 tokens).
+static bool int4_blocks_on_limbs(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, int x_dt) {
+  const int64_t E = N * K;
+  if (M <= 8 || M > 16 || wbits != 4 || bs <= 64 || E < 1 << 26 || !limb_tc_shape_ok(wbits, M, N, K, bs, x_dt, false)) return false;
+  const bool rounds = ceil_div(N, 128) > sm_count();
+  return M <= 10 ? E >= 80000000 || rounds : bs >= 256 && rounds && E < 1 << 27;
+}
+
 // Where AUTO takes the tensor-memory kernel (16-bit activations).
 //   zero points    with scale blocks wherever a tensor-core kernel is taken: it applies them in the drain it runs anyway (int4
 //                  block 128 [37888,3584] at 29 tokens 32 us against 59 on the split-activation kernel, [14336,4096] at 512: 106
@@ -241,7 +250,11 @@ static bool zp_decode_on_tc(int wbits, int64_t M, int64_t N, int64_t K, bool dec
 //   9..32 tokens   weights of 34 million values, 2^24 in int8 blocks and from 17 tokens, 2^22 for int8 from 17: int4 block 128
 //                  [14336,4096] at 16 tokens 14.3 us against 18.4, [4096,4096] at 24 11.4 against 12.2 (at 16 11.6 against 10.3); int8
 //                  per channel [1024,4096] at 32 8.8 against 11.  From 2^27 values not int4 per channel, nor int8 from 2^28, where i8tc
-//                  streams faster (int4 [28672,8192] 32 against 30), nor int4 blocks up to ten tokens (40 against 31).
+//                  streams faster (int4 [28672,8192] 32 against 30).  Nor int4 blocks where i8tc takes them, from 2^26 values on: up to ten
+//                  tokens from 80 million or with more weight tiles than SMs ([28672,8192] 40 against 31, block 128 [29741,3072] 18.6 against
+//                  13.9, [11008,8192] 18.7 against 17.4; [8192,8192] 15.1 against 15.6), up to sixteen such tiles with long blocks (block 256
+//                  [29741,3072] at 12 16.9 against 14.9; block 128 18.6 against 19.5).  i8tc leaves blocks of 64 and 384
+//                  to the others: [39078,4288] block 64 at ten 43 against 81 on tcgen05, [57344,7680] block 384 at nine 70 against 122 on mma.
 //   33..64 tokens  from 2^22 values int4, int8 blocks, and int8 per channel below 95 million: int4 block 128 [57344,8192] at 64 tokens 87 us
 //                  against 104, [4096,4096] 15 against 16.5; int8 [5120,6912] 17 against 22, [28672,8192] 55 against 51.
 //   above 64       int4 and int8 blocks, when the items fill half of the SMs (also with short K: [9728,1024] block 128 at 128 tokens 11 us
@@ -271,8 +284,9 @@ static bool use_tmem(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, int
   if (M <= 64) {
     if (out_dt == QMM_F32 && !blocked) return false;
     if (M > 32) return E >= 1 << 22 && (wbits == 4 || blocked || E < 95000000);
+    if (int4_blocks_on_limbs(wbits, M, N, K, bs, x_dt)) return false;
     if (E >= 1 << 27) {
-      if (blocked) return wbits == 8 || M > 10;
+      if (blocked) return wbits == 8 || M > 8;
       return wbits == 8 && E < 1 << 28;
     }
     if (M > 16) return E >= (wbits == 8 ? 1 << 22 : 1 << 24);
@@ -590,7 +604,8 @@ int qmm_gate_up_on_tensor_cores(int wbits, int x_dtype, int out_dtype, int64_t M
   if (M > 32) return 1;
   if (wbits != 4 && wbits != 8) return 0;
   block_size = std::max<int64_t>(block_size, 0);
-  return use_tmem(wbits, M, N2, K, block_size, x_dtype, out_dtype, false, false) || use_limb_decode(wbits, M, N2, K, block_size, x_dtype, false, false);
+  return use_tmem(wbits, M, N2, K, block_size, x_dtype, out_dtype, false, false) || use_limb_decode(wbits, M, N2, K, block_size, x_dtype, false, false) ||
+         (x_dtype != QMM_F32 && int4_blocks_on_limbs(wbits, M, N2, K, block_size, x_dtype));
 }
 
 int qmm_gate_up(int wbits, const void* x, int x_dtype, const void* w, const float* scale, void* out, int out_dtype, int64_t M,
