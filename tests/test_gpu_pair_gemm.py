@@ -50,7 +50,8 @@ def test_weight_only(M, N, K, zp, x_dt, out_dt):
   assert qo.max_abs_rel(out, exact) < {torch.float32: 1e-5, torch.float16: 3e-3, torch.bfloat16: 1e-2}[out_dt]
 
 
-@pytest.mark.parametrize("M,N,K,zp", [(129, 11008, 384, False), (256, 11008, 384, False), (100, 4096, 12288, False), (92, 5120, 640, True), (128, 5120, 640, True)])
+@pytest.mark.parametrize("M,N,K,zp", [(129, 11008, 384, False), (256, 11008, 384, False), (100, 4096, 12288, False), (92, 5120, 640, True), (128, 5120, 640, True),
+                                       (129, 3584, 12288, False), (129, 3840, 12288, True), (129, 9500, 12288, False)])
 def test_both_sides_of_the_line_between_pairs_and_single_ctas(M, N, K, zp):
   """A round of tiles less on pairs than on single CTAs, and the same number; K long enough to be split."""
   g = torch.Generator(device=DEV).manual_seed(M + N + K)

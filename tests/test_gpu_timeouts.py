@@ -128,7 +128,7 @@ def test_partial_sums_that_never_come_to_a_pair_of_ctas(short_wait, wbits, M, ou
   """The same of the kernel on pairs of CTAs (int8 per channel, long K): items split along K, three limbs and two."""
   L = short_wait
   g = torch.Generator(device=DEV).manual_seed(M)
-  N, K = 4096, 14336
+  N, K = 3072, 14336
   x = torch.randn(M, K, generator=g, device=DEV).bfloat16()
   w = torch.randint(-127, 128, (N, K), generator=g, device=DEV, dtype=torch.int8)
   s = (torch.rand(N, generator=g, device=DEV) + 0.5) / 73 / K**0.5

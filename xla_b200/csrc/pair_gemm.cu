@@ -501,13 +501,14 @@ int pair_gemm_tokens(int nl) { return nl == 3 ? Tile<3>::kTokens : kCols / nl; }
 // here, a little less, with half of the work in it.  So here where that saves a round: int8 [11008,5120] at 256 tokens, 86 items in two
 // rounds against 344 in three, 32 us, 36 there; at 129, 258 in two there as well, 31 and 27; [5120,5120] at 256 (40 items, 160)
 // 21 and 26, at 129 (40, 120) 19.5 and 17.7.  At equal rounds from 12288 inputs on, which are split over K here ([2560,28672] at 256 tokens
-// 46 and 65), and few items from 8192 ([2560,9472] at 128 22.6 and 25.2).  1832 shapes measured on both.
+// 46 and 65), and few items from 8192 ([2560,9472] at 128 22.6 and 25.2); not between 28 items and a round, which split badly ([5839,12288]
+// at 129, 46 items, 37 and 32, with three limbs at 93 40 and 34; [4096,14336] at 150, 32 items, 33.5 and 30.6).
 bool pair_gemm_preferred(int nl, int64_t M, int64_t N, int64_t K) {
   const int64_t items = ceil_div(N, 2 * kRows) * ceil_div(M, pair_gemm_tokens(nl));
   const int64_t there = ceil_div(N, kRows) * ceil_div(M, nl == 3 ? 42 : 64);  // limb_gemm.cu's items
   const int sms = sm_count();
   if (M <= (nl == 3 ? 42 : 64) || items < 16) return false;
-  return ceil_div(items, sms / 2) < ceil_div(there, sms) || K >= 12288 || (K >= 8192 && items < 24);
+  return ceil_div(items, sms / 2) < ceil_div(there, sms) || (K >= 12288 && (items <= 28 || items > sms / 2)) || (K >= 8192 && items < 24);
 }
 
 // W8A8, against w8a8_gemm.cu's 128 x 256 tiles on single CTAs: by rounds of tiles, at 0.31 us a stage here and 0.5 there, and a
