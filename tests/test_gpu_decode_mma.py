@@ -30,7 +30,7 @@ def test_every_weight_value_is_converted_exactly(dtype, wbits, bs, N, M):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("M", [1, 5, 8])
-@pytest.mark.parametrize("bs,N,K", [(128, 2368, 2048), (128, 2368, 2176), (-1, 2369, 2176), (-1, 257, 4096), (384, 2000, 4992), (128, 16, 4224)])
+@pytest.mark.parametrize("bs,N,K", [(128, 2368, 2048), (128, 2368, 2176), (-1, 2369, 2176), (-1, 257, 4096), (384, 2000, 4992), (128, 16, 4224), (-1, 512, 512), (128, 1447, 1792)])
 def test_few_row_tiles(dtype, bs, N, K, M):
   """int4 with a row tile per SM at most (2368 rows on 148) takes its activations a step ahead from 17 steps on: whole numbers again."""
   g = qc.gen(N + K + M)

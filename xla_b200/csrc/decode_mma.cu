@@ -850,12 +850,12 @@ int launch_nt(const void* x, const void* w, const ST* scale, void* out, int out_
                        (int)M, N, K, spb, shift, bw, 0, a, device_error_word());
     }
   } else if (M <= 8) {
-    // int4, a row tile per SM at most, more than a step per warp: the activations a step ahead.  There are registers to spare, and
+    // int4, a row tile per SM at most, more than a step per warp or four tokens: the activations a step ahead.  There are registers to spare, and
     // those keep the next launch's CTAs off the SMs that are in use: with 60 a thread two fit, and as the launch has fewer CTAs than
     // there are places, some SMs get two of it.  M = 7, [2048,4480] block 128: 5.8 us a launch back to back without, 4.0 with it (4.4
     // with the 70 registers of the conversion with a bias); [2048,10240] at one 8.1, 6.4; [1280,27392] at eight 21.4, 15.0.  With
     // another kernel between the launches it is 3 % at 100 steps and even at 20.
-    if (WBITS == 4 && warps >= 16 && tiles <= sms && K / VPS > 16)
+    if (WBITS == 4 && warps >= 16 && tiles <= sms && (K / VPS > 16 || M > 4))
       err = launch_pdl(decode_mma_kernel<WBITS, XT, ST, 1, 1, 16, false, false, WBITS == 4>, (unsigned)tiles, 512, 0, st, xp, wp, scale, out, out_dt,
                        (int)M, N, K, spb, shift, bw, gate_up, ArParams{}, (uint32_t*)nullptr);
     else if (warps >= 16)
