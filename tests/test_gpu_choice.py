@@ -42,6 +42,9 @@ def call_and_exact(wbits, bs, zp, M, N, K, out_dtype, dtype=torch.bfloat16):
     (4, 128, False, 9, 11008, 8192, "i8tc"), (4, 128, False, 10, 8448, 8192, "tmem"), (4, 128, False, 11, 11008, 8192, "tmem"),
     (4, 128, False, 10, 18945, 3584, "i8tc"), (4, 128, False, 10, 18944, 3584, "tmem"), (4, 256, False, 16, 22016, 3584, "i8tc"),
     (4, 128, False, 16, 22016, 3584, "tmem"), (4, 256, False, 17, 22016, 3584, "tmem"), (4, 64, False, 9, 33024, 4160, "tmem"),
+    # zero points at two to eight tokens: blocks of 64, more weight tiles than SMs
+    (4, 64, True, 8, 14336, 4096, "i8mma"), (4, 64, True, 8, 8192, 8192, "tmem"), (4, 128, True, 8, 14336, 4096, "tmem"),
+    (4, 128, True, 8, 25292, 2688, "i8mma"), (8, 128, True, 5, 28672, 2048, "i8mma"), (8, 128, True, 6, 28672, 2048, "tmem"),
     (4, 384, False, 10, 33024, 4224, "tmem"), (4, 64, False, 8, 14336, 4224, "i8mma"),
 ])
 def test_choice(wbits, bs, zp, M, N, K, kernel):

@@ -208,12 +208,17 @@ static bool use_decode_i8(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs
 //                188 at eight, 49 on tmem; int8 per channel [4096,4096] 8 at two, 13 at four, 18 at five, 14 on i8tc, [5120,6912]
 //                14 at two and 22 at three, 17 there; [28672,8192] 31 at two, 43 at five on the integer kernel, 49 on tmem, 185 on the GEMV
 //                from six on.  int8: [14336,4096] 15 us at two and 18 at four, 16 on i8tc.
-static bool zp_decode_on_tc(int wbits, int64_t M, int64_t N, int64_t K, bool decode) {
+//                Where the integer kernel goes, not with scale blocks of 64 ([25292,2688] int4 at seven 22.9 us, 30.1 on tmem; int8
+//                [28672,8192] at four 61.5, 70.6), and with other blocks later where there are more weight tiles than SMs (int4 block 128
+//                [25292,2688] at eight 19.4, 22.1 on tmem, [14336,4096] 18.8, 16.1; int8 [28672,2048] at three 16.8, 18.9, at six 19.7, 19.3).
+static bool zp_decode_on_tc(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, bool decode) {
   const int64_t E = N * K;
   if (M < 2) return false;
   if (M > 8) return true;
   if (!decode) return E >= (M == 2 ? 50000000 : M <= 4 ? 1 << 25 : 1 << 24);
-  return E >= 1 << 25 && (wbits == 8 ? M * E >= 175000000 : M >= 6);
+  if (E < 1 << 25 || bs == 64) return false;
+  const bool rounds = bs > 0 && ceil_div(N, 128) > sm_count();
+  return wbits == 8 ? M * E >= (rounds ? 350000000 : 175000000) : M >= 6 && !rounds;
 }
 
 // Batches of nine to sixteen tokens, int4 with scale blocks, that the split-activation kernel has ahead of the tensor-memory one (figures
@@ -271,9 +276,9 @@ static bool use_tmem(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, int
   const bool blocked = bs > 0;
   const int64_t E = N * K, items = ceil_div(N, 128) * ceil_div(M, 192);
   if (has_zp) {
-    if (blocked) return zp_decode_on_tc(wbits, M, N, K, decode_i8);
-    if (!limb_tc_shape_ok(wbits, M, N, K, bs, x_dt, true)) return zp_decode_on_tc(wbits, M, N, K, decode_i8);
-    if (M <= 8) return (wbits == 4 ? E < 1 << 27 : out_dt != QMM_F32) && zp_decode_on_tc(wbits, M, N, K, decode_i8);
+    if (blocked) return zp_decode_on_tc(wbits, M, N, K, bs, decode_i8);
+    if (!limb_tc_shape_ok(wbits, M, N, K, bs, x_dt, true)) return zp_decode_on_tc(wbits, M, N, K, bs, decode_i8);
+    if (M <= 8) return (wbits == 4 ? E < 1 << 27 : out_dt != QMM_F32) && zp_decode_on_tc(wbits, M, N, K, bs, decode_i8);
     if (M > 64 && wbits == 8) return items >= 64 && (K >= 4096 || (M > 1008 && N <= 4096));
     if (M > 64)
       return items >= 64 || out_dt == QMM_F32 || K >= 8192 || M > 1008 || (K >= 2048 && ceil_div(N, 128) * ceil_div(M, 42) > sm_count());
@@ -307,7 +312,7 @@ static bool use_tmem(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, int
 // against 48).
 static bool use_limb_decode(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, int x_dt, bool has_zp, bool decode_i8) {
   if (M < 2 || M > 16 || x_dt == QMM_F32 || bs == 64 || !limb_tc_shape_ok(wbits, M, N, K, bs, x_dt, has_zp)) return false;
-  if (has_zp) return M <= 8 && bs <= 0 && (!decode_i8 || K >= 3072) && zp_decode_on_tc(wbits, M, N, K, decode_i8);
+  if (has_zp) return M <= 8 && bs <= 0 && (!decode_i8 || K >= 3072) && zp_decode_on_tc(wbits, M, N, K, bs, decode_i8);
   return N * K * wbits / 8 >= 100000000;
 }
 
