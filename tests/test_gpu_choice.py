@@ -45,6 +45,8 @@ def call_and_exact(wbits, bs, zp, M, N, K, out_dtype, dtype=torch.bfloat16):
     # zero points at two to eight tokens: blocks of 64, more weight tiles than SMs
     (4, 64, True, 8, 14336, 4096, "i8mma"), (4, 64, True, 8, 8192, 8192, "tmem"), (4, 128, True, 8, 14336, 4096, "tmem"),
     (4, 128, True, 8, 25292, 2688, "i8mma"), (8, 128, True, 5, 28672, 2048, "i8mma"), (8, 128, True, 6, 28672, 2048, "tmem"),
+    # the split-activation kernel from 100 MB, at two tokens from 115
+    (4, -1, False, 2, 24576, 8192, "i8mma"), (4, -1, False, 3, 24576, 8192, "i8tc"), (4, -1, False, 2, 28672, 8192, "i8tc"),
     (4, 384, False, 10, 33024, 4224, "tmem"), (4, 64, False, 8, 14336, 4224, "i8mma"),
 ])
 def test_choice(wbits, bs, zp, M, N, K, kernel):

@@ -307,13 +307,15 @@ static bool use_tmem(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, int
 }
 
 // Where AUTO takes the split-activation kernel ahead of the decode kernels: zero points per channel at two to eight tokens (see
-// above; not on short rows where the integer decode kernel goes: int8 [21601,2208] at eight 18.0 us, 16.0 there), and weights of 100 MB
-// without at two to sixteen (int4 block 128 [57344,8192] at two tokens 46 us against 54, at five 47 against 65; int8 [28672,8192] 41
-// against 48).
+// above; where the integer decode kernel goes, on long rows and later: int8 [21601,2208] at eight 18.0 us, 16.0 there; [7864,8352] at three
+// 18.2, 16.2 there, [10000,6000] at four even, at five 17.7, 18.7), and weights of 100 MB without at two to sixteen (int4 block 128
+// [57344,8192] at two tokens 46 us against 53, at five 47 against 65; int8 [28672,8192] 41 against 48; at two tokens from 115 MB: int4
+// [49152,4096] 20.8 against 17.8, [28672,8192] even).
 static bool use_limb_decode(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, int x_dt, bool has_zp, bool decode_i8) {
   if (M < 2 || M > 16 || x_dt == QMM_F32 || bs == 64 || !limb_tc_shape_ok(wbits, M, N, K, bs, x_dt, has_zp)) return false;
-  if (has_zp) return M <= 8 && bs <= 0 && (!decode_i8 || K >= 3072) && zp_decode_on_tc(wbits, M, N, K, bs, decode_i8);
-  return N * K * wbits / 8 >= 100000000;
+  if (has_zp && decode_i8 && (K < 3072 || M * N * K < 260000000)) return false;
+  if (has_zp) return M <= 8 && bs <= 0 && zp_decode_on_tc(wbits, M, N, K, bs, decode_i8);
+  return N * K * wbits / 8 >= (M == 2 ? 115000000 : 100000000);
 }
 
 int qmm_w8a16_perchannel(const void* x, int x_dtype, const int8_t* w, const float* scale,
