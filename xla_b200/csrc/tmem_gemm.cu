@@ -19,14 +19,14 @@
 //                 64 tokens) is shared by two groups, one of 128 is a group's own; the groups take the steps in turn
 //   drain         eight warps: thread = weight row, half of the tokens in fp32 registers: tcgen05.ld, scale, add; epilogue
 //
-// What bounds it.  Up to 64 tokens the instructions of the converters and of the hand-overs: about 440 a scheduler and 128
-// values (ten for eight int4 weights, 160 of them), issued in two thirds of the cycles.  A wait for a complete barrier costs a
-// warp about 57 cycles and a dependent instruction 4 to 6, so a lone warp's loop of three waits, sixteen MMAs and a commit takes
-// 1000 cycles: hence two issuers, steps of 256 values with two scale blocks under one hand-over, barriers by address, four
-// groups of converters that wait side by side, and scales a batch at a time.  int4 block 128 [57344,8192]: 29 tokens 121 us
-// with one issuer and steps of 128 values, 74 now; 64 tokens 134 and 87.  Above 128 tokens a step of 128 values takes 1300
-// cycles for 704 of MMAs: instructions again (790 a scheduler: 96 sums a thread), at 1.65 GHz under load.  512 tokens 511 us
-// and 460.
+// What bounds it.  Up to 64 tokens the instructions of the converters and of the hand-overs: 480 to 510 a scheduler and 128
+// values all told (ten for eight int4 weights, 160 of them), issued in 61 to 65 % of the cycles, the tensor pipe busy in 14 to 26 %.
+// A wait for a complete barrier costs a warp about 57 cycles and a dependent instruction 4 to 6, so a lone warp's loop of three
+// waits, sixteen MMAs and a commit takes 1000 cycles: hence two issuers, steps of 256 values with two scale blocks under one
+// hand-over, barriers by address, four groups of converters that wait side by side, and scales a batch at a time.  int4 block 128
+// [57344,8192]: 29 tokens 121 us with one issuer and steps of 128 values, 68 now; 64 tokens 134 and 88.  Above 128 tokens a step
+// of 128 values takes 1300 cycles for 704 of MMAs: instructions again (820 a scheduler: 96 sums a thread; the tensor pipe busy in
+// half of the time), at 1.65 GHz under load.  512 tokens 511 us and 460.
 //
 // Schedule: (weight tile, token tile) items walk the CTAs whole; the items of a partly filled last round (all of them
 // when there are fewer items than SMs) are split along K over several CTAs and summed, in CTA order, from fp32 partial
