@@ -34,8 +34,11 @@ def call_and_exact(wbits, bs, zp, M, N, K, out_dtype, dtype=torch.bfloat16):
 
 
 @pytest.mark.parametrize("wbits,bs,zp,M,N,K,kernel", [
-    (4, 64, False, 33, 512, 960, "tmem"), (8, 64, False, 35, 512, 960, "tmem"), (4, 64, False, 126, 1280, 1472, "tmem"),
-    (8, 64, False, 1143, 640, 1344, "tmem"), (8, 64, False, 8, 8192, 7424, "mma"), (8, 64, False, 9, 8192, 4160, "tmem"),
+    (4, 64, False, 33, 512, 960, "tmem"), (8, 64, False, 64, 512, 960, "tmem"), (4, 64, False, 65, 512, 960, "tcgen05"),
+    (8, 64, False, 576, 512, 19968, "tcgen05"), (8, 64, False, 576, 512, 20032, "tmem"), (4, 64, False, 1152, 512, 8000, "tcgen05"),
+    (4, 64, False, 1152, 512, 8064, "tmem"), (8, 64, False, 1143, 1024, 3392, "tcgen05"), (8, 64, False, 1143, 1024, 3456, "tmem"),
+    (4, 64, False, 256, 1024, 9984, "tcgen05"), (4, 64, False, 256, 1024, 10048, "tmem"),
+    (8, 64, False, 1217, 1024, 1344, "tmem"), (8, 64, False, 8, 8192, 7424, "mma"), (8, 64, False, 9, 8192, 4160, "tmem"),
     (8, 128, False, 1100, 1024, 1152, "tmem"), (8, 256, False, 1100, 260, 1024, "tmem"), (8, 128, False, 1024, 1024, 1152, "i8tc"),
     (8, -1, False, 1100, 1024, 1040, "tmem"),
     # int4 blocks of few tokens: from 80 million values, more weight tiles than SMs (18944 outputs), long blocks, and blocks that i8tc leaves

@@ -244,9 +244,13 @@ static bool int4_blocks_on_limbs(int wbits, int64_t M, int64_t N, int64_t K, int
 //                           items: int4 with long rows, more items than SMs there (of 42 tokens), or more than one launch: [4096,14336] at
 //                           128 32 us, 38 there, [8064,7168] 28, 38, [7168,2048] at 100 16, 19, [1024,512] at 1024 15, 21; else there where
 //                           the result has 16 bits ([1024,4096] at 128 20, 17 there, [4096,4096] 21, 18)
-//   blocks of 64   above 32 tokens always: the other kernel that goes on with them there, tcgen05, has 64 tokens a pass (int4 [3584,20416] at
-//                  114 tokens 44 us against 104, int8 [1280,11328] at 1143 59 against 172, [512,960] at 35 7.3 against 10).  Not up to eight (int8
-//                  [8192,7424] at six tokens 19.5 us, 14.4 on the decode kernel).
+//   blocks of 64   above 32 tokens.  The other kernel that goes on with them there, tcgen05, has tiles of 64 tokens and splits K over a cluster
+//                  where they are few: ahead above 64 tokens while its tiles fit on the SMs, the fewer they are the longer K may be, and twice
+//                  as long where the tiles here are wider than 128 tokens (int8 [300,8704] at 620 tokens, 30 tiles, 34.4 us here and 23.4
+//                  there; [1024,4480] at 257, 40 tiles, 26 and 22, with 8704 inputs 33 and 35; [1024,1344] at 1143, 144 tiles, 18.8 and 14.6,
+//                  with 4480 28.5 and 32.6; of 128 tokens [2048,8704] at 82 26 and 23.5, [5632,1344] 15.3 and 14.3, [4096,4480] 21 and 22;
+//                  int4 [3584,20416] at 114 44 and 104; at 64 and below here throughout, [512,960] at 35 7.3 and 10).  Not up to eight
+//                  (int8 [8192,7424] at six 19.5 us, 14.4 on the decode kernel).
 //   fp32 results   per channel only where the other kernels need as many roundings: above 64 tokens, when the items fill
 //                  half of the SMs (the other kernel needs a third limb per token there; int8 [28672,8192] at 512 tokens 219 us
 //                  against 312, [2432,9248] at 763 tokens 49 against 74).
@@ -285,7 +289,12 @@ static bool use_tmem(int wbits, int64_t M, int64_t N, int64_t K, int64_t bs, int
     return wbits == 4 ? M > 42 || E < 1 << 25 : M <= 32 || N >= 12288;
   }
   if (M == 1) return false;
-  if (bs == 64 && (M <= 8 || M > 32)) return M > 32;
+  if (bs == 64 && M <= 8) return false;
+  if (bs == 64 && M > 32) {
+    const int64_t there = ceil_div(N, 128) * ceil_div(M, 64), sms = sm_count();
+    const bool wide = ceil_div(M, ceil_div(M, 192)) > 128;
+    return M <= 64 || there > sms || K > (4 * there <= sms ? 10000 : 2 * there <= sms ? 4000 : 1700) * (wide ? 2 : 1);
+  }
   if (M <= 64) {
     if (out_dt == QMM_F32 && !blocked) return false;
     if (M > 32) return E >= 1 << 22 && (wbits == 4 || blocked || E < 95000000);
